@@ -58,6 +58,7 @@ constexpr int kBQ = 64;    // rows (queries) per block
 constexpr int kBV = 128;   // candidate rows per tile
 constexpr int kBK = 16;    // dimensions per shared-memory step
 constexpr int kMaxC = 136; // screen list length (k + 8 <= 136)
+constexpr uint32_t kTcMinRows = 1024;  // below, the float32 screen's single launch is as fast
 
 __global__ void sqnorm32_kernel(const float *__restrict__ x, uint32_t n, uint32_t d, float *__restrict__ out) {
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -151,12 +152,14 @@ __global__ void __launch_bounds__(256) topk_tile_kernel(const float *__restrict_
     if (lane == 0) gcnt[row] = c;
 }
 
-// Float32 screen: for each of the kBQ rows of this block, the C candidates
-// (all rows but itself) with the smallest (||y||^2 - 2 x.y, id), over tiles of
-// kBV candidates. 256 threads: thread (ty, tx) computes a 4 x 8 block of the
+// Float32 screen: for each of the kBQ rows of this block (rows q0.. of the
+// base, or of the list `rows` of nr ids), the C candidates (all rows but
+// itself) with the smallest (||y||^2 - 2 x.y, id), over tiles of kBV
+// candidates. 256 threads: thread (ty, tx) computes a 4 x 8 block of the
 // 64 x 128 tile; then warp w inserts the tile into the lists of rows 8w..8w+7.
 __global__ void __launch_bounds__(256) screen_kernel(const float *__restrict__ x, uint32_t n, uint32_t d,
                                                      const float *__restrict__ xn, uint32_t C,
+                                                     const uint32_t *__restrict__ rows, uint32_t nr,
                                                      uint32_t *__restrict__ out_ids) {
     extern __shared__ __align__(16) uint8_t sm[];
     float *Qs = reinterpret_cast<float *>(sm);                 // [kBK][kBQ]
@@ -165,9 +168,13 @@ __global__ void __launch_bounds__(256) screen_kernel(const float *__restrict__ x
     float *ld = D + kBQ * (kBV + 1);                           // [kBQ][C]
     uint32_t *li = reinterpret_cast<uint32_t *>(ld + kBQ * C); // [kBQ][C]
     uint32_t *cnt = li + kBQ * C;                              // [kBQ]
+    uint32_t *qid = cnt + kBQ;                                 // [kBQ] row ids (~0: none)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t q0 = blockIdx.x * kBQ;
-    for (int i = tid; i < kBQ; i += 256) cnt[i] = 0;
+    for (int i = tid; i < kBQ; i += 256) {
+        cnt[i] = 0;
+        qid[i] = q0 + i < nr ? (rows ? rows[q0 + i] : q0 + i) : 0xffffffffu;
+    }
     const int ty = tid / 16, tx = tid % 16;  // rows ty*4.., cols tx*8..
     __syncthreads();
     for (uint32_t v0 = 0; v0 < n; v0 += kBV) {
@@ -179,7 +186,7 @@ __global__ void __launch_bounds__(256) screen_kernel(const float *__restrict__ x
         for (uint32_t k0 = 0; k0 < d; k0 += kBK) {
             for (int t = tid; t < kBK * kBQ; t += 256) {
                 const int kk = t % kBK, qq = t / kBK;
-                const uint32_t gq = q0 + qq, gk = k0 + kk;
+                const uint32_t gq = qid[qq], gk = k0 + kk;
                 Qs[kk * kBQ + qq] = (gq < n && gk < d) ? x[(size_t) gq * d + gk] : 0.f;
             }
             for (int t = tid; t < kBK * kBV; t += 256) {
@@ -204,7 +211,7 @@ __global__ void __launch_bounds__(256) screen_kernel(const float *__restrict__ x
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const uint32_t gq = q0 + ty * 4 + i;
+            const uint32_t gq = qid[ty * 4 + i];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const uint32_t gv = v0 + tx * 8 + j;
@@ -226,7 +233,7 @@ __global__ void __launch_bounds__(256) screen_kernel(const float *__restrict__ x
         __syncthreads();
     }
     for (int r = warp; r < kBQ; r += 8) {
-        const uint32_t gq = q0 + r;
+        const uint32_t gq = qid[r];
         if (gq >= n) continue;
         for (uint32_t e = lane; e < C; e += 32)
             out_ids[(size_t) gq * C + e] = e < cnt[r] ? li[r * C + e] : 0xffffffffu;
@@ -481,6 +488,16 @@ __global__ void dist_to_point_kernel(const float *__restrict__ x, uint32_t n, ui
 
 }  // namespace
 
+// The float32 screen of nr rows (of the list `rows`, or all without it).
+static int screen_fp32(const float *x, uint32_t n, uint32_t d, const float *xn, uint32_t C, const uint32_t *rows,
+                       uint32_t nr, uint32_t *cand, cudaStream_t s) {
+    const size_t smem = (size_t) (kBK * kBQ + kBK * kBV + kBQ * (kBV + 1)) * 4 + (size_t) kBQ * C * 8 + kBQ * 8;
+    GCU(cudaFuncSetAttribute(screen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+    screen_kernel<<<(nr + kBQ - 1) / kBQ, 256, smem, s>>>(x, n, d, xn, C, rows, nr, cand);
+    GCU(cudaGetLastError());
+    return PANNS_OK;
+}
+
 // The steps after the k-NN screen, shared by every construction: the C
 // screened candidates of each row (cand, device, n x C; ~0 = none) ranked
 // exactly by (d64, id) into k-NN lists, the MRNG prune to R, the entry (the
@@ -622,10 +639,10 @@ int panns_build_nsg_ex(int device, const float *base, uint32_t n, uint32_t d, ui
     if (screen > PANNS_SCREEN_TC) return set_error(PANNS_EINVAL, "panns_build_nsg: unknown screen");
     const uint32_t k = knn_k;
     const uint32_t C_tc = std::min(std::min(knn_k + 32u, (uint32_t) kMaxC), n - 1);
-    if (screen == PANNS_SCREEN_AUTO)
-        screen = n < 100000 ? PANNS_SCREEN_FP32
-                            : tc_screen_supported(n, d, C_tc) ? PANNS_SCREEN_TC : PANNS_SCREEN_TF32;
-    if (screen == PANNS_SCREEN_TC && !tc_screen_supported(n, d, C_tc))
+    const bool automatic = screen == PANNS_SCREEN_AUTO;
+    if (automatic)
+        screen = n >= kTcMinRows && d <= 256 ? PANNS_SCREEN_TC : n < 100000 ? PANNS_SCREEN_FP32 : PANNS_SCREEN_TF32;
+    if (!automatic && screen == PANNS_SCREEN_TC && !tc_screen_supported(n, d, C_tc))
         return set_error(PANNS_EINVAL, "panns_build_nsg: the tcgen05 screen needs d a multiple of 32 up to 128 "
                                        "and n >= 128");
     const bool tc = screen == PANNS_SCREEN_TF32;
@@ -648,13 +665,31 @@ int panns_build_nsg_ex(int device, const float *base, uint32_t n, uint32_t d, ui
     if (tcg) {
         int num_sms = 0;
         GCU(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device));
-        const int rc = tc_screen(x.p, xn.p, n, d, C, cand.p, num_sms, s);
+        Buf<uint32_t> perm, fail, nfail;
+        GCU(fail.alloc(n));
+        GCU(nfail.alloc(1));
+        int rc = PANNS_OK;
+        uint32_t slots = n;
+        if (n > 32 * kTcM) {  // below, every tile is near every other
+            GCU(perm.alloc(tc_order_slots(n, true)));
+            rc = tc_locality_order(x.p, n, d, true, perm.p, &slots, s);
+            if (rc) return rc;
+        }
+        rc = tc_screen_knn(x.p, n, d, k, C, perm.p, slots, nullptr, cand.p, fail.p, nfail.p, num_sms, s);
         if (rc) return rc;
+        // Rows that screen could not settle (long runs of equal distances,
+        // non-finite values) go through the float32 one.
+        uint32_t nf = 0;
+        GCU(cudaMemcpyAsync(&nf, nfail.p, 4, cudaMemcpyDeviceToHost, s));
+        GCU(cudaStreamSynchronize(s));
+        if (nf) {
+            rc = screen_fp32(x.p, n, d, xn.p, C, fail.p, nf, cand.p, s);
+            if (rc) return rc;
+            GCU(cudaStreamSynchronize(s));
+        }
     } else if (!tc) {
-        const size_t smem = (size_t) (kBK * kBQ + kBK * kBV + kBQ * (kBV + 1)) * 4 + (size_t) kBQ * C * 8 + kBQ * 4;
-        GCU(cudaFuncSetAttribute(screen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-        screen_kernel<<<(n + kBQ - 1) / kBQ, 256, smem, s>>>(x.p, n, d, xn.p, C, cand.p);
-        GCU(cudaGetLastError());
+        const int rc = screen_fp32(x.p, n, d, xn.p, C, nullptr, n, cand.p, s);
+        if (rc) return rc;
     } else {
         // -2 x.y for tiles of TR rows x TC candidates by TF32 tensor-core GEMMs
         // (cuBLAS, a plain library GEMM), each folded into the rows' lists.
@@ -710,7 +745,7 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
     if (cells < 1 || cells > S) return set_error(PANNS_EINVAL, "panns_build_nsg_cells: need 1 <= cells <= sample, n");
     if (probe > 8 || (probe >= cells && cells > 1)) return set_error(PANNS_EINVAL, "panns_build_nsg_cells: need probe <= 8 and probe < cells");
     const uint32_t k = knn_k, P = cells > 1 ? probe : 0u;
-    const uint32_t C = std::min(knn_k + 8u, (uint32_t) kMaxC);
+    const uint32_t C = std::min(knn_k + 16u, (uint32_t) kMaxC);
     GCU(cudaSetDevice(device));
     cudaStream_t s = nullptr;
     GCU(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -771,13 +806,63 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
     Buf<uint32_t> cand;
     GCU(cand.alloc((size_t) n * C));
     GCU(cudaMemsetAsync(cand.p, 0xff, (size_t) n * C * 4, s));
-    {
+    // Tensor-core screen: every cell padded to whole tiles, a row block of one
+    // cell against the tiles of the cell and of its near cells. Where padding
+    // would more than double the rows (cells of a few dozen rows), or its
+    // lists cannot settle a row, the float32 screen runs.
+    uint64_t slots = 0;
+    for (uint32_t c = 0; c < cells; ++c) slots += (cstart[c + 1] - cstart[c] + kTcM - 1) / kTcM * (uint64_t) kTcM;
+    bool screened = false;
+    size_t free_b = 0, total_b = 0;
+    GCU(cudaMemGetInfo(&free_b, &total_b));
+    if (d <= 256 && n >= kTcMinRows && slots <= 2ull * n && slots <= 0x7fffffffull &&
+        tc_knn_bytes(slots, d) <= free_b / 5 * 3) {
+        std::vector<uint32_t> tile0(cells + 1, 0), avail(cells, 0), order((size_t) slots, 0xffffffffu), blk;
+        blk.reserve((size_t) (slots / kTcM));
+        for (uint32_t c = 0; c < cells; ++c) {
+            const uint32_t m = cstart[c + 1] - cstart[c], t = (m + kTcM - 1) / kTcM;
+            std::copy(members.begin() + cstart[c], members.begin() + cstart[c + 1],
+                      order.begin() + (size_t) tile0[c] * kTcM);
+            blk.insert(blk.end(), t, c);
+            tile0[c + 1] = tile0[c] + t;
+            avail[c] = m;
+            for (uint32_t i = 0; i < P; ++i) {
+                const uint32_t o = nearh[(size_t) c * P + i];
+                if (o != 0xffffffffu) avail[c] += cstart[o + 1] - cstart[o];
+            }
+        }
+        int num_sms = 0;
+        GCU(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device));
+        Buf<uint32_t> dorder, dblk, dt0, dnear, davail, fail, nfail;
+        GCU(dorder.alloc(order.size()));
+        GCU(dblk.alloc(blk.size()));
+        GCU(dt0.alloc(cells + 1));
+        GCU(dnear.alloc(nearh.size()));
+        GCU(davail.alloc(cells));
+        GCU(fail.alloc(n));
+        GCU(nfail.alloc(1));
+        GCU(cudaMemcpyAsync(dorder.p, order.data(), order.size() * 4, cudaMemcpyHostToDevice, s));
+        GCU(cudaMemcpyAsync(dblk.p, blk.data(), blk.size() * 4, cudaMemcpyHostToDevice, s));
+        GCU(cudaMemcpyAsync(dt0.p, tile0.data(), (cells + 1) * 4ull, cudaMemcpyHostToDevice, s));
+        GCU(cudaMemcpyAsync(dnear.p, nearh.data(), nearh.size() * 4, cudaMemcpyHostToDevice, s));
+        GCU(cudaMemcpyAsync(davail.p, avail.data(), cells * 4ull, cudaMemcpyHostToDevice, s));
+        const TcCells tc{dblk.p, dt0.p, dnear.p, davail.p, P};
+        const int rc = tc_screen_knn(x.p, n, d, k, C, dorder.p, (uint32_t) slots, &tc, cand.p, fail.p, nfail.p, num_sms,
+                                     s);
+        if (rc) return rc;
+        uint32_t nf = 0;
+        GCU(cudaMemcpyAsync(&nf, nfail.p, 4, cudaMemcpyDeviceToHost, s));
+        GCU(cudaStreamSynchronize(s));
+        screened = nf == 0;
+    }
+    if (!screened) {
         Buf<uint32_t> dmem, dstart, dnear, dbc, dbr;
         GCU(dmem.alloc(n));
         GCU(dstart.alloc(cells + 1));
         GCU(dnear.alloc(nearh.size()));
         GCU(dbc.alloc(blk_cell.size()));
         GCU(dbr.alloc(blk_row0.size()));
+        GCU(cudaMemsetAsync(cand.p, 0xff, (size_t) n * C * 4, s));
         GCU(cudaMemcpyAsync(dmem.p, members.data(), n * 4ull, cudaMemcpyHostToDevice, s));
         GCU(cudaMemcpyAsync(dstart.p, cstart.data(), (cells + 1) * 4ull, cudaMemcpyHostToDevice, s));
         GCU(cudaMemcpyAsync(dnear.p, nearh.data(), nearh.size() * 4, cudaMemcpyHostToDevice, s));

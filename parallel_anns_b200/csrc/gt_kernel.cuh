@@ -2,9 +2,14 @@
 //
 // The k results of any search are k distinct vertices, so the largest of their
 // exact distances, tau, is an upper bound of the true k-th smallest distance.
-// One tiled pass over the base therefore only has to collect the vertices
-// whose float64 distance is <= tau (about k of them for a good search) into a
-// per-query list; an exact (distance, id) sort of that list gives the top k.
+// It is enough to collect the vertices whose float64 distance is <= tau (about
+// k of them for a good search); an exact (distance, id) sort gives the top k.
+// The collection is the tensor-core range screen (tc_screen.cu), whose lists
+// gt_rank_kernel evaluates in float64 and ranks; where its lists do not fit
+// (k > kGtMaxK, or a bound so loose that refining it does not help) one tiled
+// float64 pass over the base collects instead (gt_collect_kernel).
+// 10,000 queries x 1M x 96, k = 100: 174 ms in gt_collect_kernel, 3 ms in the
+// screen, its operands and gt_rank_kernel.
 // Distances are sum over dimensions, in order, of fma(t, t, acc) with
 // t = (double) x - (double) q, in both kernels, so the search's own results
 // meet their own bound bit for bit. Plays the role of
@@ -106,6 +111,113 @@ __global__ void __launch_bounds__(256) gt_collect_kernel(const float *__restrict
             }
         }
     }
+}
+
+constexpr uint32_t kGtMaxK = 512;     // largest k of the screened path
+constexpr uint32_t kGtList = 1024;    // vertices within the bound that gt_rank_kernel ranks
+
+// out row i = row order[i] of `rows` (width d), and tau likewise.
+__global__ void gt_gather_kernel(const float *__restrict__ rows, const double *__restrict__ tau,
+                                 const uint32_t *__restrict__ order, uint32_t nq, uint32_t d, float *__restrict__ out,
+                                 double *__restrict__ out_tau) {
+    const uint32_t i = blockIdx.x;
+    if (i >= nq) return;
+    const size_t q = order[i];
+    for (uint32_t j = threadIdx.x; j < d; j += blockDim.x) out[(size_t) i * d + j] = rows[q * d + j];
+    if (threadIdx.x == 0) out_tau[i] = tau[q];
+}
+
+// tau[order[i]] = ts[i]: bounds back in query order.
+__global__ void gt_scatter_tau_kernel(const double *__restrict__ ts, const uint32_t *__restrict__ order, uint32_t nq,
+                                      double *__restrict__ tau) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < nq) tau[order[i]] = ts[i];
+}
+
+// The vertices in layout order with every cell moved to a multiple of the
+// screen's tile: perm[to[c] + i] = orig[from[c] + i]. One block per cell.
+__global__ void gt_slots_kernel(const uint32_t *__restrict__ orig, const uint32_t *__restrict__ from,
+                                const uint32_t *__restrict__ to, uint32_t *__restrict__ perm) {
+    const uint32_t c = blockIdx.x, b = from[c], m = from[c + 1] - b;
+    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) perm[to[c] + i] = orig[b + i];
+}
+
+// One block of 128 threads per query i (row i of qs): the float64 distances of
+// the screen's entries (splits lists of up to cap; entry y = position, vertex
+// perm[position]), those within tau[i] ranked by (distance, vertex), the k best
+// written to row order[i] of out_ids / out_dist. A query whose lists overflowed,
+// or with more than kGtList vertices within tau, is not written: over[i] = 1,
+// and tau[i] becomes the k-th smallest of the distances looked at, which is a
+// bound of the answer too. d is a multiple of 4.
+__global__ void __launch_bounds__(128) gt_rank_kernel(const float *__restrict__ base, int d,
+                                                      const uint32_t *__restrict__ perm, const float *__restrict__ qs,
+                                                      uint32_t nq, const uint32_t *__restrict__ order,
+                                                      double *__restrict__ tau, uint32_t splits, uint32_t cap,
+                                                      const uint2 *__restrict__ lists, const uint32_t *__restrict__ cnt,
+                                                      uint32_t k, uint32_t *__restrict__ out_ids,
+                                                      double *__restrict__ out_dist, uint32_t *__restrict__ over) {
+    __shared__ double sd[kGtList];
+    __shared__ uint32_t si[kGtList];
+    __shared__ __align__(16) double sq[256];
+    __shared__ uint32_t found;
+    __shared__ double refined;
+    const uint32_t i = blockIdx.x, tid = threadIdx.x;
+    for (int e = tid; e < d; e += 128) sq[e] = (double) qs[(size_t) i * d + e];
+    if (tid == 0) found = 0;
+    __syncthreads();
+    const double t0 = tau[i];
+    bool full = false;
+    for (uint32_t sp = 0; sp < splits; ++sp) {
+        const uint32_t c = cnt[(size_t) sp * nq + i], m = min(c, cap);
+        full = full || c > cap;
+        const uint2 *list = lists + ((size_t) sp * nq + i) * cap;
+        for (uint32_t e = tid; e < m; e += 128) {
+            const uint32_t v = perm[list[e].y];
+            const float4 *x = reinterpret_cast<const float4 *>(base + (size_t) v * d);
+            double acc = 0.0;
+#pragma unroll 4
+            for (int j = 0; j < d / 4; ++j) {
+                const float4 f = __ldg(x + j);
+                double t = (double) f.x - sq[4 * j];
+                acc = fma(t, t, acc);
+                t = (double) f.y - sq[4 * j + 1];
+                acc = fma(t, t, acc);
+                t = (double) f.z - sq[4 * j + 2];
+                acc = fma(t, t, acc);
+                t = (double) f.w - sq[4 * j + 3];
+                acc = fma(t, t, acc);
+            }
+            if (acc <= t0) {
+                const uint32_t pos = atomicAdd(&found, 1u);
+                if (pos < kGtList) {
+                    sd[pos] = acc;
+                    si[pos] = v;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    const uint32_t n = min(found, kGtList);
+    const bool bad = full || found > kGtList;
+    if (tid == 0) {
+        over[i] = bad ? 1u : n < k ? 2u : 0u;
+        refined = t0;
+    }
+    __syncthreads();
+    for (uint32_t e = tid; e < n; e += 128) {
+        const double de = sd[e];
+        const uint32_t ie = si[e];
+        uint32_t rank = 0;
+        for (uint32_t f = 0; f < n; ++f) rank += sd[f] < de || (sd[f] == de && si[f] < ie) ? 1u : 0u;
+        if (bad) {
+            if (rank + 1 == k) refined = de;
+        } else if (rank < k) {
+            out_ids[(size_t) order[i] * k + rank] = ie;
+            if (out_dist) out_dist[(size_t) order[i] * k + rank] = de;
+        }
+    }
+    __syncthreads();
+    if (tid == 0 && bad) tau[i] = refined;
 }
 
 }  // namespace panns

@@ -21,6 +21,7 @@
 #include "block_kernel.cuh"
 #include "gt_kernel.cuh"
 #include "pss_kernel.cuh"
+#include "tc_screen.h"
 #include "kernels.h"
 
 using namespace panns;
@@ -166,6 +167,7 @@ struct panns_index {
     DevBuf<float> norms_lo, scales; // its norms; FP8 per-dimension scales
     bool ready = false;             // vec/norms/head built for the current base + graph
     std::vector<uint32_t> perm, inv;  // device id -> original id, and back
+    std::vector<uint32_t> cell_start; // device ids of each cell of the layout order (cells + 1)
     DevBuf<uint32_t> orig;
     // graph
     uint32_t width = 0, entry = 0, gn = 0, max_deg = 0;
@@ -394,6 +396,7 @@ static int finalize(panns_index *h) {
     const bool identity = (ord && std::string(ord) == "identity") || n < 4096;
     if (identity) {
         for (uint32_t v = 0; v < n; ++v) h->perm[v] = h->inv[v] = v;
+        h->cell_start = {0, n};
     } else {
         const uint32_t C = std::max(1u, std::min(4096u, n / 256));
         std::vector<uint32_t> piv(C), cell(n);
@@ -409,6 +412,7 @@ static int finalize(panns_index *h) {
         std::vector<uint32_t> start(C + 1, 0);
         for (uint32_t v = 0; v < n; ++v) start[cell[v] + 1]++;
         for (uint32_t c = 0; c < C; ++c) start[c + 1] += start[c];
+        h->cell_start = start;
         for (uint32_t v = 0; v < n; ++v) h->perm[start[cell[v]]++] = v;
         for (uint32_t u = 0; u < n; ++u) h->inv[h->perm[u]] = u;
     }
@@ -1194,8 +1198,11 @@ int panns_ground_truth(panns_index *h, const float *queries, uint32_t nq, uint32
     p.M = 8;
     p.T = 1;
     p.X = 1;
-    std::vector<uint32_t> sids((size_t) nq * k);
-    rc = panns_search_host(h, &p, queries, nq, nullptr, sids.data(), nullptr);
+    rc = check_params(h, &p);
+    if (rc) return rc;
+    const uint32_t *d_init = nullptr;
+    uint32_t stride = 0;
+    rc = stage_init(h, &p, nullptr, nq, h->stream, d_init, stride);
     if (rc) return rc;
     DevBuf<float> dq;
     DevBuf<uint32_t> dids, dcnt;
@@ -1203,13 +1210,106 @@ int panns_ground_truth(panns_index *h, const float *queries, uint32_t nq, uint32
     CU(dq.ensure((size_t) nq * h->d));
     CU(dids.ensure((size_t) nq * k));
     CU(dtau.ensure(nq));
-    CU(dcnt.ensure(nq));
+    CU(h->hq.ensure((size_t) nq * h->dpad));
+    CU(h->stats.ensure(nq));
     CU(cudaMemcpyAsync(dq.p, queries, (size_t) nq * h->d * 4, cudaMemcpyHostToDevice, h->stream));
-    CU(cudaMemcpyAsync(dids.p, sids.data(), (size_t) nq * k * 4, cudaMemcpyHostToDevice, h->stream));
+    rc = launch_search(h, &p, h->hq.p, dq.p, nq, d_init, stride, nullptr, dids.p, h->stats.p, h->stream, false);
+    if (rc) return rc;
+    uint32_t err = 0;
+    CU(cudaMemcpyAsync(&err, h->error.p, 4, cudaMemcpyDeviceToHost, h->stream));
+    CU(cudaStreamSynchronize(h->stream));
+    if (err & ERR_BAD_ID) return fail(PANNS_EDEVICE, "search: the graph holds a neighbour id >= N");
+    if (err & ERR_BAD_INIT) return fail(PANNS_EDEVICE, "search: init id >= N");
     gt_tau_kernel<<<(nq + 3) / 4, 128, 0, h->stream>>>(h->base_raw.p, (int) h->d, dq.p, nq, dids.p, k, dtau.p);
     CU(cudaGetLastError());
-    // 2. Collect every vertex within the bound. A pass scans all vertices for
-    // a set of queries with lists of `cap` entries (counts go on past cap).
+    // 2. The vertices within the bound by the tensor-core range screen, ranked
+    // exactly: the queries grouped by locality, in batches that bound the
+    // lists; those whose lists overflow again with the bound their first
+    // vertices gave, and what is still over goes to step 3.
+    std::vector<uint32_t> left;  // queries the tiled pass collects
+    if (k > kGtMaxK) {
+        left.resize(nq);
+        for (uint32_t q = 0; q < nq; ++q) left[q] = q;
+    } else {
+        // Positions: the layout order, every cell on a tile boundary.
+        const uint32_t cells = (uint32_t) h->cell_start.size() - 1;
+        std::vector<uint32_t> to(cells);
+        uint64_t slots = 0;
+        for (uint32_t c = 0; c < cells; ++c) {
+            to[c] = (uint32_t) slots;
+            slots += (h->cell_start[c + 1] - h->cell_start[c] + kTcM - 1) / kTcM * (uint64_t) kTcM;
+        }
+        if (slots > 0xfffffff0ull) return fail(PANNS_EINVAL, "panns_ground_truth: too many vertices");
+        DevBuf<uint32_t> dfrom, dto, perm, dtodo;
+        CU(dfrom.ensure(cells + 1));
+        CU(dto.ensure(cells));
+        CU(perm.ensure((size_t) slots));
+        CU(dtodo.ensure(nq));
+        CU(cudaMemcpyAsync(dfrom.p, h->cell_start.data(), (cells + 1) * 4ull, cudaMemcpyHostToDevice, h->stream));
+        CU(cudaMemcpyAsync(dto.p, to.data(), cells * 4ull, cudaMemcpyHostToDevice, h->stream));
+        CU(cudaMemsetAsync(perm.p, 0xff, (size_t) slots * 4, h->stream));
+        gt_slots_kernel<<<cells, 128, 0, h->stream>>>(h->orig.p, dfrom.p, dto.p, perm.p);
+        CU(cudaGetLastError());
+        uint32_t placed = 0;
+        rc = tc_locality_order(dq.p, nq, h->d, false, dtodo.p, &placed, h->stream);
+        if (rc) return rc;
+        std::vector<uint32_t> todo(nq);
+        CU(cudaMemcpyAsync(todo.data(), dtodo.p, nq * 4ull, cudaMemcpyDeviceToHost, h->stream));
+        CU(cudaStreamSynchronize(h->stream));
+        DevBuf<uint32_t> oid;
+        DevBuf<double> odist;
+        CU(oid.ensure((size_t) nq * k));
+        CU(odist.ensure(out_dist ? (size_t) nq * k : 1));
+        const uint32_t cap = 4 * k + 64, batch = 16384;
+        for (int pass = 0; pass < 4 && !todo.empty(); ++pass) {
+            std::vector<uint32_t> over;
+            for (size_t b0 = 0; b0 < todo.size(); b0 += batch) {
+                const uint32_t m = (uint32_t) std::min<size_t>(batch, todo.size() - b0);
+                const uint32_t splits = tc_range_splits(m, h->num_sms);
+                DevBuf<uint32_t> dorder, lcnt, dover;
+                DevBuf<float> qs;
+                DevBuf<double> ts;
+                DevBuf<uint2> lists;
+                CU(dorder.ensure(m));
+                CU(qs.ensure((size_t) m * h->d));
+                CU(ts.ensure(m));
+                CU(lists.ensure((size_t) m * splits * cap));
+                CU(lcnt.ensure((size_t) m * splits));
+                CU(dover.ensure(m));
+                CU(cudaMemcpyAsync(dorder.p, todo.data() + b0, m * 4ull, cudaMemcpyHostToDevice, h->stream));
+                gt_gather_kernel<<<m, 64, 0, h->stream>>>(dq.p, dtau.p, dorder.p, m, h->d, qs.p, ts.p);
+                CU(cudaGetLastError());
+                bool safe = false;
+                rc = tc_screen_range(h->base_raw.p, h->n, h->d, perm.p, (uint32_t) slots, dq.p, dorder.p, m, ts.p,
+                                     splits, lists.p, cap, lcnt.p, &safe, h->num_sms, h->stream);
+                if (rc) return rc;
+                if (!safe) {
+                    left.insert(left.end(), todo.begin() + b0, todo.begin() + b0 + m);
+                    continue;
+                }
+                gt_rank_kernel<<<m, 128, 0, h->stream>>>(h->base_raw.p, (int) h->d, perm.p, qs.p, m, dorder.p, ts.p,
+                                                         splits, cap, lists.p, lcnt.p, k, oid.p, out_dist ? odist.p : nullptr,
+                                                         dover.p);
+                gt_scatter_tau_kernel<<<(m + 255) / 256, 256, 0, h->stream>>>(ts.p, dorder.p, m, dtau.p);
+                CU(cudaGetLastError());
+                std::vector<uint32_t> ov(m);
+                CU(cudaMemcpyAsync(ov.data(), dover.p, m * 4ull, cudaMemcpyDeviceToHost, h->stream));
+                CU(cudaStreamSynchronize(h->stream));
+                for (uint32_t i = 0; i < m; ++i) {
+                    if (ov[i] == 1) over.push_back(todo[b0 + i]);
+                    if (ov[i] == 2) left.push_back(todo[b0 + i]);
+                }
+            }
+            todo.swap(over);
+        }
+        left.insert(left.end(), todo.begin(), todo.end());
+        CU(cudaMemcpyAsync(out_ids, oid.p, (size_t) nq * k * 4, cudaMemcpyDeviceToHost, h->stream));
+        if (out_dist) CU(cudaMemcpyAsync(out_dist, odist.p, (size_t) nq * k * 8, cudaMemcpyDeviceToHost, h->stream));
+        CU(cudaStreamSynchronize(h->stream));
+        if (left.empty()) return PANNS_OK;
+    }
+    // 3. The tiled float64 pass over all vertices for a set of queries with
+    // lists of `cap` entries (counts go on past cap).
     const uint32_t vt = (h->n + kGtV - 1) / kGtV;
     auto collect = [&](const float *qrows, const double *tau, uint32_t m, uint32_t cap, uint32_t *dc, double *cd,
                        uint32_t *ci) -> cudaError_t {
@@ -1236,30 +1336,44 @@ int panns_ground_truth(panns_index *h, const float *queries, uint32_t nq, uint32
         return PANNS_OK;
     };
     const uint32_t cap = std::max(4 * k, 64u);
-    std::vector<uint32_t> cnt(nq);
-    std::vector<uint32_t> over;  // queries whose lists overflowed
+    const uint32_t nl = (uint32_t) left.size();
+    std::vector<uint32_t> cnt(nl);
+    std::vector<uint32_t> over;  // places in `left` of the queries whose lists overflowed
+    DevBuf<float> lq;
+    DevBuf<double> ltau;
+    {
+        DevBuf<uint32_t> dleft;
+        CU(dleft.ensure(nl));
+        CU(lq.ensure((size_t) nl * h->d));
+        CU(ltau.ensure(nl));
+        CU(dcnt.ensure(nl));
+        CU(cudaMemcpyAsync(dleft.p, left.data(), nl * 4ull, cudaMemcpyHostToDevice, h->stream));
+        gt_gather_kernel<<<nl, 64, 0, h->stream>>>(dq.p, dtau.p, dleft.p, nl, h->d, lq.p, ltau.p);
+        CU(cudaGetLastError());
+        CU(cudaStreamSynchronize(h->stream));
+    }
     {
         DevBuf<double> cd;
         DevBuf<uint32_t> ci;
-        CU(cd.ensure((size_t) nq * cap));
-        CU(ci.ensure((size_t) nq * cap));
-        CU(collect(dq.p, dtau.p, nq, cap, dcnt.p, cd.p, ci.p));
-        CU(cudaMemcpyAsync(cnt.data(), dcnt.p, nq * 4ull, cudaMemcpyDeviceToHost, h->stream));
-        std::vector<double> hd((size_t) nq * cap);
-        std::vector<uint32_t> hi((size_t) nq * cap);
+        CU(cd.ensure((size_t) nl * cap));
+        CU(ci.ensure((size_t) nl * cap));
+        CU(collect(lq.p, ltau.p, nl, cap, dcnt.p, cd.p, ci.p));
+        CU(cudaMemcpyAsync(cnt.data(), dcnt.p, nl * 4ull, cudaMemcpyDeviceToHost, h->stream));
+        std::vector<double> hd((size_t) nl * cap);
+        std::vector<uint32_t> hi((size_t) nl * cap);
         CU(cudaMemcpyAsync(hd.data(), cd.p, hd.size() * 8, cudaMemcpyDeviceToHost, h->stream));
         CU(cudaMemcpyAsync(hi.data(), ci.p, hi.size() * 4, cudaMemcpyDeviceToHost, h->stream));
         CU(cudaStreamSynchronize(h->stream));
-        for (uint32_t q = 0; q < nq; ++q) {
+        for (uint32_t q = 0; q < nl; ++q) {
             if (cnt[q] > cap) {
                 over.push_back(q);
                 continue;
             }
-            rc = finish(q, hd.data() + (size_t) q * cap, hi.data() + (size_t) q * cap, cnt[q]);
+            rc = finish(left[q], hd.data() + (size_t) q * cap, hi.data() + (size_t) q * cap, cnt[q]);
             if (rc) return rc;
         }
     }
-    // 3. Queries whose bound was loose (the search missed their part of the
+    // Queries whose bound was loose (the search missed their part of the
     // graph): again, a few at a time, each list as long as its count, within
     // 4 GiB of lists per pass.
     const size_t budget = 4ull << 30;
@@ -1279,7 +1393,7 @@ int panns_ground_truth(panns_index *h, const float *queries, uint32_t nq, uint32
         std::vector<float> qh((size_t) m * h->d);
         std::vector<double> th(m);
         for (uint32_t i = 0; i < m; ++i) {
-            const uint32_t q = over[g0 + i];
+            const uint32_t q = left[over[g0 + i]];
             std::copy(queries + (size_t) q * h->d, queries + (size_t) (q + 1) * h->d, qh.begin() + (size_t) i * h->d);
         }
         DevBuf<float> gq;
@@ -1292,7 +1406,7 @@ int panns_ground_truth(panns_index *h, const float *queries, uint32_t nq, uint32
         CU(ci.ensure((size_t) m * gcap));
         CU(cudaMemcpyAsync(gq.p, qh.data(), qh.size() * 4, cudaMemcpyHostToDevice, h->stream));
         for (uint32_t i = 0; i < m; ++i)
-            CU(cudaMemcpyAsync(gt.p + i, dtau.p + over[g0 + i], 8, cudaMemcpyDeviceToDevice, h->stream));
+            CU(cudaMemcpyAsync(gt.p + i, ltau.p + over[g0 + i], 8, cudaMemcpyDeviceToDevice, h->stream));
         CU(collect(gq.p, gt.p, m, gcap, gc.p, cd.p, ci.p));
         std::vector<uint32_t> c2(m);
         std::vector<double> hd((size_t) m * gcap);
@@ -1303,7 +1417,7 @@ int panns_ground_truth(panns_index *h, const float *queries, uint32_t nq, uint32
         CU(cudaStreamSynchronize(h->stream));
         for (uint32_t i = 0; i < m; ++i) {
             if (c2[i] > gcap) return fail(PANNS_EDEVICE, "panns_ground_truth: candidate count changed between passes");
-            rc = finish(over[g0 + i], hd.data() + (size_t) i * gcap, hi.data() + (size_t) i * gcap, c2[i]);
+            rc = finish(left[over[g0 + i]], hd.data() + (size_t) i * gcap, hi.data() + (size_t) i * gcap, c2[i]);
             if (rc) return rc;
         }
         g0 = g1;

@@ -59,6 +59,7 @@ constexpr int kBV = 128;   // candidate rows per tile
 constexpr int kBK = 16;    // dimensions per shared-memory step
 constexpr int kMaxC = 136; // screen list length (k + 8 <= 136)
 constexpr uint32_t kTcMinRows = 1024;  // below, the float32 screen's single launch is as fast
+constexpr uint32_t kMaxVecD = 256;  // rerank_kernel's shared-memory copy of a row
 
 __global__ void sqnorm32_kernel(const float *__restrict__ x, uint32_t n, uint32_t d, float *__restrict__ out) {
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -405,36 +406,72 @@ __device__ __forceinline__ double d64(const float *__restrict__ a, const float *
     return acc;
 }
 
-// One warp per row a0 + r (r < na): float64 distances of its C screened
-// candidates, ranked by (d64, id); the k best go out (ids and distances, row r
-// of the chunk's knn / knn_d; a list short of k valid candidates ends in
-// invalid ids, which the caller pre-sets).
-__global__ void rerank_kernel(const float *__restrict__ x, uint32_t n, uint32_t d, const uint32_t *__restrict__ cand,
-                              uint32_t C, uint32_t k, uint32_t a0, uint32_t na, uint32_t *__restrict__ knn,
-                              double *__restrict__ knn_d) {
+// One warp per row a0 + r (r < na): float64 distances of its screened
+// candidates (C slots, ~0 = none), ranked by (d64, id); the k best go out (ids
+// and distances, row r of the chunk's knn / knn_d; a list short of k valid
+// candidates ends in invalid ids, which the caller pre-sets). Bound by the
+// float32 -> float64 conversions and the gathers of the candidates' rows: with
+// d a multiple of 4 each lane streams its candidate's row in 16-byte loads
+// against the row's float64 copy in shared memory (VEC), else by elements.
+// 250,000 x 96: 8.8 ms with 4-byte loads over k + 32 slots, 3.0 ms so.
+template <bool VEC>
+__global__ void __launch_bounds__(256) rerank_kernel(const float *__restrict__ x, uint32_t n, uint32_t d,
+                                                     const uint32_t *__restrict__ cand, uint32_t C, uint32_t k,
+                                                     uint32_t a0, uint32_t na, uint32_t *__restrict__ knn,
+                                                     double *__restrict__ knn_d) {
     __shared__ double sd[8][kMaxC];
     __shared__ uint32_t si[8][kMaxC];
+    __shared__ __align__(16) double sx[VEC ? 8 : 1][VEC ? kMaxVecD : 2];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t r = blockIdx.x * 8 + w;
     if (r >= na) return;
     const uint32_t a = a0 + r;
     const float *xa = x + (size_t) a * d;
-    for (uint32_t e = lane; e < C; e += 32) {
-        const uint32_t b = cand[(size_t) a * C + e];
-        si[w][e] = b;
-        sd[w][e] = b < n ? d64(xa, x + (size_t) b * d, d) : __longlong_as_double(0x7ff0000000000000ll);
+    if (VEC)
+        for (uint32_t e = lane; e < d; e += 32) sx[w][e] = (double) xa[e];
+    uint32_t m = 0;  // valid candidates
+    for (uint32_t e0 = 0; e0 < C; e0 += 32) {
+        const uint32_t b = e0 + lane < C ? cand[(size_t) a * C + e0 + lane] : 0xffffffffu;
+        const uint32_t bm = __ballot_sync(0xffffffffu, b < n);
+        if (b < n) si[w][m + __popc(bm & ((1u << lane) - 1u))] = b;
+        m += __popc(bm);
     }
     __syncwarp();
-    for (uint32_t e = lane; e < C; e += 32) {
+    for (uint32_t e = lane; e < m; e += 32) {
+        const float *xb = x + (size_t) si[w][e] * d;
+        double acc = 0.0;
+        if (VEC) {
+            const float4 *x4 = reinterpret_cast<const float4 *>(xb);
+#pragma unroll 4
+            for (uint32_t j = 0; j < d / 4; ++j) {
+                const float4 v = __ldg(x4 + j);
+                const double2 p = *reinterpret_cast<const double2 *>(&sx[w][4 * j]);
+                const double2 q = *reinterpret_cast<const double2 *>(&sx[w][4 * j + 2]);
+                double t = p.x - (double) v.x;
+                acc = fma(t, t, acc);
+                t = p.y - (double) v.y;
+                acc = fma(t, t, acc);
+                t = q.x - (double) v.z;
+                acc = fma(t, t, acc);
+                t = q.y - (double) v.w;
+                acc = fma(t, t, acc);
+            }
+        } else {
+            acc = d64(xa, xb, d);
+        }
+        sd[w][e] = acc;
+    }
+    __syncwarp();
+    for (uint32_t e = lane; e < m; e += 32) {
         const double de = sd[w][e];
         const uint32_t ie = si[w][e];
         uint32_t rank = 0;
-        for (uint32_t f = 0; f < C; ++f) {
+        for (uint32_t f = 0; f < m; ++f) {
             const double df = sd[w][f];
             const uint32_t jf = si[w][f];
             rank += (df < de || (df == de && jf < ie)) ? 1u : 0u;
         }
-        if (rank < k && ie < n) {
+        if (rank < k) {
             knn[(size_t) r * k + rank] = ie;
             knn_d[(size_t) r * k + rank] = de;
         }
@@ -442,7 +479,8 @@ __global__ void rerank_kernel(const float *__restrict__ x, uint32_t n, uint32_t 
 }
 
 // One warp per row a0 + r (r < na): MRNG pruning of its k-NN list (row r of
-// the chunk's knn / knn_d) to at most R (row r of out, deg).
+// the chunk's knn / knn_d) to at most R (row r of out, deg), reading the
+// candidates' rows from global memory (any d; see prune_rows_kernel).
 __global__ void prune_kernel(const float *__restrict__ x, uint32_t n, uint32_t d, const uint32_t *__restrict__ knn,
                              const double *__restrict__ knn_d, uint32_t k, uint32_t R, uint32_t na,
                              uint32_t *__restrict__ out, uint32_t *__restrict__ deg) {
@@ -470,6 +508,111 @@ __global__ void prune_kernel(const float *__restrict__ x, uint32_t n, uint32_t d
         }
     }
     for (uint32_t e = lane; e < nk; e += 32) out[(size_t) r * R + e] = kept[e];
+    if (lane == 0) deg[r] = nk;
+}
+
+// The same prune with the candidates' rows in shared memory (d a multiple of
+// 4). The walk is turned round: when a candidate c is kept, the warp tests it
+// against all later candidates that are not occluded yet (one per lane), so a
+// row takes as many dependent steps as it keeps neighbours (about 18 of 64)
+// and not one per candidate and 32 kept. d(c, b) < d(a, b) is decided in
+// float32 where the two differ by more than float32 can be off (the squared
+// differences are all positive, so the sum's relative error is at most
+// (d + 3) 2^-24; kPruneSlack is over twice that), else by the float64 chain.
+// Rows are (d / 4 rounded up to odd) 16-byte words apart, so that eight lanes
+// reading eight rows hit distinct banks. Bound by the shared-memory reads.
+// 250,000 x 96, k = 64: 61 ms with one candidate at a time in float64 from
+// global memory, 6.4 ms so.
+__host__ __device__ inline uint32_t prune_row_words(uint32_t d) { return (d / 4) | 1u; }
+__host__ __device__ inline uint32_t prune_warp_bytes(uint32_t d, uint32_t k) {
+    return k * prune_row_words(d) * 16 + ((k * 16 + 15) & ~15u);  // rows; distances, ids, list
+}
+
+__global__ void __launch_bounds__(128) prune_rows_kernel(const float *__restrict__ x, uint32_t n, uint32_t d,
+                                                         const uint32_t *__restrict__ knn,
+                                                         const double *__restrict__ knn_d, uint32_t k, uint32_t R,
+                                                         uint32_t na, uint32_t *__restrict__ out,
+                                                         uint32_t *__restrict__ deg) {
+    extern __shared__ __align__(16) uint8_t prune_sm[];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t r = blockIdx.x * (blockDim.x >> 5) + w;
+    if (r >= na) return;
+    const uint32_t d4 = d / 4, words = prune_row_words(d);
+    float4 *rows = reinterpret_cast<float4 *>(prune_sm + (size_t) w * prune_warp_bytes(d, k));
+    double *dab = reinterpret_cast<double *>(rows + (size_t) k * words);
+    uint32_t *ids = reinterpret_cast<uint32_t *>(dab + k);
+    uint32_t *al = ids + k;
+    // The list up to its first invalid id.
+    uint32_t kv = k;
+    for (uint32_t i0 = 0; i0 < k; i0 += 32) {
+        const uint32_t i = i0 + lane;
+        const uint32_t b = i < k ? knn[(size_t) r * k + i] : 0u;
+        if (i < k) {
+            ids[i] = b;
+            dab[i] = knn_d[(size_t) r * k + i];
+            al[i] = i;
+        }
+        const uint32_t bad = __ballot_sync(0xffffffffu, i < k && b >= n);
+        if (bad) {
+            kv = i0 + __ffs(bad) - 1;
+            break;
+        }
+    }
+    __syncwarp();
+    for (uint32_t e = lane; e < kv * d4; e += 32) {
+        const uint32_t i = e / d4, c = e - i * d4;
+        const uint32_t dst = (uint32_t) __cvta_generic_to_shared(rows + (size_t) i * words + c);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
+                     "l"(reinterpret_cast<const float4 *>(x + (size_t) ids[i] * d) + c)
+                     : "memory");
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+    const float slack = (float) (d + 8) * 1.2e-7f;
+    uint32_t nk = 0, alive = kv;
+    while (alive && nk < R) {
+        const uint32_t ci = al[0];
+        if (lane == 0) out[(size_t) r * R + nk] = ids[ci];
+        ++nk;
+        const float4 *rc = rows + (size_t) ci * words;
+        uint32_t left = 0;
+        for (uint32_t t0 = 1; t0 < alive; t0 += 32) {
+            const uint32_t t = t0 + lane;
+            const bool have = t < alive;
+            const uint32_t j = have ? al[t] : ci;
+            const float4 *rj = rows + (size_t) j * words;
+            float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll 4
+            for (uint32_t q = 0; q < d4; ++q) {
+                const float4 u = rc[q], v = rj[q];
+                float y = u.x - v.x;
+                s0 = fmaf(y, y, s0);
+                y = u.y - v.y;
+                s1 = fmaf(y, y, s1);
+                y = u.z - v.z;
+                s2 = fmaf(y, y, s2);
+                y = u.w - v.w;
+                s3 = fmaf(y, y, s3);
+            }
+            const float f = (s0 + s1) + (s2 + s3);
+            bool keep = false;
+            if (have) {
+                const double dj = dab[j];
+                if (f > 1e-30f && f < 1e37f && (double) f * (1.0 - (double) slack) > dj) {
+                    keep = true;
+                } else if (f > 1e-30f && f < 1e37f && (double) f * (1.0 + (double) slack) < dj) {
+                    keep = false;
+                } else {
+                    keep = !(d64(reinterpret_cast<const float *>(rc), reinterpret_cast<const float *>(rj), d) < dj);
+                }
+            }
+            const uint32_t bm = __ballot_sync(0xffffffffu, keep);
+            if (keep) al[left + __popc(bm & ((1u << lane) - 1u))] = j;
+            left += __popc(bm);
+            __syncwarp();
+        }
+        alive = left;
+    }
     if (lane == 0) deg[r] = nk;
 }
 
@@ -524,9 +667,22 @@ static int finish_graph(const float *base, const float *x, uint32_t n, uint32_t 
     for (uint32_t a0 = 0; a0 < n; a0 += chunk) {
         const uint32_t na = std::min(chunk, n - a0);
         GCU(cudaMemsetAsync(knn.p, 0xff, (size_t) na * k * 4, s));
-        rerank_kernel<<<(na + 7) / 8, 256, 0, s>>>(x, n, d, cand, C, k, a0, na, knn.p, knn_d.p);
+        if (d % 4 == 0 && d <= kMaxVecD)
+            rerank_kernel<true><<<(na + 7) / 8, 256, 0, s>>>(x, n, d, cand, C, k, a0, na, knn.p, knn_d.p);
+        else
+            rerank_kernel<false><<<(na + 7) / 8, 256, 0, s>>>(x, n, d, cand, C, k, a0, na, knn.p, knn_d.p);
         GCU(cudaGetLastError());
-        prune_kernel<<<(na + 7) / 8, 256, 8 * R * 4, s>>>(x, n, d, knn.p, knn_d.p, k, R, na, pr.p, deg.p);
+        // Rows in shared memory while two blocks of at least one warp fit an SM.
+        const uint32_t per_warp = prune_warp_bytes(d, k);
+        if (d % 4 == 0 && per_warp <= 112u * 1024u) {
+            const uint32_t wpb = std::max(1u, std::min(4u, 112u * 1024u / per_warp));
+            GCU(cudaFuncSetAttribute(prune_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int) (wpb * per_warp)));
+            prune_rows_kernel<<<(na + wpb - 1) / wpb, wpb * 32, wpb * per_warp, s>>>(x, n, d, knn.p, knn_d.p, k, R, na,
+                                                                                    pr.p, deg.p);
+        } else {
+            prune_kernel<<<(na + 7) / 8, 256, 8 * R * 4, s>>>(x, n, d, knn.p, knn_d.p, k, R, na, pr.p, deg.p);
+        }
         GCU(cudaGetLastError());
         GCU(cudaMemcpyAsync(prh.data() + (size_t) a0 * R, pr.p, (size_t) na * R * 4, cudaMemcpyDeviceToHost, s));
         GCU(cudaMemcpyAsync(degh.data() + a0, deg.p, na * 4ull, cudaMemcpyDeviceToHost, s));

@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "../../include/panns_build.h"
+#include "dev_scratch.h"
 #include "graph_types.h"
 #include "learned.h"
 #include "tc_screen.h"
@@ -46,13 +47,7 @@ namespace {
     } while (0)
 
 template <typename T>
-struct Buf {
-    T *p = nullptr;
-    ~Buf() {
-        if (p) cudaFree(p);
-    }
-    cudaError_t alloc(size_t n) { return cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)); }
-};
+using Buf = Scratch<T>;
 
 constexpr int kBQ = 64;    // rows (queries) per block
 constexpr int kBV = 128;   // candidate rows per tile
@@ -653,12 +648,12 @@ static int finish_graph(const float *base, const float *x, uint32_t n, uint32_t 
     const uint32_t chunk = std::min<uint32_t>(n, 1u << 23);
     Buf<uint32_t> knn, pr, deg;
     Buf<double> knn_d, mean, dm;
-    GCU(knn.alloc((size_t) chunk * k));
-    GCU(knn_d.alloc((size_t) chunk * k));
-    GCU(pr.alloc((size_t) chunk * R));
-    GCU(deg.alloc(chunk));
-    GCU(mean.alloc(d));
-    GCU(dm.alloc(n));
+    GCU(knn.alloc((size_t) chunk * k, s));
+    GCU(knn_d.alloc((size_t) chunk * k, s));
+    GCU(pr.alloc((size_t) chunk * R, s));
+    GCU(deg.alloc(chunk, s));
+    GCU(mean.alloc(d, s));
+    GCU(dm.alloc(n, s));
     g.reset(new panns_graph());
     g->n = n;
     g->k = k;
@@ -813,21 +808,21 @@ int panns_build_nsg_ex(int device, const float *base, uint32_t n, uint32_t d, ui
     } sg{s};
     Buf<float> x, xn;
     Buf<uint32_t> cand;
-    GCU(x.alloc((size_t) n * d));
-    GCU(xn.alloc(n));
-    GCU(cand.alloc((size_t) n * C));
+    GCU(x.alloc((size_t) n * d, s));
+    GCU(xn.alloc(n, s));
+    GCU(cand.alloc((size_t) n * C, s));
     GCU(cudaMemcpyAsync(x.p, base, (size_t) n * d * 4, cudaMemcpyHostToDevice, s));
     sqnorm32_kernel<<<(n + 255) / 256, 256, 0, s>>>(x.p, n, d, xn.p);
     if (tcg) {
         int num_sms = 0;
         GCU(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device));
         Buf<uint32_t> perm, fail, nfail;
-        GCU(fail.alloc(n));
-        GCU(nfail.alloc(1));
+        GCU(fail.alloc(n, s));
+        GCU(nfail.alloc(1, s));
         int rc = PANNS_OK;
         uint32_t slots = n;
         if (n > 32 * kTcM) {  // below, every tile is near every other
-            GCU(perm.alloc(tc_order_slots(n, true)));
+            GCU(perm.alloc(tc_order_slots(n, true), s));
             rc = tc_locality_order(x.p, n, d, true, perm.p, &slots, s);
             if (rc) return rc;
         }
@@ -852,9 +847,9 @@ int panns_build_nsg_ex(int device, const float *base, uint32_t n, uint32_t d, ui
         const uint32_t TR = std::min(n, 8192u), TC = std::min(n, 32768u);
         Buf<float> G, gld;
         Buf<uint32_t> gcnt;
-        GCU(G.alloc((size_t) TR * TC));
-        GCU(gld.alloc((size_t) n * C));
-        GCU(gcnt.alloc(n));
+        GCU(G.alloc((size_t) TR * TC, s));
+        GCU(gld.alloc((size_t) n * C, s));
+        GCU(gcnt.alloc(n, s));
         GCU(cudaMemsetAsync(gcnt.p, 0, n * 4ull, s));
         cublasHandle_t hb = nullptr;
         if (cublasCreate(&hb) != CUBLAS_STATUS_SUCCESS) return set_error(PANNS_ECUDA, "panns_build_nsg: cublasCreate failed");
@@ -910,8 +905,8 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
         ~SG() { cudaStreamDestroy(s); }
     } sg{s};
     Buf<float> x, xn;
-    GCU(x.alloc((size_t) n * d));
-    GCU(xn.alloc(n));
+    GCU(x.alloc((size_t) n * d, s));
+    GCU(xn.alloc(n, s));
     GCU(cudaMemcpyAsync(x.p, base, (size_t) n * d * 4, cudaMemcpyHostToDevice, s));
     sqnorm32_kernel<<<(n + 255) / 256, 256, 0, s>>>(x.p, n, d, xn.p);
     GCU(cudaGetLastError());
@@ -923,12 +918,12 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
         Buf<float> xs, cent;
         std::vector<uint32_t> idx(S);
         for (uint32_t i = 0; i < S; ++i) idx[i] = (uint32_t) ((uint64_t) i * n / S);
-        GCU(sidx.alloc(S));
-        GCU(xs.alloc((size_t) S * d));
-        GCU(sas.alloc(S));
-        GCU(srep.alloc(cells));
-        GCU(cent.alloc((size_t) cells * d));
-        GCU(dcell.alloc(n));
+        GCU(sidx.alloc(S, s));
+        GCU(xs.alloc((size_t) S * d, s));
+        GCU(sas.alloc(S, s));
+        GCU(srep.alloc(cells, s));
+        GCU(cent.alloc((size_t) cells * d, s));
+        GCU(dcell.alloc(n, s));
         GCU(cudaMemcpyAsync(sidx.p, idx.data(), S * 4ull, cudaMemcpyHostToDevice, s));
         gather_rows_f32_kernel<<<1024, 256, 0, s>>>(x.p, d, sidx.p, S, xs.p);
         GCU(cudaGetLastError());
@@ -938,7 +933,7 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
         if (rc) return rc;
         GCU(cudaMemcpyAsync(cellh.data(), dcell.p, n * 4ull, cudaMemcpyDeviceToHost, s));
         if (P) {
-            GCU(dnear.alloc((size_t) cells * P));
+            GCU(dnear.alloc((size_t) cells * P, s));
             near_cells_kernel<<<cells, 256, 0, s>>>(cent.p, cells, d, P, dnear.p);
             GCU(cudaGetLastError());
             GCU(cudaMemcpyAsync(nearh.data(), dnear.p, (size_t) cells * P * 4, cudaMemcpyDeviceToHost, s));
@@ -960,7 +955,7 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
             blk_row0.push_back(r);
         }
     Buf<uint32_t> cand;
-    GCU(cand.alloc((size_t) n * C));
+    GCU(cand.alloc((size_t) n * C, s));
     GCU(cudaMemsetAsync(cand.p, 0xff, (size_t) n * C * 4, s));
     // Tensor-core screen: every cell padded to whole tiles, a row block of one
     // cell against the tiles of the cell and of its near cells. Where padding
@@ -990,13 +985,13 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
         int num_sms = 0;
         GCU(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device));
         Buf<uint32_t> dorder, dblk, dt0, dnear, davail, fail, nfail;
-        GCU(dorder.alloc(order.size()));
-        GCU(dblk.alloc(blk.size()));
-        GCU(dt0.alloc(cells + 1));
-        GCU(dnear.alloc(nearh.size()));
-        GCU(davail.alloc(cells));
-        GCU(fail.alloc(n));
-        GCU(nfail.alloc(1));
+        GCU(dorder.alloc(order.size(), s));
+        GCU(dblk.alloc(blk.size(), s));
+        GCU(dt0.alloc(cells + 1, s));
+        GCU(dnear.alloc(nearh.size(), s));
+        GCU(davail.alloc(cells, s));
+        GCU(fail.alloc(n, s));
+        GCU(nfail.alloc(1, s));
         GCU(cudaMemcpyAsync(dorder.p, order.data(), order.size() * 4, cudaMemcpyHostToDevice, s));
         GCU(cudaMemcpyAsync(dblk.p, blk.data(), blk.size() * 4, cudaMemcpyHostToDevice, s));
         GCU(cudaMemcpyAsync(dt0.p, tile0.data(), (cells + 1) * 4ull, cudaMemcpyHostToDevice, s));
@@ -1013,11 +1008,11 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
     }
     if (!screened) {
         Buf<uint32_t> dmem, dstart, dnear, dbc, dbr;
-        GCU(dmem.alloc(n));
-        GCU(dstart.alloc(cells + 1));
-        GCU(dnear.alloc(nearh.size()));
-        GCU(dbc.alloc(blk_cell.size()));
-        GCU(dbr.alloc(blk_row0.size()));
+        GCU(dmem.alloc(n, s));
+        GCU(dstart.alloc(cells + 1, s));
+        GCU(dnear.alloc(nearh.size(), s));
+        GCU(dbc.alloc(blk_cell.size(), s));
+        GCU(dbr.alloc(blk_row0.size(), s));
         GCU(cudaMemsetAsync(cand.p, 0xff, (size_t) n * C * 4, s));
         GCU(cudaMemcpyAsync(dmem.p, members.data(), n * 4ull, cudaMemcpyHostToDevice, s));
         GCU(cudaMemcpyAsync(dstart.p, cstart.data(), (cells + 1) * 4ull, cudaMemcpyHostToDevice, s));

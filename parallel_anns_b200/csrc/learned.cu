@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "../../include/panns_learned.h"
+#include "dev_scratch.h"
 #include "learned.h"
 #include "mlp_infer.cuh"
 
@@ -33,22 +34,7 @@ namespace {
     } while (0)
 
 template <typename T>
-struct Dev {
-    T *p = nullptr;
-    size_t n = 0;
-    ~Dev() {
-        if (p) cudaFree(p);
-    }
-    cudaError_t alloc(size_t count) {
-        if (p) cudaFree(p);
-        p = nullptr;
-        n = 0;
-        cudaError_t e = cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T));
-        if (e == cudaSuccess) n = count;
-        else p = nullptr;
-        return e;
-    }
-};
+using Dev = Scratch<T>;
 
 __device__ __forceinline__ float to_f(float x) { return x; }
 __device__ __forceinline__ float to_f(__nv_bfloat16 x) { return __bfloat162float(x); }
@@ -324,11 +310,11 @@ struct Trainer {
     Dev<double> acc;
     Trainer(uint32_t d_, uint32_t R_, uint32_t T_, uint32_t B_) : d(d_), R(R_), T(T_), B(B_), lay(d_, R_) {}
 
-    cudaError_t alloc(bool adam) {
+    cudaError_t alloc(bool adam, cudaStream_t s) {
         cudaError_t e = cudaSuccess;
         const size_t P = lay.total;
-        auto A = [&e](auto &buf, size_t n) {
-            if (e == cudaSuccess) e = buf.alloc(n);
+        auto A = [&e, s](auto &buf, size_t n) {
+            if (e == cudaSuccess) e = buf.alloc(n, s);
         };
         A(w, P);
         A(g, P);
@@ -591,9 +577,9 @@ int kmeans_run(const float *rows, uint32_t n, uint32_t d, uint32_t k, uint32_t i
         std::mt19937_64 rng(seed);
         Dev<uint32_t> dsidx, dslot;
         Dev<float> mind;
-        LCU(dsidx.alloc(S));
-        LCU(dslot.alloc(k));
-        LCU(mind.alloc(S));
+        LCU(dsidx.alloc(S, s));
+        LCU(dslot.alloc(k, s));
+        LCU(mind.alloc(S, s));
         LCU(cudaMemcpyAsync(dsidx.p, sidx.data(), S * 4ull, cudaMemcpyHostToDevice, s));
         LCU(cudaMemsetAsync(mind.p, 0x7f, S * 4ull, s));  // 3.4e38: larger than any distance
         const uint32_t first = (uint32_t) (rng() % S);
@@ -610,11 +596,11 @@ int kmeans_run(const float *rows, uint32_t n, uint32_t d, uint32_t k, uint32_t i
     Dev<uint32_t> didx, doff, dmem;
     Dev<float> cn, G;
     const uint32_t chunk = std::min<uint32_t>(n, 65536);
-    LCU(didx.alloc(k));
-    LCU(doff.alloc(k + 1));
-    LCU(dmem.alloc(n));
-    LCU(cn.alloc(k));
-    LCU(G.alloc((size_t) chunk * k));
+    LCU(didx.alloc(k, s));
+    LCU(doff.alloc(k + 1, s));
+    LCU(dmem.alloc(n, s));
+    LCU(cn.alloc(k, s));
+    LCU(G.alloc((size_t) chunk * k, s));
     LCU(cudaMemcpyAsync(didx.p, start.data(), k * 4ull, cudaMemcpyHostToDevice, s));
     gather_rows_kernel<<<k, 128, 0, s>>>(rows, d, didx.p, k, cent);
     LCU(cudaGetLastError());
@@ -673,8 +659,8 @@ int nearest_centroid(const float *rows, uint32_t n, uint32_t d, const float *cen
                      cudaStream_t s) {
     Dev<float> cn, G;
     const uint32_t chunk = std::min<uint32_t>(n, std::max<uint32_t>(1024u, (uint32_t) std::min<uint64_t>(65536, (1ull << 29) / k)));
-    LCU(cn.alloc(k));
-    LCU(G.alloc((size_t) chunk * k));
+    LCU(cn.alloc(k, s));
+    LCU(G.alloc((size_t) chunk * k, s));
     sqnorm_kernel<<<(k + 255) / 256, 256, 0, s>>>(cent, k, d, cn.p);
     LCU(cudaGetLastError());
     for (uint32_t r0 = 0; r0 < n; r0 += chunk) {
@@ -691,7 +677,7 @@ int nearest_centroid(const float *rows, uint32_t n, uint32_t d, const float *cen
 int nearest_center(const float *rows, uint32_t n, uint32_t d, const uint32_t *center_rows, uint32_t k,
                    uint32_t *cell, cudaStream_t s) {
     Dev<float> cent;
-    LCU(cent.alloc((size_t) k * d));
+    LCU(cent.alloc((size_t) k * d, s));
     gather_rows_kernel<<<k, 128, 0, s>>>(rows, d, center_rows, k, cent.p);
     LCU(cudaGetLastError());
     return nearest_centroid(rows, n, d, cent.p, k, cell, s);
@@ -923,7 +909,7 @@ int panns_mlp_loss_grad(int device, uint32_t d, uint32_t R, uint32_t T, const fl
         ~StreamGuard() { cudaStreamDestroy(s); }
     } guard{s};
     Trainer t(d, R, T, B);
-    LCU(t.alloc(false));
+    LCU(t.alloc(false, s));
     const size_t P = t.lay.total;
     LCU(cudaMemcpyAsync(t.w.p, params, P * 4, cudaMemcpyHostToDevice, s));
     LCU(cudaMemcpyAsync(t.Xb.p, X, (size_t) B * d * 4, cudaMemcpyHostToDevice, s));
@@ -954,7 +940,7 @@ int panns_mlp_forward(int device, uint32_t d, uint32_t R, const float *params, c
     } guard{s};
     const uint32_t B = std::min<uint32_t>(n, 8192);
     Trainer t(d, R, 1, B);
-    LCU(t.alloc(false));
+    LCU(t.alloc(false, s));
     const size_t P = t.lay.total;
     LCU(cudaMemcpyAsync(t.w.p, params, P * 4, cudaMemcpyHostToDevice, s));
     to_bf16_kernel<<<256, 256, 0, s>>>(t.w.p, t.wb.p, P);
@@ -989,15 +975,15 @@ int panns_mlp_train(int device, const panns_mlp_train_params *tp, const float *X
         ~StreamGuard() { cudaStreamDestroy(s); }
     } guard{s};
     Trainer t(d, R, T, B);
-    LCU(t.alloc(true));
+    LCU(t.alloc(true, s));
     const size_t P = t.lay.total;
     Dev<float> dX, dy;
     Dev<uint16_t> dc;
     Dev<uint32_t> didx;
-    LCU(dX.alloc((size_t) n * d));
-    LCU(dy.alloc(n));
-    LCU(dc.alloc((size_t) n * T));
-    LCU(didx.alloc(n));
+    LCU(dX.alloc((size_t) n * d, s));
+    LCU(dy.alloc(n, s));
+    LCU(dc.alloc((size_t) n * T, s));
+    LCU(didx.alloc(n, s));
     LCU(cudaMemcpyAsync(dX.p, X, (size_t) n * d * 4, cudaMemcpyHostToDevice, s));
     LCU(cudaMemcpyAsync(dy.p, y, (size_t) n * 4, cudaMemcpyHostToDevice, s));
     LCU(cudaMemcpyAsync(dc.p, cells, (size_t) n * T * 2, cudaMemcpyHostToDevice, s));

@@ -47,6 +47,7 @@
 #include <vector>
 
 #include "../../include/panns_build.h"
+#include "dev_scratch.h"
 #include "graph_types.h"
 #include "learned.h"
 #include "search_kernel.cuh"
@@ -62,13 +63,7 @@ namespace {
     } while (0)
 
 template <typename T>
-struct NBuf {
-    T *p = nullptr;
-    ~NBuf() {
-        if (p) cudaFree(p);
-    }
-    cudaError_t alloc(size_t n) { return cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)); }
-};
+using NBuf = Scratch<T>;
 
 // DistanceL2::compare of rows a and b (either order gives the same bits).
 __host__ __device__ inline float l2_ref(const float *a, const float *b, uint32_t d) {
@@ -492,15 +487,15 @@ extern "C" int panns_efanna_build(int device, const float *base, uint32_t n, uin
     const uint32_t slots = blocks * kLinkWarps;
     NBuf<float> dx, dcd;
     NBuf<uint32_t> dknn, dinit, dvis, ddirty, dcid, dcn, dctl;
-    NCU(dx.alloc((size_t) n * d));
-    NCU(dknn.alloc((size_t) n * knn_k));
-    NCU(dinit.alloc((size_t) n * L));
-    NCU(dvis.alloc((size_t) slots * vis_words));
-    NCU(ddirty.alloc((size_t) slots * kLinkDirty));
-    NCU(dcid.alloc((size_t) n * R));
-    NCU(dcd.alloc((size_t) n * R));
-    NCU(dcn.alloc(n));
-    NCU(dctl.alloc(2));
+    NCU(dx.alloc((size_t) n * d, s));
+    NCU(dknn.alloc((size_t) n * knn_k, s));
+    NCU(dinit.alloc((size_t) n * L, s));
+    NCU(dvis.alloc((size_t) slots * vis_words, s));
+    NCU(ddirty.alloc((size_t) slots * kLinkDirty, s));
+    NCU(dcid.alloc((size_t) n * R, s));
+    NCU(dcd.alloc((size_t) n * R, s));
+    NCU(dcn.alloc(n, s));
+    NCU(dctl.alloc(2, s));
     NCU(cudaMemcpyAsync(dx.p, base, (size_t) n * d * 4, cudaMemcpyHostToDevice, s));
     NCU(cudaMemcpyAsync(dknn.p, knn, (size_t) n * knn_k * 4, cudaMemcpyHostToDevice, s));
     NCU(cudaMemcpyAsync(dinit.p, init.data(), init.size() * 4, cudaMemcpyHostToDevice, s));

@@ -15,6 +15,7 @@
 
 #include "../../include/panns_b200.h"
 #include "../../include/panns_learned.h"
+#include "dev_scratch.h"
 #include "graph_types.h"
 #include "learned.h"
 #include "search_kernel.cuh"
@@ -145,6 +146,12 @@ struct DevBuf {
         if (count <= n && p) return cudaSuccess;
         release();
         cudaError_t e = cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T));
+        if (e == cudaErrorMemoryAllocation) {  // the idle scratch may be what is missing
+            int device = 0;
+            cudaGetLastError();
+            if (cudaGetDevice(&device) == cudaSuccess) scratch_trim(device);
+            e = cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T));
+        }
         if (e == cudaSuccess) n = count;
         else p = nullptr;
         return e;
@@ -241,6 +248,7 @@ int panns_close(panns_index *h) {
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
     if (h->stream) cudaStreamDestroy(h->stream);
+    scratch_trim(h->device);
     delete h;
     return PANNS_OK;
 }
@@ -401,9 +409,9 @@ static int finalize(panns_index *h) {
         const uint32_t C = std::max(1u, std::min(4096u, n / 256));
         std::vector<uint32_t> piv(C), cell(n);
         for (uint32_t p = 0; p < C; ++p) piv[p] = (uint32_t) (((uint64_t) p * n) / C);
-        DevBuf<uint32_t> dpiv, dcell;
-        CU(dpiv.ensure(C));
-        CU(dcell.ensure(n));
+        Scratch<uint32_t> dpiv, dcell;
+        CU(dpiv.alloc(C, h->stream));
+        CU(dcell.alloc(n, h->stream));
         CU(cudaMemcpyAsync(dpiv.p, piv.data(), C * 4ull, cudaMemcpyHostToDevice, h->stream));
         int rc = panns::nearest_center(h->base_raw.p, n, h->d, dpiv.p, C, dcell.p, h->stream);
         if (rc) return rc;
@@ -1204,12 +1212,12 @@ int panns_ground_truth(panns_index *h, const float *queries, uint32_t nq, uint32
     uint32_t stride = 0;
     rc = stage_init(h, &p, nullptr, nq, h->stream, d_init, stride);
     if (rc) return rc;
-    DevBuf<float> dq;
-    DevBuf<uint32_t> dids, dcnt;
-    DevBuf<double> dtau;
-    CU(dq.ensure((size_t) nq * h->d));
-    CU(dids.ensure((size_t) nq * k));
-    CU(dtau.ensure(nq));
+    Scratch<float> dq;
+    Scratch<uint32_t> dids, dcnt;
+    Scratch<double> dtau;
+    CU(dq.alloc((size_t) nq * h->d, h->stream));
+    CU(dids.alloc((size_t) nq * k, h->stream));
+    CU(dtau.alloc(nq, h->stream));
     CU(h->hq.ensure((size_t) nq * h->dpad));
     CU(h->stats.ensure(nq));
     CU(cudaMemcpyAsync(dq.p, queries, (size_t) nq * h->d * 4, cudaMemcpyHostToDevice, h->stream));
@@ -1240,11 +1248,11 @@ int panns_ground_truth(panns_index *h, const float *queries, uint32_t nq, uint32
             slots += (h->cell_start[c + 1] - h->cell_start[c] + kTcM - 1) / kTcM * (uint64_t) kTcM;
         }
         if (slots > 0xfffffff0ull) return fail(PANNS_EINVAL, "panns_ground_truth: too many vertices");
-        DevBuf<uint32_t> dfrom, dto, perm, dtodo;
-        CU(dfrom.ensure(cells + 1));
-        CU(dto.ensure(cells));
-        CU(perm.ensure((size_t) slots));
-        CU(dtodo.ensure(nq));
+        Scratch<uint32_t> dfrom, dto, perm, dtodo;
+        CU(dfrom.alloc(cells + 1, h->stream));
+        CU(dto.alloc(cells, h->stream));
+        CU(perm.alloc((size_t) slots, h->stream));
+        CU(dtodo.alloc(nq, h->stream));
         CU(cudaMemcpyAsync(dfrom.p, h->cell_start.data(), (cells + 1) * 4ull, cudaMemcpyHostToDevice, h->stream));
         CU(cudaMemcpyAsync(dto.p, to.data(), cells * 4ull, cudaMemcpyHostToDevice, h->stream));
         CU(cudaMemsetAsync(perm.p, 0xff, (size_t) slots * 4, h->stream));
@@ -1256,26 +1264,26 @@ int panns_ground_truth(panns_index *h, const float *queries, uint32_t nq, uint32
         std::vector<uint32_t> todo(nq);
         CU(cudaMemcpyAsync(todo.data(), dtodo.p, nq * 4ull, cudaMemcpyDeviceToHost, h->stream));
         CU(cudaStreamSynchronize(h->stream));
-        DevBuf<uint32_t> oid;
-        DevBuf<double> odist;
-        CU(oid.ensure((size_t) nq * k));
-        CU(odist.ensure(out_dist ? (size_t) nq * k : 1));
+        Scratch<uint32_t> oid;
+        Scratch<double> odist;
+        CU(oid.alloc((size_t) nq * k, h->stream));
+        CU(odist.alloc(out_dist ? (size_t) nq * k : 1, h->stream));
         const uint32_t cap = 4 * k + 64, batch = 16384;
         for (int pass = 0; pass < 4 && !todo.empty(); ++pass) {
             std::vector<uint32_t> over;
             for (size_t b0 = 0; b0 < todo.size(); b0 += batch) {
                 const uint32_t m = (uint32_t) std::min<size_t>(batch, todo.size() - b0);
                 const uint32_t splits = tc_range_splits(m, h->num_sms);
-                DevBuf<uint32_t> dorder, lcnt, dover;
-                DevBuf<float> qs;
-                DevBuf<double> ts;
-                DevBuf<uint2> lists;
-                CU(dorder.ensure(m));
-                CU(qs.ensure((size_t) m * h->d));
-                CU(ts.ensure(m));
-                CU(lists.ensure((size_t) m * splits * cap));
-                CU(lcnt.ensure((size_t) m * splits));
-                CU(dover.ensure(m));
+                Scratch<uint32_t> dorder, lcnt, dover;
+                Scratch<float> qs;
+                Scratch<double> ts;
+                Scratch<uint2> lists;
+                CU(dorder.alloc(m, h->stream));
+                CU(qs.alloc((size_t) m * h->d, h->stream));
+                CU(ts.alloc(m, h->stream));
+                CU(lists.alloc((size_t) m * splits * cap, h->stream));
+                CU(lcnt.alloc((size_t) m * splits, h->stream));
+                CU(dover.alloc(m, h->stream));
                 CU(cudaMemcpyAsync(dorder.p, todo.data() + b0, m * 4ull, cudaMemcpyHostToDevice, h->stream));
                 gt_gather_kernel<<<m, 64, 0, h->stream>>>(dq.p, dtau.p, dorder.p, m, h->d, qs.p, ts.p);
                 CU(cudaGetLastError());
@@ -1339,24 +1347,24 @@ int panns_ground_truth(panns_index *h, const float *queries, uint32_t nq, uint32
     const uint32_t nl = (uint32_t) left.size();
     std::vector<uint32_t> cnt(nl);
     std::vector<uint32_t> over;  // places in `left` of the queries whose lists overflowed
-    DevBuf<float> lq;
-    DevBuf<double> ltau;
+    Scratch<float> lq;
+    Scratch<double> ltau;
     {
-        DevBuf<uint32_t> dleft;
-        CU(dleft.ensure(nl));
-        CU(lq.ensure((size_t) nl * h->d));
-        CU(ltau.ensure(nl));
-        CU(dcnt.ensure(nl));
+        Scratch<uint32_t> dleft;
+        CU(dleft.alloc(nl, h->stream));
+        CU(lq.alloc((size_t) nl * h->d, h->stream));
+        CU(ltau.alloc(nl, h->stream));
+        CU(dcnt.alloc(nl, h->stream));
         CU(cudaMemcpyAsync(dleft.p, left.data(), nl * 4ull, cudaMemcpyHostToDevice, h->stream));
         gt_gather_kernel<<<nl, 64, 0, h->stream>>>(dq.p, dtau.p, dleft.p, nl, h->d, lq.p, ltau.p);
         CU(cudaGetLastError());
         CU(cudaStreamSynchronize(h->stream));
     }
     {
-        DevBuf<double> cd;
-        DevBuf<uint32_t> ci;
-        CU(cd.ensure((size_t) nl * cap));
-        CU(ci.ensure((size_t) nl * cap));
+        Scratch<double> cd;
+        Scratch<uint32_t> ci;
+        CU(cd.alloc((size_t) nl * cap, h->stream));
+        CU(ci.alloc((size_t) nl * cap, h->stream));
         CU(collect(lq.p, ltau.p, nl, cap, dcnt.p, cd.p, ci.p));
         CU(cudaMemcpyAsync(cnt.data(), dcnt.p, nl * 4ull, cudaMemcpyDeviceToHost, h->stream));
         std::vector<double> hd((size_t) nl * cap);
@@ -1396,14 +1404,14 @@ int panns_ground_truth(panns_index *h, const float *queries, uint32_t nq, uint32
             const uint32_t q = left[over[g0 + i]];
             std::copy(queries + (size_t) q * h->d, queries + (size_t) (q + 1) * h->d, qh.begin() + (size_t) i * h->d);
         }
-        DevBuf<float> gq;
-        DevBuf<double> gt, cd;
-        DevBuf<uint32_t> gc, ci;
-        CU(gq.ensure(qh.size()));
-        CU(gt.ensure(m));
-        CU(gc.ensure(m));
-        CU(cd.ensure((size_t) m * gcap));
-        CU(ci.ensure((size_t) m * gcap));
+        Scratch<float> gq;
+        Scratch<double> gt, cd;
+        Scratch<uint32_t> gc, ci;
+        CU(gq.alloc(qh.size(), h->stream));
+        CU(gt.alloc(m, h->stream));
+        CU(gc.alloc(m, h->stream));
+        CU(cd.alloc((size_t) m * gcap, h->stream));
+        CU(ci.alloc((size_t) m * gcap, h->stream));
         CU(cudaMemcpyAsync(gq.p, qh.data(), qh.size() * 4, cudaMemcpyHostToDevice, h->stream));
         for (uint32_t i = 0; i < m; ++i)
             CU(cudaMemcpyAsync(gt.p + i, ltau.p + over[g0 + i], 8, cudaMemcpyDeviceToDevice, h->stream));
@@ -1673,11 +1681,11 @@ extern "C" int panns_kmeans(panns_index *h, uint32_t k, uint32_t iters, uint32_t
     if (!h) return fail(PANNS_EINVAL, "panns_kmeans: NULL handle");
     if (!h->n || !h->base_raw.p) return fail(PANNS_ESTATE, "panns_kmeans: no base vectors loaded");
     CU(cudaSetDevice(h->device));
-    DevBuf<float> cent;
-    DevBuf<uint32_t> as, rep;
-    CU(cent.ensure((size_t) k * h->d));
-    CU(as.ensure(h->n));
-    CU(rep.ensure(k));
+    Scratch<float> cent;
+    Scratch<uint32_t> as, rep;
+    CU(cent.alloc((size_t) k * h->d, h->stream));
+    CU(as.alloc(h->n, h->stream));
+    CU(rep.alloc(k, h->stream));
     int rc = panns::kmeans_run(h->base_raw.p, h->n, h->d, k, iters, seed, cent.p, as.p, rep.p, h->stream);
     if (rc) return rc;
     if (rep_ids) CU(cudaMemcpyAsync(rep_ids, rep.p, k * 4ull, cudaMemcpyDeviceToHost, h->stream));

@@ -54,6 +54,7 @@
 #include <vector>
 
 #include "../../include/panns_b200.h"
+#include "dev_scratch.h"
 #include "learned.h"
 #include "tc_screen.h"
 
@@ -1156,13 +1157,7 @@ int make_map(CUtensorMap *map, const __nv_bfloat16 *x, uint64_t rows, uint32_t w
     } while (0)
 
 template <typename T>
-struct TBuf {
-    T *p = nullptr;
-    ~TBuf() {
-        if (p) cudaFree(p);
-    }
-    cudaError_t alloc(size_t n) { return cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)); }
-};
+using TBuf = Scratch<T>;
 
 struct TcShape {
     uint32_t W, slices, stages, k_hh, k_x;
@@ -1221,9 +1216,9 @@ int tc_locality_order(const float *x, uint32_t n, uint32_t d, bool padded, uint3
     const uint32_t h = (d + 1) / 2, S = std::min(n, std::min(1024u, 200u * 1024u / (h * 4)));
     std::vector<uint32_t> count(cells);
     TBuf<uint32_t> dpiv, cell, start;
-    TCU(dpiv.alloc(cells));
-    TCU(cell.alloc(n));
-    TCU(start.alloc(cells));
+    TCU(dpiv.alloc(cells, s));
+    TCU(cell.alloc(n, s));
+    TCU(start.alloc(cells, s));
     TCU(cudaFuncSetAttribute(tc_pivot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (S * h * 4)));
     tc_pivot_kernel<<<1, 1024, S * h * 4, s>>>(x, n, d, S, cells, dpiv.p);
     TCU(cudaGetLastError());
@@ -1265,15 +1260,15 @@ int tc_screen_knn(const float *x, uint32_t n, uint32_t d, uint32_t k, uint32_t C
     uint32_t per = std::min(tiles, kTcKnnBlocks);
     if (skip) {
         per = std::min<uint32_t>(per, std::max<uint32_t>(4u * num_sms, (1u << 28) / tiles));
-        TCU(centre.alloc((size_t) tiles * d));
-        TCU(radius.alloc(tiles));
-        TCU(lb2.alloc((size_t) per * tiles));
+        TCU(centre.alloc((size_t) tiles * d, s));
+        TCU(radius.alloc(tiles, s));
+        TCU(lb2.alloc((size_t) per * tiles, s));
     }
-    TCU(A.alloc((size_t) per * kTcM * 2 * sh.W));
-    TCU(B.alloc((size_t) pad * 2 * sh.W));
-    TCU(xn.alloc(pad));
-    TCU(ctl.alloc(4));
-    TCU(shift.alloc(d));
+    TCU(A.alloc((size_t) per * kTcM * 2 * sh.W, s));
+    TCU(B.alloc((size_t) pad * 2 * sh.W, s));
+    TCU(xn.alloc(pad, s));
+    TCU(ctl.alloc(4, s));
+    TCU(shift.alloc(d, s));
     TCU(cudaMemsetAsync(ctl.p, 0, 16, s));
     TCU(cudaMemsetAsync(fail_count, 0, 4, s));
     tc_shift_kernel<<<d, 256, 0, s>>>(x, n, d, shift.p);
@@ -1282,7 +1277,7 @@ int tc_screen_knn(const float *x, uint32_t n, uint32_t d, uint32_t k, uint32_t C
                                                        per == tiles ? A.p : nullptr, B.p, xn.p, ctl.p + 2, nullptr,
                                                        centre.p, radius.p);
     TCU(cudaGetLastError());
-    TCU(lists.alloc((size_t) std::min<uint32_t>(per, (uint32_t) num_sms) * kTcM * kTcCap));
+    TCU(lists.alloc((size_t) std::min<uint32_t>(per, (uint32_t) num_sms) * kTcM * kTcCap, s));
     CUtensorMap ma, mb;
     int rc = make_map(&ma, A.p, (uint64_t) per * kTcM, 2 * sh.W);
     if (!rc) rc = make_map(&mb, B.p, pad, 2 * sh.W);
@@ -1362,15 +1357,15 @@ int tc_screen_range(const float *x, uint32_t n, uint32_t d, const uint32_t *perm
     TBuf<__nv_bfloat16> A, B;
     TBuf<float> xn, cb, rad, need, ft, shift;
     TBuf<uint32_t> ctl;  // counter, error, ymax, huge
-    TCU(A.alloc((size_t) qpad * 2 * sh.W));
-    TCU(B.alloc((size_t) chunk * 2 * sh.W));
-    TCU(xn.alloc(qpad));
-    TCU(cb.alloc((size_t) ct * d));
-    TCU(rad.alloc(ct));
-    TCU(need.alloc((size_t) rb * ct));
-    TCU(ft.alloc(nq));
-    TCU(shift.alloc(d));
-    TCU(ctl.alloc(4));
+    TCU(A.alloc((size_t) qpad * 2 * sh.W, s));
+    TCU(B.alloc((size_t) chunk * 2 * sh.W, s));
+    TCU(xn.alloc(qpad, s));
+    TCU(cb.alloc((size_t) ct * d, s));
+    TCU(rad.alloc(ct, s));
+    TCU(need.alloc((size_t) rb * ct, s));
+    TCU(ft.alloc(nq, s));
+    TCU(shift.alloc(d, s));
+    TCU(ctl.alloc(4, s));
     TCU(cudaMemsetAsync(ctl.p, 0, 16, s));
     TCU(cudaMemsetAsync(cnt, 0, (size_t) splits * nq * 4, s));
     tc_shift_kernel<<<d, 256, 0, s>>>(x, n, d, shift.p);

@@ -5,213 +5,347 @@
 //
 // One block of W warps runs one query at a time (work-stealing counter across
 // blocks). The queue lives in the block's shared memory. A search step is:
-//   1. warp 0 picks the M best unchecked candidates (as in search_kernel);
-//   2. in rounds, warp w expands candidates w, w + W, ... (at most G per warp
-//      and round, G * width <= kBuf so its fresh buffer cannot overflow):
-//      head rows, visited test-and-set on the block's bitset, distances, then
-//      the filter against the queue's L-th distance at the start of the round,
-//      then a sort of its survivors;
-//   3. the W sorted survivor lists are placed into one sorted list by rank
-//      (each element's index plus the number of smaller elements in the other
-//      lists; (distance, original id) is a total order), and the whole block
-//      merges that list into the queue (the rank merge of merge_into, spread
-//      over W * 32 threads).
+//   1. every warp finds the M best unchecked candidates by itself (the queue
+//      does not change meanwhile; they are marked after the next barrier);
+//   2. in rounds, the warps expand candidates (at most G per warp and round, G *
+//      width <= kBuf so a warp's fresh buffer cannot overflow; several warps
+//      share a candidate's row when there are fewer candidates than warps): head
+//      rows, visited test-and-set on the block's bitset, distances, the filter
+//      against the queue's L-th distance at the start of the round; the
+//      survivors of all warps are appended to one list;
+//   3. that list is ranked by counting (a thread, or several, per element; a
+//      bitonic network when it is long), each element's place in the queue is
+//      found by binary search, and the queue's elements move up by the number
+//      of list elements before them, read and written in chunks of registers.
 // Each round's merge leaves the queue equal to the L best of (queue + round
 // survivors), and the round's first insert position is the best survivor's,
 // exactly as one flush of search_kernel (see the exactness note there), so
 // ids and distance counts equal search_kernel's and the reference's.
+//
+// Bound by latency: a step is a chain of dependent loads (head row, visited
+// word, rows) and of barriers. The form before sorted every warp's survivors,
+// placed W lists into one by serial binary searches and moved the queue one
+// element per thread and barrier pair, with the original ids loaded for every
+// survivor (here only when two distances are equal): nine barriers a step, four
+// now.
 #pragma once
 
 #include "search_kernel.cuh"
 
 namespace panns {
 
-constexpr int kBlockCtl = 24;  // control words in shared memory (BC_SEG + W <= 24)
+constexpr int kBlockCtl = 16;  // control words in shared memory
+// Longest list ranked by counting; above, the bitonic network (initial queues).
+__host__ __device__ constexpr uint32_t block_rank_max(uint32_t W) { return 64u * W; }
 
 // Shared memory of one block of W warps with a queue of queue_cap entries.
 __host__ __device__ inline uint32_t block_smem_bytes(uint32_t queue_cap, uint32_t W) {
-    return queue_cap * 8u                                             // queue (dist, id)
-           + W * (kBuf * 12u + kCandGroup * kHeadWords * 4u + 64u * 4u) // per-warp lists, head rows, scratch
-           + W * kBuf * 12u                                           // merged sorted survivors
-           + kMaxM * 4u                                               // picked candidates
-           + kBlockCtl * 4u;                                          // control words
+    return queue_cap * 8u                     // queue (dist, id)
+           + W * kBuf * 8u                    // per-warp fresh ids and distances
+           + W * kBuf * 12u                   // survivors of a round (dist, id, key)
+           + block_rank_max(W) * 12u          // ranked survivors (dist, id, place)
+           + W * kMaxM * 4u                   // per-warp picked candidates / learned entries
+           + kBlockCtl * 4u;                  // control words
 }
 
-enum { BC_Q = 0, BC_SZ, BC_CNT, BC_LASTK, BC_K, BC_NK, BC_DIRTY, BC_DIST, BC_EDGES, BC_LRN, BC_LQ,
-       BC_SEG };  // BC_SEG + w, w < W <= 8
+enum { BC_Q = 0, BC_CNT, BC_CNT2, BC_TIE, BC_DIST, BC_EDGES, BC_FULL };
 
-// Number of elements of the sorted list (d, k)[0..n) that precede (dv, kv).
-__device__ __forceinline__ uint32_t list_rank(const float *d, const uint32_t *k, uint32_t n, float dv, uint32_t kv) {
-    uint32_t lo = 0, hi = n;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (plain_less(d[mid], k[mid], dv, kv)) lo = mid + 1;
-        else hi = mid;
+// Total order of distances for ranking equal ones (and NaN): floats as
+// unsigned integers that compare the same way.
+__device__ __forceinline__ uint32_t dist_key(float d) {
+    const uint32_t b = __float_as_uint(d + 0.0f);
+    return b & 0x80000000u ? ~b : b | 0x80000000u;
+}
+
+template <int W>
+struct BlockMem {
+    float *qd;
+    uint32_t *qi;
+    float *cD;       // survivors of the round
+    uint32_t *cI, *cK;
+    float *sD;       // ranked survivors
+    uint32_t *sI, *sP;
+    uint32_t *ctl;
+};
+
+// Ranks of the n <= block_rank_max(W) survivors by (distance, original id):
+// writes (sD, sI) in that order and, with PLACE, sP = the number of queue
+// elements (qd, qi)[0..sz) before each. Several adjacent threads count for one
+// element when there are fewer elements than threads; the counts of smaller and
+// of smaller or equal distances differ by more than the element itself only
+// where distances are equal (or NaN): then the block counts again by (distance,
+// original id), a total order. Called by the whole block after a barrier; ends
+// with one.
+template <int W, bool PLACE>
+__device__ __forceinline__ void block_rank(const BlockMem<W> &m, uint32_t n, uint32_t sz,
+                                           const uint32_t *__restrict__ orig) {
+    constexpr uint32_t T = W * 32;
+    const uint32_t tid = threadIdx.x;
+    uint32_t parts = 1;  // threads per element
+    while (parts < 16 && n * parts * 2 <= T) parts *= 2;
+    const uint32_t per = T / parts;  // elements per pass
+    const uint32_t quads = n / 4;
+    const uint32_t share = (quads + parts - 1) / parts;
+    const uint32_t part = tid & (parts - 1);
+    const float4 *c4 = reinterpret_cast<const float4 *>(m.cD);
+    for (uint32_t e0 = 0; e0 < n; e0 += per) {  // block-uniform: the shuffles are too
+        const uint32_t e = e0 + tid / parts;
+        const float d = e < n ? m.cD[e] : 0.f;
+        uint32_t less = 0, upto = 0;
+        const uint32_t q1 = min(quads, (part + 1) * share);
+#pragma unroll 2
+        for (uint32_t q = part * share; q < q1; ++q) {
+            const float4 x = c4[q];
+            less += x.x < d ? 1u : 0u;
+            upto += x.x <= d ? 1u : 0u;
+            less += x.y < d ? 1u : 0u;
+            upto += x.y <= d ? 1u : 0u;
+            less += x.z < d ? 1u : 0u;
+            upto += x.z <= d ? 1u : 0u;
+            less += x.w < d ? 1u : 0u;
+            upto += x.w <= d ? 1u : 0u;
+        }
+        if (part == 0)
+            for (uint32_t f = 4 * quads; f < n; ++f) {
+                less += m.cD[f] < d ? 1u : 0u;
+                upto += m.cD[f] <= d ? 1u : 0u;
+            }
+        for (uint32_t o = 1; o < parts; o <<= 1) {
+            less += __shfl_xor_sync(kFull, less, o);
+            upto += __shfl_xor_sync(kFull, upto, o);
+        }
+        if (e < n && part == 0) {
+            if (upto != less + 1) m.ctl[BC_TIE] = 1u;
+            const uint32_t r = min(less, n - 1), id = m.cI[e];
+            m.sD[r] = d;
+            m.sI[r] = id;
+            if (PLACE) m.sP[r] = queue_rank<ORDER_PANNS>(m.qd, m.qi, sz, d, id & kIdMask, orig);
+        }
     }
-    return lo;
+    __syncthreads();
+    if (m.ctl[BC_TIE]) {  // block-uniform
+        for (uint32_t e = tid; e < n; e += T) m.cK[e] = __ldg(orig + (m.cI[e] & kIdMask));
+        __syncthreads();
+        if (tid == 0) m.ctl[BC_TIE] = 0u;
+        for (uint32_t e = tid; e < n; e += T) {
+            const float d = m.cD[e];
+            const uint32_t kd = dist_key(d), ko = m.cK[e], id = m.cI[e];
+            uint32_t r = 0;
+            for (uint32_t f = 0; f < n; ++f) {
+                const uint32_t fd = dist_key(m.cD[f]);
+                r += fd < kd || (fd == kd && m.cK[f] < ko) ? 1u : 0u;
+            }
+            m.sD[r] = d;
+            m.sI[r] = id;
+            if (PLACE) m.sP[r] = queue_rank<ORDER_PANNS>(m.qd, m.qi, sz, d, id & kIdMask, orig);
+        }
+        __syncthreads();
+    }
+}
+
+// Block-wide bitonic sort of the n survivors by (distance, original id), in
+// place (the arrays hold W * kBuf entries, a power of two >= n).
+template <int W>
+__device__ __forceinline__ void block_bitonic(const BlockMem<W> &m, uint32_t n, const uint32_t *__restrict__ orig) {
+    constexpr uint32_t T = W * 32;
+    const uint32_t tid = threadIdx.x;
+    uint32_t p2 = 64;
+    while (p2 < n) p2 <<= 1;
+    for (uint32_t e = tid; e < p2; e += T) {
+        if (e < n) {
+            m.cK[e] = __ldg(orig + (m.cI[e] & kIdMask));
+        } else {
+            m.cD[e] = __int_as_float(0x7f800000);
+            m.cI[e] = kFull;
+            m.cK[e] = kFull;
+        }
+    }
+    __syncthreads();
+    for (uint32_t k = 2; k <= p2; k <<= 1)
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+            for (uint32_t p = tid; p < (p2 >> 1); p += T) {
+                const uint32_t i = ((p & ~(j - 1)) << 1) | (p & (j - 1)), x = i | j;
+                const float ad = m.cD[i], xd = m.cD[x];
+                const uint32_t ak = m.cK[i], xk = m.cK[x];
+                const bool up = (i & k) == 0;
+                if (up ? plain_less(xd, xk, ad, ak) : plain_less(ad, ak, xd, xk)) {
+                    m.cD[i] = xd;
+                    m.cD[x] = ad;
+                    m.cK[i] = xk;
+                    m.cK[x] = ak;
+                    const uint32_t t = m.cI[i];
+                    m.cI[i] = m.cI[x];
+                    m.cI[x] = t;
+                }
+            }
+            __syncthreads();
+        }
+}
+
+// Merge the n survivors (cD, cI) into the queue of size sz and capacity L.
+// Returns the position of the best one (L when none is inserted); sz is
+// updated. Called by the whole block with n and sz uniform, after a barrier;
+// ends with one.
+template <int W>
+__device__ __forceinline__ uint32_t block_merge(const BlockMem<W> &m, uint32_t n, uint32_t &sz, uint32_t L,
+                                                const uint32_t *__restrict__ orig) {
+    constexpr uint32_t T = W * 32;
+    constexpr int CH = 4;  // queue elements a thread moves between two barriers
+    const uint32_t tid = threadIdx.x;
+    if (n == 0) {
+        __syncthreads();
+        return L;
+    }
+    const float *sD = m.sD;
+    const uint32_t *sI = m.sI;
+    uint32_t *sP = m.sP;
+    if (n <= block_rank_max(W)) {
+        block_rank<W, true>(m, n, sz, orig);
+    } else {
+        block_bitonic<W>(m, n, orig);
+        sD = m.cD;
+        sI = m.cI;
+        sP = m.cK;
+        for (uint32_t i = tid; i < n; i += T)
+            sP[i] = queue_rank<ORDER_PANNS>(m.qd, m.qi, sz, sD[i], sI[i] & kIdMask, orig);
+        __syncthreads();
+    }
+    const uint32_t p0 = sP[0];
+    const uint32_t end = min(L, sz + n);
+    if (p0 >= L) {
+        __syncthreads();  // sP is read before the next round writes it
+        return L;
+    }
+    // A queue element moves up by the number of survivors before it: those
+    // whose own count of queue elements before them is at most its index.
+    uint32_t steps = 0;
+    while ((1u << steps) <= n) ++steps;
+    uint32_t top = sz;
+    while (true) {
+        float d[CH];
+        uint32_t id[CH], np[CH];
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+            np[c] = L;
+            const uint32_t back = c * T + tid + 1;
+            if (back <= top && top - back >= p0) {
+                const uint32_t j = top - back;
+                d[c] = m.qd[j];
+                id[c] = m.qi[j];
+                uint32_t lo = 0;  // survivors with sP <= j
+                for (uint32_t b = 1u << (steps - 1); b > 0; b >>= 1)
+                    if (lo + b <= n && sP[lo + b - 1] <= j) lo += b;
+                np[c] = j + lo;
+            }
+        }
+        const bool last = top <= p0 + CH * T;
+        __syncthreads();
+#pragma unroll
+        for (int c = 0; c < CH; ++c)
+            if (np[c] < L) {
+                m.qd[np[c]] = d[c];
+                m.qi[np[c]] = id[c];
+            }
+        if (last) break;
+        top -= CH * T;  // (the next chunk reads below what this one wrote)
+    }
+    for (uint32_t i = tid; i < n; i += T) {
+        const uint32_t np = i + sP[i];
+        if (np < L) {
+            m.qd[np] = sD[i];
+            m.qi[np] = sI[i];
+        }
+    }
+    sz = end;
+    __syncthreads();
+    return p0;
 }
 
 template <int KIND, int CL, int W, int STORE>
 __device__ void block_search_one(const SearchArgs &a, uint32_t q, uint8_t *smem, uint32_t *vis, uint32_t *dirty) {
-    constexpr int T = W * 32;
+    constexpr uint32_t T = W * 32;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const uint32_t qcap = a.queue_cap;
-    float *qd = reinterpret_cast<float *>(smem);
-    uint32_t *qi = reinterpret_cast<uint32_t *>(qd + qcap);
-    float *segD = reinterpret_cast<float *>(qi + qcap);
-    uint32_t *segI = reinterpret_cast<uint32_t *>(segD + W * kBuf);
-    uint32_t *segK = segI + W * kBuf;
-    uint32_t *hrowAll = segK + W * kBuf;
-    uint32_t *preAll = hrowAll + W * kCandGroup * kHeadWords;
-    float *cD = reinterpret_cast<float *>(preAll + W * 64);
-    uint32_t *cI = reinterpret_cast<uint32_t *>(cD + W * kBuf);
-    uint32_t *cK = cI + W * kBuf;
-    uint32_t *cand = cK + W * kBuf;
-    uint32_t *ctl = cand + kMaxM;
-    float *bd = segD + w * kBuf;
-    uint32_t *bi = segI + w * kBuf;
-    uint32_t *bk = segK + w * kBuf;
-    uint32_t *hrow = hrowAll + w * kCandGroup * kHeadWords;
-    uint32_t *pre = preAll + w * 64;
+    BlockMem<W> m;
+    m.qd = reinterpret_cast<float *>(smem);
+    m.qi = reinterpret_cast<uint32_t *>(m.qd + a.queue_cap);
+    float *bd = reinterpret_cast<float *>(m.qi + a.queue_cap) + w * kBuf;
+    uint32_t *bi = reinterpret_cast<uint32_t *>(m.qi + a.queue_cap) + W * kBuf + w * kBuf;
+    m.cD = reinterpret_cast<float *>(m.qi + a.queue_cap + 2 * W * kBuf);
+    m.cI = reinterpret_cast<uint32_t *>(m.cD + W * kBuf);
+    m.cK = m.cI + W * kBuf;
+    m.sD = reinterpret_cast<float *>(m.cK + W * kBuf);
+    m.sI = reinterpret_cast<uint32_t *>(m.sD + block_rank_max(W));
+    m.sP = m.sI + block_rank_max(W);
+    uint32_t *cand = m.sP + block_rank_max(W) + w * kMaxM;
+    m.ctl = m.sP + block_rank_max(W) + W * kMaxM;
+    uint32_t *ctl = m.ctl;
 
     uint32_t L = a.Lq ? __ldg(a.Lq + q) : a.L;
     // Init ids: n_lrn learned entries (cand) then n_plain of the init list.
     uint32_t n_lrn = 0, n_plain = L;
     if (a.decisions) {
-        if (w == 0) {
-            const uint2 r = mlp_read_decision(a.decisions, a.dec_L_init, q, cand, lane);
-            if (lane == 0) {
-                ctl[BC_LRN] = r.x;
-                ctl[BC_LQ] = r.y;
-            }
-        }
-        __syncthreads();
-        n_lrn = ctl[BC_LRN] & 0xffu;
-        n_plain = ctl[BC_LRN] >> 8;
-        L = ctl[BC_LQ];
+        const uint2 r = mlp_read_decision(a.decisions, a.dec_L_init, q, cand, lane);  // every warp its own copy
+        n_lrn = r.x & 0xffu;
+        n_plain = r.x >> 8;
+        L = r.y;
     }
     const uint32_t n_init = n_lrn + n_plain;
     Dist<KIND, CL, STORE> D;
     D.load(a, q, lane);
-    if (tid == 0) {
-        ctl[BC_SZ] = 0;
-        ctl[BC_DIRTY] = 0;
-        ctl[BC_DIST] = 0;
-        ctl[BC_EDGES] = 0;
-        ctl[BC_K] = 0;
-    }
+    if (tid < kBlockCtl && tid != BC_Q) ctl[tid] = 0;
     __syncthreads();
 
-    // Block-wide list of the visited words that went from zero to non-zero.
-    auto note_dirty_block = [&](bool first, uint32_t word) {
-        const uint32_t bm = __ballot_sync(kFull, first);
-        uint32_t base = 0;
-        if (lane == 0 && bm) base = atomicAdd(&ctl[BC_DIRTY], (uint32_t) __popc(bm));
-        base = __shfl_sync(kFull, base, 0);
-        if (first) {
-            const uint32_t pos = base + __popc(bm & lanemask_lt());
-            if (pos < a.dirty_cap) dirty[pos] = word;
-        }
-    };
+    uint32_t sz = 0, dcount = 0, n_dist = 0, n_edges = 0, n_expand = 0, n_iter = 0;
+    // The warp's part of the list of visited words that went from zero to non-zero.
+    const uint32_t dcap = a.dirty_cap / W;
+    uint32_t *my_dirty = dirty + (size_t) w * dcap;
+    uint32_t turn = 0;  // which of the two list counters the round uses
 
-    // Merge the W sorted lists (counts in ctl[BC_SEG + w]) into the queue.
-    // Returns nothing; updates ctl[BC_SZ] and ctl[BC_NK].
-    auto block_merge = [&]() {
-        const uint32_t my = ctl[BC_SEG + w];
-        uint32_t total = 0;
-#pragma unroll
-        for (int v = 0; v < W; ++v) total += ctl[BC_SEG + v];
-        for (uint32_t i = lane; i < my; i += 32) {
-            const float dv = bd[i];
-            const uint32_t kv = bk[i];
-            uint32_t r = i;
-#pragma unroll
-            for (int v = 0; v < W; ++v)
-                if (v != w) r += list_rank(segD + v * kBuf, segK + v * kBuf, ctl[BC_SEG + v], dv, kv);
-            cD[r] = dv;
-            cI[r] = bi[i];
-        }
-        __syncthreads();
-        const uint32_t qsz = ctl[BC_SZ];
-        if (total == 0) return;  // uniform
-        for (uint32_t i = tid; i < total; i += T)
-            cK[i] = i + queue_rank<ORDER_PANNS>(qd, qi, qsz, cD[i], cI[i] & kIdMask, a.orig);
-        __syncthreads();
-        const uint32_t p0 = cK[0];
-        if (p0 < L) {
-            for (int32_t top = (int32_t) qsz - 1; top >= (int32_t) p0; top -= T) {
-                const int32_t j = top - tid;
-                float d = 0.f;
-                uint32_t id = 0, np = L;
-                if (j >= (int32_t) p0) {
-                    d = qd[j];
-                    id = qi[j];
-                    np = (uint32_t) j + fresh_rank<ORDER_PANNS>(cD, cI, total, d, id & kIdMask, a.orig);
-                }
-                __syncthreads();
-                if (np < L) {
-                    qd[np] = d;
-                    qi[np] = id;
-                }
-                __syncthreads();
-            }
-            for (uint32_t i = tid; i < total; i += T) {
-                const uint32_t np = cK[i];
-                if (np < L) {
-                    qd[np] = cD[i];
-                    qi[np] = cI[i];
-                }
-            }
-        }
-        __syncthreads();
-        if (tid == 0) {
-            ctl[BC_SZ] = min(L, qsz + total);
-            ctl[BC_NK] = min(ctl[BC_NK], p0 < L ? p0 : L);
-        }
-        __syncthreads();
-    };
-
-    // Distances, filter against the queue's L-th (bound), keys, sort; leaves
-    // the warp's survivor count in ctl[BC_SEG + w].
+    // Distances of the warp's fresh vertices, the filter against the queue's
+    // L-th, the survivors appended to the round's list.
     auto finish_list = [&](uint32_t nb, bool filter) {
-        if constexpr (STORE == STORE_FP32) distances_wide<KIND, CL>(a, D.qv, bi, bd, nb, lane);
-        else D.distances(a, bi, bd, nb, lane);
-        if (lane == 0 && nb) atomicAdd(&ctl[BC_DIST], nb);
-        const uint32_t sz = ctl[BC_SZ];
+        if (nb) {
+            if constexpr (STORE == STORE_FP32) distances_wide<KIND, CL>(a, D.qv, bi, bd, nb, lane);
+            else D.distances(a, bi, bd, nb, lane);
+        }
+        n_dist += nb;
         const bool any_bound = filter && sz >= L;
-        const float bound = any_bound ? qd[L - 1] : __int_as_float(0x7f800000);
-        uint32_t cnt = 0;
+        const float bound = any_bound ? m.qd[L - 1] : __int_as_float(0x7f800000);
         for (uint32_t b0 = 0; b0 < nb; b0 += 32) {
             const uint32_t b = b0 + lane;
-            float d = 0.f;
-            uint32_t id = 0;
-            bool keep = false;
-            if (b < nb) {
-                d = bd[b];
-                id = bi[b];
-                keep = !any_bound || !(d > bound);
-            }
+            const float d = b < nb ? bd[b] : 0.f;
+            const bool keep = b < nb && (!any_bound || !(d > bound));
             const uint32_t bm = __ballot_sync(kFull, keep);
-            __syncwarp();
+            if (!bm) continue;
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(&ctl[BC_CNT + turn], (uint32_t) __popc(bm));
+            base = __shfl_sync(kFull, base, 0);
             if (keep) {
-                const uint32_t pos = cnt + __popc(bm & lanemask_lt());
-                bd[pos] = d;
-                bi[pos] = id;
-                bk[pos] = __ldg(a.orig + id);
+                const uint32_t pos = base + __popc(bm & lanemask_lt());
+                m.cD[pos] = d;
+                m.cI[pos] = bi[b];
             }
-            cnt += __popc(bm);
-            __syncwarp();
         }
-        warp_sort<ORDER_PANNS>(bd, bi, bk, cnt, a.orig, lane);
-        if (lane == 0) ctl[BC_SEG + w] = cnt;
+    };
+    // The barrier after finish_list, and the list's length. The rounds count
+    // alternately in two words: the other one is cleared here, which the
+    // barriers of block_merge put before its next use.
+    auto close_list = [&]() -> uint32_t {
+        __syncthreads();
+        const uint32_t n = ctl[BC_CNT + turn];
+        turn ^= 1u;
+        if (tid == 0) ctl[BC_CNT + turn] = 0;
+        return n;
     };
 
     // Initial queue: the init ids (learned entries first, a repeated id
-    // entering once), W * kBuf at a time.
+    // entering once), spread evenly over the warps.
     const uint32_t *init = a.init_ids + (size_t) q * a.init_stride;
     for (uint32_t r0 = 0; r0 < n_init; r0 += W * kBuf) {
+        const uint32_t rest = min(n_init - r0, (uint32_t) (W * kBuf));
+        const uint32_t per = ((rest + W - 1) / W + 15) & ~15u;  // <= kBuf, whole distance passes
         uint32_t nb = 0;
-        const uint32_t lo = r0 + w * kBuf, hi = min(n_init, lo + kBuf);
+        const uint32_t lo = r0 + w * per, hi = min(r0 + rest, lo + per);
         for (uint32_t i0 = lo; i0 < hi; i0 += 32) {
             const uint32_t i = i0 + lane;
             const bool valid = i < hi;
@@ -219,7 +353,7 @@ __device__ void block_search_one(const SearchArgs &a, uint32_t q, uint8_t *smem,
             const bool ok = valid && id < a.n;
             if (valid && !ok) atomicOr(a.error, ERR_BAD_INIT);
             const uint32_t old = visit_issue(vis, id, ok);
-            note_dirty_block(ok && old == 0, id >> 5);
+            note_dirty(my_dirty, dcap, dcount, ok && old == 0, id >> 5);
             const bool fresh = ok && !(old & (1u << (id & 31)));
             const uint32_t bm = __ballot_sync(kFull, fresh);
             if (fresh) bi[nb + __popc(bm & lanemask_lt())] = id;
@@ -227,167 +361,161 @@ __device__ void block_search_one(const SearchArgs &a, uint32_t q, uint8_t *smem,
             __syncwarp();
         }
         finish_list(nb, false);
-        if (tid == 0) ctl[BC_NK] = L;
-        __syncthreads();
-        block_merge();
+        const uint32_t n = close_list();
+        block_merge<W>(m, n, sz, L, a.orig);
     }
 
-    uint32_t n_expand = 0, n_iter = 0;
-    const uint32_t M = a.M;
-    const uint32_t G = a.block_round;
+    const uint32_t M = a.M, G = a.block_round;
+    uint32_t k = 0;
     for (;;) {
-        // 1. Pick (warp 0), exactly as search_kernel.
-        if (w == 0) {
-            const uint32_t k = ctl[BC_K], sz = ctl[BC_SZ];
-            uint32_t cnt = 0, last_k = L;
-            for (uint32_t p0 = k; p0 < sz && cnt < M; p0 += 32) {
-                const uint32_t p = p0 + lane;
-                const bool un = p < sz && !(qi[p] & kChecked);
-                const uint32_t bm = __ballot_sync(kFull, un);
-                const uint32_t take = min((uint32_t) __popc(bm), M - cnt);
-                const uint32_t r = __popc(bm & lanemask_lt());
-                if (un && r < take) {
-                    const uint32_t id = qi[p];
-                    qi[p] = id | kChecked;
-                    cand[cnt + r] = id;
-                }
-                if (take) {
-                    uint32_t x = bm;
-                    for (uint32_t t = 1; t < take; ++t) x &= x - 1;
-                    last_k = p0 + (__ffs(x) - 1);
-                }
-                cnt += take;
-                __syncwarp();
-            }
-            if (lane == 0) {
-                ctl[BC_CNT] = cnt;
-                ctl[BC_LASTK] = last_k;
-                ctl[BC_NK] = L;
-            }
+        // 1. The step's candidates: every warp scans for itself.
+        uint32_t cnt = 0, last_k = L;
+        for (uint32_t p0 = k; p0 < sz && cnt < M; p0 += 32) {
+            const uint32_t p = p0 + lane;
+            const uint32_t id = p < sz ? m.qi[p] : kChecked;
+            const uint32_t bm = __ballot_sync(kFull, !(id & kChecked));
+            const uint32_t take = min((uint32_t) __popc(bm), M - cnt);
+            const uint32_t r = __popc(bm & lanemask_lt());
+            const bool mine = !(id & kChecked) && r < take;
+            if (mine) cand[cnt + r] = id;
+            const uint32_t tm = __ballot_sync(kFull, mine);
+            if (tm) last_k = p0 + 31 - __clz(tm);
+            cnt += take;
         }
-        __syncthreads();
-        const uint32_t cnt = ctl[BC_CNT];
-        if (cnt == 0) break;
+        __syncwarp();
+        if (cnt == 0) break;  // block-uniform
         ++n_iter;
         n_expand += cnt;
+        uint32_t nk = L;
+        // Warps per candidate when there are fewer candidates than warps.
+        uint32_t parts = 1;
+        while (parts < W && cnt * parts * 2 <= W) parts *= 2;
+        const uint32_t lead = W / parts;  // candidates expanded at once
+        const uint32_t ci = w / parts, part = w & (parts - 1);
         // 2-3. Rounds of at most G candidates per warp.
-        for (uint32_t r0 = 0; r0 < cnt; r0 += W * G) {
-            // this warp's candidates: r0 + w + W * t, t < G
+        for (uint32_t r0 = 0; r0 < cnt; r0 += lead * G) {
             uint32_t gc = 0;
-            for (uint32_t t = 0; t < G; ++t)
-                if (r0 + w + W * t < cnt) ++gc;
+            while (gc < G && r0 + ci + lead * gc < cnt) ++gc;
             uint32_t nb = 0;
             if (gc) {
-                uint32_t hv[kCandGroup];
+                uint32_t hv[kCandGroup], olds[kCandGroup];
 #pragma unroll
-                for (int j = 0; j < kCandGroup; ++j)
-                    hv[j] = (uint32_t) j < gc ? __ldg(a.head + (size_t) cand[r0 + w + W * j] * kHeadWords + lane) : 0u;
+                for (int j = 0; j < kCandGroup; ++j) {
+                    if ((uint32_t) j >= gc) break;
+                    hv[j] = __ldg(a.head + (size_t) cand[r0 + ci + lead * j] * kHeadWords + lane);
+                }
+                bool any_long = false;
 #pragma unroll
-                for (int j = 0; j < kCandGroup; ++j)
-                    if ((uint32_t) j < gc) hrow[j * kHeadWords + lane] = hv[j];
-            }
-            __syncwarp();
-            uint32_t deg = 0, hcount = 0;
-            if (lane < (int) gc) {
-                deg = hrow[lane * kHeadWords];
-                hcount = min(deg, (uint32_t) kHeadNbrs);
-            }
-            uint32_t incl = hcount;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t t = __shfl_up_sync(kFull, incl, o);
-                if (lane >= o) incl += t;
-            }
-            const uint32_t total = __shfl_sync(kFull, incl, 31);
-            if (lane < (int) gc) pre[lane] = incl - hcount;
-            uint32_t degsum = deg;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) degsum += __shfl_xor_sync(kFull, degsum, o);
-            if (lane == 0 && gc) atomicAdd(&ctl[BC_EDGES], gc + degsum);
-            const bool any_long = __any_sync(kFull, deg > (uint32_t) kHeadNbrs);
-            __syncwarp();
-            // Head-row neighbours: every visited test-and-set of the round is
-            // issued before any result is used (total <= kCandGroup * 31).
-            uint32_t ids[kGroupChunks], olds[kGroupChunks];
-#pragma unroll
-            for (int ch = 0; ch < kGroupChunks; ++ch) {
-                const uint32_t f = ch * 32 + lane;
-                uint32_t id = 0;
-                bool valid = f < total;
-                if (valid) {
-                    uint32_t j = 0;
-                    while (j + 1 < gc && pre[j + 1] <= f) ++j;
-                    id = hrow[j * kHeadWords + 1 + (f - pre[j])];
-                    if (id >= a.n) {
+                for (int j = 0; j < kCandGroup; ++j) {
+                    if ((uint32_t) j >= gc) break;
+                    const uint32_t dj = __shfl_sync(kFull, hv[j], 0);
+                    if (part == 0) n_edges += 1 + dj;
+                    any_long = any_long || dj > (uint32_t) kHeadNbrs;
+                    bool valid = lane >= 1 && (uint32_t) lane <= min(dj, (uint32_t) kHeadNbrs) &&
+                                 ((uint32_t) lane & (parts - 1)) == part;
+                    if (valid && hv[j] >= a.n) {
                         atomicOr(a.error, ERR_BAD_ID);
                         valid = false;
                     }
+                    if (!valid) hv[j] = kFull;
+                    olds[j] = visit_issue(vis, hv[j], valid);
                 }
-                ids[ch] = valid ? id : kFull;
-                olds[ch] = visit_issue(vis, id, valid);
-            }
 #pragma unroll
-            for (int ch = 0; ch < kGroupChunks; ++ch) {
-                if (ch * 32 >= (int) total) break;
-                const uint32_t id = ids[ch];
-                const bool valid = id != kFull;
-                const bool fresh = valid && !(olds[ch] & (1u << (id & 31)));
-                note_dirty_block(valid && olds[ch] == 0, id >> 5);
-                const uint32_t bm = __ballot_sync(kFull, fresh);
-                if (fresh) bi[nb + __popc(bm & lanemask_lt())] = id;
-                nb += __popc(bm);
-                __syncwarp();
-            }
-            if (any_long) {
-                for (uint32_t j = 0; j < gc; ++j) {
-                    const uint32_t dj = hrow[j * kHeadWords];
-                    if (dj <= (uint32_t) kHeadNbrs) continue;
-                    const uint64_t off = __ldg(a.ovf_off + cand[r0 + w + W * j]);
-                    for (uint32_t s0 = kHeadNbrs; s0 < dj; s0 += 32) {
-                        const uint32_t s = s0 + lane;
-                        bool valid = s < dj;
-                        const uint32_t id = valid ? __ldg(a.ovf + off + (s - kHeadNbrs)) : 0u;
-                        if (valid && id >= a.n) {
-                            atomicOr(a.error, ERR_BAD_ID);
-                            valid = false;
+                for (int j = 0; j < kCandGroup; ++j) {
+                    if ((uint32_t) j >= gc) break;
+                    const uint32_t id = hv[j];
+                    const bool valid = id != kFull;
+                    const bool fresh = valid && !(olds[j] & (1u << (id & 31)));
+                    note_dirty(my_dirty, dcap, dcount, valid && olds[j] == 0, id >> 5);
+                    const uint32_t bm = __ballot_sync(kFull, fresh);
+                    if (fresh) bi[nb + __popc(bm & lanemask_lt())] = id;
+                    nb += __popc(bm);
+                }
+                if (any_long) {
+                    for (uint32_t j = 0; j < gc; ++j) {
+                        const uint32_t c = cand[r0 + ci + lead * j];
+                        const uint32_t dj = __ldg(a.head + (size_t) c * kHeadWords);
+                        if (dj <= (uint32_t) kHeadNbrs) continue;
+                        const uint64_t off = __ldg(a.ovf_off + c);
+                        for (uint32_t s0 = kHeadNbrs; s0 < dj; s0 += 32 * parts) {
+                            const uint32_t s = s0 + part * 32 + lane;
+                            bool valid = s < dj;
+                            const uint32_t id = valid ? __ldg(a.ovf + off + (s - kHeadNbrs)) : 0u;
+                            if (valid && id >= a.n) {
+                                atomicOr(a.error, ERR_BAD_ID);
+                                valid = false;
+                            }
+                            const uint32_t old = visit_issue(vis, id, valid);
+                            const bool fresh = valid && !(old & (1u << (id & 31)));
+                            note_dirty(my_dirty, dcap, dcount, valid && old == 0, id >> 5);
+                            const uint32_t bm = __ballot_sync(kFull, fresh);
+                            if (fresh) bi[nb + __popc(bm & lanemask_lt())] = id;
+                            nb += __popc(bm);
                         }
-                        const uint32_t old = visit_issue(vis, id, valid);
-                        const bool fresh = valid && !(old & (1u << (id & 31)));
-                        note_dirty_block(valid && old == 0, id >> 5);
-                        const uint32_t bm = __ballot_sync(kFull, fresh);
-                        if (fresh) bi[nb + __popc(bm & lanemask_lt())] = id;
-                        nb += __popc(bm);
-                        __syncwarp();
                     }
                 }
+                __syncwarp();
             }
             finish_list(nb, true);
-            __syncthreads();
-            block_merge();
+            const uint32_t n = close_list();
+            // Every warp has its candidates: mark them (block_merge reads the
+            // marks after its next barrier at the earliest).
+            if (r0 == 0 && w == 0) {
+                uint32_t left = cnt;
+                for (uint32_t p0 = k; left; p0 += 32) {
+                    const uint32_t p = p0 + lane;
+                    const uint32_t id = p < sz ? m.qi[p] : kChecked;
+                    const uint32_t bm = __ballot_sync(kFull, !(id & kChecked));
+                    const uint32_t take = min((uint32_t) __popc(bm), left);
+                    if (!(id & kChecked) && (uint32_t) __popc(bm & lanemask_lt()) < take) m.qi[p] = id | kChecked;
+                    left -= take;
+                }
+            }
+            nk = min(nk, block_merge<W>(m, n, sz, L, a.orig));
         }
-        if (tid == 0) {
-            const uint32_t nk = ctl[BC_NK], last_k = ctl[BC_LASTK];
-            ctl[BC_K] = nk <= last_k ? nk : last_k + 1;
-        }
-        __syncthreads();
+        k = nk <= last_k ? nk : last_k + 1;
     }
 
     if constexpr (STORE != STORE_FP32) {
-        // Re-rank the final L in exact float32 (warp 0), as search_kernel does.
-        if (w == 0) {
-            Dist<KIND, CL, STORE_FP32> E;
-            E.load(a, q, lane);
-            const uint32_t sz = ctl[BC_SZ];
-            E.distances(a, qi, qd, sz, lane);
-            rerank_output(qd, qi, sz, a.K, a.orig, a.out_ids + (size_t) q * a.K, lane);
+        // Re-rank the final queue in exact float32 (reference lane order); the K
+        // best by (distance, original id) go out.
+        Dist<KIND, CL, STORE_FP32> E;
+        E.load(a, q, lane);
+        const uint32_t per = ((sz + W - 1) / W + 7) & ~7u;
+        const uint32_t lo = min(sz, w * per), hi = min(sz, lo + per);
+        E.distances(a, m.qi + lo, m.qd + lo, hi - lo, lane);
+        __syncthreads();
+        if (sz <= W * kBuf) {
+            for (uint32_t i = tid; i < sz; i += T) {
+                m.cD[i] = m.qd[i];
+                m.cI[i] = m.qi[i] & kIdMask;
+            }
+            __syncthreads();
+            const uint32_t *ids = m.sI;
+            if (sz <= block_rank_max(W)) {
+                block_rank<W, false>(m, sz, 0, a.orig);
+            } else {
+                block_bitonic<W>(m, sz, a.orig);
+                ids = m.cI;
+            }
+            for (uint32_t i = tid; i < a.K; i += T) a.out_ids[(size_t) q * a.K + i] = __ldg(a.orig + ids[i]);
+        } else if (w == 0) {
+            rerank_output(m.qd, m.qi, sz, a.K, a.orig, a.out_ids + (size_t) q * a.K, lane);
         }
     } else {
-        for (uint32_t i = tid; i < a.K; i += T) a.out_ids[(size_t) q * a.K + i] = __ldg(a.orig + (qi[i] & kIdMask));
+        for (uint32_t i = tid; i < a.K; i += T)
+            a.out_ids[(size_t) q * a.K + i] = __ldg(a.orig + (m.qi[i] & kIdMask));
     }
+    if (lane == 0) {
+        atomicAdd(&ctl[BC_DIST], n_dist);
+        atomicAdd(&ctl[BC_EDGES], n_edges);
+        if (dcount > dcap) ctl[BC_FULL] = 1u;
+    }
+    __syncthreads();
     if (tid == 0 && a.out_stats) a.out_stats[q] = make_uint4(ctl[BC_DIST], n_expand, ctl[BC_EDGES], n_iter);
-    const uint32_t dcount = ctl[BC_DIRTY];
-    if (dcount <= a.dirty_cap) {
-        for (uint32_t i = tid; i < dcount; i += T) vis[dirty[i]] = 0u;
+    // Clear the visited words this query set.
+    if (!ctl[BC_FULL]) {
+        for (uint32_t i = lane; i < dcount; i += 32) vis[my_dirty[i]] = 0u;
     } else {
         for (uint32_t i = tid; i < a.vis_words; i += T) vis[i] = 0u;
     }

@@ -42,6 +42,12 @@ struct Scratch {
         p = nullptr;
         n = 0;
     }
+    T *take() {  // the caller frees it (scratch_free)
+        T *q = p;
+        p = nullptr;
+        n = 0;
+        return q;
+    }
     cudaError_t alloc(size_t count, cudaStream_t stream) {
         release();
         s = stream;

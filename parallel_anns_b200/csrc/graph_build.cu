@@ -25,7 +25,6 @@
 
 #include <algorithm>
 #include <cstring>
-#include <deque>
 #include <memory>
 #include <string>
 #include <vector>
@@ -624,6 +623,275 @@ __global__ void dist_to_point_kernel(const float *__restrict__ x, uint32_t n, ui
     out[r] = acc;
 }
 
+// The float64 mean of the rows, every dimension summed in row order (the order
+// that fixes its last bits): one thread per dimension, a chain of n additions
+// fed 64 rows ahead. The addition's latency bounds it (250,000 rows: 2 ms), so
+// it runs beside the screen on a stream of its own; the same sum on the host
+// took 10 ms.
+__global__ void __launch_bounds__(32) mean_kernel(const float *__restrict__ x, uint32_t n, uint32_t d,
+                                                  double *__restrict__ mean) {
+    constexpr int U = 64;
+    const uint32_t j = blockIdx.x * 32 + threadIdx.x;
+    if (j >= d) return;
+    const float *c = x + j;
+    double s = 0.0;
+    float cur[U];
+    uint32_t r = 0;
+    if (n >= U) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) cur[u] = __ldg(c + (size_t) u * d);
+        for (; r + 2 * U <= n; r += U) {
+            float nxt[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) nxt[u] = __ldg(c + (size_t) (r + U + u) * d);
+#pragma unroll
+            for (int u = 0; u < U; ++u) s += (double) cur[u];
+#pragma unroll
+            for (int u = 0; u < U; ++u) cur[u] = nxt[u];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) s += (double) cur[u];
+        r += U;
+    }
+    for (; r < n; ++r) s += (double) __ldg(c + (size_t) r * d);
+    mean[j] = s / (double) n;
+}
+
+// The lowest index of the smallest value (one block); 0 if value 0 is a NaN.
+__global__ void __launch_bounds__(1024) argmin64_kernel(const double *__restrict__ v, uint32_t n,
+                                                        uint32_t *__restrict__ out) {
+    __shared__ double bv[32];
+    __shared__ uint32_t bi[32];
+    double best = __longlong_as_double(0x7ff0000000000000ll);
+    uint32_t at = 0xffffffffu;
+    for (uint32_t i = threadIdx.x; i < n; i += 1024) {
+        const double t = v[i];
+        if (t < best || (t == best && i < at)) {
+            best = t;
+            at = i;
+        }
+    }
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int round = 0; round < 2; ++round) {
+        for (int o = 16; o > 0; o >>= 1) {
+            const double v2 = __shfl_xor_sync(0xffffffffu, best, o);
+            const uint32_t i2 = __shfl_xor_sync(0xffffffffu, at, o);
+            if (v2 < best || (v2 == best && i2 < at)) {
+                best = v2;
+                at = i2;
+            }
+        }
+        if (round == 1) break;
+        if (lane == 0) {
+            bv[w] = best;
+            bi[w] = at;
+        }
+        __syncthreads();
+        if (w) return;
+        best = bv[lane];
+        at = bi[lane];
+    }
+    if (lane == 0) *out = v[0] != v[0] || at >= n ? 0u : at;
+}
+
+// Exclusive prefix sums of n words into out[0..n] (64 bits; out[n] = the
+// total): sums of 4,096-word blocks, one block that scans those, the blocks again.
+constexpr uint32_t kScanBlock = 4096;
+
+__device__ __forceinline__ uint64_t block_scan_1024(uint64_t v, uint64_t *red, uint64_t &total) {
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint64_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint64_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if ((int) lane >= o) incl += t;
+    }
+    __syncthreads();
+    if (lane == 31) red[w] = incl;
+    __syncthreads();
+    uint64_t before = 0;
+    total = 0;
+    for (uint32_t i = 0; i < 32; ++i) {
+        if (i < w) before += red[i];
+        total += red[i];
+    }
+    return before + incl - v;
+}
+
+__global__ void __launch_bounds__(1024) scan_sums_kernel(const uint32_t *__restrict__ in, uint32_t n,
+                                                         uint64_t *__restrict__ sums) {
+    __shared__ uint64_t red[32];
+    uint64_t v = 0;
+    for (uint32_t e = 0; e < 4; ++e) {
+        const uint64_t i = (uint64_t) blockIdx.x * kScanBlock + threadIdx.x * 4 + e;
+        v += i < n ? in[i] : 0u;
+    }
+    uint64_t total;
+    block_scan_1024(v, red, total);
+    if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(1024) scan_blocks_kernel(uint64_t *__restrict__ sums, uint32_t m) {
+    __shared__ uint64_t red[32];
+    uint64_t base = 0;
+    for (uint32_t b0 = 0; b0 < m; b0 += 1024) {
+        const uint32_t b = b0 + threadIdx.x;
+        const uint64_t v = b < m ? sums[b] : 0;
+        uint64_t total;
+        const uint64_t ex = block_scan_1024(v, red, total);
+        if (b < m) sums[b] = base + ex;
+        base += total;
+    }
+}
+
+__global__ void __launch_bounds__(1024) scan_write_kernel(const uint32_t *__restrict__ in, uint32_t n,
+                                                          const uint64_t *__restrict__ sums,
+                                                          uint64_t *__restrict__ out) {
+    __shared__ uint64_t red[32];
+    const uint64_t i0 = (uint64_t) blockIdx.x * kScanBlock + threadIdx.x * 4;
+    uint32_t x[4];
+    uint64_t v = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        x[e] = i0 + e < n ? in[i0 + e] : 0u;
+        v += x[e];
+    }
+    uint64_t total;
+    uint64_t at = sums[blockIdx.x] + block_scan_1024(v, red, total);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        if (i0 + e <= n) out[i0 + e] = at;
+        at += x[e];
+    }
+}
+
+cudaError_t scan_words(const uint32_t *in, uint32_t n, uint64_t *out, cudaStream_t s) {
+    // One block more than the words need, so that out[n] is always written.
+    const uint32_t m = n / kScanBlock + 1;
+    Scratch<uint64_t> sums;
+    cudaError_t e = sums.alloc(m, s);
+    if (e != cudaSuccess) return e;
+    scan_sums_kernel<<<m, 1024, 0, s>>>(in, n, sums.p);
+    scan_blocks_kernel<<<1, 1024, 0, s>>>(sums.p, m);
+    scan_write_kernel<<<m, 1024, 0, s>>>(in, n, sums.p, out);
+    return cudaGetLastError();
+}
+
+// Rows of up to R (deg[a] used) into CSR; one warp per row.
+__global__ void __launch_bounds__(256) compact_kernel(const uint32_t *__restrict__ rows, uint32_t R,
+                                                      const uint32_t *__restrict__ deg,
+                                                      const uint64_t *__restrict__ off, uint32_t n,
+                                                      uint32_t *__restrict__ out) {
+    const uint32_t a = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (a >= n) return;
+    const uint32_t m = deg[a];
+    for (uint32_t e = lane; e < m; e += 32) out[off[a] + e] = rows[(size_t) a * R + e];
+}
+
+// Reverse edges. For every pruned edge a -> b (a ascending, then list order),
+// b -> a is appended to b's list while it holds fewer than R and does not
+// contain a already (efanna2e's InterInsert plays this part, with a re-prune on
+// overflow instead of the cap). What b gets depends on b alone: the smallest
+// ids among its in-neighbours that its pruned list lacks, ascending. So the
+// pruned edges are transposed (counts, offsets, ids in any order), and one warp
+// per vertex picks them. 200,000 vertices: 115 ms edge by edge on the host.
+__global__ void __launch_bounds__(256) indegree_kernel(const uint32_t *__restrict__ rows, uint32_t R,
+                                                       const uint32_t *__restrict__ deg, uint32_t n,
+                                                       uint32_t *__restrict__ indeg) {
+    const uint32_t a = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (a >= n) return;
+    for (uint32_t e = lane; e < deg[a]; e += 32) atomicAdd(indeg + rows[(size_t) a * R + e], 1u);
+}
+
+__global__ void __launch_bounds__(256) transpose_kernel(const uint32_t *__restrict__ rows, uint32_t R,
+                                                        const uint32_t *__restrict__ deg, uint32_t n,
+                                                        const uint64_t *__restrict__ ioff,
+                                                        uint32_t *__restrict__ fill, uint32_t *__restrict__ in) {
+    const uint32_t a = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (a >= n) return;
+    for (uint32_t e = lane; e < deg[a]; e += 32) {
+        const uint32_t b = rows[(size_t) a * R + e];
+        in[ioff[b] + atomicAdd(fill + b, 1u)] = a;
+    }
+}
+
+constexpr uint32_t kRevList = 256;  // in-neighbours ranked in shared memory
+__global__ void __launch_bounds__(256) reverse_kernel(uint32_t *__restrict__ rows, uint32_t R,
+                                                      const uint32_t *__restrict__ deg, uint32_t n,
+                                                      const uint64_t *__restrict__ ioff,
+                                                      const uint32_t *__restrict__ in,
+                                                      uint32_t *__restrict__ newdeg) {
+    __shared__ uint32_t list[8][kRevList];
+    const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31, b = blockIdx.x * 8 + w;
+    if (b >= n) return;
+    const uint32_t d0 = deg[b];
+    uint32_t *row = rows + (size_t) b * R;
+    const uint32_t *src = in + ioff[b];
+    const uint64_t m = ioff[b + 1] - ioff[b];
+    const uint32_t want = R - d0;
+    auto fresh = [&](uint32_t a) {  // not in b's pruned list
+        bool has = false;
+        for (uint32_t e = 0; e < d0; ++e) has = has || __ldg(row + e) == a;
+        return !has;
+    };
+    uint32_t got = 0;
+    if (m <= kRevList) {
+        uint32_t c = 0;
+        for (uint32_t i0 = 0; i0 < (uint32_t) m; i0 += 32) {
+            const uint32_t i = i0 + lane;
+            const uint32_t a = i < m ? src[i] : 0u;
+            const bool keep = i < m && fresh(a);
+            const uint32_t bm = __ballot_sync(0xffffffffu, keep);
+            if (keep) list[w][c + __popc(bm & ((1u << lane) - 1u))] = a;
+            c += __popc(bm);
+        }
+        __syncwarp();
+        for (uint32_t i = lane; i < c; i += 32) {
+            const uint32_t a = list[w][i];
+            uint32_t rank = 0;
+            for (uint32_t e = 0; e < c; ++e) rank += list[w][e] < a ? 1u : 0u;
+            if (rank < want) row[d0 + rank] = a;
+        }
+        got = min(c, want);
+    } else {
+        // Many in-neighbours: the smallest one above the last, one at a time.
+        uint32_t last = 0;
+        while (got < want) {
+            uint32_t best = 0xffffffffu;
+            for (uint64_t i = lane; i < m; i += 32) {
+                const uint32_t a = src[i];
+                if (a < best && (got == 0 || a > last) && fresh(a)) best = a;
+            }
+            best = __reduce_min_sync(0xffffffffu, best);
+            if (best == 0xffffffffu) break;
+            if (lane == 0) row[d0 + got] = best;
+            last = best;
+            ++got;
+        }
+    }
+    if (lane == 0) newdeg[b] = d0 + got;
+}
+
+// Parents of the repair's roots: the first vertex of root i's k-NN list that an
+// earlier walk reached (walk[c] = 1 for the entry's, i + 2 for root i's), else
+// the entry.
+__global__ void __launch_bounds__(256) parent_kernel(const uint32_t *__restrict__ knn, uint32_t k, uint32_t n,
+                                                     const uint32_t *__restrict__ roots, uint32_t m,
+                                                     const uint32_t *__restrict__ walk, uint32_t entry,
+                                                     uint32_t *__restrict__ parent) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m) return;
+    uint32_t p = entry;
+    for (uint32_t e = 0; e < k; ++e) {
+        const uint32_t c = knn[(size_t) roots[i] * k + e];
+        if (c < n && walk[c] <= i + 1) {
+            p = c;
+            break;
+        }
+    }
+    parent[i] = p;
+}
+
 }  // namespace
 
 // The float32 screen of nr rows (of the list `rows`, or all without it).
@@ -636,135 +904,218 @@ static int screen_fp32(const float *x, uint32_t n, uint32_t d, const float *xn, 
     return PANNS_OK;
 }
 
+// The float64 mean of the base, computed beside the screen.
+struct MeanJob {
+    cudaStream_t s = nullptr;
+    cudaEvent_t ready = nullptr, done = nullptr;
+    Scratch<double> mean;
+    ~MeanJob() {
+        if (s) cudaStreamSynchronize(s);
+        mean.release();
+        if (ready) cudaEventDestroy(ready);
+        if (done) cudaEventDestroy(done);
+        if (s) cudaStreamDestroy(s);
+    }
+    // x is complete on `from` at this point; `from` may use `mean` after wait().
+    int start(const float *x, uint32_t n, uint32_t d, cudaStream_t from) {
+        GCU(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        GCU(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
+        GCU(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+        GCU(mean.alloc(d, s));
+        GCU(cudaEventRecord(ready, from));
+        GCU(cudaStreamWaitEvent(s, ready, 0));
+        mean_kernel<<<(d + 31) / 32, 32, 0, s>>>(x, n, d, mean.p);
+        GCU(cudaGetLastError());
+        GCU(cudaEventRecord(done, s));
+        return PANNS_OK;
+    }
+    int wait(cudaStream_t to) {
+        GCU(cudaStreamWaitEvent(to, done, 0));
+        return PANNS_OK;
+    }
+};
+
 // The steps after the k-NN screen, shared by every construction: the C
 // screened candidates of each row (cand, device, n x C; ~0 = none) ranked
-// exactly by (d64, id) into k-NN lists, the MRNG prune to R, the entry (the
-// row nearest the float64 mean of base, summed in id order) and the
-// reachability repair. The rows go through the rerank and the prune in
-// chunks, so the per-row float64 lists never exist for all n at once.
-static int finish_graph(const float *base, const float *x, uint32_t n, uint32_t d, uint32_t k, uint32_t R,
-                        const uint32_t *cand, uint32_t C, cudaStream_t s, std::unique_ptr<panns_graph> &g,
-                        bool reverse = false) {
+// exactly by (d64, id) into k-NN lists, the MRNG prune to R, reverse edges, the
+// entry (the row nearest the float64 mean) and the reachability repair. The
+// lists stay on the device until they are a CSR graph; the walks of the repair
+// follow it on the host, one after the other, and the lists of the vertices
+// they start from are looked up on the device again. Rows go through the rank
+// and the prune in chunks; k-NN lists above kKnnOnDevice bytes go to the host
+// as they come.
+constexpr size_t kKnnOnDevice = 4ull << 30;
+
+static int finish_graph(int device, const float *x, uint32_t n, uint32_t d, uint32_t k, uint32_t R,
+                        const uint32_t *cand, uint32_t C, MeanJob &mean, cudaStream_t s,
+                        std::unique_ptr<panns_graph> &g, bool reverse = false) {
     const uint32_t chunk = std::min<uint32_t>(n, 1u << 23);
-    Buf<uint32_t> knn, pr, deg;
-    Buf<double> knn_d, mean, dm;
-    GCU(knn.alloc((size_t) chunk * k, s));
+    const bool knn_host = (size_t) n * k * 4 > kKnnOnDevice;
+    Buf<uint32_t> knn, pr, deg, entry;
+    Buf<double> knn_d, dm;
+    Buf<uint64_t> off;
+    GCU(knn.alloc(knn_host ? (size_t) chunk * k : (size_t) n * k, s));
     GCU(knn_d.alloc((size_t) chunk * k, s));
-    GCU(pr.alloc((size_t) chunk * R, s));
-    GCU(deg.alloc(chunk, s));
-    GCU(mean.alloc(d, s));
+    GCU(pr.alloc((size_t) n * R, s));
+    GCU(deg.alloc(n, s));
     GCU(dm.alloc(n, s));
+    GCU(entry.alloc(1, s));
+    GCU(off.alloc((size_t) n + 1, s));
     g.reset(new panns_graph());
     g->n = n;
     g->k = k;
-    std::vector<uint32_t> prh((size_t) n * R), degh(n);
-    g->knn.resize((size_t) n * k);
+    g->device = device;
+    if (knn_host) g->knn.resize((size_t) n * k);
     for (uint32_t a0 = 0; a0 < n; a0 += chunk) {
         const uint32_t na = std::min(chunk, n - a0);
-        GCU(cudaMemsetAsync(knn.p, 0xff, (size_t) na * k * 4, s));
+        uint32_t *kn = knn_host ? knn.p : knn.p + (size_t) a0 * k;
+        GCU(cudaMemsetAsync(kn, 0xff, (size_t) na * k * 4, s));
         if (d % 4 == 0 && d <= kMaxVecD)
-            rerank_kernel<true><<<(na + 7) / 8, 256, 0, s>>>(x, n, d, cand, C, k, a0, na, knn.p, knn_d.p);
+            rerank_kernel<true><<<(na + 7) / 8, 256, 0, s>>>(x, n, d, cand, C, k, a0, na, kn, knn_d.p);
         else
-            rerank_kernel<false><<<(na + 7) / 8, 256, 0, s>>>(x, n, d, cand, C, k, a0, na, knn.p, knn_d.p);
+            rerank_kernel<false><<<(na + 7) / 8, 256, 0, s>>>(x, n, d, cand, C, k, a0, na, kn, knn_d.p);
         GCU(cudaGetLastError());
         // Rows in shared memory while two blocks of at least one warp fit an SM.
         const uint32_t per_warp = prune_warp_bytes(d, k);
+        uint32_t *prc = pr.p + (size_t) a0 * R;
         if (d % 4 == 0 && per_warp <= 112u * 1024u) {
             const uint32_t wpb = std::max(1u, std::min(4u, 112u * 1024u / per_warp));
             GCU(cudaFuncSetAttribute(prune_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int) (wpb * per_warp)));
-            prune_rows_kernel<<<(na + wpb - 1) / wpb, wpb * 32, wpb * per_warp, s>>>(x, n, d, knn.p, knn_d.p, k, R, na,
-                                                                                    pr.p, deg.p);
+            prune_rows_kernel<<<(na + wpb - 1) / wpb, wpb * 32, wpb * per_warp, s>>>(x, n, d, kn, knn_d.p, k, R, na, prc,
+                                                                                    deg.p + a0);
         } else {
-            prune_kernel<<<(na + 7) / 8, 256, 8 * R * 4, s>>>(x, n, d, knn.p, knn_d.p, k, R, na, pr.p, deg.p);
+            prune_kernel<<<(na + 7) / 8, 256, 8 * R * 4, s>>>(x, n, d, kn, knn_d.p, k, R, na, prc, deg.p + a0);
         }
         GCU(cudaGetLastError());
-        GCU(cudaMemcpyAsync(prh.data() + (size_t) a0 * R, pr.p, (size_t) na * R * 4, cudaMemcpyDeviceToHost, s));
-        GCU(cudaMemcpyAsync(degh.data() + a0, deg.p, na * 4ull, cudaMemcpyDeviceToHost, s));
-        GCU(cudaMemcpyAsync(g->knn.data() + (size_t) a0 * k, knn.p, (size_t) na * k * 4, cudaMemcpyDeviceToHost, s));
+        if (knn_host)
+            GCU(cudaMemcpyAsync(g->knn.data() + (size_t) a0 * k, kn, (size_t) na * k * 4, cudaMemcpyDeviceToHost, s));
+    }
+    knn_d.release();
+    // Entry: the row nearest the mean.
+    int rc = mean.wait(s);
+    if (rc) return rc;
+    dist_to_point_kernel<<<(n + 255) / 256, 256, 0, s>>>(x, n, d, mean.mean.p, dm.p);
+    argmin64_kernel<<<1, 1024, 0, s>>>(dm.p, n, entry.p);
+    GCU(cudaGetLastError());
+    GCU(cudaMemcpyAsync(&g->entry, entry.p, 4, cudaMemcpyDeviceToHost, s));
+    if (reverse) {
+        Buf<uint32_t> fill, in, deg2;
+        Buf<uint64_t> ioff;
+        GCU(fill.alloc(n, s));
+        GCU(deg2.alloc(n, s));
+        GCU(ioff.alloc((size_t) n + 1, s));
+        GCU(cudaMemsetAsync(fill.p, 0, (size_t) n * 4, s));
+        indegree_kernel<<<(n + 7) / 8, 256, 0, s>>>(pr.p, R, deg.p, n, fill.p);
+        GCU(cudaGetLastError());
+        GCU(scan_words(fill.p, n, ioff.p, s));
+        uint64_t edges = 0;
+        GCU(cudaMemcpyAsync(&edges, ioff.p + n, 8, cudaMemcpyDeviceToHost, s));
+        GCU(cudaStreamSynchronize(s));
+        GCU(in.alloc((size_t) edges, s));
+        GCU(cudaMemsetAsync(fill.p, 0, (size_t) n * 4, s));
+        transpose_kernel<<<(n + 7) / 8, 256, 0, s>>>(pr.p, R, deg.p, n, ioff.p, fill.p, in.p);
+        reverse_kernel<<<(n + 7) / 8, 256, 0, s>>>(pr.p, R, deg.p, n, ioff.p, in.p, deg2.p);
+        GCU(cudaGetLastError());
+        GCU(cudaMemcpyAsync(deg.p, deg2.p, (size_t) n * 4, cudaMemcpyDeviceToDevice, s));
+    }
+    // The lists as a CSR graph, to the host (with room for one repair edge per vertex).
+    GCU(scan_words(deg.p, n, off.p, s));
+    std::vector<uint64_t> &go = g->off;
+    go.resize((size_t) n + 1);
+    GCU(cudaMemcpyAsync(go.data(), off.p, ((size_t) n + 1) * 8, cudaMemcpyDeviceToHost, s));
+    GCU(cudaStreamSynchronize(s));
+    const uint64_t edges = go[n];
+    {
+        Buf<uint32_t> csr;
+        GCU(csr.alloc((size_t) edges, s));
+        compact_kernel<<<(n + 7) / 8, 256, 0, s>>>(pr.p, R, deg.p, off.p, n, csr.p);
+        GCU(cudaGetLastError());
+        pr.release();
+        g->nbrs.resize((size_t) edges, (size_t) edges + n);
+        GCU(cudaMemcpyAsync(g->nbrs.data(), csr.p, (size_t) edges * 4, cudaMemcpyDeviceToHost, s));
         GCU(cudaStreamSynchronize(s));
     }
-    // Entry: float64 mean of the rows in id order (host), then the nearest row.
-    std::vector<double> mh(d, 0.0);
-    for (uint32_t r = 0; r < n; ++r)
-        for (uint32_t j = 0; j < d; ++j) mh[j] += (double) base[(size_t) r * d + j];
-    for (uint32_t j = 0; j < d; ++j) mh[j] /= (double) n;
-    GCU(cudaMemcpyAsync(mean.p, mh.data(), d * 8ull, cudaMemcpyHostToDevice, s));
-    dist_to_point_kernel<<<(n + 255) / 256, 256, 0, s>>>(x, n, d, mean.p, dm.p);
-    GCU(cudaGetLastError());
-    std::vector<double> dmh(n);
-    GCU(cudaMemcpyAsync(dmh.data(), dm.p, n * 8ull, cudaMemcpyDeviceToHost, s));
-    GCU(cudaStreamSynchronize(s));
-    uint32_t entry = 0;
-    for (uint32_t r = 1; r < n; ++r)
-        if (dmh[r] < dmh[entry]) entry = r;
-    g->entry = entry;
-    if (reverse) {
-        // Reverse edges: for every pruned edge a -> b (a ascending, then list
-        // order), b -> a is appended to b's list while it holds fewer than R
-        // and does not contain a already (efanna2e's InterInsert plays this
-        // part, with a re-prune on overflow instead of the cap).
-        const std::vector<uint32_t> deg0(degh);
-        for (uint32_t a = 0; a < n; ++a) {
-            const uint32_t *la = prh.data() + (size_t) a * R;
-            for (uint32_t e = 0; e < deg0[a]; ++e) {
-                const uint32_t b = la[e];
-                uint32_t *lb = prh.data() + (size_t) b * R;
-                if (degh[b] >= R || std::find(lb, lb + degh[b], a) != lb + degh[b]) continue;
-                lb[degh[b]++] = a;
+    // Reachability repair: walks over the lists, from the entry and then from
+    // every vertex no walk has reached yet, in id order. walk[v] is the number of
+    // the walk that reached v. A repair edge parent -> root is followed at once by
+    // the walk from the root, so walks never need the repair edges themselves.
+    std::vector<uint32_t> walk(n, 0), queue(n), roots;
+    const uint32_t *nb = g->nbrs.data();
+    auto follow = [&](uint32_t src, uint32_t number) {  // breadth-first
+        size_t head = 0, tail = 0;
+        walk[src] = number;
+        queue[tail++] = src;
+        while (head < tail) {
+            if (head + 8 < tail) __builtin_prefetch(&go[queue[head + 8]]);
+            if (head + 4 < tail) {
+                const uint32_t *p = nb + go[queue[head + 4]];
+                __builtin_prefetch(p);
+                __builtin_prefetch(p + 16);
             }
-        }
-    }
-    // Reachability repair from the entry over the pruned lists. A repair edge
-    // parent -> u is followed at once by a walk from u, so walks never need
-    // the repair edges themselves; they are appended to their parents' lists
-    // (in the order they were made) when the CSR is built.
-    std::vector<uint8_t> reached(n, 0);
-    std::vector<uint32_t> stack;
-    auto walk = [&](uint32_t src) {  // breadth-first from src over the pruned lists
-        reached[src] = 1;
-        stack.assign(1, src);
-        for (size_t h = 0; h < stack.size(); ++h) {
-            const uint32_t v = stack[h];
-            const uint32_t *lv = prh.data() + (size_t) v * R;
-            for (uint32_t e = 0; e < degh[v]; ++e)
-                if (!reached[lv[e]]) {
-                    reached[lv[e]] = 1;
-                    stack.push_back(lv[e]);
+            const uint32_t v = queue[head++];
+            for (uint64_t e = go[v]; e < go[v + 1]; ++e) {
+                const uint32_t u = nb[e];
+                if (!walk[u]) {
+                    walk[u] = number;
+                    queue[tail++] = u;
                 }
+            }
         }
     };
-    walk(entry);
-    std::vector<std::pair<uint32_t, uint32_t>> extra;  // (parent, u)
-    std::vector<uint32_t> nextra(n, 0);
-    for (uint32_t u = 0; u < n; ++u) {
-        if (reached[u]) continue;
-        uint32_t parent = entry;
-        for (uint32_t i = 0; i < k; ++i) {
-            const uint32_t c = g->knn[(size_t) u * k + i];
-            if (c < n && reached[c]) {
-                parent = c;
-                break;
+    follow(g->entry, 1);
+    for (uint32_t u = 0; u < n; ++u)
+        if (!walk[u]) {
+            roots.push_back(u);
+            follow(u, (uint32_t) roots.size() + 1);
+        }
+    const uint32_t m = (uint32_t) roots.size();
+    std::vector<uint32_t> parent(m);
+    if (m && !knn_host) {
+        Buf<uint32_t> droots, dwalk, dparent;
+        GCU(droots.alloc(m, s));
+        GCU(dwalk.alloc(n, s));
+        GCU(dparent.alloc(m, s));
+        GCU(cudaMemcpyAsync(droots.p, roots.data(), m * 4ull, cudaMemcpyHostToDevice, s));
+        GCU(cudaMemcpyAsync(dwalk.p, walk.data(), (size_t) n * 4, cudaMemcpyHostToDevice, s));
+        parent_kernel<<<(m + 255) / 256, 256, 0, s>>>(knn.p, k, n, droots.p, m, dwalk.p, g->entry, dparent.p);
+        GCU(cudaGetLastError());
+        GCU(cudaMemcpyAsync(parent.data(), dparent.p, m * 4ull, cudaMemcpyDeviceToHost, s));
+        GCU(cudaStreamSynchronize(s));
+    } else {
+        for (uint32_t i = 0; i < m; ++i) {
+            parent[i] = g->entry;
+            for (uint32_t e = 0; e < k; ++e) {
+                const uint32_t c = g->knn[(size_t) roots[i] * k + e];
+                if (c < n && walk[c] <= i + 1) {
+                    parent[i] = c;
+                    break;
+                }
             }
         }
-        extra.emplace_back(parent, u);
-        ++nextra[parent];
-        ++g->repaired;
-        walk(u);
     }
-    g->off.assign((size_t) n + 1, 0);
-    for (uint32_t a = 0; a < n; ++a) {
-        const uint32_t da = degh[a] + nextra[a];
-        g->off[a + 1] = g->off[a] + da;
-        g->width = std::max(g->width, da);
+    g->repaired = m;
+    // The repair edges at the ends of their parents' lists, in the order they
+    // were made: rows move up, the last first.
+    if (m) {
+        std::vector<uint32_t> &more = queue;  // repair edges per vertex
+        std::fill(more.begin(), more.end(), 0u);
+        for (uint32_t i = 0; i < m; ++i) ++more[parent[i]];
+        uint64_t shift = m;
+        uint64_t end = go[n];
+        go[n] += m;
+        g->nbrs.n += m;
+        for (uint32_t a = n; a-- > 0 && shift;) {
+            const uint64_t b0 = go[a];
+            shift -= more[a];
+            memmove(g->nbrs.data() + b0 + shift, g->nbrs.data() + b0, (size_t) (end - b0) * 4);
+            end = b0;
+            go[a] = b0 + shift;
+        }
+        for (uint32_t i = 0; i < m; ++i) g->nbrs[(size_t) (go[parent[i] + 1] - more[parent[i]]--)] = roots[i];
     }
-    g->nbrs.resize(g->off[n]);
-    std::vector<uint64_t> fill(n);
-    for (uint32_t a = 0; a < n; ++a) {
-        std::copy(prh.begin() + (size_t) a * R, prh.begin() + (size_t) a * R + degh[a], g->nbrs.begin() + g->off[a]);
-        fill[a] = g->off[a] + degh[a];
-    }
-    for (const auto &pe : extra) g->nbrs[fill[pe.first]++] = pe.second;
+    for (uint32_t a = 0; a < n; ++a) g->width = std::max(g->width, (uint32_t) (go[a + 1] - go[a]));
+    if (!knn_host) g->knn_dev = knn.take();
     return PANNS_OK;
 }
 
@@ -812,6 +1163,11 @@ int panns_build_nsg_ex(int device, const float *base, uint32_t n, uint32_t d, ui
     GCU(xn.alloc(n, s));
     GCU(cand.alloc((size_t) n * C, s));
     GCU(cudaMemcpyAsync(x.p, base, (size_t) n * d * 4, cudaMemcpyHostToDevice, s));
+    MeanJob mean;
+    {
+        const int rc = mean.start(x.p, n, d, s);
+        if (rc) return rc;
+    }
     sqnorm32_kernel<<<(n + 255) / 256, 256, 0, s>>>(x.p, n, d, xn.p);
     if (tcg) {
         int num_sms = 0;
@@ -877,7 +1233,7 @@ int panns_build_nsg_ex(int device, const float *base, uint32_t n, uint32_t d, ui
         GCU(cudaStreamSynchronize(s));
     }
     std::unique_ptr<panns_graph> g;
-    const int rc = finish_graph(base, x.p, n, d, k, R, cand.p, C, s, g);
+    const int rc = finish_graph(device, x.p, n, d, k, R, cand.p, C, mean, s, g);
     if (rc) return rc;
     *out = g.release();
     return PANNS_OK;
@@ -908,6 +1264,11 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
     GCU(x.alloc((size_t) n * d, s));
     GCU(xn.alloc(n, s));
     GCU(cudaMemcpyAsync(x.p, base, (size_t) n * d * 4, cudaMemcpyHostToDevice, s));
+    MeanJob mean;
+    {
+        const int rc = mean.start(x.p, n, d, s);
+        if (rc) return rc;
+    }
     sqnorm32_kernel<<<(n + 255) / 256, 256, 0, s>>>(x.p, n, d, xn.p);
     GCU(cudaGetLastError());
     // Cells: Lloyd k-means on S rows at a fixed stride, then every row to its
@@ -1028,7 +1389,7 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
         GCU(cudaStreamSynchronize(s));
     }
     std::unique_ptr<panns_graph> g;
-    const int rc = finish_graph(base, x.p, n, d, k, R, cand.p, C, s, g, reverse != 0);
+    const int rc = finish_graph(device, x.p, n, d, k, R, cand.p, C, mean, s, g, reverse != 0);
     if (rc) return rc;
     g->cells = cells;
     g->probe = P;
@@ -1062,7 +1423,12 @@ int panns_graph_copy(const panns_graph *g, uint64_t *offsets, uint32_t *nbrs, ui
     if (!g) return set_error(PANNS_EINVAL, "panns_graph_copy: NULL graph");
     if (offsets) memcpy(offsets, g->off.data(), g->off.size() * 8);
     if (nbrs && !g->nbrs.empty()) memcpy(nbrs, g->nbrs.data(), g->nbrs.size() * 4);
-    if (knn) memcpy(knn, g->knn.data(), g->knn.size() * 4);
+    if (knn && g->knn_dev) {
+        GCU(cudaSetDevice(g->device));
+        GCU(cudaMemcpy(knn, g->knn_dev, (size_t) g->n * g->k * 4, cudaMemcpyDeviceToHost));
+    } else if (knn) {
+        memcpy(knn, g->knn.data(), g->knn.size() * 4);
+    }
     return PANNS_OK;
 }
 

@@ -33,7 +33,7 @@ def build_nsg(base: np.ndarray, R: int = 50, knn_k: int = 64, device: int = 0, w
         N.check(lib.panns_graph_copy(g, N.ptr(off), N.ptr(nbrs), N.ptr(knn) if with_knn else None))
     finally:
         lib.panns_graph_free(g)
-    graph = NSGGraph(int(width), int(entry), off.astype(np.int64), nbrs[:n_edges].copy())
+    graph = NSGGraph(int(width), int(entry), off.view(np.int64), nbrs[:n_edges])
     graph.repaired = repaired
     return (graph, knn) if with_knn else graph
 
@@ -71,7 +71,7 @@ def build_nsg_cells(base: np.ndarray, R: int = 48, knn_k: int = 64, cells: int =
             part = (cell, near[:, :npb.value])
     finally:
         lib.panns_graph_free(g)
-    graph = NSGGraph(int(width), int(entry), off.astype(np.int64), nbrs[:n_edges].copy())
+    graph = NSGGraph(int(width), int(entry), off.view(np.int64), nbrs[:n_edges])
     graph.repaired = repaired
     out = [graph]
     if with_knn:
@@ -113,4 +113,4 @@ def efanna_build(base: np.ndarray, knn: np.ndarray, L: int, R: int, C: int, rand
         N.check(lib.panns_graph_copy(g, N.ptr(off), N.ptr(nbrs), None))
     finally:
         lib.panns_graph_free(g)
-    return NSGGraph(int(width), int(entry), off.astype(np.int64), nbrs[:n_edges].copy())
+    return NSGGraph(int(width), int(entry), off.view(np.int64), nbrs[:n_edges])

@@ -8,7 +8,7 @@
 //   1. every warp finds the M best unchecked candidates by itself (the queue
 //      does not change meanwhile; they are marked after the next barrier);
 //   2. in rounds, the warps expand candidates (at most G per warp and round, G *
-//      width <= kBuf so a warp's fresh buffer cannot overflow; several warps
+//      degree <= buffer so a warp's fresh buffer cannot overflow; several warps
 //      share a candidate's row when there are fewer candidates than warps): head
 //      rows, visited test-and-set on the block's bitset, distances, the filter
 //      against the queue's L-th distance at the start of the round; the
@@ -38,14 +38,16 @@ constexpr int kBlockCtl = 16;  // control words in shared memory
 // Longest list ranked by counting; above, the bitonic network (initial queues).
 __host__ __device__ constexpr uint32_t block_rank_max(uint32_t W) { return 64u * W; }
 
-// Shared memory of one block of W warps with a queue of queue_cap entries.
-__host__ __device__ inline uint32_t block_smem_bytes(uint32_t queue_cap, uint32_t W) {
+// Shared memory of one block of W warps with a queue of queue_cap entries and
+// warp buffers of buf.
+__host__ __device__ inline uint32_t block_smem_bytes(uint32_t queue_cap, uint32_t W, uint32_t buf, uint32_t vis_smem) {
     return queue_cap * 8u                     // queue (dist, id)
-           + W * kBuf * 8u                    // per-warp fresh ids and distances
-           + W * kBuf * 12u                   // survivors of a round (dist, id, key)
+           + W * buf * 8u                     // per-warp fresh ids and distances
+           + W * buf * 12u                    // survivors of a round (dist, id, key)
            + block_rank_max(W) * 12u          // ranked survivors (dist, id, place)
-           + W * kMaxM * 4u                   // per-warp picked candidates / learned entries
-           + kBlockCtl * 4u;                  // control words
+           + W * kMaxM * 8u                   // per-warp picked candidates (id, place) / learned entries
+           + kBlockCtl * 4u                   // control words
+           + vis_smem * 4u;                   // visited bitset, where it fits
 }
 
 enum { BC_Q = 0, BC_CNT, BC_CNT2, BC_TIE, BC_DIST, BC_EDGES, BC_FULL };
@@ -81,45 +83,89 @@ __device__ __forceinline__ void block_rank(const BlockMem<W> &m, uint32_t n, uin
                                            const uint32_t *__restrict__ orig) {
     constexpr uint32_t T = W * 32;
     const uint32_t tid = threadIdx.x;
-    uint32_t parts = 1;  // threads per element
-    while (parts < 16 && n * parts * 2 <= T) parts *= 2;
-    const uint32_t per = T / parts;  // elements per pass
-    const uint32_t quads = n / 4;
-    const uint32_t share = (quads + parts - 1) / parts;
-    const uint32_t part = tid & (parts - 1);
     const float4 *c4 = reinterpret_cast<const float4 *>(m.cD);
-    for (uint32_t e0 = 0; e0 < n; e0 += per) {  // block-uniform: the shuffles are too
-        const uint32_t e = e0 + tid / parts;
-        const float d = e < n ? m.cD[e] : 0.f;
-        uint32_t less = 0, upto = 0;
-        const uint32_t q1 = min(quads, (part + 1) * share);
-#pragma unroll 2
-        for (uint32_t q = part * share; q < q1; ++q) {
-            const float4 x = c4[q];
-            less += x.x < d ? 1u : 0u;
-            upto += x.x <= d ? 1u : 0u;
-            less += x.y < d ? 1u : 0u;
-            upto += x.y <= d ? 1u : 0u;
-            less += x.z < d ? 1u : 0u;
-            upto += x.z <= d ? 1u : 0u;
-            less += x.w < d ? 1u : 0u;
-            upto += x.w <= d ? 1u : 0u;
-        }
-        if (part == 0)
-            for (uint32_t f = 4 * quads; f < n; ++f) {
-                less += m.cD[f] < d ? 1u : 0u;
-                upto += m.cD[f] <= d ? 1u : 0u;
+    const uint32_t quads = n / 4;
+    if (n <= T / 4) {
+        // Short lists (the usual case): eight lanes per element, which also
+        // search the queue together, eight ways a step.
+        const uint32_t part = tid & 7u, shift = tid & 24u;
+        uint32_t width = 1;  // the search's first stride: sz <= 8 * width
+        while (PLACE && width * 8 < sz) width *= 8;
+        for (uint32_t e0 = 0; e0 < n; e0 += T / 8) {
+            const uint32_t e = e0 + tid / 8;
+            if (e0 + (tid & ~31u) / 8 >= n) break;  // warp-uniform
+            const float d = e < n ? m.cD[e] : 0.f;
+            const uint32_t id = e < n ? m.cI[e] : 0u;
+            uint32_t less = 0, upto = 0;
+            for (uint32_t q = part; q < quads; q += 8) {
+                const float4 x = c4[q];
+                less += (x.x < d ? 1u : 0u) + (x.y < d ? 1u : 0u) + (x.z < d ? 1u : 0u) + (x.w < d ? 1u : 0u);
+                upto += (x.x <= d ? 1u : 0u) + (x.y <= d ? 1u : 0u) + (x.z <= d ? 1u : 0u) + (x.w <= d ? 1u : 0u);
             }
-        for (uint32_t o = 1; o < parts; o <<= 1) {
-            less += __shfl_xor_sync(kFull, less, o);
-            upto += __shfl_xor_sync(kFull, upto, o);
+            if (4 * quads + part < n) {
+                const float x = m.cD[4 * quads + part];
+                less += x < d ? 1u : 0u;
+                upto += x <= d ? 1u : 0u;
+            }
+            uint32_t both = less | upto << 16;
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) both += __shfl_xor_sync(kFull, both, o);
+            less = both & 0xffffu;
+            upto = both >> 16;
+            uint32_t place = 0;
+            if (PLACE) {
+                for (uint32_t wd = width; wd > 0; wd /= 8) {
+                    const uint32_t p = place + (part + 1) * wd - 1;
+                    bool before = false;
+                    if (p < sz) {
+                        const float md = m.qd[p];
+                        before = md < d ||
+                                 (md == d && __ldg(orig + (m.qi[p] & kIdMask)) < __ldg(orig + (id & kIdMask)));
+                    }
+                    place += wd * __popc((__ballot_sync(kFull, before) >> shift) & 0xffu);
+                }
+            }
+            if (e < n && part == 0) {
+                if (upto != less + 1) m.ctl[BC_TIE] = 1u;
+                const uint32_t r = min(less, n - 1);
+                m.sD[r] = d;
+                m.sI[r] = id;
+                if (PLACE) m.sP[r] = place;
+            }
         }
-        if (e < n && part == 0) {
-            if (upto != less + 1) m.ctl[BC_TIE] = 1u;
-            const uint32_t r = min(less, n - 1), id = m.cI[e];
-            m.sD[r] = d;
-            m.sI[r] = id;
-            if (PLACE) m.sP[r] = queue_rank<ORDER_PANNS>(m.qd, m.qi, sz, d, id & kIdMask, orig);
+    } else {
+        uint32_t parts = 1;  // threads per element
+        while (parts < 4 && n * parts * 2 <= T) parts *= 2;
+        const uint32_t per = T / parts;  // elements per pass
+        const uint32_t share = (quads + parts - 1) / parts;
+        const uint32_t part = tid & (parts - 1);
+        for (uint32_t e0 = 0; e0 < n; e0 += per) {  // block-uniform: the shuffles are too
+            const uint32_t e = e0 + tid / parts;
+            const float d = e < n ? m.cD[e] : 0.f;
+            uint32_t less = 0, upto = 0;
+            const uint32_t q1 = min(quads, (part + 1) * share);
+#pragma unroll 2
+            for (uint32_t q = part * share; q < q1; ++q) {
+                const float4 x = c4[q];
+                less += (x.x < d ? 1u : 0u) + (x.y < d ? 1u : 0u) + (x.z < d ? 1u : 0u) + (x.w < d ? 1u : 0u);
+                upto += (x.x <= d ? 1u : 0u) + (x.y <= d ? 1u : 0u) + (x.z <= d ? 1u : 0u) + (x.w <= d ? 1u : 0u);
+            }
+            if (part == 0)
+                for (uint32_t f = 4 * quads; f < n; ++f) {
+                    less += m.cD[f] < d ? 1u : 0u;
+                    upto += m.cD[f] <= d ? 1u : 0u;
+                }
+            for (uint32_t o = 1; o < parts; o <<= 1) {
+                less += __shfl_xor_sync(kFull, less, o);
+                upto += __shfl_xor_sync(kFull, upto, o);
+            }
+            if (e < n && part == 0) {
+                if (upto != less + 1) m.ctl[BC_TIE] = 1u;
+                const uint32_t r = min(less, n - 1), id = m.cI[e];
+                m.sD[r] = d;
+                m.sI[r] = id;
+                if (PLACE) m.sP[r] = queue_rank<ORDER_PANNS>(m.qd, m.qi, sz, d, id & kIdMask, orig);
+            }
         }
     }
     __syncthreads();
@@ -144,7 +190,7 @@ __device__ __forceinline__ void block_rank(const BlockMem<W> &m, uint32_t n, uin
 }
 
 // Block-wide bitonic sort of the n survivors by (distance, original id), in
-// place (the arrays hold W * kBuf entries, a power of two >= n).
+// place (the arrays hold a power of two >= n entries).
 template <int W>
 __device__ __forceinline__ void block_bitonic(const BlockMem<W> &m, uint32_t n, const uint32_t *__restrict__ orig) {
     constexpr uint32_t T = W * 32;
@@ -218,25 +264,41 @@ __device__ __forceinline__ uint32_t block_merge(const BlockMem<W> &m, uint32_t n
     }
     // A queue element moves up by the number of survivors before it: those
     // whose own count of queue elements before them is at most its index.
-    uint32_t steps = 0;
-    while ((1u << steps) <= n) ++steps;
+    const uint32_t steps = 32 - __clz(n);  // 2^steps > n
     uint32_t top = sz;
     while (true) {
         float d[CH];
         uint32_t id[CH], np[CH];
+        if (top - p0 > T) {
+            uint32_t j[CH], lo[CH];  // lo: survivors with sP <= j
 #pragma unroll
-        for (int c = 0; c < CH; ++c) {
-            np[c] = L;
-            const uint32_t back = c * T + tid + 1;
-            if (back <= top && top - back >= p0) {
-                const uint32_t j = top - back;
-                d[c] = m.qd[j];
-                id[c] = m.qi[j];
-                uint32_t lo = 0;  // survivors with sP <= j
-                for (uint32_t b = 1u << (steps - 1); b > 0; b >>= 1)
-                    if (lo + b <= n && sP[lo + b - 1] <= j) lo += b;
-                np[c] = j + lo;
+            for (int c = 0; c < CH; ++c) {
+                const uint32_t back = c * T + tid + 1;
+                const bool have = back <= top - p0;
+                j[c] = have ? top - back : 0u;
+                d[c] = m.qd[j[c]];
+                id[c] = m.qi[j[c]];
+                lo[c] = 0;
+                np[c] = have ? j[c] : L;
             }
+            for (uint32_t b = 1u << (steps - 1); b > 0; b >>= 1) {
+#pragma unroll
+                for (int c = 0; c < CH; ++c)
+                    if (lo[c] + b <= n && sP[lo[c] + b - 1] <= j[c]) lo[c] += b;
+            }
+#pragma unroll
+            for (int c = 0; c < CH; ++c) np[c] += lo[c];
+        } else {  // one element a thread
+#pragma unroll
+            for (int c = 1; c < CH; ++c) np[c] = L;
+            const bool have = (uint32_t) tid < top - p0;
+            const uint32_t j = have ? top - 1 - tid : 0u;
+            d[0] = m.qd[j];
+            id[0] = m.qi[j];
+            uint32_t lo = 0;
+            for (uint32_t b = 1u << (steps - 1); b > 0; b >>= 1)
+                if (lo + b <= n && sP[lo + b - 1] <= j) lo += b;
+            np[0] = have ? j + lo : L;
         }
         const bool last = top <= p0 + CH * T;
         __syncthreads();
@@ -268,17 +330,21 @@ __device__ void block_search_one(const SearchArgs &a, uint32_t q, uint8_t *smem,
     BlockMem<W> m;
     m.qd = reinterpret_cast<float *>(smem);
     m.qi = reinterpret_cast<uint32_t *>(m.qd + a.queue_cap);
-    float *bd = reinterpret_cast<float *>(m.qi + a.queue_cap) + w * kBuf;
-    uint32_t *bi = reinterpret_cast<uint32_t *>(m.qi + a.queue_cap) + W * kBuf + w * kBuf;
-    m.cD = reinterpret_cast<float *>(m.qi + a.queue_cap + 2 * W * kBuf);
-    m.cI = reinterpret_cast<uint32_t *>(m.cD + W * kBuf);
-    m.cK = m.cI + W * kBuf;
-    m.sD = reinterpret_cast<float *>(m.cK + W * kBuf);
+    const uint32_t buf = a.block_buf;
+    float *bd = reinterpret_cast<float *>(m.qi + a.queue_cap) + w * buf;
+    uint32_t *bi = m.qi + a.queue_cap + W * buf + w * buf;
+    m.cD = reinterpret_cast<float *>(m.qi + a.queue_cap + 2 * W * buf);
+    m.cI = reinterpret_cast<uint32_t *>(m.cD + W * buf);
+    m.cK = m.cI + W * buf;
+    m.sD = reinterpret_cast<float *>(m.cK + W * buf);
     m.sI = reinterpret_cast<uint32_t *>(m.sD + block_rank_max(W));
     m.sP = m.sI + block_rank_max(W);
-    uint32_t *cand = m.sP + block_rank_max(W) + w * kMaxM;
-    m.ctl = m.sP + block_rank_max(W) + W * kMaxM;
+    uint32_t *cand = m.sP + block_rank_max(W) + w * 2 * kMaxM;
+    uint32_t *cpos = cand + kMaxM;  // the candidates' places in the queue
+    m.ctl = m.sP + block_rank_max(W) + W * 2 * kMaxM;
     uint32_t *ctl = m.ctl;
+    uint32_t *svis = ctl + kBlockCtl;
+    const bool in_smem = a.vis_smem != 0;
 
     uint32_t L = a.Lq ? __ldg(a.Lq + q) : a.L;
     // Init ids: n_lrn learned entries (cand) then n_plain of the init list.
@@ -293,6 +359,7 @@ __device__ void block_search_one(const SearchArgs &a, uint32_t q, uint8_t *smem,
     Dist<KIND, CL, STORE> D;
     D.load(a, q, lane);
     if (tid < kBlockCtl && tid != BC_Q) ctl[tid] = 0;
+    for (uint32_t i = tid; i < a.vis_smem; i += T) svis[i] = 0;
     __syncthreads();
 
     uint32_t sz = 0, dcount = 0, n_dist = 0, n_edges = 0, n_expand = 0, n_iter = 0;
@@ -301,12 +368,29 @@ __device__ void block_search_one(const SearchArgs &a, uint32_t q, uint8_t *smem,
     uint32_t *my_dirty = dirty + (size_t) w * dcap;
     uint32_t turn = 0;  // which of the two list counters the round uses
 
+    // Test-and-set of a vertex's visited bit: was it clear? In shared memory
+    // where the bitset fits beside the queue without costing resident blocks
+    // (an atomic there takes a tenth of one in L2, and nothing is left to
+    // clear), else in the block's slot of global memory.
+    auto visit = [&](uint32_t id, bool valid) -> bool {
+        const uint32_t bit = 1u << (id & 31);
+        if (in_smem) return valid && !(atomicOr(svis + (id >> 5), bit) & bit);
+        const uint32_t old = visit_issue(vis, id, valid);
+        note_dirty(my_dirty, dcap, dcount, valid && old == 0, id >> 5);
+        return valid && !(old & bit);
+    };
     // Distances of the warp's fresh vertices, the filter against the queue's
     // L-th, the survivors appended to the round's list.
     auto finish_list = [&](uint32_t nb, bool filter) {
         if (nb) {
-            if constexpr (STORE == STORE_FP32) distances_wide<KIND, CL>(a, D.qv, bi, bd, nb, lane);
-            else D.distances(a, bi, bd, nb, lane);
+            if constexpr (STORE == STORE_FP32) {
+                // 16 rows a pass; eight or fewer left over in a pass of eight
+                const uint32_t wide = (nb & 15u) > 8u ? nb : nb & ~15u;
+                if (wide) distances_wide<KIND, CL>(a, D.qv, bi, bd, wide, lane);
+                if (wide < nb) D.distances(a, bi + wide, bd + wide, nb - wide, lane);
+            } else {
+                D.distances(a, bi, bd, nb, lane);
+            }
         }
         n_dist += nb;
         const bool any_bound = filter && sz >= L;
@@ -341,9 +425,9 @@ __device__ void block_search_one(const SearchArgs &a, uint32_t q, uint8_t *smem,
     // Initial queue: the init ids (learned entries first, a repeated id
     // entering once), spread evenly over the warps.
     const uint32_t *init = a.init_ids + (size_t) q * a.init_stride;
-    for (uint32_t r0 = 0; r0 < n_init; r0 += W * kBuf) {
-        const uint32_t rest = min(n_init - r0, (uint32_t) (W * kBuf));
-        const uint32_t per = ((rest + W - 1) / W + 15) & ~15u;  // <= kBuf, whole distance passes
+    for (uint32_t r0 = 0; r0 < n_init; r0 += W * buf) {
+        const uint32_t rest = min(n_init - r0, W * buf);
+        const uint32_t per = ((rest + W - 1) / W + 15) & ~15u;  // <= buf, whole distance passes
         uint32_t nb = 0;
         const uint32_t lo = r0 + w * per, hi = min(r0 + rest, lo + per);
         for (uint32_t i0 = lo; i0 < hi; i0 += 32) {
@@ -352,9 +436,7 @@ __device__ void block_search_one(const SearchArgs &a, uint32_t q, uint8_t *smem,
             const uint32_t id = valid ? (i < n_lrn ? cand[i] : __ldg(init + (i - n_lrn))) : 0u;
             const bool ok = valid && id < a.n;
             if (valid && !ok) atomicOr(a.error, ERR_BAD_INIT);
-            const uint32_t old = visit_issue(vis, id, ok);
-            note_dirty(my_dirty, dcap, dcount, ok && old == 0, id >> 5);
-            const bool fresh = ok && !(old & (1u << (id & 31)));
+            const bool fresh = visit(id, ok);
             const uint32_t bm = __ballot_sync(kFull, fresh);
             if (fresh) bi[nb + __popc(bm & lanemask_lt())] = id;
             nb += __popc(bm);
@@ -368,19 +450,37 @@ __device__ void block_search_one(const SearchArgs &a, uint32_t q, uint8_t *smem,
     const uint32_t M = a.M, G = a.block_round;
     uint32_t k = 0;
     for (;;) {
-        // 1. The step's candidates: every warp scans for itself.
+        // 1. The step's candidates: every warp scans for itself, four entries
+        // a lane (the queue's room is a multiple of 32).
         uint32_t cnt = 0, last_k = L;
-        for (uint32_t p0 = k; p0 < sz && cnt < M; p0 += 32) {
-            const uint32_t p = p0 + lane;
-            const uint32_t id = p < sz ? m.qi[p] : kChecked;
-            const uint32_t bm = __ballot_sync(kFull, !(id & kChecked));
-            const uint32_t take = min((uint32_t) __popc(bm), M - cnt);
-            const uint32_t r = __popc(bm & lanemask_lt());
-            const bool mine = !(id & kChecked) && r < take;
-            if (mine) cand[cnt + r] = id;
-            const uint32_t tm = __ballot_sync(kFull, mine);
-            if (tm) last_k = p0 + 31 - __clz(tm);
-            cnt += take;
+        for (uint32_t p0 = k & ~3u; p0 < sz && cnt < M; p0 += 128) {
+            const uint32_t p = p0 + 4 * lane;
+            uint4 e = make_uint4(kChecked, kChecked, kChecked, kChecked);
+            if (p < sz) e = *reinterpret_cast<const uint4 *>(m.qi + p);
+            const uint32_t v[4] = {e.x, e.y, e.z, e.w};
+            bool un[4];
+            uint32_t before = 0, total = 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                un[i] = !(v[i] & kChecked) && p + i >= k && p + i < sz;
+                const uint32_t bm = __ballot_sync(kFull, un[i]);
+                before += __popc(bm & lanemask_lt());
+                total += __popc(bm);
+            }
+            uint32_t r = cnt + before, mine = 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (un[i]) {
+                    if (r < M) {
+                        cand[r] = v[i];
+                        cpos[r] = p + i;
+                        mine = p + i + 1;
+                    }
+                    ++r;
+                }
+            mine = __reduce_max_sync(kFull, mine);
+            if (mine) last_k = mine - 1;
+            cnt = min(M, cnt + total);
         }
         __syncwarp();
         if (cnt == 0) break;  // block-uniform
@@ -418,15 +518,20 @@ __device__ void block_search_one(const SearchArgs &a, uint32_t q, uint8_t *smem,
                         valid = false;
                     }
                     if (!valid) hv[j] = kFull;
-                    olds[j] = visit_issue(vis, hv[j], valid);
+                    if (!in_smem) olds[j] = visit_issue(vis, hv[j], valid);
                 }
 #pragma unroll
                 for (int j = 0; j < kCandGroup; ++j) {
                     if ((uint32_t) j >= gc) break;
                     const uint32_t id = hv[j];
                     const bool valid = id != kFull;
-                    const bool fresh = valid && !(olds[j] & (1u << (id & 31)));
-                    note_dirty(my_dirty, dcap, dcount, valid && olds[j] == 0, id >> 5);
+                    bool fresh;
+                    if (in_smem) {
+                        fresh = visit(id, valid);
+                    } else {  // (all of them issued before any is used)
+                        fresh = valid && !(olds[j] & (1u << (id & 31)));
+                        note_dirty(my_dirty, dcap, dcount, valid && olds[j] == 0, id >> 5);
+                    }
                     const uint32_t bm = __ballot_sync(kFull, fresh);
                     if (fresh) bi[nb + __popc(bm & lanemask_lt())] = id;
                     nb += __popc(bm);
@@ -445,9 +550,7 @@ __device__ void block_search_one(const SearchArgs &a, uint32_t q, uint8_t *smem,
                                 atomicOr(a.error, ERR_BAD_ID);
                                 valid = false;
                             }
-                            const uint32_t old = visit_issue(vis, id, valid);
-                            const bool fresh = valid && !(old & (1u << (id & 31)));
-                            note_dirty(my_dirty, dcap, dcount, valid && old == 0, id >> 5);
+                            const bool fresh = visit(id, valid);
                             const uint32_t bm = __ballot_sync(kFull, fresh);
                             if (fresh) bi[nb + __popc(bm & lanemask_lt())] = id;
                             nb += __popc(bm);
@@ -460,17 +563,8 @@ __device__ void block_search_one(const SearchArgs &a, uint32_t q, uint8_t *smem,
             const uint32_t n = close_list();
             // Every warp has its candidates: mark them (block_merge reads the
             // marks after its next barrier at the earliest).
-            if (r0 == 0 && w == 0) {
-                uint32_t left = cnt;
-                for (uint32_t p0 = k; left; p0 += 32) {
-                    const uint32_t p = p0 + lane;
-                    const uint32_t id = p < sz ? m.qi[p] : kChecked;
-                    const uint32_t bm = __ballot_sync(kFull, !(id & kChecked));
-                    const uint32_t take = min((uint32_t) __popc(bm), left);
-                    if (!(id & kChecked) && (uint32_t) __popc(bm & lanemask_lt()) < take) m.qi[p] = id | kChecked;
-                    left -= take;
-                }
-            }
+            if (r0 == 0)
+                for (uint32_t c = w + W * lane; c < cnt; c += W * 32) m.qi[cpos[c]] = cand[c] | kChecked;
             nk = min(nk, block_merge<W>(m, n, sz, L, a.orig));
         }
         k = nk <= last_k ? nk : last_k + 1;
@@ -485,7 +579,7 @@ __device__ void block_search_one(const SearchArgs &a, uint32_t q, uint8_t *smem,
         const uint32_t lo = min(sz, w * per), hi = min(sz, lo + per);
         E.distances(a, m.qi + lo, m.qd + lo, hi - lo, lane);
         __syncthreads();
-        if (sz <= W * kBuf) {
+        if (sz <= W * buf) {
             for (uint32_t i = tid; i < sz; i += T) {
                 m.cD[i] = m.qd[i];
                 m.cI[i] = m.qi[i] & kIdMask;
@@ -514,7 +608,8 @@ __device__ void block_search_one(const SearchArgs &a, uint32_t q, uint8_t *smem,
     __syncthreads();
     if (tid == 0 && a.out_stats) a.out_stats[q] = make_uint4(ctl[BC_DIST], n_expand, ctl[BC_EDGES], n_iter);
     // Clear the visited words this query set.
-    if (!ctl[BC_FULL]) {
+    if (in_smem) {
+    } else if (!ctl[BC_FULL]) {
         for (uint32_t i = lane; i < dcount; i += 32) vis[my_dirty[i]] = 0u;
     } else {
         for (uint32_t i = tid; i < a.vis_words; i += T) vis[i] = 0u;
@@ -528,7 +623,7 @@ __global__ void __launch_bounds__(W * 32) search_block_kernel(SearchArgs a) {
     const uint32_t slot = blockIdx.x;
     uint32_t *vis = a.visited + (size_t) slot * a.vis_words;
     uint32_t *dirty = a.dirty + (size_t) slot * a.dirty_cap;
-    uint32_t *ctl = reinterpret_cast<uint32_t *>(smem + block_smem_bytes(a.queue_cap, W) - kBlockCtl * 4);
+    uint32_t *ctl = reinterpret_cast<uint32_t *>(smem + block_smem_bytes(a.queue_cap, W, a.block_buf, 0) - kBlockCtl * 4);
     for (;;) {
         if (threadIdx.x == 0) ctl[BC_Q] = atomicAdd(a.counter, 1u);
         __syncthreads();

@@ -196,6 +196,14 @@ struct panns_index {
     DevBuf<uint32_t> init_def;  // default PANNS init list (device ids) for init_def_L
     uint32_t init_def_L = 0;
     DevBuf<float> dq;           // chain-major copy of device-pointer queries
+    // Resident blocks per SM by (kernel, threads, shared memory), asked for once.
+    struct Resident {
+        const void *kern;
+        int threads;
+        size_t smem;
+        int per_sm, max_threads;
+    };
+    std::vector<Resident> resident;
     // Captured launch (PANNS_FLAG_CUDA_GRAPH): replayed while its key matches.
     cudaGraphExec_t gexec = nullptr;
     std::vector<uint8_t> gkey;
@@ -797,6 +805,85 @@ static int enqueue_launch(panns_index *h, const LaunchDesc &l, cudaStream_t s, b
     return PANNS_OK;
 }
 
+constexpr size_t kSmemLimit = 227u << 10;  // dynamic shared memory of one block
+
+// Resident blocks per SM of a search kernel, and its largest block, kept per handle.
+static int resident_blocks(panns_index *h, const void *kern, int threads, size_t smem, panns_index::Resident &out) {
+    for (const auto &r : h->resident)
+        if (r.kern == kern && r.threads == threads && r.smem == smem) {
+            out = r;
+            return PANNS_OK;
+        }
+    panns_index::Resident r{kern, threads, smem, 0, 0};
+    cudaFuncAttributes fa;
+    CU(cudaFuncGetAttributes(&fa, kern));
+    r.max_threads = fa.maxThreadsPerBlock;
+    CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kSmemLimit));
+    CU(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, -1));
+    if (threads <= r.max_threads)
+        CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r.per_sm, kern, threads, smem));
+    if (h->resident.size() >= 64) h->resident.clear();  // a handle that keeps changing its sizes
+    h->resident.push_back(r);
+    out = r;
+    return PANNS_OK;
+}
+
+// Entries of a block kernel's warp buffer: the neighbours of the warp's share of
+// a step's candidates (at most max_deg per candidate) in one round, up to kBuf.
+static uint32_t block_buffer(uint32_t max_deg, uint32_t M, uint32_t W) {
+    const uint64_t want = (uint64_t) std::max(1u, max_deg) * ((M + W - 1) / W);
+    uint32_t b = 64;
+    while (b < (uint32_t) kBuf && b < want) b *= 2;
+    return b;
+}
+
+// Warps per query where the caller leaves the choice open (same ids either
+// way). More warps shorten a query but fewer queries are resident at once, and a
+// batch takes as many waves as its residents make it, so the choice is the
+// smallest waves x cost, cost relative to one warp. Measured on 1M x 96, M = 8
+// (ms per wave at L = 384, float32: 1.33 / 0.82 / 0.55 / 0.36-0.42 / 0.33 with 1 /
+// 2 / 4 / 8 / 16 warps; the ratios at L = 100 and 1,024 and with the FP8 copy are
+// within a fifth of it, but at L = 1,024 16 warps take 0.92 against 0.78 ms with
+// 8) and on 100k x 128 at L = 2,048 (9.8 / 3.5 / 2.0 / 1.7). Examples, ms with 1 /
+// 2 / 4 / 8 warps: 220 queries 1.34 / 0.82 / 0.52 / 0.42, 500 1.33 / 0.85 / 0.58 /
+// 0.80, 740 1.37 / 0.88 / 1.02 / 1.16, 1,480 1.48 / 1.68 / 1.57 / 1.98; 1,000 at
+// L = 2,048 10.6 / 9.1 / 6.4 / 7.1.
+static int choose_warps(panns_index *h, const panns_search_params *p, uint32_t kind, int CL, uint32_t M, uint32_t nq,
+                        uint32_t &wpq) {
+    static const uint32_t warps[5] = {1, 2, 4, 8, 16};
+    static const float short_cost[5] = {1.f, 0.61f, 0.40f, 0.28f, 0.25f};
+    static const float long_cost[5] = {1.f, 0.36f, 0.20f, 0.175f, 0.2f};
+    const float *cost = p->L < 2048 ? short_cost : long_cost;
+    const uint32_t qcap = ((p->L + 31) / 32) * 32;
+    float best = 0.f;
+    wpq = 1;
+    for (int i = 0; i < 5; ++i) {
+        const uint32_t W = warps[i];
+        if (W == 16 && (p->L > 512 || nq > (uint32_t) h->num_sms)) continue;
+        uint32_t wpb = 4;
+        if (W == 1)
+            while (wpb > 1 && wpb * warp_smem_bytes(qcap) > kSmemLimit) --wpb;
+        const size_t smem = W == 1 ? (size_t) wpb * warp_smem_bytes(qcap)
+                                   : (size_t) block_smem_bytes(qcap, W, block_buffer(h->max_deg, M, W), 0);
+        if (smem > kSmemLimit) continue;
+        const void *kern = W == 1 ? search_kernel_ptr(kind, ORDER_PANNS, CL, p->storage)
+                                  : search_block_kernel_ptr(kind, CL, W, p->storage);
+        if (!kern) continue;
+        panns_index::Resident r;
+        const int rc = resident_blocks(h, kern, (int) (W == 1 ? wpb : W) * 32, smem, r);
+        if (rc) return rc;
+        if (r.per_sm < 1) continue;
+        const uint32_t at_once = (uint32_t) r.per_sm * (uint32_t) h->num_sms * (W == 1 ? wpb : 1u);
+        if (W == 1 && p->L < 2048 && nq > at_once) break;  // one warp each keeps every SM full
+        const float c = (float) ((nq + at_once - 1) / at_once) * cost[i];
+        if (best == 0.f || c < best) {
+            best = c;
+            wpq = W;
+        }
+    }
+    return PANNS_OK;
+}
+
 // Launch the search for nq device queries (chain-major at d_queries_cm; when
 // d_rows is set they are first laid out there from row-major d_rows), with
 // device init ids and optional per-query queue lengths; everything enqueued
@@ -809,21 +896,17 @@ static int launch_search(panns_index *h, const panns_search_params *p, float *d_
     const uint32_t order = p->mode == PANNS_MODE_EFANNA ? ORDER_EFANNA : ORDER_PANNS;
     const uint32_t kind = p->distance == PANNS_DIST_L2 ? KIND_L2 : KIND_IP;
     const bool pss = p->mode == PANNS_MODE_PSS_V5 && p->T > 1;
+    const uint32_t M = p->mode == PANNS_MODE_TOP_M ? p->M : 1u;
     uint32_t wpq = p->warps_per_query > 1 ? p->warps_per_query : 1u;
     if (p->warps_per_query == 0 && p->warps_per_block == 0 && p->blocks_per_sm == 0 &&
         (p->mode == PANNS_MODE_NSG_SEQ || p->mode == PANNS_MODE_TOP_M || (p->mode == PANNS_MODE_PSS_V5 && p->T == 1)) &&
         h->max_deg <= (uint32_t) kBuf) {
-        // Automatic block shape (same ids either way), from the 1M x 96 and
-        // 1M x 128 measurements: 8 warps per query up to one query per SM and
-        // for queues of 2048 and more, 2 up to ten queries per SM, else one.
-        const uint32_t sms = (uint32_t) h->num_sms;
-        if (p->L >= 2048 || nq <= sms) wpq = 8;
-        else if (nq <= 10 * sms) wpq = 2;
+        const int rc = choose_warps(h, p, kind, CL, M, nq, wpq);
+        if (rc) return rc;
     }
     const void *kern = wpq > 1 ? search_block_kernel_ptr(kind, CL, wpq, p->storage)
                                : pss ? pss_kernel_ptr(kind, CL) : search_kernel_ptr(kind, order, CL, p->storage);
     if (!kern) return fail(PANNS_EINVAL, "search: unsupported dimension");
-    const uint32_t M = p->mode == PANNS_MODE_TOP_M ? p->M : 1u;
     const uint32_t qcap = ((p->L + 31) / 32) * 32;
     const uint32_t L_local = p->L_local ? p->L_local : p->L;
     const uint32_t wcap = ((L_local + 31) / 32) * 32;
@@ -838,25 +921,43 @@ static int launch_search(panns_index *h, const panns_search_params *p, float *d_
     }
     if (per_warp > (227u << 10))
         return fail(PANNS_EINVAL, "search: the queues (L, T x L_local) do not fit in shared memory");
-    const size_t smem = wpq > 1 ? (size_t) block_smem_bytes(qcap, wpq) : (size_t) wpb * per_warp;
-    if (smem > (227u << 10)) return fail(PANNS_EINVAL, "search: the queue does not fit in shared memory");
+    const uint32_t bbuf = wpq > 1 ? block_buffer(h->max_deg, M, wpq) : 0;
+    uint32_t vis_smem = 0;
+    size_t smem = wpq > 1 ? (size_t) block_smem_bytes(qcap, wpq, bbuf, 0) : (size_t) wpb * per_warp;
+    if (smem > kSmemLimit) return fail(PANNS_EINVAL, "search: the queue does not fit in shared memory");
     const uint32_t qpb = wpq > 1 ? 1u : wpb;  // queries in flight per block
+    panns_index::Resident res;
     {
-        cudaFuncAttributes fa;
-        CU(cudaFuncGetAttributes(&fa, kern));
-        if ((int) (wpb * 32) > fa.maxThreadsPerBlock)
-            return fail(PANNS_EINVAL, "search: warps_per_block must be <= " + std::to_string(fa.maxThreadsPerBlock / 32) +
+        int rc = resident_blocks(h, kern, (int) wpb * 32, smem, res);
+        if (rc) return rc;
+        if ((int) (wpb * 32) > res.max_threads)
+            return fail(PANNS_EINVAL, "search: warps_per_block must be <= " + std::to_string(res.max_threads / 32) +
                                           " for this kernel");
+        if (wpq > 1) {
+            // The visited bitset in shared memory too, where that costs no
+            // resident query: as many blocks per SM as without it, or as the
+            // batch needs. One query on 1M x 96: 280 -> 240 us, 1,000 at L =
+            // 2,048 on 100k x 128 9.9 -> 7.1 ms (with the smaller warp buffers).
+            const uint32_t words = (h->n + 31) / 32;
+            const size_t with = (size_t) words * 4 < kSmemLimit ? (size_t) block_smem_bytes(qcap, wpq, bbuf, words)
+                                                                : kSmemLimit + 1;
+            const uint32_t need = (nq + (uint32_t) h->num_sms - 1) / (uint32_t) h->num_sms;
+            if (with <= kSmemLimit &&
+                (228u << 10) / (with + 1024) >= std::min<uint32_t>((uint32_t) std::max(res.per_sm, 1), need)) {
+                vis_smem = words;
+                smem = with;
+                rc = resident_blocks(h, kern, (int) wpb * 32, smem, res);
+                if (rc) return rc;
+            }
+        }
     }
-    CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
     // The L1 / shared-memory split: the driver's first (enough shared memory
     // for the most resident blocks); with a block count (blocks_per_sm, or the
     // default below), just enough shared memory for that many blocks, the rest
     // of the array left to L1, which caches the gathered rows.
     CU(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                             carveout_percent(smem, p->blocks_per_sm)));
-    int per_sm = 0;
-    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int) wpb * 32, smem));
+    int per_sm = res.per_sm;
     if (per_sm < 1) return fail(PANNS_EINVAL, "search: L too large for shared memory");
     uint32_t bps = p->blocks_per_sm;
     if (!bps) {
@@ -950,8 +1051,10 @@ static int launch_search(panns_index *h, const panns_search_params *p, float *d_
     a.error = h->error.p;
     a.queue_cap = qcap;
     // Block kernel: candidates per warp and merge round, so that a warp's
-    // fresh neighbours (at most max_deg per candidate) fit its list.
-    a.block_round = std::max(1u, std::min<uint32_t>(kCandGroup, kBuf / std::max(1u, h->max_deg)));
+    // fresh neighbours (at most max_deg per candidate) fit its buffer.
+    a.block_round = std::max(1u, std::min<uint32_t>(kCandGroup, bbuf / std::max(1u, h->max_deg)));
+    a.block_buf = bbuf;
+    a.vis_smem = vis_smem;
     PssArgs pa;
     memset(&pa, 0, sizeof(pa));
     memcpy(&pa.s, &a, sizeof(a));
@@ -1600,7 +1703,7 @@ extern "C" int panns_search_static(panns_index *h, const panns_search_params *p,
             return fail(PANNS_EINVAL, "search: warps_per_block must be <= " + std::to_string(fa.maxThreadsPerBlock / 32) +
                                           " for this kernel");
     }
-    CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+    CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kSmemLimit));
     CU(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, -1));
     int per_sm = 0;
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int) wpb * 32, smem));

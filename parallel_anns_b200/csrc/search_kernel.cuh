@@ -118,7 +118,10 @@ struct SearchArgs {
     const uint32_t *Lq;       // per-query queue length (K <= Lq[q] <= L), or null: L for all
     const uint32_t *decisions;  // per-query records of the entry / L-budget network (mlp_decide), or null
     uint32_t dec_L_init;      // plain init ids kept after learned entries
-    uint32_t block_round;     // search_block_kernel: candidates per warp and merge round
+    // search_block_kernel:
+    uint32_t block_round;     // candidates per warp and merge round
+    uint32_t block_buf;       // fresh vertices per warp and round (a power of two)
+    uint32_t vis_smem;        // words of the visited bitset in shared memory (0: in global memory)
 };
 
 // Bytes of shared memory one warp needs.

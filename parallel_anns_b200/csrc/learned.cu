@@ -48,106 +48,153 @@ __device__ __forceinline__ void split_tf32(float x, uint32_t &hi, uint32_t &lo) 
 
 // c += a * b for one m16n8k8 tile (A row-major, B column-major, TF32, float32 accumulate).
 __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-    asm volatile(
+    asm(
         "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
         "{%0, %1, %2, %3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// C[M x N] = A(M x K) * B(K x N) (+ bias[n]) (relu) (or C += when accumulate).
+// C[M x N] = A(M x K) * B(K x N) (+ bias[n]) (relu) (or, with mask, 0 where the
+// element of `mask`, laid out as C, is not positive: a ReLU's backward pass).
 // A(m, k) = AT ? A[k * lda + m] : A[m * lda + k]; B(k, n) = BT ? B[n * ldb + k]
-// : B[k * ldb + n]. 64 x 64 tiles staged through shared memory 32 deep, the
-// next slice's loads in flight (registers) while the tensor cores work on the
-// current one (split TF32, float32 accumulation); the order of every sum is
-// fixed (k ascending in steps of 8), so results are deterministic.
-template <typename TA, typename TB, bool AT, bool BT>
-__global__ void __launch_bounds__(256) gemm_kernel(const TA *__restrict__ A, int lda, const TB *__restrict__ B,
-                                                   int ldb, float *__restrict__ C, int ldc, int M, int N, int K,
-                                                   const float *__restrict__ bias, int relu, int accumulate) {
-    constexpr int BK = 32;
+// : B[k * ldb + n]. BM x BN tiles staged through shared memory 32 deep by WR * WC
+// warps (each (BM / WR) x (BN / WC) of the tile), AHEAD slices of global loads in
+// flight in registers while the tensor cores work on the one in shared memory
+// (split TF32, float32 accumulation). A staged tile runs along the index that is
+// contiguous in global memory, its rows padded so that both the stores and the
+// fragment loads go without bank conflicts. The order of every sum is fixed
+// (k ascending in steps of 8, whatever the tile), so results are deterministic
+// and do not depend on the tile chosen.
+// Large products are bound by the rate of the TF32 MMAs, the training step's
+// (1,024 x 256 x 256 and the like) by the latency of their slices and MMA
+// chains: gemm() has the rule and both sides' times.
+template <typename TA, typename TB, bool AT, bool BT, int BM, int BN, int WR, int WC, int AHEAD>
+__global__ void __launch_bounds__(WR *WC * 32) gemm_kernel(const TA *__restrict__ A, int lda, const TB *__restrict__ B,
+                                                          int ldb, float *__restrict__ C, int ldc, int M, int N, int K,
+                                                          const float *__restrict__ bias, int relu, const float *__restrict__ mask) {
+    constexpr int BK = 32, NT = WR * WC * 32;
+    constexpr int NA = BM * BK / NT, NB = BN * BK / NT;  // elements a thread loads of a slice
+    constexpr int TN = BN / WC / 8;                      // 8-wide MMA tiles of a warp
+    static_assert(BM / WR == 16 && BN % (8 * WC) == 0 && NA * NT == BM * BK && NB * NT == BN * BK, "tile");
     constexpr bool kBExact = std::is_same<TB, __nv_bfloat16>::value;  // BF16 is exact in TF32
-    __shared__ float As[2][BK][64 + 4];
-    __shared__ float Bs[2][BK][64 + 4];
+    constexpr int LA = AT ? BM + 8 : BK + 4, LB = BT ? BK + 4 : BN + 8;  // padded rows
+    __shared__ float As[2][AT ? BK * LA : BM * LA];
+    __shared__ float Bs[2][BT ? BN * LB : BK * LB];
+    auto ia = [](int m, int k) { return AT ? k * LA + m : m * LA + k; };
+    auto ib = [](int k, int n) { return BT ? n * LB + k : k * LB + n; };
     const int tid = threadIdx.x;
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-    // 8 warps: warp w computes rows wm..wm+15 and columns wn..wn+31 of the tile.
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int warp = tid >> 5, lane = tid & 31;
-    const int wm = (warp & 3) * 16, wn = (warp >> 2) * 32;
+    const int wm = (warp % WR) * 16, wn = (warp / WR) * (BN / WC);
     const int g = lane >> 2, tq = lane & 3;  // MMA fragment coordinates
-    float acc[4][4];
+    float acc[TN][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < TN; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-    // Element e = tid + 256 i of a slice: A as (m, k), B as (k, n), each in
+    // Element e = tid + NT i of a slice: A as (m, k), B as (k, n), each in
     // the order that keeps a warp's global loads contiguous.
-    float ra[8], rb[8];
-    auto load = [&](int k0) {
+    struct Slice {
+        float a[NA], b[NB];
+    };
+    auto load = [&](int k0, Slice &r) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int e = tid + 256 * i;
-            const int mm = AT ? e % 64 : e / BK, kk = AT ? e / 64 : e % BK;
+        for (int i = 0; i < NA; ++i) {
+            const int e = tid + NT * i;
+            const int mm = AT ? e % BM : e / BK, kk = AT ? e / BM : e % BK;
             const int gm = m0 + mm, gk = k0 + kk;
-            ra[i] = (gm < M && gk < K) ? to_f(AT ? A[(size_t) gk * lda + gm] : A[(size_t) gm * lda + gk]) : 0.f;
-            const int nn = BT ? e / BK : e % 64, kb = BT ? e % BK : e / 64;
-            const int gn = n0 + nn, gkb = k0 + kb;
-            rb[i] = (gn < N && gkb < K) ? to_f(BT ? B[(size_t) gn * ldb + gkb] : B[(size_t) gkb * ldb + gn]) : 0.f;
+            r.a[i] = (gm < M && gk < K) ? to_f(AT ? A[(size_t) gk * lda + gm] : A[(size_t) gm * lda + gk]) : 0.f;
         }
-    };
-    auto store = [&](int buf) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int e = tid + 256 * i;
-            As[buf][AT ? e / 64 : e % BK][AT ? e % 64 : e / BK] = ra[i];
-            Bs[buf][BT ? e % BK : e / 64][BT ? e / BK : e % 64] = rb[i];
+        for (int i = 0; i < NB; ++i) {
+            const int e = tid + NT * i;
+            const int nn = BT ? e / BK : e % BN, kk = BT ? e % BK : e / BN;
+            const int gn = n0 + nn, gk = k0 + kk;
+            r.b[i] = (gn < N && gk < K) ? to_f(BT ? B[(size_t) gn * ldb + gk] : B[(size_t) gk * ldb + gn]) : 0.f;
         }
     };
-    load(0);
-    store(0);
-    __syncthreads();
-    int buf = 0;
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        const bool more = k0 + BK < K;
-        if (more) load(k0 + BK);  // in flight during the MMAs below
-        // Tensor cores: per 8-deep k step, the warp's 16 x 32 block of C as
-        // four m16n8k8 TF32 MMAs. A float32 operand is split into a TF32 high
-        // part and the TF32 rounding of its remainder, and the products
-        // hi*hi + hi*lo + lo*hi accumulate in float32, which keeps float32
-        // accuracy; a BF16 operand is exact in TF32 (no low part, one MMA less).
+    auto store = [&](int buf, const Slice &r) {
+#pragma unroll
+        for (int i = 0; i < NA; ++i) {
+            const int e = tid + NT * i;
+            As[buf][AT ? ia(e % BM, e / BM) : ia(e / BK, e % BK)] = r.a[i];
+        }
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+            const int e = tid + NT * i;
+            Bs[buf][BT ? ib(e % BK, e / BK) : ib(e / BN, e % BN)] = r.b[i];
+        }
+    };
+    // Tensor cores: per 8-deep k step, the warp's block of C as m16n8k8 TF32
+    // MMAs. A float32 operand is split into a TF32 high part and the TF32
+    // rounding of its remainder, and the products hi*hi + hi*lo + lo*hi
+    // accumulate in float32, which keeps float32 accuracy; a BF16 operand is
+    // exact in TF32 (no low part, one MMA less).
+    auto multiply = [&](int buf) {
 #pragma unroll
         for (int kk = 0; kk < BK; kk += 8) {
             uint32_t ah[4], al[4];
-            {
-                const float av[4] = {As[buf][kk + tq][wm + g], As[buf][kk + tq][wm + g + 8],
-                                     As[buf][kk + tq + 4][wm + g], As[buf][kk + tq + 4][wm + g + 8]};
+            const float av[4] = {As[buf][ia(wm + g, kk + tq)], As[buf][ia(wm + g + 8, kk + tq)],
+                                 As[buf][ia(wm + g, kk + tq + 4)], As[buf][ia(wm + g + 8, kk + tq + 4)]};
 #pragma unroll
-                for (int i = 0; i < 4; ++i) split_tf32(av[i], ah[i], al[i]);
-            }
+            for (int i = 0; i < 4; ++i) split_tf32(av[i], ah[i], al[i]);
+uint32_t bh[TN][2], bl[TN][2];
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                const int nb = wn + nt * 8;
-                uint32_t bh[2], bl[2];
+            for (int nt = 0; nt < TN; ++nt) {
+                const float b0 = Bs[buf][ib(kk + tq, wn + nt * 8 + g)], b1 = Bs[buf][ib(kk + tq + 4, wn + nt * 8 + g)];
                 if (kBExact) {
-                    bh[0] = __float_as_uint(Bs[buf][kk + tq][nb + g]);
-                    bh[1] = __float_as_uint(Bs[buf][kk + tq + 4][nb + g]);
-                    mma_tf32(acc[nt], ah, bh);
-                    mma_tf32(acc[nt], al, bh);
+                    bh[nt][0] = __float_as_uint(b0);
+                    bh[nt][1] = __float_as_uint(b1);
                 } else {
-                    split_tf32(Bs[buf][kk + tq][nb + g], bh[0], bl[0]);
-                    split_tf32(Bs[buf][kk + tq + 4][nb + g], bh[1], bl[1]);
-                    mma_tf32(acc[nt], ah, bh);
-                    mma_tf32(acc[nt], ah, bl);
-                    mma_tf32(acc[nt], al, bh);
+                    split_tf32(b0, bh[nt][0], bl[nt][0]);
+                    split_tf32(b1, bh[nt][1], bl[nt][1]);
                 }
             }
+#pragma unroll
+            for (int nt = 0; nt < TN; ++nt) mma_tf32(acc[nt], ah, bh[nt]);
+            if (!kBExact) {
+#pragma unroll
+                for (int nt = 0; nt < TN; ++nt) mma_tf32(acc[nt], ah, bl[nt]);
+            }
+#pragma unroll
+            for (int nt = 0; nt < TN; ++nt) mma_tf32(acc[nt], al, bh[nt]);
         }
-        if (more) store(buf ^ 1);
+    };
+    Slice r0;
+    load(0, r0);
+    if constexpr (AHEAD == 1) {
+        store(0, r0);
         __syncthreads();
-        buf ^= 1;
+        int buf = 0;
+        for (int k0 = 0; k0 < K; k0 += BK) {
+            const bool more = k0 + BK < K;
+            if (more) load(k0 + BK, r0);  // in flight during the MMAs below
+            multiply(buf);
+            if (more) store(buf ^ 1, r0);
+            __syncthreads();
+            buf ^= 1;
+        }
+    } else {
+        // Slice s sits in shared memory buffer s & 1; s + 1 and s + 2 are in flight.
+        Slice r1;
+        load(BK, r1);
+        store(0, r0);
+        load(2 * BK, r0);
+        __syncthreads();
+        for (int k0 = 0; k0 < K; k0 += 2 * BK) {
+            multiply(0);
+            store(1, r1);  // zeros past K
+            load(k0 + 3 * BK, r1);
+            __syncthreads();
+            if (k0 + BK < K) multiply(1);
+            store(0, r0);
+            load(k0 + 4 * BK, r0);
+            __syncthreads();
+        }
     }
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
+    for (int nt = 0; nt < TN; ++nt) {
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
             const int gm = m0 + wm + g + (h >= 2 ? 8 : 0);
@@ -156,17 +203,33 @@ __global__ void __launch_bounds__(256) gemm_kernel(const TA *__restrict__ A, int
             float v = acc[nt][h];
             if (bias) v += bias[gn];
             if (relu) v = fmaxf(v, 0.f);
-            float *c = C + (size_t) gm * ldc + gn;
-            *c = accumulate ? *c + v : v;
+            const size_t at = (size_t) gm * ldc + gn;
+            if (mask && !(mask[at] > 0.f)) v = 0.f;
+            C[at] = v;
         }
     }
 }
 
+// Tiles: 64 x 64 with one slice ahead from 256 blocks on (the operands are read
+// least often and several blocks share an SM); else 64 x 32 with two slices ahead
+// from 128 blocks on; else 16 x 32. Measured (us; before: 64 x 64, conflicts in the
+// staging): 10,000 x 1,024 x 256 142 -> 130, 1,024 x 1,025 x 256 22.7 -> 20.5
+// (64 x 32: 26.7), 1,024 x 256 x 1,025 55 -> 24.6 (64 x 64: 45), 1,024 x 256 x 256
+// 16.5 -> 10.3, 256 x 1,025 x 1,024 49 -> 29 (64 x 64: 45), 256 x 256 x 1,024
+// 49 -> 18.5 (64 x 32: 28.7).
 template <typename TA, typename TB, bool AT, bool BT>
 cudaError_t gemm(const TA *A, int lda, const TB *B, int ldb, float *C, int ldc, int M, int N, int K,
-                 const float *bias, int relu, cudaStream_t s) {
-    dim3 grid((N + 63) / 64, (M + 63) / 64);
-    gemm_kernel<TA, TB, AT, BT><<<grid, 256, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K, bias, relu, 0);
+                 const float *bias, int relu, cudaStream_t s, const float *mask = nullptr) {
+    const uint32_t m64 = (M + 63) / 64, n64 = (N + 63) / 64, n32 = (N + 31) / 32;
+    if ((uint64_t) m64 * n64 >= 256)
+        gemm_kernel<TA, TB, AT, BT, 64, 64, 4, 2, 1><<<dim3(n64, m64), 256, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K, bias,
+                                                                                  relu, mask);
+    else if ((uint64_t) m64 * n32 >= 128)
+        gemm_kernel<TA, TB, AT, BT, 64, 32, 4, 2, 2><<<dim3(n32, m64), 256, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K, bias,
+                                                                                  relu, mask);
+    else
+        gemm_kernel<TA, TB, AT, BT, 16, 32, 1, 4, 2><<<dim3(n32, (M + 15) / 16), 128, 0, s>>>(A, lda, B, ldb, C, ldc, M, N,
+                                                                                            K, bias, relu, mask);
     return cudaGetLastError();
 }
 
@@ -230,26 +293,78 @@ __global__ void __launch_bounds__(256) loss_kernel(const float *__restrict__ Z, 
     }
 }
 
-__global__ void relu_bwd_kernel(float *__restrict__ dH, const float *__restrict__ H, size_t n) {
-    for (size_t i = blockIdx.x * (size_t) blockDim.x + threadIdx.x; i < n; i += (size_t) gridDim.x * blockDim.x)
-        if (!(H[i] > 0.f)) dH[i] = 0.f;
-}
-
-// db[n] = sum over the B rows of dY[., n], rows in order.
-__global__ void colsum_kernel(const float *__restrict__ dY, int B, int N, float *__restrict__ db) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
+// db[n] = sum over the B rows of dY[., n], rows in order: a chain of B additions
+// per column. 32 columns a block; 8 warps bring 128 rows at a time through
+// registers into shared memory while the first warp adds the 128 before (1,024
+// rows: 23 us with the loads in the chain, 4 us so; the chain itself is 2 us).
+__global__ void __launch_bounds__(256) colsum_kernel(const float *__restrict__ dY, int B, int N,
+                                                     float *__restrict__ db) {
+    constexpr int ROWS = 128, U = ROWS / 8;
+    __shared__ float t[2][ROWS][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, n = blockIdx.x * 32 + lane;
+    float r[U];
+    auto load = [&](int b0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int b = b0 + u * 8 + w;
+            r[u] = b < B && n < N ? __ldg(dY + (size_t) b * N + n) : 0.f;
+        }
+    };
+    auto store = [&](int buf) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) t[buf][u * 8 + w][lane] = r[u];
+    };
     float s = 0.f;
-    for (int b = 0; b < B; ++b) s += dY[(size_t) b * N + n];
-    db[n] = s;
+    load(0);
+    store(0);
+    __syncthreads();
+    int buf = 0;
+    for (int b0 = 0; b0 < B; b0 += ROWS) {
+        const bool more = b0 + ROWS < B;
+        if (more) load(b0 + ROWS);
+        if (w == 0) {
+            const int m = min(ROWS, B - b0);
+            if (m == ROWS) {
+#pragma unroll 32
+                for (int i = 0; i < ROWS; ++i) s += t[buf][i][lane];
+            } else {
+                for (int i = 0; i < m; ++i) s += t[buf][i][lane];
+            }
+        }
+        if (more) store(buf ^ 1);
+        __syncthreads();
+        buf ^= 1;
+    }
+    if (w == 0 && n < N) db[n] = s;
 }
 
-// Mean of the per-row losses, summed in row order by one thread.
-__global__ void loss_mean_kernel(const float *__restrict__ loss, int B, double *__restrict__ acc) {
+// Mean of every batch's per-row losses, each summed in row order by one thread
+// (block b: batch b; a chain of B float64 additions, 19 us at B = 1,024, so the
+// batches of an epoch go at once when it is over), and the batches' means added
+// up in order.
+__global__ void __launch_bounds__(32) loss_mean_kernel(const float *__restrict__ loss, int B,
+                                                       double *__restrict__ mean) {
+    const float *l = loss + (size_t) blockIdx.x * B;
+    double s = 0.0;
+    float v = (int) threadIdx.x < B ? l[threadIdx.x] : 0.f;
+    for (int b0 = 0; b0 < B; b0 += 32) {
+        const int i = b0 + 32 + (int) threadIdx.x;
+        const float nxt = i < B ? l[i] : 0.f;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const float x = __shfl_sync(0xffffffffu, v, j);
+            if (b0 + j < B) s += x;
+        }
+        v = nxt;
+    }
+    if (threadIdx.x == 0) mean[blockIdx.x] = s / B;
+}
+
+__global__ void loss_sum_kernel(const double *__restrict__ mean, int nb, double *__restrict__ acc) {
     if (threadIdx.x || blockIdx.x) return;
     double s = 0.0;
-    for (int b = 0; b < B; ++b) s += loss[b];
-    *acc += s / B;
+    for (int b = 0; b < nb; ++b) s += mean[b];
+    *acc = s;
 }
 
 __global__ void to_bf16_kernel(const float *__restrict__ w, __nv_bfloat16 *__restrict__ wb, size_t n) {
@@ -307,10 +422,10 @@ struct Trainer {
     Dev<float> w, g, m, v, H1, H2, Z, dZ, dH2, dH1, Xb, yb, loss;
     Dev<__nv_bfloat16> wb;
     Dev<uint16_t> cb;
-    Dev<double> acc;
+    Dev<double> acc, means;
     Trainer(uint32_t d_, uint32_t R_, uint32_t T_, uint32_t B_) : d(d_), R(R_), T(T_), B(B_), lay(d_, R_) {}
 
-    cudaError_t alloc(bool adam, cudaStream_t s) {
+    cudaError_t alloc(bool adam, uint32_t nb, cudaStream_t s) {  // nb: batches whose losses are kept
         cudaError_t e = cudaSuccess;
         const size_t P = lay.total;
         auto A = [&e, s](auto &buf, size_t n) {
@@ -331,7 +446,8 @@ struct Trainer {
         A(dH1, (size_t) B * kMlpH);
         A(Xb, (size_t) B * d);
         A(yb, B);
-        A(loss, B);
+        A(loss, (size_t) nb * B);
+        A(means, nb);
         A(cb, (size_t) B * T);
         A(acc, 1);
         return e;
@@ -350,47 +466,41 @@ struct Trainer {
         return e;
     }
 
-    // Loss (mean over the batch, added to acc) and gradient g of the batch in Xb, cb, yb.
-    cudaError_t loss_grad(float lam, cudaStream_t s) {
+    // Per-row losses (loss_rows, B) and gradient g of the batch in Xb, cb, yb.
+    cudaError_t loss_grad(float lam, float *loss_rows, cudaStream_t s) {
         const int H = kMlpH;
         cudaError_t e = forward(Xb.p, B, H1.p, H2.p, Z.p, s);
         if (e != cudaSuccess) return e;
-        loss_kernel<<<B, 256, R * sizeof(float), s>>>(Z.p, R, cb.p, T, yb.p, lam, 1.f / B, dZ.p, loss.p);
-        loss_mean_kernel<<<1, 32, 0, s>>>(loss.p, B, acc.p);
-        const int rb = (int) std::min<size_t>(((size_t) B * H + 255) / 256, 4096);
+        loss_kernel<<<B, 256, R * sizeof(float), s>>>(Z.p, R, cb.p, T, yb.p, lam, 1.f / B, dZ.p, loss_rows);
         e = cudaGetLastError();
+        auto colsum = [&](const float *dY, int N, float *db) {
+            if (e != cudaSuccess) return;
+            colsum_kernel<<<(N + 31) / 32, 256, 0, s>>>(dY, B, N, db);
+            e = cudaGetLastError();
+        };
         if (e == cudaSuccess)
             e = gemm<float, float, true, false>(H2.p, H, dZ.p, R + 1, g.p + lay.w3, R + 1, H, R + 1, B, nullptr, 0, s);
-        if (e == cudaSuccess) {
-            colsum_kernel<<<(R + 1 + 255) / 256, 256, 0, s>>>(dZ.p, B, R + 1, g.p + lay.b3);
-            e = cudaGetLastError();
-        }
+        colsum(dZ.p, R + 1, g.p + lay.b3);
         if (e == cudaSuccess)
             e = gemm<float, __nv_bfloat16, false, true>(dZ.p, R + 1, wb.p + lay.w3, R + 1, dH2.p, H, B, H, R + 1,
-                                                        nullptr, 0, s);
-        if (e == cudaSuccess) {
-            relu_bwd_kernel<<<rb, 256, 0, s>>>(dH2.p, H2.p, (size_t) B * H);
-            e = cudaGetLastError();
-        }
+                                                        nullptr, 0, s, H2.p);
         if (e == cudaSuccess)
             e = gemm<float, float, true, false>(H1.p, H, dH2.p, H, g.p + lay.w2, H, H, H, B, nullptr, 0, s);
-        if (e == cudaSuccess) {
-            colsum_kernel<<<1, 256, 0, s>>>(dH2.p, B, H, g.p + lay.b2);
-            e = cudaGetLastError();
-        }
+        colsum(dH2.p, H, g.p + lay.b2);
         if (e == cudaSuccess)
-            e = gemm<float, __nv_bfloat16, false, true>(dH2.p, H, wb.p + lay.w2, H, dH1.p, H, B, H, H, nullptr, 0, s);
-        if (e == cudaSuccess) {
-            relu_bwd_kernel<<<rb, 256, 0, s>>>(dH1.p, H1.p, (size_t) B * H);
-            e = cudaGetLastError();
-        }
+            e = gemm<float, __nv_bfloat16, false, true>(dH2.p, H, wb.p + lay.w2, H, dH1.p, H, B, H, H, nullptr, 0, s,
+                                                        H1.p);
         if (e == cudaSuccess)
             e = gemm<float, float, true, false>(Xb.p, d, dH1.p, H, g.p + lay.w1, H, d, H, B, nullptr, 0, s);
-        if (e == cudaSuccess) {
-            colsum_kernel<<<1, 256, 0, s>>>(dH1.p, B, H, g.p + lay.b1);
-            e = cudaGetLastError();
-        }
+        colsum(dH1.p, H, g.p + lay.b1);
         return e;
+    }
+
+    // acc = the sum over nb batches of their mean losses (loss: nb x B).
+    cudaError_t sum_losses(uint32_t nb, cudaStream_t s) {
+        loss_mean_kernel<<<nb, 32, 0, s>>>(loss.p, (int) B, means.p);
+        loss_sum_kernel<<<1, 32, 0, s>>>(means.p, (int) nb, acc.p);
+        return cudaGetLastError();
     }
 };
 
@@ -909,16 +1019,16 @@ int panns_mlp_loss_grad(int device, uint32_t d, uint32_t R, uint32_t T, const fl
         ~StreamGuard() { cudaStreamDestroy(s); }
     } guard{s};
     Trainer t(d, R, T, B);
-    LCU(t.alloc(false, s));
+    LCU(t.alloc(false, 1, s));
     const size_t P = t.lay.total;
     LCU(cudaMemcpyAsync(t.w.p, params, P * 4, cudaMemcpyHostToDevice, s));
     LCU(cudaMemcpyAsync(t.Xb.p, X, (size_t) B * d * 4, cudaMemcpyHostToDevice, s));
     LCU(cudaMemcpyAsync(t.cb.p, cells, (size_t) B * T * 2, cudaMemcpyHostToDevice, s));
     LCU(cudaMemcpyAsync(t.yb.p, y, (size_t) B * 4, cudaMemcpyHostToDevice, s));
-    LCU(cudaMemsetAsync(t.acc.p, 0, 8, s));
     to_bf16_kernel<<<256, 256, 0, s>>>(t.w.p, t.wb.p, P);
     LCU(cudaGetLastError());
-    LCU(t.loss_grad(lambda_L, s));
+    LCU(t.loss_grad(lambda_L, t.loss.p, s));
+    LCU(t.sum_losses(1, s));
     LCU(cudaMemcpyAsync(grad, t.g.p, P * 4, cudaMemcpyDeviceToHost, s));
     LCU(cudaMemcpyAsync(loss, t.acc.p, 8, cudaMemcpyDeviceToHost, s));
     LCU(cudaStreamSynchronize(s));
@@ -940,7 +1050,7 @@ int panns_mlp_forward(int device, uint32_t d, uint32_t R, const float *params, c
     } guard{s};
     const uint32_t B = std::min<uint32_t>(n, 8192);
     Trainer t(d, R, 1, B);
-    LCU(t.alloc(false, s));
+    LCU(t.alloc(false, 1, s));
     const size_t P = t.lay.total;
     LCU(cudaMemcpyAsync(t.w.p, params, P * 4, cudaMemcpyHostToDevice, s));
     to_bf16_kernel<<<256, 256, 0, s>>>(t.w.p, t.wb.p, P);
@@ -975,7 +1085,7 @@ int panns_mlp_train(int device, const panns_mlp_train_params *tp, const float *X
         ~StreamGuard() { cudaStreamDestroy(s); }
     } guard{s};
     Trainer t(d, R, T, B);
-    LCU(t.alloc(true, s));
+    LCU(t.alloc(true, n / B, s));
     const size_t P = t.lay.total;
     Dev<float> dX, dy;
     Dev<uint16_t> dc;
@@ -1001,12 +1111,11 @@ int panns_mlp_train(int device, const panns_mlp_train_params *tp, const float *X
         std::iota(order.begin(), order.end(), 0u);
         for (uint32_t i = n - 1; i > 0; --i) std::swap(order[i], order[rng() % (i + 1)]);
         LCU(cudaMemcpyAsync(didx.p, order.data(), (size_t) n * 4, cudaMemcpyHostToDevice, s));
-        LCU(cudaMemsetAsync(t.acc.p, 0, 8, s));
         for (uint32_t b = 0; b < nb; ++b) {
             gather_batch_kernel<<<B, 128, 0, s>>>(dX.p, d, dc.p, T, dy.p, didx.p + (size_t) b * B, B, t.Xb.p, t.cb.p,
                                                   t.yb.p);
             LCU(cudaGetLastError());
-            LCU(t.loss_grad(tp->lambda_L, s));
+            LCU(t.loss_grad(tp->lambda_L, t.loss.p + (size_t) b * B, s));
             ++step;
             c1p *= tp->beta1;
             c2p *= tp->beta2;
@@ -1014,6 +1123,7 @@ int panns_mlp_train(int device, const panns_mlp_train_params *tp, const float *X
                                             tp->weight_decay, (float) (1.0 - c1p), (float) (1.0 - c2p), t.wb.p);
             LCU(cudaGetLastError());
         }
+        LCU(t.sum_losses(nb, s));
         // The order vector is rewritten next epoch: wait for its copy.
         double l = 0.0;
         LCU(cudaMemcpyAsync(&l, t.acc.p, 8, cudaMemcpyDeviceToHost, s));

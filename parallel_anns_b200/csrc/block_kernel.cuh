@@ -46,6 +46,7 @@ __host__ __device__ inline uint32_t block_smem_bytes(uint32_t queue_cap, uint32_
            + W * buf * 12u                    // survivors of a round (dist, id, key)
            + block_rank_max(W) * 12u          // ranked survivors (dist, id, place)
            + W * kMaxM * 8u                   // per-warp picked candidates (id, place) / learned entries
+           + W * 1024u                        // per-warp distance chains
            + kBlockCtl * 4u                   // control words
            + vis_smem * 4u;                   // visited bitset, where it fits
 }
@@ -341,7 +342,8 @@ __device__ void block_search_one(const SearchArgs &a, uint32_t q, uint8_t *smem,
     m.sP = m.sI + block_rank_max(W);
     uint32_t *cand = m.sP + block_rank_max(W) + w * 2 * kMaxM;
     uint32_t *cpos = cand + kMaxM;  // the candidates' places in the queue
-    m.ctl = m.sP + block_rank_max(W) + W * 2 * kMaxM;
+    float *tmp = reinterpret_cast<float *>(m.sP + block_rank_max(W) + W * 2 * kMaxM) + w * 256;
+    m.ctl = m.sP + block_rank_max(W) + W * 2 * kMaxM + W * 256;
     uint32_t *ctl = m.ctl;
     uint32_t *svis = ctl + kBlockCtl;
     const bool in_smem = a.vis_smem != 0;
@@ -386,10 +388,10 @@ __device__ void block_search_one(const SearchArgs &a, uint32_t q, uint8_t *smem,
             if constexpr (STORE == STORE_FP32) {
                 // 16 rows a pass; eight or fewer left over in a pass of eight
                 const uint32_t wide = (nb & 15u) > 8u ? nb : nb & ~15u;
-                if (wide) distances_wide<KIND, CL>(a, D.qv, bi, bd, wide, lane);
-                if (wide < nb) D.distances(a, bi + wide, bd + wide, nb - wide, lane);
+                if (wide) distances_wide<KIND, CL>(a, D.qv, bi, bd, wide, lane, tmp);
+                if (wide < nb) D.distances(a, bi + wide, bd + wide, nb - wide, lane, tmp);
             } else {
-                D.distances(a, bi, bd, nb, lane);
+                D.distances(a, bi, bd, nb, lane, tmp);
             }
         }
         n_dist += nb;
@@ -577,7 +579,7 @@ __device__ void block_search_one(const SearchArgs &a, uint32_t q, uint8_t *smem,
         E.load(a, q, lane);
         const uint32_t per = ((sz + W - 1) / W + 7) & ~7u;
         const uint32_t lo = min(sz, w * per), hi = min(sz, lo + per);
-        E.distances(a, m.qi + lo, m.qd + lo, hi - lo, lane);
+        E.distances(a, m.qi + lo, m.qd + lo, hi - lo, lane, tmp);
         __syncthreads();
         if (sz <= W * buf) {
             for (uint32_t i = tid; i < sz; i += T) {

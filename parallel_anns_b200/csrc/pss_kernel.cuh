@@ -54,20 +54,8 @@ struct PssMem {
 // L-th distance, sort, merge into (qd, qi) of size *sz and capacity cap.
 template <int KIND, int CL>
 __device__ uint32_t pss_flush(const SearchArgs &a, const PssMem &m, uint32_t nb, float *qd, uint32_t *qi,
-                              uint32_t *sz, uint32_t cap, const float4 (&qv)[CL], int lane) {
-    const int g = lane >> 3;
-    for (uint32_t b0 = 0; b0 < nb; b0 += 8) {
-        const uint32_t b = b0 + g, bb = b0 + 4 + g;
-        const bool act0 = b < nb, act1 = bb < nb;
-        const uint32_t v0 = act0 ? m.bi[b] : 0u, v1 = act1 ? m.bi[bb] : 0u;
-        float d0, d1;
-        group_distance2<KIND, CL>(a.vec, a.norms, v0, act0, v1, act1, qv, lane, d0, d1);
-        if ((lane & 7) == 0) {
-            if (act0) m.bd[b] = d0;
-            if (act1) m.bd[bb] = d1;
-        }
-    }
-    __syncwarp();
+                              uint32_t *sz, uint32_t cap, const Dist<KIND, CL, STORE_FP32> &D, int lane) {
+    D.distances(a, m.bi, m.bd, nb, lane, reinterpret_cast<float *>(m.bk));
     const float bound = m.md[a.L - 1];
     uint32_t cnt = 0;
     for (uint32_t b0 = 0; b0 < nb; b0 += 32) {
@@ -86,12 +74,14 @@ __device__ uint32_t pss_flush(const SearchArgs &a, const PssMem &m, uint32_t nb,
             const uint32_t pos = cnt + __popc(bm & lanemask_lt());
             m.bd[pos] = d;
             m.bi[pos] = id;
-            m.bk[pos] = __ldg(a.orig + id);
         }
         cnt += __popc(bm);
         __syncwarp();
     }
     if (cnt == 0) return cap;
+    if (cnt <= 32) return rank_merge32<ORDER_PANNS>(qd, qi, sz, cap, m.bd, m.bi, cnt, a.orig, lane);
+    for (uint32_t b = lane; b < cnt; b += 32) m.bk[b] = __ldg(a.orig + m.bi[b]);
+    __syncwarp();
     warp_sort<ORDER_PANNS>(m.bd, m.bi, m.bk, cnt, a.orig, lane);
     return merge_into<ORDER_PANNS>(qd, qi, sz, cap, m.bd, m.bi, m.bk, cnt, a.orig, lane);
 }
@@ -103,7 +93,7 @@ template <int KIND, int CL>
 __device__ uint32_t pss_expand(const SearchArgs &a, const PssMem &m, uint32_t v, float *qd, uint32_t *qi,
                                uint32_t *sz, uint32_t cap, uint32_t *vis, uint32_t *dirty,
                                uint32_t &dcount, uint32_t &n_dist, uint32_t &n_edges,
-                               const float4 (&qv)[CL], int lane) {
+                               const Dist<KIND, CL, STORE_FP32> &D, int lane) {
     const uint32_t hw = __ldg(a.head + (size_t) v * kHeadWords + lane);
     const uint32_t deg = __shfl_sync(kFull, hw, 0);
     n_edges += 1 + deg;
@@ -126,7 +116,7 @@ __device__ uint32_t pss_expand(const SearchArgs &a, const PssMem &m, uint32_t v,
         note_dirty(dirty, a.dirty_cap, dcount, valid && old == 0, id >> 5);
         if (nb + 32 > kBuf) {
             n_dist += nb;
-            nk = min(nk, pss_flush<KIND, CL>(a, m, nb, qd, qi, sz, cap, qv, lane));
+            nk = min(nk, pss_flush<KIND, CL>(a, m, nb, qd, qi, sz, cap, D, lane));
             nb = 0;
         }
         const uint32_t bm = __ballot_sync(kFull, fresh);
@@ -136,7 +126,7 @@ __device__ uint32_t pss_expand(const SearchArgs &a, const PssMem &m, uint32_t v,
     }
     if (nb) {
         n_dist += nb;
-        nk = min(nk, pss_flush<KIND, CL>(a, m, nb, qd, qi, sz, cap, qv, lane));
+        nk = min(nk, pss_flush<KIND, CL>(a, m, nb, qd, qi, sz, cap, D, lane));
     }
     return nk;
 }
@@ -208,12 +198,8 @@ __device__ void pss_one(const PssArgs &pa, const PssMem &m, uint32_t q, uint32_t
                         int lane) {
     const SearchArgs &a = pa.s;
     const uint32_t L = a.L, T = pa.T, Ll = pa.L_local, X = pa.X, wcap = pa.wcap;
-    float4 qv[CL];
-    {
-        const float4 *qrow = a.queries + (size_t) q * (CL * 8);
-#pragma unroll
-        for (int i = 0; i < CL; ++i) qv[i] = __ldg(qrow + 8 * i + (lane & 7));
-    }
+    Dist<KIND, CL, STORE_FP32> D;
+    D.load(a, q, lane);
     uint32_t dcount = 0, n_dist = 0, n_expand = 0, n_edges = 0, n_iter = 0;
     // Initial master queue (initialize_set_L_para :897-935).
     uint32_t msz = 0;
@@ -233,19 +219,7 @@ __device__ void pss_one(const PssArgs &pa, const PssMem &m, uint32_t q, uint32_t
             __syncwarp();
             if (nb > kBuf - 32 || i0 + 32 >= L) {
                 // no bound yet: distances, sort, merge
-                const int g = lane >> 3;
-                for (uint32_t b0 = 0; b0 < nb; b0 += 8) {
-                    const uint32_t b = b0 + g, bb = b0 + 4 + g;
-                    const bool act0 = b < nb, act1 = bb < nb;
-                    float d0, d1;
-                    group_distance2<KIND, CL>(a.vec, a.norms, act0 ? m.bi[b] : 0u, act0,
-                                              act1 ? m.bi[bb] : 0u, act1, qv, lane, d0, d1);
-                    if ((lane & 7) == 0) {
-                        if (act0) m.bd[b] = d0;
-                        if (act1) m.bd[bb] = d1;
-                    }
-                }
-                __syncwarp();
+                D.distances(a, m.bi, m.bd, nb, lane, reinterpret_cast<float *>(m.bk));
                 for (uint32_t b = lane; b < nb; b += 32) m.bk[b] = __ldg(a.orig + m.bi[b]);
                 __syncwarp();
                 warp_sort<ORDER_PANNS>(m.bd, m.bi, m.bk, nb, a.orig, lane);
@@ -265,7 +239,7 @@ __device__ void pss_one(const PssArgs &pa, const PssMem &m, uint32_t q, uint32_t
             if (lane == 0) m.mi[0] = v | kChecked;
             __syncwarp();
             ++n_expand;
-            r = pss_expand<KIND, CL>(a, m, v, m.md, m.mi, &msz, L, vis, dirty, dcount, n_dist, n_edges, qv, lane);
+            r = pss_expand<KIND, CL>(a, m, v, m.md, m.mi, &msz, L, vis, dirty, dcount, n_dist, n_edges, D, lane);
         }
         k_master = r <= k_master ? r : k_master + 1;
     }
@@ -325,7 +299,7 @@ __device__ void pss_one(const PssArgs &pa, const PssMem &m, uint32_t q, uint32_t
                 __syncwarp();
                 ++n_expand;
                 const uint32_t r = pss_expand<KIND, CL>(a, m, v & kIdMask, qd, qi, &size, cap, vis, dirty,
-                                                        dcount, n_dist, n_edges, qv, lane);
+                                                        dcount, n_dist, n_edges, D, lane);
                 if (master) msz = size;
                 __syncwarp();
                 if (lane == 0) {

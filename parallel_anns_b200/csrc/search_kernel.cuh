@@ -60,9 +60,6 @@ constexpr int kHeadNbrs = kHeadWords - 1;
 #ifndef PANNS_KBUF
 #define PANNS_KBUF 256
 #endif
-#ifndef PANNS_WIDE_DIST
-#define PANNS_WIDE_DIST 0  // 1: 16 rows in flight per warp pass in the one-warp kernel too
-#endif
 #ifndef PANNS_FP8_MIXED
 #define PANNS_FP8_MIXED 1  // FP8 rows times a half-precision query by mixed-precision FMAs
 #endif
@@ -76,6 +73,8 @@ constexpr int kCandGroup = 8;    // candidates whose head rows are loaded at onc
 constexpr int kGroupChunks = (kCandGroup * kHeadNbrs + 31) / 32;
 // A group's head-row neighbours go into the fresh buffer without a flush in between.
 static_assert(kCandGroup * kHeadNbrs <= kBuf, "kBuf must hold a group's head-row neighbours");
+// The key buffer doubles as the distance pass's scratch (32 vertices x 8 chains).
+static_assert(kBuf >= 256, "the distance pass needs 256 words of scratch");
 constexpr int kOvfChunks = 2;    // overflow neighbours per batch of loads: kOvfChunks * 32
 constexpr int kMaxM = 64;
 
@@ -158,10 +157,9 @@ static __device__ __forceinline__ uint32_t lanemask_lt() {
 }
 
 // ---------------------------------------------------------------------------
-// Distances of two vertices per 8-lane group (c = lane & 7 is the lane
-// accumulator this thread owns): both rows are loaded before either is used.
-// Lane sum: ((u0 + u1) + u2) + ... + u7; norm trick: -2 * dot + norm, which
-// is one rounding either way because -2 * dot is exact.
+// Distances with 8 lanes per vertex: lane c of a group runs lane accumulator c's
+// chain of the reference. Lane sum: ((u0 + u1) + u2) + ... + u7; norm trick: -2 *
+// dot + norm, which is one rounding either way because -2 * dot is exact.
 // ---------------------------------------------------------------------------
 template <int KIND, int CL>
 __device__ __forceinline__ float chain(const float4 (&x)[CL], const float4 (&qv)[CL]) {
@@ -184,42 +182,18 @@ __device__ __forceinline__ float chain(const float4 (&x)[CL], const float4 (&qv)
     return acc;
 }
 
-static __device__ __forceinline__ float lane_sum8(float acc, int lane) {
-    const int base = lane & ~7;
-    float s = __shfl_sync(kFull, acc, base);
-#pragma unroll
-    for (int j = 1; j < 8; ++j) s = __fadd_rn(s, __shfl_sync(kFull, acc, base + j));
-    return s;
-}
-
-template <int KIND, int CL>
-__device__ __forceinline__ void group_distance2(const float4 *__restrict__ vec,
-                                                const float *__restrict__ norms, uint32_t v0,
-                                                bool a0, uint32_t v1, bool a1,
-                                                const float4 (&qv)[CL], int lane, float &d0,
-                                                float &d1) {
-    const int c = lane & 7;
-    float4 x0[CL], x1[CL];
-    float n0 = 0.f, n1 = 0.f;
-    const float4 *r0 = vec + (size_t) v0 * (CL * 8) + c;
-    const float4 *r1 = vec + (size_t) v1 * (CL * 8) + c;
-#pragma unroll
-    for (int i = 0; i < CL; ++i) {
-        x0[i] = a0 ? __ldg(r0 + 8 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
-        x1[i] = a1 ? __ldg(r1 + 8 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    if (KIND == KIND_IP) {
-        n0 = a0 ? __ldg(norms + v0) : 0.f;
-        n1 = a1 ? __ldg(norms + v1) : 0.f;
-    }
-    float s0 = lane_sum8(chain<KIND, CL>(x0, qv), lane);
-    float s1 = lane_sum8(chain<KIND, CL>(x1, qv), lane);
-    if (KIND == KIND_IP) {
-        s0 = __fmaf_rn(-2.0f, s0, n0);
-        s1 = __fmaf_rn(-2.0f, s1, n1);
-    }
-    d0 = s0;
-    d1 = s1;
+// The lane sum of a vertex's eight chains (tmp, 16-byte aligned) and the norm trick.
+template <int KIND>
+__device__ __forceinline__ float finish_sum(const float *tmp, float norm) {
+    const float4 x = *reinterpret_cast<const float4 *>(tmp), y = *reinterpret_cast<const float4 *>(tmp + 4);
+    float s = __fadd_rn(x.x, x.y);
+    s = __fadd_rn(s, x.z);
+    s = __fadd_rn(s, x.w);
+    s = __fadd_rn(s, y.x);
+    s = __fadd_rn(s, y.y);
+    s = __fadd_rn(s, y.z);
+    s = __fadd_rn(s, y.w);
+    return KIND == KIND_IP ? __fmaf_rn(-2.0f, s, norm) : s;
 }
 
 // (dist, key) order. PANNS: key is a device id and equal distances compare
@@ -409,6 +383,86 @@ __device__ __forceinline__ uint32_t warp_merge(const WarpMem &m, uint32_t *sz, u
     return merge_into<ORDER>(m.qd, m.qi, sz, L, m.bd, m.bi, m.bk, cnt, orig, lane);
 }
 
+// Sort and merge for up to 32 fresh elements (bd, bi)[0..cnt), in arrival order,
+// one per lane: the usual case (27 survivors a step at L = 384, M = 8). An
+// element's rank among them is the number of smaller distances (where two are
+// equal, PANNS order decides by original id, EFANNA order by arrival); its
+// merged position is its rank plus its rank in the queue. The queue is then
+// filled from the top in windows of 32 positions: the fresh positions of a
+// window are one word (a reduction over the lanes), every other position takes
+// the queue element as many places down as there are fresh positions below it.
+// Against warp_sort and merge_into, which compare keys pairwise and search the
+// fresh list once per moved element, this executes about a quarter fewer
+// instructions per step. bd has room for three entries past cnt. Returns as
+// merge_into.
+template <int ORDER>
+__device__ __forceinline__ uint32_t rank_merge32(float *qd, uint32_t *qi, uint32_t *sz, uint32_t cap, float *bd,
+                                                 const uint32_t *bi, uint32_t cnt, const uint32_t *__restrict__ orig,
+                                                 int lane) {
+    const uint32_t qsz = *sz;
+    const bool have = (uint32_t) lane < cnt;
+    const float d = have ? bd[lane] : 0.f;
+    const uint32_t id = have ? bi[lane] : 0u;
+    if (lane < 3) bd[cnt + lane] = __int_as_float(0x7f800000);
+    __syncwarp();
+    uint32_t less = 0, upto = 0;
+    for (uint32_t s = 0; s < cnt; s += 4) {
+        const float4 x = *reinterpret_cast<const float4 *>(bd + s);
+        less += x.x < d ? 1u : 0u;
+        upto += x.x <= d ? 1u : 0u;
+        less += x.y < d ? 1u : 0u;
+        upto += x.y <= d ? 1u : 0u;
+        less += x.z < d ? 1u : 0u;
+        upto += x.z <= d ? 1u : 0u;
+        less += x.w < d ? 1u : 0u;
+        upto += x.w <= d ? 1u : 0u;
+    }
+    uint32_t r = less;
+    if (__any_sync(kFull, have && upto != less + 1)) {
+        // Equal distances, infinities or NaN: by (distance, key) as integers, a total order.
+        const uint32_t b = __float_as_uint(d + 0.0f);
+        const uint32_t kd = have ? (b & 0x80000000u ? ~b : b | 0x80000000u) : kFull;
+        const uint32_t ko = !have ? kFull : ORDER == ORDER_PANNS ? __ldg(orig + (id & kIdMask)) : (uint32_t) lane;
+        r = 0;
+        for (uint32_t s = 0; s < cnt; ++s) {
+            const uint32_t fd = __shfl_sync(kFull, kd, s), fo = __shfl_sync(kFull, ko, s);
+            r += fd < kd || (fd == kd && fo < ko) ? 1u : 0u;
+        }
+    }
+    const uint32_t np = have ? r + queue_rank<ORDER>(qd, qi, qsz, d, id & kIdMask, orig) : kFull;
+    const uint32_t p0 = __reduce_min_sync(kFull, np);
+    if (p0 >= cap) return cap;
+    const uint32_t nsz = min(cap, qsz + cnt);
+    // Windows from the top; a window's reads come before its writes, and the
+    // windows below read below what it writes.
+    for (int32_t c = (int32_t) ((nsz - 1) >> 5); c >= (int32_t) (p0 >> 5); --c) {
+        const uint32_t lo = (uint32_t) c << 5, p = lo + lane;
+        const uint32_t word = __reduce_or_sync(kFull, (np >> 5) == (uint32_t) c ? 1u << (np & 31) : 0u);
+        const uint32_t below = __popc(__ballot_sync(kFull, np < lo));
+        const bool move = p < nsz && p >= p0 && !((word >> lane) & 1u);
+        const uint32_t j = p - below - __popc(word & lanemask_lt());
+        float md = 0.f;
+        uint32_t mi = 0;
+        if (move) {
+            md = qd[j];
+            mi = qi[j];
+        }
+        __syncwarp();
+        if (move) {
+            qd[p] = md;
+            qi[p] = mi;
+        }
+    }
+    __syncwarp();
+    if (np < cap) {
+        qd[np] = d;
+        qi[np] = id;
+    }
+    __syncwarp();
+    *sz = nsz;
+    return p0;
+}
+
 // Visited bitset: test-and-set returns the previous word.
 static __device__ __forceinline__ uint32_t visit_issue(uint32_t *vis, uint32_t id, bool valid) {
     return valid ? atomicOr(vis + (id >> 5), 1u << (id & 31)) : kFull;
@@ -442,58 +496,65 @@ struct Dist<KIND, CL, STORE_FP32> {
 #pragma unroll
         for (int i = 0; i < CL; ++i) qv[i] = __ldg(qrow + 8 * i + (lane & 7));
     }
-    __device__ __forceinline__ void distances(const SearchArgs &a, const uint32_t *ids, float *out,
-                                              uint32_t nb, int lane) const {
-        const int g = lane >> 3;
-        // 8 vertices per round (2 per 8-lane group, loads issued together).
-        for (uint32_t b0 = 0; b0 < nb; b0 += 8) {
-            const uint32_t b = b0 + g, bb = b0 + 4 + g;
-            const bool act0 = b < nb, act1 = bb < nb;
-            const uint32_t v0 = act0 ? ids[b] & kIdMask : 0u, v1 = act1 ? ids[bb] & kIdMask : 0u;
-            float d0, d1;
-            group_distance2<KIND, CL>(a.vec, a.norms, v0, act0, v1, act1, qv, lane, d0, d1);
-            if ((lane & 7) == 0) {
-                if (act0) out[b] = d0;
-                if (act1) out[bb] = d1;
+    // 32 vertices at a time, 8 rows in flight (2 per 8-lane group). The lanes
+    // leave their chains in tmp (256 floats), then lane i adds the eight of vertex
+    // i in order: a store per lane and vertex and one sum per 32 vertices, where
+    // shuffling the sum together on every lane took as many instructions as
+    // the rest of the pass.
+    __device__ __forceinline__ void distances(const SearchArgs &a, const uint32_t *ids, float *out, uint32_t nb,
+                                              int lane, float *tmp) const {
+        const uint32_t g = lane >> 3, c = lane & 7;
+        for (uint32_t b0 = 0; b0 < nb; b0 += 32) {
+            const uint32_t m = min(32u, nb - b0);
+            const bool have = (uint32_t) lane < m;
+            const uint32_t mine = have ? ids[b0 + lane] & kIdMask : 0u;
+            const float nrm = KIND == KIND_IP && have ? __ldg(a.norms + mine) : 0.f;
+            for (uint32_t p = 0; p < m; p += 8) {
+                const bool a0 = p + g < m, a1 = p + 4 + g < m;
+                const float4 *r0 = a.vec + (size_t) __shfl_sync(kFull, mine, p + g) * (CL * 8) + c;
+                const float4 *r1 = a.vec + (size_t) __shfl_sync(kFull, mine, p + 4 + g) * (CL * 8) + c;
+                float4 x0[CL], x1[CL];
+#pragma unroll
+                for (int i = 0; i < CL; ++i) {
+                    x0[i] = a0 ? __ldg(r0 + 8 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    x1[i] = a1 ? __ldg(r1 + 8 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+                tmp[p * 8 + lane] = chain<KIND, CL>(x0, qv);
+                tmp[p * 8 + 32 + lane] = chain<KIND, CL>(x1, qv);
             }
+            __syncwarp();
+            if (have) out[b0 + lane] = finish_sum<KIND>(tmp + lane * 8, nrm);
+            __syncwarp();
         }
-        __syncwarp();
     }
 };
 
 // Four vertices per 8-lane group (16 per warp pass), all rows loaded before
-// any is used: the same per-vertex arithmetic as group_distance2, with twice
-// the loads in flight, for kernels with registers to spare.
+// any is used: the same per-vertex arithmetic with twice the loads in flight,
+// for kernels with registers to spare. tmp: 128 floats.
 template <int KIND, int CL>
 __device__ __forceinline__ void distances_wide(const SearchArgs &a, const float4 (&qv)[CL], const uint32_t *ids,
-                                               float *out, uint32_t nb, int lane) {
-    const int g = lane >> 3, c = lane & 7;
+                                               float *out, uint32_t nb, int lane, float *tmp) {
+    const uint32_t g = lane >> 3, c = lane & 7;
     for (uint32_t b0 = 0; b0 < nb; b0 += 16) {
-        uint32_t v[4];
-        bool act[4];
+        const uint32_t m = min(16u, nb - b0);
+        const bool have = (uint32_t) lane < m;
+        const uint32_t mine = have ? ids[b0 + lane] & kIdMask : 0u;
+        const float nrm = KIND == KIND_IP && have ? __ldg(a.norms + mine) : 0.f;
         float4 x[4][CL];
-        float nrm[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const uint32_t b = b0 + 4 * u + g;
-            act[u] = b < nb;
-            v[u] = act[u] ? ids[b] & kIdMask : 0u;
+            const float4 *r = a.vec + (size_t) __shfl_sync(kFull, mine, 4 * u + g) * (CL * 8) + c;
+            const bool act = 4 * u + g < m;
+#pragma unroll
+            for (int i = 0; i < CL; ++i) x[u][i] = act ? __ldg(r + 8 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const float4 *r = a.vec + (size_t) v[u] * (CL * 8) + c;
-#pragma unroll
-            for (int i = 0; i < CL; ++i) x[u][i] = act[u] ? __ldg(r + 8 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
-            nrm[u] = (KIND == KIND_IP && act[u]) ? __ldg(a.norms + v[u]) : 0.f;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            float s = lane_sum8(chain<KIND, CL>(x[u], qv), lane);
-            if (KIND == KIND_IP) s = __fmaf_rn(-2.0f, s, nrm[u]);
-            if (c == 0 && act[u]) out[b0 + 4 * u + g] = s;
-        }
+        for (int u = 0; u < 4; ++u) tmp[32 * u + lane] = chain<KIND, CL>(x[u], qv);
+        __syncwarp();
+        if (have) out[b0 + lane] = finish_sum<KIND>(tmp + lane * 8, nrm);
+        __syncwarp();
     }
-    __syncwarp();
 }
 
 // Position of natural element e in a chain-major padded row (inverse of the
@@ -618,8 +679,8 @@ struct Dist {
         }
         return acc;
     }
-    __device__ __forceinline__ void distances(const SearchArgs &a, const uint32_t *ids, float *out,
-                                              uint32_t nb, int lane) const {
+    __device__ __forceinline__ void distances(const SearchArgs &a, const uint32_t *ids, float *out, uint32_t nb,
+                                              int lane, float *) const {
         const int g = lane >> 2, t = lane & 3;
         // 16 vertices per round (2 per 4-lane group, loads issued together).
         for (uint32_t b0 = 0; b0 < nb; b0 += 16) {
@@ -738,12 +799,7 @@ template <int KIND, int ORDER, int CL, int STORE>
 __device__ uint32_t flush(const SearchArgs &a, const WarpMem &m, uint32_t nb, uint32_t *sz, uint32_t L,
                           bool filter, const Dist<KIND, CL, STORE> &D, int lane) {
     constexpr bool kLazyKeys = ORDER == ORDER_PANNS && STORE != STORE_FP8;
-#if PANNS_WIDE_DIST
-    if constexpr (STORE == STORE_FP32) distances_wide<KIND, CL>(a, D.qv, m.bi, m.bd, nb, lane);
-    else D.distances(a, m.bi, m.bd, nb, lane);
-#else
-    D.distances(a, m.bi, m.bd, nb, lane);
-#endif
+    D.distances(a, m.bi, m.bd, nb, lane, reinterpret_cast<float *>(m.bk));
     // Keep the survivors, in arrival order.
     const float bound = (filter && *sz >= L) ? m.qd[L - 1] : __int_as_float(0x7f800000);
     const bool any_bound = filter && *sz >= L;
@@ -770,6 +826,7 @@ __device__ uint32_t flush(const SearchArgs &a, const WarpMem &m, uint32_t nb, ui
         __syncwarp();
     }
     if (cnt == 0) return L;
+    if (cnt <= 32) return rank_merge32<ORDER>(m.qd, m.qi, sz, L, m.bd, m.bi, cnt, a.orig, lane);
     // With lazy keys the survivors are sorted by (distance, device id); PANNS
     // order breaks equal distances by original id, so if the sorted
     // survivors hold equal distances (rare) they are sorted once more with
@@ -855,17 +912,15 @@ __device__ void search_one(const SearchArgs &a, const WarpMem &m, uint32_t q, ui
             const uint32_t bm = __ballot_sync(kFull, un);
             const uint32_t take = min((uint32_t) __popc(bm), M - cnt);
             const uint32_t r = __popc(bm & lanemask_lt());
-            if (un && r < take) {
+            const bool mine = un && r < take;
+            if (mine) {
                 const uint32_t id = m.qi[p];
                 m.qi[p] = id | kChecked;
                 m.cand[cnt + r] = id;
             }
-            if (take) {
-                // position of the take-th unchecked slot in this window
-                uint32_t x = bm;
-                for (uint32_t t = 1; t < take; ++t) x &= x - 1;
-                last_k = p0 + (__ffs(x) - 1);
-            }
+            // position of the take-th unchecked slot in this window
+            const uint32_t taken = __ballot_sync(kFull, mine);
+            if (taken) last_k = p0 + 31 - __clz(taken);
             cnt += take;
             __syncwarp();
         }
@@ -1000,7 +1055,7 @@ __device__ void search_one(const SearchArgs &a, const WarpMem &m, uint32_t q, ui
         // order); the K best by (distance, original id) go out.
         Dist<KIND, CL, STORE_FP32> E;
         E.load(a, q, lane);
-        E.distances(a, m.qi, m.qd, sz, lane);
+        E.distances(a, m.qi, m.qd, sz, lane, reinterpret_cast<float *>(m.bk));
         rerank_output(m.qd, m.qi, sz, a.K, a.orig, a.out_ids + (size_t) q * a.K, lane);
     } else {
         // Results (original ids).

@@ -828,6 +828,14 @@ static int resident_blocks(panns_index *h, const void *kern, int threads, size_t
     return PANNS_OK;
 }
 
+// Of per_sm blocks that fit an SM, those that fit in 196 KB of shared memory (at
+// least one block): the default number of resident blocks, see launch_search.
+static uint32_t blocks_in_196kb(int per_sm, size_t smem) {
+    const size_t per_block = smem + 1024;
+    const uint32_t fit = (uint32_t) ((196u << 10) / per_block);
+    return (size_t) per_sm * per_block > (196u << 10) && fit >= 1 ? fit : (uint32_t) per_sm;
+}
+
 // Entries of a block kernel's warp buffer: the neighbours of the warp's share of
 // a step's candidates (at most max_deg per candidate) in one round, up to kBuf.
 static uint32_t block_buffer(uint32_t max_deg, uint32_t M, uint32_t W) {
@@ -933,22 +941,25 @@ static int launch_search(panns_index *h, const panns_search_params *p, float *d_
         if ((int) (wpb * 32) > res.max_threads)
             return fail(PANNS_EINVAL, "search: warps_per_block must be <= " + std::to_string(res.max_threads / 32) +
                                           " for this kernel");
-        if (wpq > 1) {
-            // The visited bitset in shared memory too, where that costs no
-            // resident query: as many blocks per SM as without it, or as the
-            // batch needs. One query on 1M x 96: 280 -> 240 us, 1,000 at L =
-            // 2,048 on 100k x 128 9.9 -> 7.1 ms (with the smaller warp buffers).
-            const uint32_t words = (h->n + 31) / 32;
-            const size_t with = (size_t) words * 4 < kSmemLimit ? (size_t) block_smem_bytes(qcap, wpq, bbuf, words)
-                                                                : kSmemLimit + 1;
-            const uint32_t need = (nq + (uint32_t) h->num_sms - 1) / (uint32_t) h->num_sms;
-            if (with <= kSmemLimit &&
-                (228u << 10) / (with + 1024) >= std::min<uint32_t>((uint32_t) std::max(res.per_sm, 1), need)) {
-                vis_smem = words;
-                smem = with;
-                rc = resident_blocks(h, kern, (int) wpb * 32, smem, res);
-                if (rc) return rc;
-            }
+        // The visited bitset in shared memory too, where that costs no resident
+        // query: as many blocks per SM as without it, or as the batch needs. One
+        // query on 1M x 96: 280 -> 240 us, 1,000 at L = 2,048 on 100k x 128 9.9 ->
+        // 7.1 ms (with the smaller warp buffers).
+        const uint32_t words = (h->n + 31) / 32;
+        size_t with = kSmemLimit + 1;
+        if ((size_t) words * 4 < kSmemLimit)
+            with = wpq > 1 ? (size_t) block_smem_bytes(qcap, wpq, bbuf, words)
+                           : wpb * (size_t) (pss ? pss_smem_bytes(qcap, p->T, wcap, words) : warp_smem_bytes(qcap, words));
+        const uint32_t at_once = qpb * (uint32_t) h->num_sms, need = (nq + at_once - 1) / at_once;
+        const uint32_t now = p->blocks_per_sm ? std::min(p->blocks_per_sm, (uint32_t) std::max(res.per_sm, 1))
+                                              : blocks_in_196kb(std::max(res.per_sm, 1), smem);
+        const uint32_t fit = (uint32_t) ((228u << 10) / (with + 1024));
+        if (with <= kSmemLimit &&
+            (p->blocks_per_sm ? fit : blocks_in_196kb((int) fit, with)) >= std::min(now, need)) {
+            vis_smem = words;
+            smem = with;
+            rc = resident_blocks(h, kern, (int) wpb * 32, smem, res);
+            if (rc) return rc;
         }
     }
     // The L1 / shared-memory split: the driver's first (enough shared memory
@@ -965,9 +976,8 @@ static int launch_search(panns_index *h, const panns_search_params *p, float *d_
         // array as shared memory (28 KB of L1 left): then as many as fit in
         // 196 KB. Measured on the 1M set: L = 448, 8.9 ms (5 blocks) against
         // 10.0 ms (6 blocks); L = 512 with 2-warp blocks, 9.8 ms (10) against 11.0 (12).
-        const size_t per_block = smem + 1024;
-        const int fit = (int) ((196u << 10) / per_block);
-        if ((size_t) per_sm * per_block > (196u << 10) && fit >= 1) bps = (uint32_t) fit;
+        const uint32_t fit = blocks_in_196kb(per_sm, smem);
+        if (fit < (uint32_t) per_sm) bps = fit;
     }
     if (bps) {
         CU(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, carveout_percent(smem, bps)));
@@ -1125,13 +1135,16 @@ static int stage_init(panns_index *h, const panns_search_params *p, const uint32
         }
         ids = buf.data();
     }
-    // Valid, distinct vertices per list; handed over as device ids in the same order.
+    // Valid, distinct vertices per list (the caller's are checked; the ones made
+    // above are); handed over as device ids in the same order.
     const uint32_t groups = efanna ? nq : 1;
     std::vector<uint32_t> dev((size_t) groups * L);
+    if (!init_ids)
+        for (size_t i = 0; i < dev.size(); ++i) dev[i] = h->inv[ids[i]];
     const bool by_sort = (uint64_t) groups * L * 16 < h->n;
-    std::vector<uint8_t> seen(by_sort ? 0 : h->n, 0);
+    std::vector<uint8_t> seen(by_sort || !init_ids ? 0 : h->n, 0);
     std::vector<uint32_t> tmp;
-    for (uint32_t g = 0; g < groups; ++g) {
+    for (uint32_t g = 0; g < groups && init_ids; ++g) {
         const uint32_t *x = ids + (size_t) g * L;
         for (uint32_t i = 0; i < L; ++i) {
             if (x[i] >= h->n) return fail(PANNS_EINVAL, "search: init id out of range");

@@ -33,8 +33,10 @@ struct PssArgs {
     uint32_t wcap;  // shared-memory entries per worker queue (>= L_local)
 };
 
-__host__ __device__ inline uint32_t pss_smem_bytes(uint32_t qcap, uint32_t T, uint32_t wcap) {
-    return qcap * 8u + (T - 1) * wcap * 8u + kBuf * 12u + 4u * ((3u * T + 31u) / 32u * 32u) + 64u * 4u;
+// Shared memory of one warp; vis_words: its visited bitset, where that fits too.
+__host__ __device__ inline uint32_t pss_smem_bytes(uint32_t qcap, uint32_t T, uint32_t wcap, uint32_t vis_words = 0) {
+    return qcap * 8u + (T - 1) * wcap * 8u + kBuf * 12u + 4u * ((3u * T + 31u) / 32u * 32u) + 64u * 4u +
+           (vis_words + 3u) / 4u * 16u;
 }
 
 struct PssMem {
@@ -55,7 +57,11 @@ struct PssMem {
 template <int KIND, int CL>
 __device__ uint32_t pss_flush(const SearchArgs &a, const PssMem &m, uint32_t nb, float *qd, uint32_t *qi,
                               uint32_t *sz, uint32_t cap, const Dist<KIND, CL, STORE_FP32> &D, int lane) {
-    D.distances(a, m.bi, m.bd, nb, lane, reinterpret_cast<float *>(m.bk));
+    // 16 rows in flight; eight or fewer left over in a pass of eight.
+    const uint32_t wide = (nb & 15u) > 8u ? nb : nb & ~15u;
+    float *tmp = reinterpret_cast<float *>(m.bk);
+    if (wide) distances_wide<KIND, CL>(a, D.qv, m.bi, m.bd, wide, lane, tmp);
+    if (wide < nb) D.distances(a, m.bi + wide, m.bd + wide, nb - wide, lane, tmp);
     const float bound = m.md[a.L - 1];
     uint32_t cnt = 0;
     for (uint32_t b0 = 0; b0 < nb; b0 += 32) {
@@ -113,7 +119,7 @@ __device__ uint32_t pss_expand(const SearchArgs &a, const PssMem &m, uint32_t v,
         }
         const uint32_t old = visit_issue(vis, id, valid);
         const bool fresh = valid && !(old & (1u << (id & 31)));
-        note_dirty(dirty, a.dirty_cap, dcount, valid && old == 0, id >> 5);
+        if (!a.vis_smem) note_dirty(dirty, a.dirty_cap, dcount, valid && old == 0, id >> 5);
         if (nb + 32 > kBuf) {
             n_dist += nb;
             nk = min(nk, pss_flush<KIND, CL>(a, m, nb, qd, qi, sz, cap, D, lane));
@@ -201,6 +207,8 @@ __device__ void pss_one(const PssArgs &pa, const PssMem &m, uint32_t q, uint32_t
     Dist<KIND, CL, STORE_FP32> D;
     D.load(a, q, lane);
     uint32_t dcount = 0, n_dist = 0, n_expand = 0, n_edges = 0, n_iter = 0;
+    for (uint32_t i = lane; i < a.vis_smem; i += 32) vis[i] = 0u;
+    __syncwarp();
     // Initial master queue (initialize_set_L_para :897-935).
     uint32_t msz = 0;
     {
@@ -212,7 +220,7 @@ __device__ void pss_one(const PssArgs &pa, const PssMem &m, uint32_t q, uint32_t
             const bool ok = valid && id < a.n;
             if (valid && !ok) atomicOr(a.error, ERR_BAD_INIT);
             const uint32_t old = visit_issue(vis, id, ok);
-            note_dirty(dirty, a.dirty_cap, dcount, ok && old == 0, id >> 5);
+            if (!a.vis_smem) note_dirty(dirty, a.dirty_cap, dcount, ok && old == 0, id >> 5);
             const uint32_t bm = __ballot_sync(kFull, ok);
             if (ok) m.bi[nb + __popc(bm & lanemask_lt())] = id;
             nb += __popc(bm);
@@ -325,7 +333,8 @@ __device__ void pss_one(const PssArgs &pa, const PssMem &m, uint32_t q, uint32_t
     for (uint32_t i = lane; i < a.K; i += 32)
         a.out_ids[(size_t) q * a.K + i] = __ldg(a.orig + (m.mi[i] & kIdMask));
     if (lane == 0 && a.out_stats) a.out_stats[q] = make_uint4(n_dist, n_expand, n_edges, n_iter);
-    if (dcount <= a.dirty_cap) {
+    if (a.vis_smem) {  // zeroed by the next query
+    } else if (dcount <= a.dirty_cap) {
         for (uint32_t i = lane; i < dcount; i += 32) vis[dirty[i]] = 0u;
     } else {
         for (uint32_t i = lane; i < a.vis_words; i += 32) vis[i] = 0u;
@@ -340,7 +349,8 @@ __global__ void __launch_bounds__(128, 4) pss_kernel(PssArgs pa) {
     const int wid = threadIdx.x >> 5;
     const SearchArgs &a = pa.s;
     const uint32_t qcap = a.queue_cap;
-    uint8_t *base = smem + (size_t) wid * pss_smem_bytes(qcap, pa.T, pa.wcap);
+    const uint32_t per_warp = pss_smem_bytes(qcap, pa.T, pa.wcap, a.vis_smem);
+    uint8_t *base = smem + (size_t) wid * per_warp;
     PssMem m;
     m.md = reinterpret_cast<float *>(base);
     m.mi = reinterpret_cast<uint32_t *>(m.md + qcap);
@@ -353,7 +363,10 @@ __global__ void __launch_bounds__(128, 4) pss_kernel(PssArgs pa) {
     m.kuc = m.wsz + pa.T;
     m.iters = m.kuc + pa.T;
     const uint32_t slot = blockIdx.x * (blockDim.x >> 5) + wid;
-    uint32_t *vis = a.visited + (size_t) slot * a.vis_words;
+    // The visited bitset: in shared memory where it fits beside the queues without
+    // costing resident queries (an atomic there takes a tenth of one in L2).
+    uint32_t *vis = a.vis_smem ? reinterpret_cast<uint32_t *>(base + per_warp - (a.vis_smem + 3u) / 4u * 16u)
+                               : a.visited + (size_t) slot * a.vis_words;
     uint32_t *dirty = a.dirty + (size_t) slot * a.dirty_cap;
     for (;;) {
         uint32_t q = 0;

@@ -117,17 +117,19 @@ struct SearchArgs {
     const uint32_t *Lq;       // per-query queue length (K <= Lq[q] <= L), or null: L for all
     const uint32_t *decisions;  // per-query records of the entry / L-budget network (mlp_decide), or null
     uint32_t dec_L_init;      // plain init ids kept after learned entries
+    uint32_t vis_smem;        // words of the visited bitset in shared memory (0: in global memory)
     // search_block_kernel:
     uint32_t block_round;     // candidates per warp and merge round
     uint32_t block_buf;       // fresh vertices per warp and round (a power of two)
-    uint32_t vis_smem;        // words of the visited bitset in shared memory (0: in global memory)
 };
 
-// Bytes of shared memory one warp needs.
-__host__ __device__ inline uint32_t warp_smem_bytes(uint32_t queue_cap) {
+// Bytes of shared memory one warp needs; vis_words: its visited bitset, where that
+// fits too (16-byte multiples throughout).
+__host__ __device__ inline uint32_t warp_smem_bytes(uint32_t queue_cap, uint32_t vis_words = 0) {
     return queue_cap * 8u                 // queue dist + id
            + kBuf * 12u                   // buffer dist + id + key
-           + kMaxM * 4u;                  // picked candidate ids / learned entries
+           + kMaxM * 4u                   // picked candidate ids / learned entries
+           + (vis_words + 3u) / 4u * 16u; // visited bitset
 }
 
 struct WarpMem {
@@ -798,7 +800,6 @@ static __device__ void rerank_output(float *qd, uint32_t *qi, uint32_t sz, uint3
 template <int KIND, int ORDER, int CL, int STORE>
 __device__ uint32_t flush(const SearchArgs &a, const WarpMem &m, uint32_t nb, uint32_t *sz, uint32_t L,
                           bool filter, const Dist<KIND, CL, STORE> &D, int lane) {
-    constexpr bool kLazyKeys = ORDER == ORDER_PANNS && STORE != STORE_FP8;
     D.distances(a, m.bi, m.bd, nb, lane, reinterpret_cast<float *>(m.bk));
     // Keep the survivors, in arrival order.
     const float bound = (filter && *sz >= L) ? m.qd[L - 1] : __int_as_float(0x7f800000);
@@ -820,23 +821,23 @@ __device__ uint32_t flush(const SearchArgs &a, const WarpMem &m, uint32_t nb, ui
             const uint32_t pos = cnt + __popc(bm & lanemask_lt());
             m.bd[pos] = d;
             m.bi[pos] = id;
-            m.bk[pos] = ORDER == ORDER_PANNS ? (kLazyKeys ? id : __ldg(a.orig + id)) : pos;
         }
         cnt += __popc(bm);
         __syncwarp();
     }
     if (cnt == 0) return L;
     if (cnt <= 32) return rank_merge32<ORDER>(m.qd, m.qi, sz, L, m.bd, m.bi, cnt, a.orig, lane);
-    // With lazy keys the survivors are sorted by (distance, device id); PANNS
-    // order breaks equal distances by original id, so if the sorted
-    // survivors hold equal distances (rare) they are sorted once more with
+    // Longer lists are sorted by (distance, device id) or, EFANNA, (distance,
+    // arrival); PANNS order breaks equal distances by original id, so if the
+    // sorted survivors hold equal distances (rare) they are sorted once more with
     // the original ids as keys (one inlined copy of warp_sort either way).
-    // Measured (10,000 queries, L = 384, M = 8, same ids): float32 rows
-    // 5.42 -> 5.31 ms, BF16 5.08 -> 5.02 ms, FP8 5.03 -> 5.08 ms, so the FP8
-    // kernel keeps loading the original ids in the filter.
+    // Loading every survivor's original id in the filter instead cost 2 % of the
+    // float32 and BF16 kernels' time.
+    for (uint32_t i = lane; i < cnt; i += 32) m.bk[i] = ORDER == ORDER_PANNS ? m.bi[i] & kIdMask : i;
+    __syncwarp();
     for (int pass = 0;; ++pass) {
         warp_sort<ORDER>(m.bd, m.bi, m.bk, cnt, a.orig, lane);
-        if (!kLazyKeys || pass) break;
+        if (ORDER != ORDER_PANNS || pass) break;
         bool tie = false;
         for (uint32_t i = lane; i + 1 < cnt; i += 32) tie |= m.bd[i] == m.bd[i + 1];
         if (!__any_sync(kFull, tie)) break;
@@ -874,6 +875,8 @@ __device__ void search_one(const SearchArgs &a, const WarpMem &m, uint32_t q, ui
     uint32_t dcount = 0;
     uint32_t n_dist = 0, n_expand = 0, n_edges = 0, n_iter = 0;
     uint32_t sz = 0;
+    for (uint32_t i = lane; i < a.vis_smem; i += 32) vis[i] = 0u;
+    __syncwarp();
 
     // Initial queue: the init ids, all marked visited, sorted (init order
     // breaks equal distances for efanna2e). A repeated id (a learned entry
@@ -888,7 +891,7 @@ __device__ void search_one(const SearchArgs &a, const WarpMem &m, uint32_t q, ui
         const bool ok = valid && id < a.n;
         if (valid && !ok) atomicOr(a.error, ERR_BAD_INIT);
         const uint32_t old = visit_issue(vis, id, ok);
-        note_dirty(dirty, a.dirty_cap, dcount, ok && old == 0, id >> 5);
+        if (!a.vis_smem) note_dirty(dirty, a.dirty_cap, dcount, ok && old == 0, id >> 5);
         const bool fresh = ok && !(old & (1u << (id & 31)));
         const uint32_t bm = __ballot_sync(kFull, fresh);
         if (fresh) m.bi[nb + __popc(bm & lanemask_lt())] = id;
@@ -984,7 +987,7 @@ __device__ void search_one(const SearchArgs &a, const WarpMem &m, uint32_t q, ui
                     const uint32_t id = hv[j];
                     const bool valid = id != kFull;
                     const bool fresh = valid && !(olds[j] & (1u << (id & 31)));
-                    note_dirty(dirty, a.dirty_cap, dcount, valid && olds[j] == 0, id >> 5);
+                    if (!a.vis_smem) note_dirty(dirty, a.dirty_cap, dcount, valid && olds[j] == 0, id >> 5);
                     append_ids(m, nb, fresh, id, lane);
                 }
                 // Rows longer than the head row: the rest from the overflow
@@ -1036,7 +1039,7 @@ __device__ void search_one(const SearchArgs &a, const WarpMem &m, uint32_t q, ui
                     const uint32_t id = oid[ch];
                     const bool valid = id != kFull;
                     const bool fresh = valid && !(oold[ch] & (1u << (id & 31)));
-                    note_dirty(dirty, a.dirty_cap, dcount, valid && oold[ch] == 0, id >> 5);
+                    if (!a.vis_smem) note_dirty(dirty, a.dirty_cap, dcount, valid && oold[ch] == 0, id >> 5);
                     append_ids(m, nb, fresh, id, lane);
                 }
                 f0 += 32 * kOvfChunks;
@@ -1064,7 +1067,8 @@ __device__ void search_one(const SearchArgs &a, const WarpMem &m, uint32_t q, ui
     }
     if (lane == 0 && a.out_stats) a.out_stats[q] = make_uint4(n_dist, n_expand, n_edges, n_iter);
     // Clear the visited words this query set.
-    if (dcount <= a.dirty_cap) {
+    if (a.vis_smem) {  // zeroed by the next query
+    } else if (dcount <= a.dirty_cap) {
         for (uint32_t i = lane; i < dcount; i += 32) vis[dirty[i]] = 0u;
     } else {
         for (uint32_t i = lane; i < a.vis_words; i += 32) vis[i] = 0u;
@@ -1077,9 +1081,14 @@ __global__ void __launch_bounds__(128, PANNS_SEARCH_MIN_BLOCKS) search_kernel(Se
     extern __shared__ __align__(16) uint8_t smem[];
     const int lane = threadIdx.x & 31;
     const int wid = threadIdx.x >> 5;
-    const WarpMem m = carve(smem + (size_t) wid * warp_smem_bytes(a.queue_cap), a.queue_cap);
+    const uint32_t per_warp = warp_smem_bytes(a.queue_cap, a.vis_smem);
+    uint8_t *base = smem + (size_t) wid * per_warp;
+    const WarpMem m = carve(base, a.queue_cap);
     const uint32_t slot = blockIdx.x * (blockDim.x >> 5) + wid;
-    uint32_t *vis = a.visited + (size_t) slot * a.vis_words;
+    // The visited bitset: in shared memory where it fits beside the queue without
+    // costing resident queries, else the warp's slot of global memory.
+    uint32_t *vis = a.vis_smem ? reinterpret_cast<uint32_t *>(base + warp_smem_bytes(a.queue_cap))
+                               : a.visited + (size_t) slot * a.vis_words;
     uint32_t *dirty = a.dirty + (size_t) slot * a.dirty_cap;
     for (;;) {
         uint32_t q = 0;

@@ -332,6 +332,16 @@ __global__ void __launch_bounds__(256) screen_cells_kernel(
     }
 }
 
+// The cells' rows, each cell from the start of its first tile (the rest of the
+// order is filled beforehand).
+__global__ void __launch_bounds__(256) pad_cells_kernel(const uint32_t *__restrict__ members,
+                                                        const uint32_t *__restrict__ start,
+                                                        const uint32_t *__restrict__ tile0,
+                                                        uint32_t *__restrict__ order) {
+    const uint32_t c = blockIdx.x, b = start[c], m = start[c + 1] - b;
+    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) order[(size_t) tile0[c] * kTcM + i] = members[b + i];
+}
+
 // For every cell c (one block each), the P other cells whose centroids are
 // nearest by (float64 squared distance, index); ~0 where there are fewer.
 __global__ void __launch_bounds__(256) near_cells_kernel(const float *__restrict__ cent, uint32_t cells, uint32_t d,
@@ -1273,7 +1283,10 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
     GCU(cudaGetLastError());
     // Cells: Lloyd k-means on S rows at a fixed stride, then every row to its
     // nearest centroid; each cell's P nearest cells by centroid distance.
-    std::vector<uint32_t> cellh(n), nearh((size_t) cells * std::max(P, 1u), 0xffffffffu);
+    std::vector<uint32_t> cellh(n), nearh((size_t) cells * std::max(P, 1u), 0xffffffffu), cstart(cells + 1);
+    Buf<uint32_t> dmem, dstart;
+    GCU(dmem.alloc(n, s));
+    GCU(dstart.alloc(cells + 1, s));
     {
         Buf<uint32_t> sidx, sas, srep, dcell, dnear;
         Buf<float> xs, cent;
@@ -1292,7 +1305,10 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
         if (rc) return rc;
         rc = nearest_centroid(x.p, n, d, cent.p, cells, dcell.p, s);
         if (rc) return rc;
+        // Members of each cell in id order.
+        GCU(cell_sort(dcell.p, n, cells, dstart.p, dmem.p, s));
         GCU(cudaMemcpyAsync(cellh.data(), dcell.p, n * 4ull, cudaMemcpyDeviceToHost, s));
+        GCU(cudaMemcpyAsync(cstart.data(), dstart.p, (cells + 1) * 4ull, cudaMemcpyDeviceToHost, s));
         if (P) {
             GCU(dnear.alloc((size_t) cells * P, s));
             near_cells_kernel<<<cells, 256, 0, s>>>(cent.p, cells, d, P, dnear.p);
@@ -1301,20 +1317,6 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
         }
         GCU(cudaStreamSynchronize(s));
     }
-    // Members of each cell in id order, and the screen's blocks of up to kBQ
-    // rows of one cell.
-    std::vector<uint32_t> cstart(cells + 1, 0), members(n), blk_cell, blk_row0;
-    for (uint32_t i = 0; i < n; ++i) ++cstart[cellh[i] + 1];
-    for (uint32_t c = 0; c < cells; ++c) cstart[c + 1] += cstart[c];
-    {
-        std::vector<uint32_t> pos(cstart.begin(), cstart.end() - 1);
-        for (uint32_t i = 0; i < n; ++i) members[pos[cellh[i]]++] = i;
-    }
-    for (uint32_t c = 0; c < cells; ++c)
-        for (uint32_t r = cstart[c]; r < cstart[c + 1]; r += kBQ) {
-            blk_cell.push_back(c);
-            blk_row0.push_back(r);
-        }
     Buf<uint32_t> cand;
     GCU(cand.alloc((size_t) n * C, s));
     GCU(cudaMemsetAsync(cand.p, 0xff, (size_t) n * C * 4, s));
@@ -1329,12 +1331,10 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
     GCU(cudaMemGetInfo(&free_b, &total_b));
     if (d <= 256 && n >= kTcMinRows && slots <= 2ull * n && slots <= 0x7fffffffull &&
         tc_knn_bytes(slots, d) <= free_b / 5 * 3) {
-        std::vector<uint32_t> tile0(cells + 1, 0), avail(cells, 0), order((size_t) slots, 0xffffffffu), blk;
+        std::vector<uint32_t> tile0(cells + 1, 0), avail(cells, 0), blk;
         blk.reserve((size_t) (slots / kTcM));
         for (uint32_t c = 0; c < cells; ++c) {
             const uint32_t m = cstart[c + 1] - cstart[c], t = (m + kTcM - 1) / kTcM;
-            std::copy(members.begin() + cstart[c], members.begin() + cstart[c + 1],
-                      order.begin() + (size_t) tile0[c] * kTcM);
             blk.insert(blk.end(), t, c);
             tile0[c + 1] = tile0[c] + t;
             avail[c] = m;
@@ -1346,16 +1346,18 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
         int num_sms = 0;
         GCU(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device));
         Buf<uint32_t> dorder, dblk, dt0, dnear, davail, fail, nfail;
-        GCU(dorder.alloc(order.size(), s));
+        GCU(dorder.alloc((size_t) slots, s));
         GCU(dblk.alloc(blk.size(), s));
         GCU(dt0.alloc(cells + 1, s));
         GCU(dnear.alloc(nearh.size(), s));
         GCU(davail.alloc(cells, s));
         GCU(fail.alloc(n, s));
         GCU(nfail.alloc(1, s));
-        GCU(cudaMemcpyAsync(dorder.p, order.data(), order.size() * 4, cudaMemcpyHostToDevice, s));
+        GCU(cudaMemsetAsync(dorder.p, 0xff, (size_t) slots * 4, s));
         GCU(cudaMemcpyAsync(dblk.p, blk.data(), blk.size() * 4, cudaMemcpyHostToDevice, s));
         GCU(cudaMemcpyAsync(dt0.p, tile0.data(), (cells + 1) * 4ull, cudaMemcpyHostToDevice, s));
+        pad_cells_kernel<<<cells, 256, 0, s>>>(dmem.p, dstart.p, dt0.p, dorder.p);
+        GCU(cudaGetLastError());
         GCU(cudaMemcpyAsync(dnear.p, nearh.data(), nearh.size() * 4, cudaMemcpyHostToDevice, s));
         GCU(cudaMemcpyAsync(davail.p, avail.data(), cells * 4ull, cudaMemcpyHostToDevice, s));
         const TcCells tc{dblk.p, dt0.p, dnear.p, davail.p, P};
@@ -1368,15 +1370,18 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
         screened = nf == 0;
     }
     if (!screened) {
-        Buf<uint32_t> dmem, dstart, dnear, dbc, dbr;
-        GCU(dmem.alloc(n, s));
-        GCU(dstart.alloc(cells + 1, s));
+        // Blocks of up to kBQ rows of one cell.
+        std::vector<uint32_t> blk_cell, blk_row0;
+        for (uint32_t c = 0; c < cells; ++c)
+            for (uint32_t r = cstart[c]; r < cstart[c + 1]; r += kBQ) {
+                blk_cell.push_back(c);
+                blk_row0.push_back(r);
+            }
+        Buf<uint32_t> dnear, dbc, dbr;
         GCU(dnear.alloc(nearh.size(), s));
         GCU(dbc.alloc(blk_cell.size(), s));
         GCU(dbr.alloc(blk_row0.size(), s));
         GCU(cudaMemsetAsync(cand.p, 0xff, (size_t) n * C * 4, s));
-        GCU(cudaMemcpyAsync(dmem.p, members.data(), n * 4ull, cudaMemcpyHostToDevice, s));
-        GCU(cudaMemcpyAsync(dstart.p, cstart.data(), (cells + 1) * 4ull, cudaMemcpyHostToDevice, s));
         GCU(cudaMemcpyAsync(dnear.p, nearh.data(), nearh.size() * 4, cudaMemcpyHostToDevice, s));
         GCU(cudaMemcpyAsync(dbc.p, blk_cell.data(), blk_cell.size() * 4, cudaMemcpyHostToDevice, s));
         GCU(cudaMemcpyAsync(dbr.p, blk_row0.data(), blk_row0.size() * 4, cudaMemcpyHostToDevice, s));

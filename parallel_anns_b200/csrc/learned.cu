@@ -526,63 +526,67 @@ __global__ void gather_rows_kernel(const float *__restrict__ rows, uint32_t d, c
     for (uint32_t j = threadIdx.x; j < d; j += blockDim.x) out[(size_t) c * d + j] = rows[(size_t) idx[c] * d + j];
 }
 
-// Farthest-point seeding, all on the GPU. mind[s] = the squared distance of
-// sample row sidx[s] to the nearest centre chosen so far; kpp_update folds
-// in the newest centre (sample slot *slot).
-__global__ void kpp_update_kernel(const float *__restrict__ rows, uint32_t d, const uint32_t *__restrict__ sidx,
-                                  uint32_t S, const uint32_t *__restrict__ slot, float *__restrict__ mind) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= S) return;
-    const float *x = rows + (size_t) sidx[t] * d;
-    const float *c = rows + (size_t) sidx[*slot] * d;
+// Farthest-point seeding, one launch per centre. mind[t] = the squared distance
+// of sample t (row t n / S) to the nearest centre chosen so far. A step folds in
+// the newest centre (the sample ~(low word of *key)) and leaves the farthest
+// sample in *next as (distance bits, ~sample): distances are not negative, so
+// the largest word is the largest distance, ties to the lower sample.
+//
+// Bound by latency: 200 dependent steps of 6,400 rows x 96. A block stages 64
+// rows (all loads in flight at once, whole lines) and two warps run one chain
+// a row over shared memory, so a step costs one memory latency and d steps of
+// the chain: 3.4 us. A thread that walked its row in memory, and a second
+// launch for the maximum, took 18.9 us a step.
+constexpr int kSeedRows = 64, kSeedDims = 128;
+
+__global__ void __launch_bounds__(256) seed_step_kernel(const float *__restrict__ rows, uint32_t n, uint32_t d,
+                                                        uint32_t S, const unsigned long long *__restrict__ key,
+                                                        unsigned long long *__restrict__ next,
+                                                        float *__restrict__ mind) {
+    __shared__ float tile[kSeedRows][kSeedDims + 1];
+    __shared__ float cen[kSeedDims];
+    const uint32_t tid = threadIdx.x, w = tid >> 5, lane = tid & 31, t0 = blockIdx.x * kSeedRows;
+    const uint64_t crow = (uint64_t) ~(uint32_t) *key * n / S;
+    const uint64_t mine = (uint64_t) min(t0 + w + 8 * (lane & 7), S - 1) * n / S;
     float acc = 0.f;
-    for (uint32_t j = 0; j < d; ++j) {
-        const float u = x[j] - c[j];
-        acc = fmaf(u, u, acc);
+    for (uint32_t j0 = 0; j0 < d; j0 += kSeedDims) {
+        const uint32_t m = min((uint32_t) kSeedDims, d - j0);
+        if (j0) __syncthreads();
+        if (tid < m) cen[tid] = rows[crow * d + j0 + tid];
+#pragma unroll
+        for (uint32_t q = 0; q < kSeedRows / 8; ++q) {
+            const float *src = rows + __shfl_sync(0xffffffffu, mine, q) * d + j0;
+#pragma unroll
+            for (uint32_t j = lane; j < (uint32_t) kSeedDims; j += 32)
+                if (j < m) tile[w + 8 * q][j] = src[j];
+        }
+        __syncthreads();
+        if (tid < kSeedRows)
+#pragma unroll 8
+            for (uint32_t j = 0; j < m; ++j) {
+                const float u = tile[tid][j] - cen[j];
+                acc = fmaf(u, u, acc);
+            }
     }
-    mind[t] = fminf(mind[t], acc);
+    if (tid >= kSeedRows) return;
+    unsigned long long best = 0;
+    if (t0 + tid < S) {
+        const float v = fminf(mind[t0 + tid], acc);
+        mind[t0 + tid] = v;
+        best = (unsigned long long) __float_as_uint(v) << 32 | ~(t0 + tid);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long b2 = __shfl_xor_sync(0xffffffffu, best, o);
+        best = b2 > best ? b2 : best;
+    }
+    if (lane == 0) atomicMax(next, best);
 }
 
-// One block of 1024 threads: the next centre, the sample slot with the
-// largest mind (ties to the lower slot).
-__global__ void __launch_bounds__(1024) kpp_pick_kernel(const float *__restrict__ mind, uint32_t S,
-                                                        uint32_t *__restrict__ slot) {
-    __shared__ float bv[32];
-    __shared__ uint32_t bi[32];
-    float best = -1.f;
-    uint32_t bidx = 0xffffffffu;
-    for (uint32_t i = threadIdx.x; i < S; i += blockDim.x)
-        if (mind[i] > best) {  // ascending i: the lower slot wins ties
-            best = mind[i];
-            bidx = i;
-        }
-    for (int o = 16; o > 0; o >>= 1) {
-        const float v2 = __shfl_xor_sync(0xffffffffu, best, o);
-        const uint32_t i2 = __shfl_xor_sync(0xffffffffu, bidx, o);
-        if (v2 > best || (v2 == best && i2 < bidx)) {
-            best = v2;
-            bidx = i2;
-        }
-    }
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) {
-        bv[w] = best;
-        bi[w] = bidx;
-    }
-    __syncthreads();
-    if (w == 0) {
-        best = bv[l];
-        bidx = bi[l];
-        for (int o = 16; o > 0; o >>= 1) {
-            const float v2 = __shfl_xor_sync(0xffffffffu, best, o);
-            const uint32_t i2 = __shfl_xor_sync(0xffffffffu, bidx, o);
-            if (v2 > best || (v2 == best && i2 < bidx)) {
-                best = v2;
-                bidx = i2;
-            }
-        }
-        if (l == 0) *slot = bidx < S ? bidx : 0u;
-    }
+// idx[c] = the row of the chosen sample c.
+__global__ void seed_rows_kernel(const unsigned long long *__restrict__ key, uint32_t k, uint32_t n, uint32_t S,
+                                 uint32_t *__restrict__ idx) {
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < k) idx[c] = (uint32_t) ((uint64_t) ~(uint32_t) key[c] * n / S);
 }
 
 __global__ void sqnorm_kernel(const float *__restrict__ rows, uint32_t n, uint32_t d, float *__restrict__ out) {
@@ -619,20 +623,99 @@ __global__ void argmin_kernel(const float *__restrict__ G, uint32_t rows, uint32
     if (lane == 0) assign[w] = bi < k ? bi : 0u;
 }
 
+// Stable counting sort of the rows by cell. A warp owns `step` consecutive rows
+// and the column `chunk` of the counters tab[cell][chunk]; PLACE = false counts,
+// PLACE = true (after the two scans below) writes every row id to its place: a
+// warp takes 32 rows at a time in order, so ids ascend within a cell.
+// Both passes take 27 us (200 cells); the same lists made on the host between
+// two copies took about 1 ms a round.
+template <bool PLACE>
+__global__ void __launch_bounds__(256) cell_sort_kernel(const uint32_t *__restrict__ cell, uint32_t n, uint32_t step,
+                                                        uint32_t chunks, uint32_t *__restrict__ tab,
+                                                        const uint32_t *__restrict__ off,
+                                                        uint32_t *__restrict__ members) {
+    const uint32_t chunk = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (chunk >= chunks) return;
+    const uint64_t b = (uint64_t) chunk * step, e = min(b + step, (uint64_t) n);
+    for (uint64_t i0 = b; i0 < e; i0 += 32) {
+        const uint64_t i = i0 + lane;
+        const uint32_t c = i < e ? cell[i] : 0xffffffffu;
+        const uint32_t same = __match_any_sync(0xffffffffu, c);
+        const int lead = __ffs(same) - 1;
+        uint32_t pos = 0;
+        if (i < e && (int) lane == lead) pos = atomicAdd(&tab[(size_t) c * chunks + chunk], (uint32_t) __popc(same));
+        if constexpr (PLACE) {
+            pos = __shfl_sync(0xffffffffu, pos, lead);
+            if (i < e) members[off[c] + pos + __popc(same & ((1u << lane) - 1))] = (uint32_t) i;
+        }
+    }
+}
+
+// Exclusive prefix sums of each row of `m` words in place, one block per row,
+// the row's sum to total[row].
+__global__ void __launch_bounds__(256) scan_rows_kernel(uint32_t *__restrict__ tab, uint32_t m,
+                                                        uint32_t *__restrict__ total) {
+    __shared__ uint32_t ws[8];
+    uint32_t *t = tab + (size_t) blockIdx.x * m;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t carry = 0;
+    for (uint32_t i0 = 0; i0 < m; i0 += 256) {
+        const uint32_t i = i0 + threadIdx.x, v = i < m ? t[i] : 0u;
+        uint32_t x = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= (uint32_t) o) x += y;
+        }
+        if (lane == 31) ws[w] = x;
+        __syncthreads();
+        uint32_t before = carry;
+        for (uint32_t u = 0; u < 8; ++u) {
+            if (u < w) before += ws[u];
+            carry += ws[u];
+        }
+        if (i < m) t[i] = before + x - v;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) total[blockIdx.x] = carry;
+}
+
 // One block per cell: the centroid = mean of its rows (listed in id order in
 // members[off[c]..off[c+1])), kept when the cell is empty; with rep != null,
 // the member nearest to the centroid (exact float32 squared distance, ties to
 // the lower id) instead.
-__global__ void cell_kernel(const float *__restrict__ rows, uint32_t d, const uint32_t *__restrict__ members,
-                            const uint32_t *__restrict__ off, float *__restrict__ cent, uint32_t *__restrict__ rep) {
+//
+// The mean is one float64 chain a dimension (its order is part of the result),
+// so the rows are loaded sixteen at a time and what is left is the longest
+// cell's chain of additions: 292 us a round for 200 uneven cells x 96
+// dimensions, 371 us with one row in flight.
+__global__ void __launch_bounds__(256) cell_kernel(const float *__restrict__ rows, uint32_t d,
+                                                   const uint32_t *__restrict__ members,
+                                                   const uint32_t *__restrict__ off, float *__restrict__ cent,
+                                                   uint32_t *__restrict__ rep) {
     const uint32_t c = blockIdx.x;
     const uint32_t b = off[c], e = off[c + 1];
     if (!rep) {
         if (b == e) return;
-        for (uint32_t j = threadIdx.x; j < d; j += blockDim.x) {
+        __shared__ uint32_t ids[256];
+        for (uint32_t j0 = 0; j0 < d; j0 += 256) {
+            const uint32_t j = j0 + threadIdx.x;
             double s = 0.0;
-            for (uint32_t i = b; i < e; ++i) s += rows[(size_t) members[i] * d + j];
-            cent[(size_t) c * d + j] = (float) (s / (double) (e - b));
+            for (uint32_t i0 = b; i0 < e; i0 += 256) {
+                const uint32_t m = min(256u, e - i0);
+                __syncthreads();
+                if (threadIdx.x < m) ids[threadIdx.x] = members[i0 + threadIdx.x];
+                __syncthreads();
+                if (j >= d) continue;
+                for (uint32_t i = 0; i < m; i += 16) {
+                    float v[16];
+#pragma unroll
+                    for (uint32_t u = 0; u < 16; ++u) v[u] = rows[(size_t) ids[min(i + u, m - 1)] * d + j];
+#pragma unroll
+                    for (uint32_t u = 0; u < 16; ++u)
+                        if (i + u < m) s += v[u];
+                }
+            }
+            if (j < d) cent[(size_t) c * d + j] = (float) (s / (double) (e - b));
         }
         return;
     }
@@ -671,38 +754,25 @@ __global__ void cell_kernel(const float *__restrict__ rows, uint32_t d, const ui
 
 }  // namespace
 
+cudaError_t cell_sort(const uint32_t *cell, uint32_t n, uint32_t k, uint32_t *off, uint32_t *members,
+                      cudaStream_t s) {
+    // 512 rows a warp, or more where the counters would pass 16 M words.
+    const uint32_t step = (uint32_t) std::max<uint64_t>(512, ((uint64_t) n * k / (16u << 20) + 32) / 32 * 32);
+    const uint32_t chunks = (n + step - 1) / step;
+    Dev<uint32_t> tab;
+    cudaError_t e = tab.alloc((size_t) k * chunks, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(tab.p, 0, (size_t) k * chunks * 4, s);
+    if (e != cudaSuccess) return e;
+    cell_sort_kernel<false><<<(chunks + 7) / 8, 256, 0, s>>>(cell, n, step, chunks, tab.p, nullptr, nullptr);
+    scan_rows_kernel<<<k, 256, 0, s>>>(tab.p, chunks, off);
+    scan_rows_kernel<<<1, 256, 0, s>>>(off, k, off + k);
+    cell_sort_kernel<true><<<(chunks + 7) / 8, 256, 0, s>>>(cell, n, step, chunks, tab.p, off, members);
+    return cudaGetLastError();
+}
+
 int kmeans_run(const float *rows, uint32_t n, uint32_t d, uint32_t k, uint32_t iters, uint32_t seed,
                float *cent, uint32_t *assign, uint32_t *rep, cudaStream_t s) {
     if (k == 0 || k > n) return set_error(PANNS_EINVAL, "kmeans: need 0 < k <= N");
-    // Start: farthest-point seeding (Gonzalez, 1985) on S rows at a fixed
-    // stride: a seeded first centre, then each next one the sample row
-    // farthest from the centres so far (on the GPU). Far-apart clusters then
-    // each get a centre before any is split, which random starts (and D^2
-    // sampling, with as many centres as clusters) miss.
-    std::vector<uint32_t> start(k);
-    {
-        const uint32_t S = (uint32_t) std::min<uint64_t>(n, std::max<uint64_t>(k, 32ull * k));
-        std::vector<uint32_t> sidx(S), slots(k);
-        for (uint32_t i = 0; i < S; ++i) sidx[i] = (uint32_t) ((uint64_t) i * n / S);
-        std::mt19937_64 rng(seed);
-        Dev<uint32_t> dsidx, dslot;
-        Dev<float> mind;
-        LCU(dsidx.alloc(S, s));
-        LCU(dslot.alloc(k, s));
-        LCU(mind.alloc(S, s));
-        LCU(cudaMemcpyAsync(dsidx.p, sidx.data(), S * 4ull, cudaMemcpyHostToDevice, s));
-        LCU(cudaMemsetAsync(mind.p, 0x7f, S * 4ull, s));  // 3.4e38: larger than any distance
-        const uint32_t first = (uint32_t) (rng() % S);
-        LCU(cudaMemcpyAsync(dslot.p, &first, 4, cudaMemcpyHostToDevice, s));
-        for (uint32_t c = 0; c < k; ++c) {
-            kpp_update_kernel<<<(S + 255) / 256, 256, 0, s>>>(rows, d, dsidx.p, S, dslot.p + c, mind.p);
-            if (c + 1 < k) kpp_pick_kernel<<<1, 1024, 0, s>>>(mind.p, S, dslot.p + c + 1);
-        }
-        LCU(cudaGetLastError());
-        LCU(cudaMemcpyAsync(slots.data(), dslot.p, k * 4ull, cudaMemcpyDeviceToHost, s));
-        LCU(cudaStreamSynchronize(s));
-        for (uint32_t c = 0; c < k; ++c) start[c] = sidx[slots[c]];
-    }
     Dev<uint32_t> didx, doff, dmem;
     Dev<float> cn, G;
     const uint32_t chunk = std::min<uint32_t>(n, 65536);
@@ -711,10 +781,30 @@ int kmeans_run(const float *rows, uint32_t n, uint32_t d, uint32_t k, uint32_t i
     LCU(dmem.alloc(n, s));
     LCU(cn.alloc(k, s));
     LCU(G.alloc((size_t) chunk * k, s));
-    LCU(cudaMemcpyAsync(didx.p, start.data(), k * 4ull, cudaMemcpyHostToDevice, s));
+    // Start: farthest-point seeding (Gonzalez, 1985) on S rows at a fixed
+    // stride: a seeded first centre, then each next one the sample row
+    // farthest from the centres so far (on the GPU). Far-apart clusters then
+    // each get a centre before any is split, which random starts (and D^2
+    // sampling, with as many centres as clusters) miss.
+    {
+        const uint32_t S = (uint32_t) std::min<uint64_t>(n, std::max<uint64_t>(k, 32ull * k));
+        std::mt19937_64 rng(seed);
+        Dev<unsigned long long> key;
+        Dev<float> mind;
+        LCU(key.alloc(k, s));
+        LCU(mind.alloc(S, s));
+        LCU(cudaMemsetAsync(mind.p, 0x7f, S * 4ull, s));  // 3.4e38: larger than any distance
+        LCU(cudaMemsetAsync(key.p, 0, k * 8ull, s));
+        const unsigned long long first = (uint32_t) ~(uint32_t) (rng() % S);
+        LCU(cudaMemcpyAsync(key.p, &first, 8, cudaMemcpyHostToDevice, s));
+        for (uint32_t c = 0; c + 1 < k; ++c)
+            seed_step_kernel<<<(S + kSeedRows - 1) / kSeedRows, 256, 0, s>>>(rows, n, d, S, key.p + c, key.p + c + 1,
+                                                                             mind.p);
+        seed_rows_kernel<<<(k + 255) / 256, 256, 0, s>>>(key.p, k, n, S, didx.p);
+        LCU(cudaGetLastError());
+    }
     gather_rows_kernel<<<k, 128, 0, s>>>(rows, d, didx.p, k, cent);
     LCU(cudaGetLastError());
-    std::vector<uint32_t> h_assign(n), off(k + 1), members(n);
     for (uint32_t it = 0; it <= iters; ++it) {
         sqnorm_kernel<<<(k + 255) / 256, 256, 0, s>>>(cent, k, d, cn.p);
         LCU(cudaGetLastError());
@@ -725,40 +815,29 @@ int kmeans_run(const float *rows, uint32_t n, uint32_t d, uint32_t k, uint32_t i
             argmin_kernel<<<(rows_c * 32 + 255) / 256, 256, 0, s>>>(G.p, rows_c, k, cn.p, assign + r0);
             LCU(cudaGetLastError());
         }
-        // Members of each cell in id order (counting sort on the host).
-        LCU(cudaMemcpyAsync(h_assign.data(), assign, n * 4ull, cudaMemcpyDeviceToHost, s));
-        LCU(cudaStreamSynchronize(s));
-        std::fill(off.begin(), off.end(), 0u);
-        for (uint32_t i = 0; i < n; ++i) ++off[h_assign[i] + 1];
-        for (uint32_t c = 0; c < k; ++c) off[c + 1] += off[c];
-        {
-            std::vector<uint32_t> pos(off.begin(), off.end() - 1);
-            for (uint32_t i = 0; i < n; ++i) members[pos[h_assign[i]]++] = i;
-        }
-        LCU(cudaMemcpyAsync(doff.p, off.data(), (k + 1) * 4ull, cudaMemcpyHostToDevice, s));
-        LCU(cudaMemcpyAsync(dmem.p, members.data(), n * 4ull, cudaMemcpyHostToDevice, s));
+        LCU(cell_sort(assign, n, k, doff.p, dmem.p, s));
         // Last round: representatives of the final cells; otherwise new centroids.
         cell_kernel<<<k, 256, 0, s>>>(rows, d, dmem.p, doff.p, cent, it == iters ? rep : nullptr);
         LCU(cudaGetLastError());
-        LCU(cudaStreamSynchronize(s));  // the host vectors are rewritten next iteration
     }
     // Empty cells: give each a row that no other cell uses.
-    std::vector<uint32_t> h_rep(k);
+    std::vector<uint32_t> h_rep(k), off(k + 1);
     LCU(cudaMemcpyAsync(h_rep.data(), rep, k * 4ull, cudaMemcpyDeviceToHost, s));
+    LCU(cudaMemcpyAsync(off.data(), doff.p, (k + 1) * 4ull, cudaMemcpyDeviceToHost, s));
     LCU(cudaStreamSynchronize(s));
-    std::vector<uint8_t> used(n, 0);
     bool fix = false;
-    for (uint32_t c = 0; c < k; ++c)
-        if (off[c + 1] > off[c]) used[h_rep[c]] = 1;
-    uint32_t next = 0;
-    for (uint32_t c = 0; c < k; ++c) {
-        if (off[c + 1] > off[c]) continue;
-        while (used[next]) ++next;
-        used[next] = 1;
-        h_rep[c] = next;
-        fix = true;
-    }
+    for (uint32_t c = 0; c < k; ++c) fix |= off[c + 1] == off[c];
     if (fix) {
+        std::vector<uint8_t> used(n, 0);
+        for (uint32_t c = 0; c < k; ++c)
+            if (off[c + 1] > off[c]) used[h_rep[c]] = 1;
+        uint32_t next = 0;
+        for (uint32_t c = 0; c < k; ++c) {
+            if (off[c + 1] > off[c]) continue;
+            while (used[next]) ++next;
+            used[next] = 1;
+            h_rep[c] = next;
+        }
         LCU(cudaMemcpyAsync(rep, h_rep.data(), k * 4ull, cudaMemcpyHostToDevice, s));
         LCU(cudaStreamSynchronize(s));
     }

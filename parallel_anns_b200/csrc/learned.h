@@ -25,6 +25,12 @@ int set_error(int code, const std::string &msg);
 int kmeans_run(const float *rows, uint32_t n, uint32_t d, uint32_t k, uint32_t iters, uint32_t seed,
                float *centroids, uint32_t *assign, uint32_t *rep, cudaStream_t stream);
 
+// members = the n rows (device ids) listed by their cell (cell[i] < k), ids
+// ascending within a cell; cell c's rows are members[off[c]..off[c + 1]). All
+// device pointers, off of k + 1 words. Only enqueues on `stream`.
+cudaError_t cell_sort(const uint32_t *cell, uint32_t n, uint32_t k, uint32_t *off, uint32_t *members,
+                      cudaStream_t stream);
+
 // cell[i] = the nearest (squared L2, via ||c||^2 - 2 x.c; ties to the lower
 // index) of the k rows center_rows[0..k) (device) for each of the n rows
 // (device, row-major, width d). Enqueued on `stream`, synchronised.

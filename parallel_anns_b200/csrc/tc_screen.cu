@@ -45,6 +45,7 @@
 // still releases its tensor memory. No multicast anywhere.
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 #include <stdint.h>
@@ -59,6 +60,8 @@
 #include "tc_screen.h"
 
 namespace panns {
+
+namespace cg = cooperative_groups;
 namespace {
 
 constexpr uint32_t kTcSliceW = 64;     // BF16 per TMA box row (128 bytes)
@@ -929,40 +932,64 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
 // its 128 queries, each part rounded to the safe side. Per query rather than
 // ball against ball: a block's queries may lie in several clusters. One block
 // per (row block, 64 tiles), 8 x 4 distances per thread.
+//
+// Bound by the float32 distances (two operations an element; 10,000 queries x
+// 7,813 tiles x 96: 0.42 ms of them). Slices of 16 dimensions are fetched into
+// registers while the slice before is worked on and go to the other half of
+// shared memory, one barrier a slice: 0.97 ms with loads between two barriers,
+// 0.76 ms so.
 __global__ void __launch_bounds__(256) tc_need_kernel(const float *__restrict__ q, const uint32_t *__restrict__ qperm,
                                                       uint32_t nq, const float *__restrict__ tau,
                                                       const float *__restrict__ cb, const float *__restrict__ rb,
                                                       uint32_t nb, uint32_t d, float *__restrict__ need) {
-    __shared__ __align__(16) float sa[16][kTcM + 4];
-    __shared__ __align__(16) float sb[16][68];
-    __shared__ uint32_t rows[kTcM];
+    __shared__ __align__(16) float sa[2][16][kTcM + 4];
+    __shared__ __align__(16) float sb[2][16][68];
     __shared__ float st[kTcM];
     __shared__ uint32_t any[64];
     const uint32_t i0 = blockIdx.y * kTcM, t0 = blockIdx.x * 64, tid = threadIdx.x;
     const uint32_t ty = tid / 16, tx = tid % 16;
-    if (tid < kTcM) {
-        rows[tid] = i0 + tid < nq ? qperm[i0 + tid] : kNone;
-        st[tid] = i0 + tid < nq ? tau[i0 + tid] : -1.f;
-    }
+    // Thread tid brings 8 values of query tid / 2 and 4 of tile tid / 4 a slice.
+    const uint32_t ra = tid / 2, ka = tid % 2 * 8, rc = tid / 4, kc = tid % 4 * 4;
+    const float *qr = i0 + ra < nq ? q + (size_t) qperm[i0 + ra] * d : nullptr;
+    const float *cr = t0 + rc < nb ? cb + (size_t) (t0 + rc) * d : nullptr;
+    if (tid < kTcM) st[tid] = i0 + tid < nq ? tau[i0 + tid] : -1.f;
     if (tid < 64) any[tid] = 0;
-    __syncthreads();
+    float va[8], vc[4];
+    const bool quads = d % 4 == 0;
+    auto fetch4 = [&](const float *r, uint32_t k, float *v) {
+        if (quads && r && k < d) {
+            const float4 f = __ldg(reinterpret_cast<const float4 *>(r + k));
+            v[0] = f.x, v[1] = f.y, v[2] = f.z, v[3] = f.w;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = !quads && r && k + e < d ? __ldg(r + k + e) : 0.f;
+        }
+    };
+    auto fetch = [&](uint32_t k0) {
+        fetch4(qr, k0 + ka, va);
+        fetch4(qr, k0 + ka + 4, va + 4);
+        fetch4(cr, k0 + kc, vc);
+    };
+    auto store = [&](int buf) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sa[buf][ka + e][ra] = va[e];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sb[buf][kc + e][rc] = vc[e];
+    };
     float acc[8][4] = {};
-    for (uint32_t k0 = 0; k0 < d; k0 += 16) {
-        for (uint32_t e = tid; e < kTcM * 16; e += 256) {
-            const uint32_t rr = e / 16, kk = e % 16;
-            sa[kk][rr] = rows[rr] != kNone && k0 + kk < d ? q[(size_t) rows[rr] * d + k0 + kk] : 0.f;
-        }
-        for (uint32_t e = tid; e < 64 * 16; e += 256) {
-            const uint32_t rr = e / 16, kk = e % 16;
-            sb[kk][rr] = t0 + rr < nb && k0 + kk < d ? cb[(size_t) (t0 + rr) * d + k0 + kk] : 0.f;
-        }
-        __syncthreads();
+    fetch(0);
+    store(0);
+    __syncthreads();
+    int buf = 0;
+    for (uint32_t k0 = 0; k0 < d; k0 += 16, buf ^= 1) {
+        const bool more = k0 + 16 < d;
+        if (more) fetch(k0 + 16);
 #pragma unroll
         for (int kk = 0; kk < 16; ++kk) {
             float av[8];
-            const float4 a0 = *reinterpret_cast<const float4 *>(&sa[kk][ty * 8]);
-            const float4 a1 = *reinterpret_cast<const float4 *>(&sa[kk][ty * 8 + 4]);
-            const float4 b0 = *reinterpret_cast<const float4 *>(&sb[kk][tx * 4]);
+            const float4 a0 = *reinterpret_cast<const float4 *>(&sa[buf][kk][ty * 8]);
+            const float4 a1 = *reinterpret_cast<const float4 *>(&sa[buf][kk][ty * 8 + 4]);
+            const float4 b0 = *reinterpret_cast<const float4 *>(&sb[buf][kk][tx * 4]);
             av[0] = a0.x; av[1] = a0.y; av[2] = a0.z; av[3] = a0.w;
             av[4] = a1.x; av[5] = a1.y; av[6] = a1.z; av[7] = a1.w;
             const float bv[4] = {b0.x, b0.y, b0.z, b0.w};
@@ -974,7 +1001,10 @@ __global__ void __launch_bounds__(256) tc_need_kernel(const float *__restrict__ 
                     acc[i][j] = fmaf(u, u, acc[i][j]);
                 }
         }
-        __syncthreads();
+        if (more) {
+            store(buf ^ 1);
+            __syncthreads();
+        }
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -1044,72 +1074,82 @@ __global__ void __launch_bounds__(256) tc_bound_kernel(const float *__restrict__
 }
 
 // `cells` pivots by farthest-point seeding (Gonzalez, 1985) over S rows at a
-// fixed stride, S * d BF16 values in shared memory: one block of 1,024 threads,
-// thread t holding row t's distance to the pivots so far. Far-apart clusters
-// each get a pivot before any gets two, which rows taken at a stride only give
-// with many times more of them. A round is one pass over the shared rows (about
-// 1 us); BF16 distances only decide which rows are taken.
-__global__ void __launch_bounds__(1024) tc_pivot_kernel(const float *__restrict__ x, uint32_t n, uint32_t d,
-                                                        uint32_t S, uint32_t cells, uint32_t *__restrict__ pivots) {
-    extern __shared__ __align__(16) __nv_bfloat162 srow[];  // [ceil(d / 2)][S]: thread t reads column t
-    __shared__ float bv[32];
-    __shared__ uint32_t bi[32];
-    __shared__ uint32_t pick;
-    const uint32_t t = threadIdx.x, lane = t & 31, w = t >> 5, h = (d + 1) / 2;
-    for (uint32_t e = t; e < S * h; e += 1024) {
-        const uint32_t i = e / h, q = 2 * (e - i * h);
-        const float *r = x + ((uint64_t) i * n / S) * d;
-        srow[(size_t) (e - i * h) * S + i] = __floats2bfloat162_rn(r[q], q + 1 < d ? r[q + 1] : 0.f);
+// fixed stride, held as BF16 values in the shared memory of one cluster of 8
+// CTAs, 128 rows each, four threads a row. Far-apart clusters each get a pivot
+// before any gets two, which rows taken at a stride only give with many times
+// more of them. BF16 distances only decide which rows are taken.
+//
+// Bound by the latency of a round: each CTA's farthest row goes to all eight
+// (distributed shared memory), one cluster barrier, then every CTA fetches the
+// winner's row from its owner. One CTA of 1,024 threads, bound by issue, took
+// 3.6 us a round (256 rounds, d = 96); this takes 1.4 us.
+constexpr int kPivCtas = 8, kPivRows = 128;
+
+// Words per row: h rounded up to 4 mod 8, so that a warp's 8 rows x 4 words lie in 32 banks.
+__host__ __device__ constexpr uint32_t piv_stride(uint32_t h) { return (h + 3) / 8 * 8 + 4; }
+
+__global__ void __cluster_dims__(kPivCtas, 1, 1) __launch_bounds__(4 * kPivRows)
+    tc_pivot_kernel(const float *__restrict__ x, uint32_t n, uint32_t d, uint32_t S, uint32_t cells,
+                    uint32_t *__restrict__ pivots) {
+    extern __shared__ __align__(16) __nv_bfloat162 srow[];  // [kPivRows][piv_stride(h)]
+    __shared__ float2 prow[128];                             // the newest pivot's row
+    __shared__ unsigned long long wkey[16], keys[2][kPivCtas];
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, h = (d + 1) / 2, hp = piv_stride(h);
+    const uint32_t rank = cluster.block_rank(), row = tid / 4, sub = tid % 4, slot = rank * kPivRows + row;
+    for (uint32_t e = tid; e < kPivRows * h; e += 4 * kPivRows) {
+        const uint32_t i = e / h, q = 2 * (e - i * h), g = rank * kPivRows + i;
+        if (g >= S) break;
+        const float *r = x + ((uint64_t) g * n / S) * d;
+        srow[(size_t) i * hp + q / 2] = __floats2bfloat162_rn(r[q], q + 1 < d ? r[q + 1] : 0.f);
     }
-    float mind = t < S ? 3e38f : -1.f;
+    float mind = 3e38f;
     uint32_t cur = 0;
-    __syncthreads();
-    for (uint32_t c = 0; c < cells; ++c) {
-        if (t == 0) pivots[c] = (uint32_t) ((uint64_t) cur * n / S);
-        if (t < S) {
-            float s = 0.f;
-            for (uint32_t q = 0; q < h; ++q) {
-                const float2 a = __bfloat1622float2(srow[(size_t) q * S + t]);
-                const float2 b = __bfloat1622float2(srow[(size_t) q * S + cur]);
-                const float u = a.x - b.x, v = a.y - b.y;
-                s = fmaf(u, u, s);
-                s = fmaf(v, v, s);
-            }
-            mind = fminf(mind, s);
+    cluster.sync();
+    for (uint32_t c = 0;; ++c) {
+        if (rank == 0 && tid == 0) pivots[c] = (uint32_t) ((uint64_t) cur * n / S);
+        if (c + 1 == cells) break;
+        if (tid < h) {
+            const __nv_bfloat162 *owner = cluster.map_shared_rank(srow, cur / kPivRows);
+            prow[tid] = __bfloat1622float2(owner[(size_t) (cur % kPivRows) * hp + tid]);
         }
-        float best = mind;
-        uint32_t bt = t;
+        __syncthreads();
+        float s = 0.f;
+        for (uint32_t q = sub; q < h; q += 4) {
+            const float2 a = __bfloat1622float2(srow[(size_t) row * hp + q]), b = prow[q];
+            const float u = a.x - b.x, v = a.y - b.y;
+            s = fmaf(u, u, s);
+            s = fmaf(v, v, s);
+        }
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        mind = fminf(mind, s);
+        // (distance, ~slot): the farthest row, ties to the lower slot.
+        unsigned long long key = slot < S ? (unsigned long long) __float_as_uint(mind) << 32 | ~slot : 0ull;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float v2 = __shfl_xor_sync(0xffffffffu, best, o);
-            const uint32_t i2 = __shfl_xor_sync(0xffffffffu, bt, o);
-            if (v2 > best || (v2 == best && i2 < bt)) {
-                best = v2;
-                bt = i2;
-            }
+        for (int o = 4; o < 32; o *= 2) {
+            const unsigned long long k2 = __shfl_xor_sync(0xffffffffu, key, o);
+            key = k2 > key ? k2 : key;
         }
-        if (lane == 0) {
-            bv[w] = best;
-            bi[w] = bt;
-        }
+        if (lane == 0) wkey[w] = key;
         __syncthreads();
         if (w == 0) {
-            best = bv[lane];
-            bt = bi[lane];
+            key = wkey[lane % 16];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float v2 = __shfl_xor_sync(0xffffffffu, best, o);
-                const uint32_t i2 = __shfl_xor_sync(0xffffffffu, bt, o);
-                if (v2 > best || (v2 == best && i2 < bt)) {
-                    best = v2;
-                    bt = i2;
-                }
+            for (int o = 1; o < 16; o *= 2) {
+                const unsigned long long k2 = __shfl_xor_sync(0xffffffffu, key, o);
+                key = k2 > key ? k2 : key;
             }
-            if (lane == 0) pick = bt < S ? bt : 0u;
+            if (lane < kPivCtas) *cluster.map_shared_rank(&keys[c & 1][rank], lane) = key;
         }
-        __syncthreads();
-        cur = pick;
+        // Keys of the next round go to the other half, so one barrier a round is enough.
+        cluster.sync();
+        key = keys[c & 1][0];
+#pragma unroll
+        for (int i = 1; i < kPivCtas; ++i) key = keys[c & 1][i] > key ? keys[c & 1][i] : key;
+        cur = ~(uint32_t) key;
     }
+    cluster.sync();  // no CTA leaves while another may read its rows
 }
 
 // Counting sort of the rows by cell: the order within a cell is the order the
@@ -1200,9 +1240,9 @@ bool tc_screen_supported(uint32_t n, uint32_t d, uint32_t C) {
     return d % 32 == 0 && d >= 32 && d <= 128 && C >= 1 && C <= 128 && C < n && n >= kTcM;
 }
 
-// Two tiles' worth of rows per pivot up to 256 of them: the pivots are chosen
-// one after the other (256 take 0.3 ms), and on a base of 64 clusters 64 are
-// enough.
+// 32 rows a pivot (two tiles' worth where cells are padded) up to 256 pivots: they
+// are chosen one after the other (256 take 0.37 ms), and on a base of 64 clusters
+// 64 are enough.
 static uint32_t tc_pivots(uint32_t n, bool padded) {
     return std::max(1u, std::min(256u, n / (padded ? 2 * kTcM : 32)));
 }
@@ -1213,14 +1253,15 @@ int tc_locality_order(const float *x, uint32_t n, uint32_t d, bool padded, uint3
                       cudaStream_t s) {
     if (d == 0 || d > 256) return set_error(PANNS_EINVAL, "tc screen: unsupported shape");
     const uint32_t cells = tc_pivots(n, padded);
-    const uint32_t h = (d + 1) / 2, S = std::min(n, std::min(1024u, 200u * 1024u / (h * 4)));
+    const uint32_t h = (d + 1) / 2, S = std::min(n, (uint32_t) (kPivCtas * kPivRows));
+    const uint32_t psmem = kPivRows * piv_stride(h) * 4;
     std::vector<uint32_t> count(cells);
     TBuf<uint32_t> dpiv, cell, start;
     TCU(dpiv.alloc(cells, s));
     TCU(cell.alloc(n, s));
     TCU(start.alloc(cells, s));
-    TCU(cudaFuncSetAttribute(tc_pivot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (S * h * 4)));
-    tc_pivot_kernel<<<1, 1024, S * h * 4, s>>>(x, n, d, S, cells, dpiv.p);
+    TCU(cudaFuncSetAttribute(tc_pivot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) psmem));
+    tc_pivot_kernel<<<kPivCtas, 4 * kPivRows, psmem, s>>>(x, n, d, S, cells, dpiv.p);
     TCU(cudaGetLastError());
     const int rc = nearest_center(x, n, d, dpiv.p, cells, cell.p, s);
     if (rc) return rc;

@@ -56,4 +56,12 @@ void scratch_trim(int device) {
     if (pool) cudaMemPoolTrimTo(pool, 0);
 }
 
+cudaError_t allow_shared(const void *kern) {
+    cudaFuncAttributes a{};
+    const cudaError_t e = cudaFuncGetAttributes(&a, kern);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int) ((227u << 10) - a.sharedSizeBytes));
+}
+
 }  // namespace panns

@@ -28,6 +28,12 @@ void scratch_free(void *p, cudaStream_t s);
 // Give the device's idle pool memory back to the driver.
 void scratch_trim(int device);
 
+// Let `kern` be launched with as much dynamic shared memory as a block can have.
+// The limit is a property of the kernel, not of a launch: set to each launch's
+// own size, one thread's launch could fail on the smaller size another thread has
+// set in between.
+cudaError_t allow_shared(const void *kern);
+
 template <typename T>
 struct Scratch {
     T *p = nullptr;

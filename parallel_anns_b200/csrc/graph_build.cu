@@ -908,7 +908,7 @@ __global__ void __launch_bounds__(256) parent_kernel(const uint32_t *__restrict_
 static int screen_fp32(const float *x, uint32_t n, uint32_t d, const float *xn, uint32_t C, const uint32_t *rows,
                        uint32_t nr, uint32_t *cand, cudaStream_t s) {
     const size_t smem = (size_t) (kBK * kBQ + kBK * kBV + kBQ * (kBV + 1)) * 4 + (size_t) kBQ * C * 8 + kBQ * 8;
-    GCU(cudaFuncSetAttribute(screen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+    GCU(allow_shared((const void *) screen_kernel));
     screen_kernel<<<(nr + kBQ - 1) / kBQ, 256, smem, s>>>(x, n, d, xn, C, rows, nr, cand);
     GCU(cudaGetLastError());
     return PANNS_OK;
@@ -990,8 +990,7 @@ static int finish_graph(int device, const float *x, uint32_t n, uint32_t d, uint
         uint32_t *prc = pr.p + (size_t) a0 * R;
         if (d % 4 == 0 && per_warp <= 112u * 1024u) {
             const uint32_t wpb = std::max(1u, std::min(4u, 112u * 1024u / per_warp));
-            GCU(cudaFuncSetAttribute(prune_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int) (wpb * per_warp)));
+            GCU(allow_shared((const void *) prune_rows_kernel));
             prune_rows_kernel<<<(na + wpb - 1) / wpb, wpb * 32, wpb * per_warp, s>>>(x, n, d, kn, knn_d.p, k, R, na, prc,
                                                                                     deg.p + a0);
         } else {
@@ -1387,7 +1386,7 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
         GCU(cudaMemcpyAsync(dbr.p, blk_row0.data(), blk_row0.size() * 4, cudaMemcpyHostToDevice, s));
         const size_t smem = (size_t) (kBK * kBQ + kBK * kBV + kBQ * (kBV + 1)) * 4 + (size_t) kBQ * C * 8 +
                             (size_t) kBQ * 8 + (size_t) kBV * 4;
-        GCU(cudaFuncSetAttribute(screen_cells_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+        GCU(allow_shared((const void *) screen_cells_kernel));
         screen_cells_kernel<<<(unsigned) blk_cell.size(), 256, smem, s>>>(x.p, n, d, xn.p, C, dmem.p, dstart.p,
                                                                            dnear.p, P, dbc.p, dbr.p, cand.p);
         GCU(cudaGetLastError());

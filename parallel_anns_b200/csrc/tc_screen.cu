@@ -1218,8 +1218,7 @@ TcShape tc_shape(uint32_t d) {
 
 template <int FORM>
 int tc_launch(const CUtensorMap &ma, const CUtensorMap &mb, const TcArgs &a, size_t smem, int num_sms, cudaStream_t s) {
-    TCU(cudaFuncSetAttribute((const void *) tc_screen_kernel<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int) smem));
+    TCU(allow_shared((const void *) tc_screen_kernel<FORM>));
     TCU(cudaMemsetAsync(a.counter, 0, 4, s));
     tc_screen_kernel<FORM><<<std::min<uint32_t>(a.items, (uint32_t) num_sms), kTcThreads, smem, s>>>(ma, mb, a);
     TCU(cudaGetLastError());
@@ -1260,7 +1259,7 @@ int tc_locality_order(const float *x, uint32_t n, uint32_t d, bool padded, uint3
     TCU(dpiv.alloc(cells, s));
     TCU(cell.alloc(n, s));
     TCU(start.alloc(cells, s));
-    TCU(cudaFuncSetAttribute(tc_pivot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) psmem));
+    TCU(allow_shared((const void *) tc_pivot_kernel));
     tc_pivot_kernel<<<kPivCtas, 4 * kPivRows, psmem, s>>>(x, n, d, S, cells, dpiv.p);
     TCU(cudaGetLastError());
     const int rc = nearest_center(x, n, d, dpiv.p, cells, cell.p, s);
@@ -1313,7 +1312,7 @@ int tc_screen_knn(const float *x, uint32_t n, uint32_t d, uint32_t k, uint32_t C
     TCU(cudaMemsetAsync(ctl.p, 0, 16, s));
     TCU(cudaMemsetAsync(fail_count, 0, 4, s));
     tc_shift_kernel<<<d, 256, 0, s>>>(x, n, d, shift.p);
-    TCU(cudaFuncSetAttribute(tc_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (kTcM * d * 4)));
+    TCU(allow_shared((const void *) tc_prepare_kernel));
     tc_prepare_kernel<<<tiles, 256, kTcM * d * 4, s>>>(x, n, d, perm, 0, slots, sh.W, shift.p,
                                                        per == tiles ? A.p : nullptr, B.p, xn.p, ctl.p + 2, nullptr,
                                                        centre.p, radius.p);
@@ -1411,7 +1410,7 @@ int tc_screen_range(const float *x, uint32_t n, uint32_t d, const uint32_t *perm
     TCU(cudaMemsetAsync(cnt, 0, (size_t) splits * nq * 4, s));
     tc_shift_kernel<<<d, 256, 0, s>>>(x, n, d, shift.p);
     tc_tau_kernel<<<(nq + 255) / 256, 256, 0, s>>>(tau, nq, ft.p);
-    TCU(cudaFuncSetAttribute(tc_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (kTcM * d * 4)));
+    TCU(allow_shared((const void *) tc_prepare_kernel));
     tc_prepare_kernel<<<rb, 256, kTcM * d * 4, s>>>(queries, kNone, d, qperm, 0, nq, sh.W, shift.p, A.p, nullptr, xn.p,
                                                     nullptr, ctl.p + 3, nullptr, nullptr);
     TCU(cudaGetLastError());

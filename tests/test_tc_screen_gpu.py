@@ -75,3 +75,31 @@ def test_ground_truth_with_loose_bounds():
     oids, odist = O.ground_truth(x, q, 20)
     assert np.array_equal(ids, oids)
     np.testing.assert_allclose(dist, odist, rtol=34 * 2.0 ** -52, atol=0)
+
+
+def test_threads_with_different_widths():
+    """Constructions and ground truths of different widths at the same time."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    from parallel_anns_b200.graph import build_nsg
+    from parallel_anns_b200.searching import Index, ground_truth
+
+    def work(d):
+        x, q = _data("mix", 3000, d, d), _data("mix", 70, d, d)
+        got = []
+        for _ in range(6):
+            g = build_nsg(x, R=16, knn_k=24)
+            with Index(0) as ix:
+                ix.set_base(x)
+                ix.set_graph(g)
+                got.append((g.entry, g.nbrs, *ground_truth(ix, q, 10)))
+        return got
+
+    widths = [8, 64, 136, 256]
+    with ThreadPoolExecutor(len(widths)) as pool:
+        for d, got in zip(widths, pool.map(work, widths)):
+            x, q = _data("mix", 3000, d, d), _data("mix", 70, d, d)
+            og, _ = O.build_nsg(x, 24, 16)
+            oids, _ = O.ground_truth(x, q, 10)
+            for entry, nbrs, ids, _ in got:
+                assert entry == og.entry and np.array_equal(nbrs, og.nbrs) and np.array_equal(ids, oids), d

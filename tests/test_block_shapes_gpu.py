@@ -46,3 +46,31 @@ def test_block_shapes_equal_one_warp_and_oracle(n, d, deg, L, M, integer):
         assert np.array_equal(many, np.repeat(one, 80, axis=0)) and sm["n_dist"] == 80 * s1["n_dist"]
     ref, nd = O.search_top_m(x, O.Graph.from_nsg(g), q, K, L, M)
     assert np.array_equal(one, ref) and s1["n_dist"] == nd
+
+
+@pytest.mark.parametrize("n,shared", [(2_000_003, False), (40_000, True)])
+def test_one_warp_and_pss_with_either_bitset(n, shared):
+    """PSS_v5, efanna2e and the one-warp kernel on a base whose visited bits fit
+    shared memory and on one where they do not."""
+    from parallel_anns_b200 import native as N
+    from parallel_anns_b200.searching import Index
+    rng = np.random.default_rng(n)
+    d, L, K = 16, 60, 20
+    x, q = rng.random((n, d), dtype=np.float32), rng.random((70, d), dtype=np.float32)
+    g = _random_graph(n, 12, 3)
+    og = O.Graph.from_nsg(g)
+    assert shared == (n // 8 < 200_000)
+    with Index(0) as ix:
+        ix.set_base(x)
+        ix.set_graph(g)
+        for T, X in ((1, 1), (4, 2), (7, 1)):
+            ids, s = ix.search(q, K=K, L=L, mode=N.MODE_PSS_V5, distance=N.DIST_L2, T=T, X=X)
+            ref, nd = O.search_pss(x, og, q, K, L, L, X, T, kind=O.DIST_L2)
+            assert np.array_equal(ids, ref) and s["n_dist"] == nd, (T, X)
+        init = ix.efanna_init_ids(L, q.shape[0])
+        ids, s = ix.search(q, K=K, L=L, mode=N.MODE_EFANNA, distance=N.DIST_L2, init_ids=init)
+        ref, nd = O.search_efanna(x, og, q, K, L, init_ids=init)
+        assert np.array_equal(ids, ref) and s["n_dist"] == nd
+        ids, s = ix.search(q, K=K, L=L, mode=N.MODE_TOP_M, M=3, distance=N.DIST_L2, warps_per_query=1)
+        ref, nd = O.search_top_m(x, og, q, K, L, 3, kind=O.DIST_L2)
+        assert np.array_equal(ids, ref) and s["n_dist"] == nd

@@ -93,8 +93,8 @@ typedef struct {
                                  block; NSG_SEQ, TOP_M, PSS_V5 at T = 1, any storage, with or
                                  without PANNS_FLAG_LEARNED), for small batches and long queues; same
                                  ids and counts.
-                                 0: chosen from nq and L (8 up to one query per SM or for L >= 2048,
-                                 2 up to ten per SM, else 1) when the mode allows it and
+                                 0: chosen (1, 2, 4, 8 or 16) by how many waves of queries each
+                                 takes and how long a wave is, when the mode allows it and
                                  warps_per_block and blocks_per_sm are 0, else 1 */
 } panns_search_params;
 
@@ -124,7 +124,8 @@ uint32_t panns_version(void);
  * PANNS::Searching (PSS.h:30-226) / efanna2e::IndexNSG (NSG.h:17-43). */
 int panns_open(panns_index **out, int device);
 /* Release all host and device memory of the handle (Searching::~Searching,
- * PSS.h:213-226). */
+ * PSS.h:213-226), and the device's idle scratch memory (a pool of at most 2 GiB
+ * that constructions, training and ground truths share). */
 int panns_close(panns_index *h);
 
 /* Base vectors, n x d float32 row-major (host pointer, copied).
@@ -218,9 +219,10 @@ int panns_recall(const uint32_t *result_ids, uint32_t nq, uint32_t K, const uint
 /* Float64 brute-force ground truth on the GPU: the top-k ids (original ids)
  * by exact squared L2 in float64, ties by id, for nq host queries (nq x d
  * float32); out_dist (optional) gets the float64 distances. Needs the base
- * and the graph: a search gives each query a distance bound, one float64
- * pass over all N collects the vertices within it, and an exact sort of those
- * gives the answer. Plays the role of tools/save_true_nearest_neighbors.cpp:16-64
+ * and the graph: a search gives each query a distance bound, a tensor-core
+ * screen with a proven error bound collects the vertices within it (k <= 512;
+ * one float64 pass over all N beyond that, and for queries whose bound holds
+ * too many), and those are ranked exactly in float64. Plays the role of tools/save_true_nearest_neighbors.cpp:16-64
  * (which scans in float32). */
 int panns_ground_truth(panns_index *h, const float *queries, uint32_t nq, uint32_t k, uint32_t *out_ids,
                        double *out_dist);

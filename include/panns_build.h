@@ -14,8 +14,8 @@
  * entry = argmin over v of (d64(v, mean), v) with mean = the float64 mean of
  * the rows; repair: every vertex not reachable from the entry, in id order,
  * gets an in-edge from the first reachable vertex of its k-NN list (else from
- * the entry). The k-NN lists come from a float32 screen of all pairs keeping
- * k + 8 candidates per row, ranked exactly in float64.
+ * the entry). The k-NN lists come from a screen of all pairs (below), ranked
+ * exactly in float64.
  */
 #ifndef PANNS_BUILD_H
 #define PANNS_BUILD_H
@@ -30,11 +30,15 @@ typedef struct panns_graph panns_graph;
 
 /* k-NN screen of the build: all pairs in float32 on CUDA cores keeping k + 8
  * candidates per row; by TF32 tensor-core GEMMs (cuBLAS) keeping k + 32; or
- * by the library's own tcgen05 kernel (TF32 MMAs into tensor memory, TMA-fed,
- * the per-row selection in the epilogue, no distance tile written; d a
- * multiple of 32 up to 128) keeping k + 32. Either way the candidates are
- * ranked exactly in float64. AUTO: the tcgen05 kernel from 100,000 vectors on
- * where it applies, else TF32 from 100,000 vectors on, else float32. */
+ * by the library's own tcgen05 kernel (operands split in two BF16 parts, TMA
+ * into shared memory, accumulators in tensor memory), which hands on every
+ * pair within a threshold that provably holds all k nearest, and skips tiles
+ * whose ball is out of reach. Either way the candidates are ranked exactly in
+ * float64. AUTO: the tcgen05 kernel for n >= 1,024 and d <= 256 (rows it
+ * cannot settle - non-finite values, more equal distances than its lists
+ * hold - go through the float32 screen), else float32 below 100,000 vectors
+ * and TF32 from there on. Chosen by name, PANNS_SCREEN_TC asks for d a
+ * multiple of 32 up to 128. */
 #define PANNS_SCREEN_AUTO 0u
 #define PANNS_SCREEN_FP32 1u
 #define PANNS_SCREEN_TF32 2u
@@ -56,9 +60,11 @@ int panns_build_nsg_ex(int device, const float *base, uint32_t n, uint32_t d, ui
  * vertex goes to its nearest centroid), and the k-NN list of vertex a holds
  * the knn_k vertices b != a with the smallest (d64(a, b), b) among the
  * members of a's cell and of the `probe` cells whose centroids are nearest to
- * it (by float64 squared distance, then index). The candidates come from a
- * float32 screen keeping k + 8 per row, ranked exactly in float64; prune,
- * entry and repair are those of panns_build_nsg. probe <= 8; a list with
+ * it (by float64 squared distance, then index). The candidates come from the
+ * tcgen05 screen with every cell padded to whole tiles where d <= 256, padding
+ * at most doubles the rows and its operands fit the free memory, else from a
+ * float32 screen keeping k + 8 per row; they are ranked exactly in float64.
+ * Prune, entry and repair are those of panns_build_nsg. probe <= 8; a list with
  * fewer than knn_k candidates is shorter. With `reverse` set, before the
  * repair every pruned edge a -> b (a ascending, then list order) also gives
  * b -> a while b has fewer than R neighbours and not a already (the part
@@ -86,6 +92,8 @@ int panns_graph_copy(const panns_graph *g, uint64_t *offsets, uint32_t *nbrs, ui
  * panns_load_nsg / Searching::load_nsg_graph read. */
 int panns_graph_save_nsg(const panns_graph *g, const char *path);
 
+/* Release the graph. Its k-NN lists stay in device memory until then (lists of
+ * more than 4 GiB are kept on the host). */
 int panns_graph_free(panns_graph *g);
 
 /* efanna2e's own NSG construction, IndexNSG::Build

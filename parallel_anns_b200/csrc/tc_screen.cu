@@ -767,11 +767,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 
 // ---- operands, balls, bounds -------------------------------------------------
 
-__device__ __forceinline__ void bf16_split(float x, __nv_bfloat16 &h, __nv_bfloat16 &l) {
-    h = __float2bfloat16_rn(x);
-    l = __float2bfloat16_rn(x - __bfloat162float(h));
-}
-
 // shift = the mean of up to 4,096 rows at a fixed stride (one block per
 // dimension). Distances do not change under a shift, and the error bound
 // follows the norms, so data far from the origin loses nothing. (x - shift
@@ -804,7 +799,11 @@ __global__ void __launch_bounds__(256) tc_shift_kernel(const float *__restrict__
 //   leaves float32's safe range;
 //   the tile's centre (mean of its rows) and radius (rounded up; a tile without
 //   rows gets one that puts it out of every reach), not shifted.
-// Null outputs are skipped. Bound by HBM: 1M x 96 as columns, 1.0 GB moved.
+// Null outputs are skipped. Bound by issue: a lane keeps its column pairs in
+// registers from the norm to the two operands. 1M x 96 as columns: 0.72 ms with
+// 440 instructions a row, 0.49 ms so.
+constexpr int kPrepSteps = 5;  // 64-wide steps of an operand row: W <= 320
+
 __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict__ x, uint32_t n, uint32_t d,
                                                          const uint32_t *__restrict__ perm, uint32_t p0,
                                                          uint32_t valid, uint32_t W, const float *__restrict__ shift,
@@ -817,20 +816,29 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
     __shared__ float c[256], sh[256];
     __shared__ float rmax[8], nmax[8];
     const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, t0 = blockIdx.x * kTcM;
+    bool filled = false;
     if (tid < kTcM) {
         const uint32_t p = p0 + t0 + tid;
         const uint32_t row = p < valid ? (perm ? perm[p] : p) : kNone;
-        rows[tid] = row < n ? row : kNone;
+        filled = row < n;
+        rows[tid] = filled ? row : kNone;
     }
     if (tid < d) sh[tid] = shift[tid];
-    __syncthreads();
+    const uint32_t count = (uint32_t) __syncthreads_count(filled);
     if (d % 4 == 0) {
-        const uint32_t d4 = d / 4;
+        const uint32_t d4 = d / 4, di = 256 / d4, dq = 256 - di * d4;
         float4 *t4 = reinterpret_cast<float4 *>(tile);
+        uint32_t i = tid / d4, q = tid - i * d4;
+#pragma unroll 4
         for (uint32_t e = tid; e < kTcM * d4; e += 256) {
-            const uint32_t i = e / d4, q = e - i * d4;
             t4[e] = rows[i] != kNone ? __ldg(reinterpret_cast<const float4 *>(x + (size_t) rows[i] * d) + q)
                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+            i += di;
+            q += dq;
+            if (q >= d4) {
+                q -= d4;
+                ++i;
+            }
         }
     } else {
         for (uint32_t e = tid; e < kTcM * d; e += 256) {
@@ -841,13 +849,26 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
     __syncthreads();
     float nm = 0.f;
     bool big = false;
+    const bool even = d % 2 == 0;
     for (uint32_t i = w; i < kTcM; i += 8) {
         const bool have = rows[i] != kNone;
         const float *xr = tile + (size_t) i * d;
+        // The lane's column pairs 2 lane + 64 t, shifted.
+        float2 v[kPrepSteps];
         double s = 0.0;
-        for (uint32_t e = lane; e < d; e += 32) {
-            const double v = have ? (double) (xr[e] - sh[e]) : 0.0;
-            s = fma(v, v, s);
+#pragma unroll
+        for (int t = 0; t < kPrepSteps; ++t) {
+            const uint32_t e = 2 * lane + 64 * t;
+            v[t] = make_float2(0.f, 0.f);
+            if (64u * t >= d) continue;
+            if (have && e + 1 < d) {
+                float2 y = even ? *reinterpret_cast<const float2 *>(xr + e) : make_float2(xr[e], xr[e + 1]);
+                v[t] = make_float2(y.x - sh[e], y.y - sh[e + 1]);
+            } else if (have && e < d) {
+                v[t].x = xr[e] - sh[e];
+            }
+            s = fma((double) v[t].x, (double) v[t].x, s);
+            s = fma((double) v[t].y, (double) v[t].y, s);
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -859,30 +880,34 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
         const float r1 = have ? nf - __bfloat162float(n1) : 0.f;
         const __nv_bfloat16 n2 = __float2bfloat16_rn(r1);
         const __nv_bfloat16 n3 = __float2bfloat16_rn(r1 - __bfloat162float(n2));
-        for (uint32_t e = 2 * lane; e < W; e += 64) {
-            __nv_bfloat16 ah[2], al[2], bh[2], bl[2];
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const uint32_t q = e + j;
-                ah[j] = al[j] = bh[j] = bl[j] = __float2bfloat16_rn(0.f);
-                if (q < d) {
-                    const float v = have ? xr[q] - sh[q] : 0.f;
-                    bf16_split(v, ah[j], al[j]);
-                    bh[j] = __float2bfloat16_rn(-2.f * __bfloat162float(ah[j]));
-                    bl[j] = __float2bfloat16_rn(-2.f * __bfloat162float(al[j]));
-                } else if (q < d + 3) {
-                    ah[j] = __float2bfloat16_rn(1.f);
-                    bh[j] = q == d ? n1 : q == d + 1 ? n2 : n3;
-                }
-            }
+        for (int t = 0; t < kPrepSteps; ++t) {
+            const uint32_t e = 2 * lane + 64 * t;
+            if (64u * t >= W) break;
+            __nv_bfloat162 hi = __floats2bfloat162_rn(v[t].x, v[t].y);
+            const float2 hf = __bfloat1622float2(hi);
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(v[t].x - hf.x, v[t].y - hf.y);
             const size_t at = (size_t) (t0 + i) * 2 * W + e;
+            const __nv_bfloat16 one = __float2bfloat16_rn(1.f);
+            const uint32_t k0 = e - d, k1 = e + 1 - d;  // 0, 1, 2: the norm's parts
             if (A) {
-                *reinterpret_cast<__nv_bfloat162 *>(A + at) = __halves2bfloat162(ah[0], ah[1]);
-                *reinterpret_cast<__nv_bfloat162 *>(A + at + W) = __halves2bfloat162(al[0], al[1]);
+                __nv_bfloat162 a = hi;
+                if (e + 1 >= d) {
+                    if (k0 < 3u) a.x = one;
+                    if (k1 < 3u) a.y = one;
+                }
+                *reinterpret_cast<__nv_bfloat162 *>(A + at) = a;
+                *reinterpret_cast<__nv_bfloat162 *>(A + at + W) = lo;
             }
             if (B) {
-                *reinterpret_cast<__nv_bfloat162 *>(B + at) = __halves2bfloat162(bh[0], bh[1]);
-                *reinterpret_cast<__nv_bfloat162 *>(B + at + W) = __halves2bfloat162(bl[0], bl[1]);
+                const float2 lf = __bfloat1622float2(lo);
+                __nv_bfloat162 b = __floats2bfloat162_rn(-2.f * hf.x, -2.f * hf.y);
+                if (e + 1 >= d) {
+                    if (k0 < 3u) b.x = k0 == 0 ? n1 : k0 == 1 ? n2 : n3;
+                    if (k1 < 3u) b.y = k1 == 0 ? n1 : k1 == 1 ? n2 : n3;
+                }
+                *reinterpret_cast<__nv_bfloat162 *>(B + at) = b;
+                *reinterpret_cast<__nv_bfloat162 *>(B + at + W) = __floats2bfloat162_rn(-2.f * lf.x, -2.f * lf.y);
             }
         }
     }
@@ -894,15 +919,11 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
         atomicMax(ymax, __float_as_uint(nm));
     }
     if (!centre) return;
-    uint32_t have = 0;
-    float s = 0.f;
-    for (uint32_t i = 0; i < kTcM; ++i) {
-        if (rows[i] == kNone) continue;
-        ++have;
-        if (tid < d) s += tile[(size_t) i * d + tid];
-    }
-    if (tid < d) {
-        c[tid] = have ? s / (float) have : 0.f;
+    if (tid < d) {  // positions without a row hold zeros
+        float s = 0.f;
+#pragma unroll 16
+        for (uint32_t i = 0; i < kTcM; ++i) s += tile[(size_t) i * d + tid];
+        c[tid] = count ? s / (float) count : 0.f;
         centre[(size_t) blockIdx.x * d + tid] = c[tid];
     }
     __syncthreads();
@@ -923,7 +944,7 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
     if (tid == 0) {
         float q = 0.f;
         for (int i = 0; i < 8; ++i) q = rmax[i] > q || rmax[i] != rmax[i] ? rmax[i] : q;
-        radius[blockIdx.x] = have ? sqrtf(q) * 1.00002f + 1e-18f : -1e30f;
+        radius[blockIdx.x] = count ? sqrtf(q) * 1.00002f + 1e-18f : -1e30f;
     }
 }
 

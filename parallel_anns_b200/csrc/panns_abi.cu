@@ -1358,8 +1358,20 @@ int panns_ground_truth(panns_index *h, const float *queries, uint32_t nq, uint32
     // exactly: the queries grouped by locality, in batches that bound the
     // lists; those whose lists overflow again with the bound their first
     // vertices gave, and what is still over goes to step 3.
+    //
+    // A few queries go to step 3 at once: it costs 2e-10 ms for each (query, with
+    // the 64 of a tile filled, x vertex x dimension) and 6e-5 ms for each of the
+    // nq k results sorted on the host, the screen at least 0.25 ms and a pass over
+    // the base's operands, more with the tiles that a whole row block of queries
+    // reaches. Screen / step 3 in ms: 20,000 x 56, k = 10: 1 query 0.40 / 0.20, 256
+    // 0.45 / 0.37, 600 0.62 / 0.61; 100,000 x 96, k = 10: 64 queries 0.78 / 0.38, 256
+    // 0.79 / 0.82; k = 100: 10 queries 0.66 / 0.41, 128 0.88 / 1.27; 400,000 x 96, k =
+    // 10: 1 query 0.77 / 0.74, 128 1.61 / 1.27, 256 1.49 / 2.25.
+    const double base_work = (double) h->n * h->d;
+    const double direct_ms = 2e-10 * base_work * ((nq + kGtQ - 1) / kGtQ * kGtQ) + 6e-5 * nq * k;
+    const double screen_ms = 0.25 + 7e-9 * base_work * (nq >= 32 ? 3 : 1);
     std::vector<uint32_t> left;  // queries the tiled pass collects
-    if (k > kGtMaxK) {
+    if (k > kGtMaxK || (direct_ms <= screen_ms && direct_ms <= 1.5)) {
         left.resize(nq);
         for (uint32_t q = 0; q < nq; ++q) left[q] = q;
     } else {

@@ -55,6 +55,24 @@ def test_ground_truth_equals_oracle(n, d, nq, k, kind):
     np.testing.assert_allclose(dist, odist, rtol=(d + 2) * 2.0 ** -52, atol=0)
 
 
+@pytest.mark.parametrize("n,d,k,kind", [(6000, 32, 10, "ties"), (3001, 96, 1, "far"), (6000, 24, 100, "mix")])
+def test_ground_truth_of_few_and_of_many_queries(n, d, k, kind):
+    """Few queries take the tiled pass, many the screen: the same answers."""
+    from parallel_anns_b200.graph import build_nsg
+    from parallel_anns_b200.searching import Index, ground_truth
+    x = _data(kind, n, d, n)
+    q = _data("far" if kind == "far" else "mix", 5000, d, n)
+    q[-1] = x[0]
+    oids, odist = O.ground_truth(x, q, k)
+    with Index(0) as ix:
+        ix.set_base(x)
+        ix.set_graph(build_nsg(x, R=16, knn_k=24))
+        for nq in (1, 31, 33, 5000):
+            ids, dist = ground_truth(ix, q[-nq:], k)
+            assert np.array_equal(ids, oids[-nq:]), nq
+            np.testing.assert_allclose(dist, odist[-nq:], rtol=(d + 2) * 2.0 ** -52, atol=0)
+
+
 def test_ground_truth_with_loose_bounds():
     """Two groups no edge joins: searches for the second see only the first, so
     their bounds hold more vertices than a list does and are refined."""
@@ -68,6 +86,28 @@ def test_ground_truth_with_loose_bounds():
     off = np.concatenate([half.offsets, half.offsets[1:] + half.offsets[-1]])
     nbrs = np.concatenate([half.nbrs, half.nbrs + 5000]).astype(np.uint32)
     q = (rng.random((150, 32), dtype=np.float32) + np.float32(0.5)).astype(np.float32)
+    with Index(0) as ix:
+        ix.set_base(x)
+        ix.set_graph(NSGGraph(half.width, half.entry, off, nbrs))
+        ids, dist = ground_truth(ix, q, 20)
+    oids, odist = O.ground_truth(x, q, 20)
+    assert np.array_equal(ids, oids)
+    np.testing.assert_allclose(dist, odist, rtol=34 * 2.0 ** -52, atol=0)
+
+
+def test_ground_truth_with_loose_bounds_of_many_queries():
+    """The same with as many queries as the screen takes, so that its lists
+    overflow and are refined."""
+    from parallel_anns_b200.formats import NSGGraph
+    from parallel_anns_b200.graph import build_nsg
+    from parallel_anns_b200.searching import Index, ground_truth
+    rng = np.random.default_rng(4)
+    a = rng.random((5000, 32), dtype=np.float32)
+    x = np.concatenate([a, a + np.float32(0.5)])
+    half = build_nsg(a, R=16, knn_k=24)
+    off = np.concatenate([half.offsets, half.offsets[1:] + half.offsets[-1]])
+    nbrs = np.concatenate([half.nbrs, half.nbrs + 5000]).astype(np.uint32)
+    q = (rng.random((3000, 32), dtype=np.float32) + np.float32(0.5)).astype(np.float32)
     with Index(0) as ix:
         ix.set_base(x)
         ix.set_graph(NSGGraph(half.width, half.entry, off, nbrs))

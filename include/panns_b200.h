@@ -221,8 +221,8 @@ int panns_recall(const uint32_t *result_ids, uint32_t nq, uint32_t K, const uint
  * float32); out_dist (optional) gets the float64 distances. Needs the base
  * and the graph: a search gives each query a distance bound, a tensor-core
  * screen with a proven error bound collects the vertices within it (k <= 512;
- * one float64 pass over all N beyond that, and for queries whose bound holds
- * too many), and those are ranked exactly in float64. Plays the role of tools/save_true_nearest_neighbors.cpp:16-64
+ * one float64 pass over all N beyond that, for a few queries, and for queries
+ * whose bound holds too many), and those are ranked exactly in float64. Plays the role of tools/save_true_nearest_neighbors.cpp:16-64
  * (which scans in float32). */
 int panns_ground_truth(panns_index *h, const float *queries, uint32_t nq, uint32_t k, uint32_t *out_ids,
                        double *out_dist);

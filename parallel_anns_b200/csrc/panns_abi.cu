@@ -178,6 +178,7 @@ struct panns_index {
     DevBuf<uint32_t> orig;
     // graph
     uint32_t width = 0, entry = 0, gn = 0, max_deg = 0;
+    uint32_t entry_distinct = 0;  // leading neighbours of the entry before the first repeated one
     std::vector<uint64_t> off;
     std::vector<uint32_t> nbrs;
     DevBuf<uint32_t> head, ovf;
@@ -391,6 +392,12 @@ int panns_set_graph(panns_index *h, uint32_t width, uint32_t entry, const uint64
     h->width = width;
     h->entry = entry;
     h->gn = n;
+    {
+        std::vector<uint8_t> seen(n, 0);
+        uint64_t e = offsets[entry];
+        for (; e < offsets[entry + 1] && !seen[nbrs[e]]; ++e) seen[nbrs[e]] = 1;
+        h->entry_distinct = (uint32_t) (e - offsets[entry]);
+    }
     h->ready = false;
     return PANNS_OK;
 }
@@ -1123,6 +1130,11 @@ static int stage_init(panns_index *h, const panns_search_params *p, const uint32
     const uint32_t *ids = init_ids;
     if (!ids) {
         if (efanna) {
+            // The lists begin with the entry's neighbours as the graph holds them
+            // (the rest is drawn without repeats), so one that is there twice is in
+            // every list.
+            if (std::min<uint64_t>(L, h->off[h->entry + 1] - h->off[h->entry]) > h->entry_distinct)
+                return fail(PANNS_EINVAL, "search: duplicate init id");
             int32_t st[40];
             panns_rand_seed(st, 1);
             buf.resize((size_t) nq * L);
@@ -1135,8 +1147,9 @@ static int stage_init(panns_index *h, const panns_search_params *p, const uint32
         }
         ids = buf.data();
     }
-    // Valid, distinct vertices per list (the caller's are checked; the ones made
-    // above are); handed over as device ids in the same order.
+    // Valid, distinct vertices per list (the caller's are checked one by one; the
+    // ones made above are distinct by construction or were refused there); handed
+    // over as device ids in the same order.
     const uint32_t groups = efanna ? nq : 1;
     std::vector<uint32_t> dev((size_t) groups * L);
     if (!init_ids)

@@ -170,8 +170,10 @@ int panns_efanna_init_ids(const panns_index *h, uint32_t L, uint32_t nq, int32_t
  * init_ids: L ids shared by all queries (NSG_SEQ, TOP_M, PSS_V5; NULL = the
  * panns_prepare_init_ids list) or nq x L per query (EFANNA; NULL = replay
  * of a fresh seed-1 rand() stream). out_ids: nq x K row-major, query i's K ids
- * at out_ids + i*K (the set_K_list order of the reference apps). Replaces the
- * per-query loops over para_search_PSS_v5_dist_thresh_profiling
+ * at out_ids + i*K (the set_K_list order of the reference apps); 0xffffffff in the
+ * slots past the vertices a search reached, where those are fewer than K (short
+ * init lists of PANNS_FLAG_LEARNED). Replaces the per-query loops over
+ * para_search_PSS_v5_dist_thresh_profiling
  * (app/PSS_v5_distance_threshold_profiling.cpp:132-152), seq_search_simple_search,
  * para_search_with_top_m_pure and IndexNSG::Search / SearchWithOptGraph. */
 int panns_search(panns_index *h, const panns_search_params *p, const uint32_t *init_ids,

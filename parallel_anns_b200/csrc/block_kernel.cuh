@@ -594,13 +594,14 @@ __device__ void block_search_one(const SearchArgs &a, uint32_t q, uint8_t *smem,
                 block_bitonic<W>(m, sz, a.orig);
                 ids = m.cI;
             }
-            for (uint32_t i = tid; i < a.K; i += T) a.out_ids[(size_t) q * a.K + i] = __ldg(a.orig + ids[i]);
+            for (uint32_t i = tid; i < a.K; i += T)
+                a.out_ids[(size_t) q * a.K + i] = i < sz ? __ldg(a.orig + ids[i]) : kFull;
         } else if (w == 0) {
             rerank_output(m.qd, m.qi, sz, a.K, a.orig, a.out_ids + (size_t) q * a.K, lane);
         }
     } else {
         for (uint32_t i = tid; i < a.K; i += T)
-            a.out_ids[(size_t) q * a.K + i] = __ldg(a.orig + (m.qi[i] & kIdMask));
+            a.out_ids[(size_t) q * a.K + i] = i < sz ? __ldg(a.orig + (m.qi[i] & kIdMask)) : kFull;
     }
     if (lane == 0) {
         atomicAdd(&ctl[BC_DIST], n_dist);

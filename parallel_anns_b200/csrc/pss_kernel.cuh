@@ -331,7 +331,7 @@ __device__ void pss_one(const PssArgs &pa, const PssMem &m, uint32_t q, uint32_t
         if (nk <= k_master) k_master = nk;
     }
     for (uint32_t i = lane; i < a.K; i += 32)
-        a.out_ids[(size_t) q * a.K + i] = __ldg(a.orig + (m.mi[i] & kIdMask));
+        a.out_ids[(size_t) q * a.K + i] = i < msz ? __ldg(a.orig + (m.mi[i] & kIdMask)) : kFull;
     if (lane == 0 && a.out_stats) a.out_stats[q] = make_uint4(n_dist, n_expand, n_edges, n_iter);
     if (a.vis_smem) {  // zeroed by the next query
     } else if (dcount <= a.dirty_cap) {

@@ -758,7 +758,7 @@ static __device__ void rank_sort(float *qd, uint32_t *qi, uint32_t sz, const uin
 // place by rank_sort (a power of two, so it needs no padding) and an entry's
 // output position is its index in its run plus, for every other run, the
 // number of that run's entries that precede it. The queue therefore needs no
-// room beyond sz.
+// room beyond sz. Outputs past sz are ~0.
 static __device__ void rerank_output(float *qd, uint32_t *qi, uint32_t sz, uint32_t K, const uint32_t *orig,
                                      uint32_t *out, int lane) {
     for (uint32_t start = 0, b = 32; b-- > 0;) {
@@ -792,6 +792,7 @@ static __device__ void rerank_output(float *qd, uint32_t *qi, uint32_t sz, uint3
         }
         if (rank < K) out[rank] = key;
     }
+    for (uint32_t i = sz + lane; i < K; i += 32) out[i] = kFull;
 }
 
 // Compute distances of the buffered fresh vertices bi[0..nb), keep the ones
@@ -1061,9 +1062,10 @@ __device__ void search_one(const SearchArgs &a, const WarpMem &m, uint32_t q, ui
         E.distances(a, m.qi, m.qd, sz, lane, reinterpret_cast<float *>(m.bk));
         rerank_output(m.qd, m.qi, sz, a.K, a.orig, a.out_ids + (size_t) q * a.K, lane);
     } else {
-        // Results (original ids).
+        // Results (original ids); a search can end with fewer than K vertices (short
+        // init lists of PANNS_FLAG_LEARNED in a graph whose parts do not meet).
         for (uint32_t i = lane; i < a.K; i += 32)
-            a.out_ids[(size_t) q * a.K + i] = __ldg(a.orig + (m.qi[i] & kIdMask));
+            a.out_ids[(size_t) q * a.K + i] = i < sz ? __ldg(a.orig + (m.qi[i] & kIdMask)) : kFull;
     }
     if (lane == 0 && a.out_stats) a.out_stats[q] = make_uint4(n_dist, n_expand, n_edges, n_iter);
     // Clear the visited words this query set.

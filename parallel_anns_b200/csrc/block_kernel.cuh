@@ -53,8 +53,8 @@ __host__ __device__ inline uint32_t block_smem_bytes(uint32_t queue_cap, uint32_
 
 enum { BC_Q = 0, BC_CNT, BC_CNT2, BC_TIE, BC_DIST, BC_EDGES, BC_FULL };
 
-// Total order of distances for ranking equal ones (and NaN): floats as
-// unsigned integers that compare the same way.
+// Total order of distances for ranking equal ones: floats as unsigned integers
+// that compare the same way.
 __device__ __forceinline__ uint32_t dist_key(float d) {
     const uint32_t b = __float_as_uint(d + 0.0f);
     return b & 0x80000000u ? ~b : b | 0x80000000u;
@@ -76,7 +76,7 @@ struct BlockMem {
 // elements (qd, qi)[0..sz) before each. Several adjacent threads count for one
 // element when there are fewer elements than threads; the counts of smaller and
 // of smaller or equal distances differ by more than the element itself only
-// where distances are equal (or NaN): then the block counts again by (distance,
+// where distances are equal: then the block counts again by (distance,
 // original id), a total order. Called by the whole block after a barrier; ends
 // with one.
 template <int W, bool PLACE>

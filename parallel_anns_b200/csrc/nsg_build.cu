@@ -65,7 +65,8 @@ namespace {
 template <typename T>
 using NBuf = Scratch<T>;
 
-// DistanceL2::compare of rows a and b (either order gives the same bits).
+// DistanceL2::compare of rows a and b (either order gives the same bits); a NaN
+// counts as +infinity, as in the search kernels (ordered, search_kernel.cuh).
 __host__ __device__ inline float l2_ref(const float *a, const float *b, uint32_t d) {
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     const uint32_t DR = d % 16, DD = d - DR;
@@ -82,7 +83,7 @@ __host__ __device__ inline float l2_ref(const float *a, const float *b, uint32_t
         }
     float r = acc[0];
     for (int j = 1; j < 8; ++j) r = r + acc[j];
-    return r;
+    return fminf(r, INFINITY);
 }
 
 constexpr uint32_t kLinkBuf = 256;     // fresh vertices per flush

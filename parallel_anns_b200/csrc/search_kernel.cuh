@@ -184,6 +184,11 @@ __device__ __forceinline__ float chain(const float4 (&x)[CL], const float4 (&qv)
     return acc;
 }
 
+// A distance as the queues take it: a NaN counts as +infinity. Ranks and merges
+// need an order; with a NaN in it a merge leaves places of the queue unwritten,
+// and what happens to be there is followed as a vertex.
+static __device__ __forceinline__ float ordered(float d) { return fminf(d, __int_as_float(0x7f800000)); }
+
 // The lane sum of a vertex's eight chains (tmp, 16-byte aligned) and the norm trick.
 template <int KIND>
 __device__ __forceinline__ float finish_sum(const float *tmp, float norm) {
@@ -195,7 +200,7 @@ __device__ __forceinline__ float finish_sum(const float *tmp, float norm) {
     s = __fadd_rn(s, y.y);
     s = __fadd_rn(s, y.z);
     s = __fadd_rn(s, y.w);
-    return KIND == KIND_IP ? __fmaf_rn(-2.0f, s, norm) : s;
+    return ordered(KIND == KIND_IP ? __fmaf_rn(-2.0f, s, norm) : s);
 }
 
 // (dist, key) order. PANNS: key is a device id and equal distances compare
@@ -421,7 +426,7 @@ __device__ __forceinline__ uint32_t rank_merge32(float *qd, uint32_t *qi, uint32
     }
     uint32_t r = less;
     if (__any_sync(kFull, have && upto != less + 1)) {
-        // Equal distances, infinities or NaN: by (distance, key) as integers, a total order.
+        // Equal distances (infinities among them): by (distance, key) as integers, a total order.
         const uint32_t b = __float_as_uint(d + 0.0f);
         const uint32_t kd = have ? (b & 0x80000000u ? ~b : b | 0x80000000u) : kFull;
         const uint32_t ko = !have ? kFull : ORDER == ORDER_PANNS ? __ldg(orig + (id & kIdMask)) : (uint32_t) lane;
@@ -699,8 +704,8 @@ struct Dist {
                 s0 += __shfl_xor_sync(kFull, s0, 2);
                 s1 += __shfl_xor_sync(kFull, s1, 2);
                 if (t == 0) {
-                    if (act0) out[b] = fmaf(-2.f, s0, n0);
-                    if (act1) out[bb] = fmaf(-2.f, s1, n1);
+                    if (act0) out[b] = ordered(fmaf(-2.f, s0, n0));
+                    if (act1) out[bb] = ordered(fmaf(-2.f, s1, n1));
                 }
                 continue;
             }
@@ -712,8 +717,8 @@ struct Dist {
             if (t == 0) {
                 const float m2 = kMixed ? -2.f / kMixedScale : -2.f;
                 const float2 r = __ffma2_rn(make_float2(m2, m2), s, make_float2(n0, n1));
-                if (act0) out[b] = r.x;
-                if (act1) out[bb] = r.y;
+                if (act0) out[b] = ordered(r.x);
+                if (act1) out[bb] = ordered(r.y);
             }
         }
         __syncwarp();

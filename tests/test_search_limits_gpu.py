@@ -1,5 +1,5 @@
 """Searches at the edge of what the kernels may assume: init lists with a repeated
-vertex, searches that reach fewer than K vertices."""
+vertex, searches that reach fewer than K vertices, distances that are not numbers."""
 import numpy as np
 import pytest
 
@@ -76,3 +76,83 @@ def test_learned_search_that_reaches_fewer_than_k(storage):
                 reach = {int(u) // 5 * 5 + j for u in [plain, *entries[i]] for j in range(5)}
                 assert {int(u) for u in ids[i, :len(reach)]} == reach, (w, i)
                 assert (ids[i, len(reach):] == 0xFFFFFFFF).all(), (w, i)
+
+
+def _graph(n, deg, seed):
+    from parallel_anns_b200.formats import NSGGraph
+    rng = np.random.default_rng(seed)
+    nb = rng.integers(0, n, size=(n, deg), dtype=np.int64)
+    nb[:, 0] = (np.arange(n) + 1) % n
+    nb = (nb + (nb == np.arange(n)[:, None])) % n
+    return NSGGraph(deg, 0, np.arange(n + 1, dtype=np.int64) * deg, nb.reshape(-1).astype(np.uint32))
+
+
+@pytest.mark.parametrize("n,d,deg,L,M,K", [(5000, 24, 30, 64, 4, 50), (3000, 40, 60, 700, 8, 100),
+                                           (9000, 16, 12, 300, 16, 300)])
+def test_nan_counts_as_infinity(n, d, deg, L, M, K):
+    """Rows and queries with a NaN: the same ids as with rows and queries whose
+    squared distances overflow to infinity, in every kernel of the float32 search."""
+    from parallel_anns_b200 import native as N
+    from parallel_anns_b200.searching import Index
+    rng = np.random.default_rng(n)
+    x, q = rng.random((n, d), dtype=np.float32), rng.random((40, d), dtype=np.float32)
+    bad = rng.permutation(n)[:n // 3]
+    xn, xi, qn, qi = x.copy(), x.copy(), q.copy(), q.copy()
+    xn[bad, 3], xi[bad, 3] = np.nan, 1e30
+    qn[::7, 1], qi[::7, 1] = np.nan, -1e30  # away from the rows': no difference is zero
+    g = _graph(n, deg, L)
+    og = O.Graph.from_nsg(g)
+    with Index(0) as ix:
+        ix.set_base(xn)
+        ix.set_graph(g)
+        ref, nd = O.search_top_m(xi, og, qi, K, L, M, kind=O.DIST_L2)
+        for w in (0, 1, 2, 4, 8):
+            ids, s = ix.search(qn, K=K, L=L, mode=N.MODE_TOP_M, M=M, distance=N.DIST_L2, warps_per_query=w)
+            assert np.array_equal(ids, ref) and s["n_dist"] == nd, w
+        ref, nd = O.search_pss(xi, og, qi, K, L, L, 2, 3, kind=O.DIST_L2)
+        ids, s = ix.search(qn, K=K, L=L, mode=N.MODE_PSS_V5, distance=N.DIST_L2, T=3, X=2)
+        assert np.array_equal(ids, ref) and s["n_dist"] == nd
+        init = ix.efanna_init_ids(L, q.shape[0])
+        ref, nd = O.search_efanna(xi, og, qi, K, L, init_ids=init)
+        ids, s = ix.search(qn, K=K, L=L, mode=N.MODE_EFANNA, distance=N.DIST_L2, init_ids=init)
+        assert np.array_equal(ids, ref) and s["n_dist"] == nd
+        # the norm trick, where such rows have no counterpart: K different vertices
+        for w in (1, 2, 8):
+            ids, _ = ix.search(qn, K=K, L=L, mode=N.MODE_TOP_M, M=M, warps_per_query=w)
+            assert ids.max() < n and all(np.unique(r).size == K for r in ids)
+
+
+@pytest.mark.parametrize("storage", [1, 2])
+def test_nan_in_reduced_copies(storage):
+    """K different vertices, the same with any number of warps, where the reduced rows,
+    their norms and the exact distances hold NaNs."""
+    from parallel_anns_b200 import native as N
+    from parallel_anns_b200.searching import Index
+    rng = np.random.default_rng(storage)
+    n, d, K, L = 6000, 32, 60, 200
+    x, q = rng.random((n, d), dtype=np.float32), rng.random((40, d), dtype=np.float32)
+    x[rng.permutation(n)[:n // 3], 5] = np.nan
+    q[::5, 2] = np.nan
+    with Index(0) as ix:
+        ix.set_base(x, storage=storage)
+        ix.set_graph(_graph(n, 20, 1))
+        one, _ = ix.search(q, K=K, L=L, mode=N.MODE_TOP_M, M=8, storage=storage, warps_per_query=1)
+        assert one.max() < n and all(np.unique(r).size == K for r in one)
+        for w in (0, 2, 4, 8):
+            ids, _ = ix.search(q, K=K, L=L, mode=N.MODE_TOP_M, M=8, storage=storage, warps_per_query=w)
+            assert np.array_equal(ids, one), w
+
+
+def test_efanna_build_with_nan_rows():
+    """IndexNSG::Build on rows with NaNs equals the build on rows with infinities in
+    their place: every distance to such a row, its own included, is infinite."""
+    from parallel_anns_b200.graph import efanna_build
+    rng = np.random.default_rng(5)
+    n, d = 600, 16
+    x = rng.random((n, d), dtype=np.float32)
+    knn = O.host_knn(x, None, 20)[0]
+    xn, xi = x.copy(), x.copy()
+    xn[::9, 2], xi[::9, 2] = np.nan, np.inf
+    a, b = efanna_build(xn, knn, 60, 12, 80), efanna_build(xi, knn, 60, 12, 80)
+    assert a.entry < n and a.nbrs.max() < n
+    assert np.array_equal(a.offsets, b.offsets) and np.array_equal(a.nbrs, b.nbrs)

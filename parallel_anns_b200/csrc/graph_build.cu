@@ -1191,15 +1191,16 @@ int panns_build_nsg_ex(int device, const float *base, uint32_t n, uint32_t d, ui
             rc = tc_locality_order(x.p, n, d, true, perm.p, &slots, s);
             if (rc) return rc;
         }
-        rc = tc_screen_knn(x.p, n, d, k, C, perm.p, slots, nullptr, cand.p, fail.p, nfail.p, num_sms, s);
+        bool safe = false;
+        rc = tc_screen_knn(x.p, n, d, k, C, perm.p, slots, nullptr, cand.p, fail.p, nfail.p, &safe, num_sms, s);
         if (rc) return rc;
         // Rows that screen could not settle (long runs of equal distances,
         // non-finite values) go through the float32 one.
-        uint32_t nf = 0;
-        GCU(cudaMemcpyAsync(&nf, nfail.p, 4, cudaMemcpyDeviceToHost, s));
+        uint32_t nf = n;
+        if (safe) GCU(cudaMemcpyAsync(&nf, nfail.p, 4, cudaMemcpyDeviceToHost, s));
         GCU(cudaStreamSynchronize(s));
         if (nf) {
-            rc = screen_fp32(x.p, n, d, xn.p, C, fail.p, nf, cand.p, s);
+            rc = screen_fp32(x.p, n, d, xn.p, C, safe ? fail.p : nullptr, nf, cand.p, s);
             if (rc) return rc;
             GCU(cudaStreamSynchronize(s));
         }
@@ -1360,13 +1361,14 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
         GCU(cudaMemcpyAsync(dnear.p, nearh.data(), nearh.size() * 4, cudaMemcpyHostToDevice, s));
         GCU(cudaMemcpyAsync(davail.p, avail.data(), cells * 4ull, cudaMemcpyHostToDevice, s));
         const TcCells tc{dblk.p, dt0.p, dnear.p, davail.p, P};
-        const int rc = tc_screen_knn(x.p, n, d, k, C, dorder.p, (uint32_t) slots, &tc, cand.p, fail.p, nfail.p, num_sms,
-                                     s);
+        bool safe = false;
+        const int rc = tc_screen_knn(x.p, n, d, k, C, dorder.p, (uint32_t) slots, &tc, cand.p, fail.p, nfail.p, &safe,
+                                     num_sms, s);
         if (rc) return rc;
         uint32_t nf = 0;
         GCU(cudaMemcpyAsync(&nf, nfail.p, 4, cudaMemcpyDeviceToHost, s));
         GCU(cudaStreamSynchronize(s));
-        screened = nf == 0;
+        screened = safe && nf == 0;
     }
     if (!screened) {
         // Blocks of up to kBQ rows of one cell.

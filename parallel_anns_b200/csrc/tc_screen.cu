@@ -11,15 +11,25 @@
 //           ties) or holds non-finite values is reported instead.
 //   range   per query, every column with s below a fixed threshold + e.
 //
-// Precision. Each float32 operand is split in two BF16 parts, x = x1 + x2 + r
-// with |r| <= 2^-18 |x|, and x.y is taken as x1.y1 + x1.y2 + x2.y1 in float32
-// accumulators: what is left out is at most 3 * 2^-18 |x||y|, and the
-// accumulation of at most 35 steps adds less than 35 * 2^-22 of the terms'
-// sum; e = 2^-14 |x| max|y| + 2^-16 max|y|^2 is larger than both together.
-// Against a single TF32 product (the form before) this costs 1.5 times the
+// Precision. The rows of both sides are shifted to the base's mean and multiplied
+// by a power of two (exact) that brings the base's spread to about 1; s, the
+// thresholds and the bounds below are all in these units. Each float32 operand is
+// split in two BF16 parts, x = x1 + x2 + r with |r| <= 2^-18 |x|, and x.y is taken
+// as x1.y1 + x1.y2 + x2.y1 in float32 accumulators, ||y||^2 riding in the
+// contraction as three BF16 parts against ones. Left out of s: 2 * 3 * 2^-18
+// |x||y|. The accumulation takes ceil((d + 3) / 16) + 2 ceil(d / 16) <= 49 steps,
+// each within 2^-22 of the sum of the terms' sizes, 2 |x||y| + |y|^2. Together
+// 2^-14.4 |x||y| + 2^-16.4 |y|^2. The float32 shift moves a squared distance by
+// at most 2^-23 (|x| + |y|)^2, and a threshold's own roundings add 2^-23 (|x|^2 +
+// |y|^2). Parts below BF16's or float32's normal range (2^-126) are off
+// absolutely: by 2^-122 (|x| + |y|), which the terms above cover unless it is
+// below 1e-60, and by 2^-117 in sums. e = 2^-14 |x| max|y| + 2^-16 max|y|^2 +
+// 2^-21 |x|^2 + 1e-30 is larger than all of it for squared norms below 1e36
+// (kTcLarge); a screen that meets a larger finite one says so (the spread is taken
+// from a sample), a row with an infinity or a NaN is reported.
+// Against a single TF32 product (the form before) the split costs 1.5 times the
 // tensor time for 2^-16 instead of 2^-10, which makes the lists both short
-// (about k + 3 entries instead of k + 32) and safe. ||y||^2 rides in the
-// contraction as three BF16 parts against ones.
+// (about k + 3 entries instead of k + 32) and safe.
 //
 // Skipping. Rows and columns are processed in a locality order; every tile has
 // a centre and a radius, and a tile whose ball is further from the row block's
@@ -75,10 +85,12 @@ constexpr uint32_t kTcCap = 384;       // list entries per row of the k-NN form
 constexpr uint32_t kTcEnd = 0xffffffffu, kTcExit = 0xfffffffeu, kTcTighten = 0xfffffffdu;
 constexpr uint32_t kTcFirst = 0x80000000u;
 constexpr float kTcBig = 1e38f;        // threshold of a list that is not full yet
+constexpr float kTcLarge = 1e36f;      // squared norms the error bound holds up to
 constexpr uint32_t kTcKnnBlocks = 32768;  // row blocks whose operand is held at a time (2 GB at d = 96)
 constexpr uint32_t kNone = 0xffffffffu;
 
 enum : uint32_t { TC_ERR_TIMEOUT = 1u };
+enum : uint32_t { TC_NORM_BAD = 1u, TC_NORM_LARGE = 2u };  // a norm not below kTcLarge; one of finite values
 enum { TC_KNN = 0, TC_RANGE = 1 };
 
 struct TcArgs {
@@ -698,13 +710,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 thr = -kInf;
                 if (live) {
                     xn = a.xn[row];
-                    eps = 0x1p-14f * sqrtf(xn) * sqrtf(ymax2) + 0x1p-16f * ymax2 + 0x1p-22f * xn;
+                    eps = 0x1p-14f * sqrtf(xn) * sqrtf(ymax2) + 0x1p-16f * ymax2 + 0x1p-21f * xn + 1e-30f;
                     if (FORM == TC_RANGE) {
                         cnt = a.cnt[(size_t) sp * a.rows + row];
                         thr = a.tau[row] - xn + eps;
                         list = a.lists + ((size_t) sp * a.rows + row) * a.cap;
                     } else {
-                        thr = kTcBig;
+                        thr = xn < kTcLarge ? kTcBig : -kInf;  // (a NaN is not): reported
                         list = my_lists + (size_t) r * kTcCap;
                     }
                 }
@@ -768,15 +780,22 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 // ---- operands, balls, bounds -------------------------------------------------
 
 // shift = the mean of up to 4,096 rows at a fixed stride (one block per
-// dimension). Distances do not change under a shift, and the error bound
-// follows the norms, so data far from the origin loses nothing. (x - shift
-// rounds by 2^-24 of itself, inside the bound's slack.)
+// dimension), spread = the largest finite distance of one of their values to it
+// (float bits, zeroed beforehand). Distances do not change under a shift, and the
+// error bound follows the norms, so data far from the origin loses nothing.
 __global__ void __launch_bounds__(256) tc_shift_kernel(const float *__restrict__ x, uint32_t n, uint32_t d,
-                                                       float *__restrict__ shift) {
+                                                       float *__restrict__ shift, uint32_t *__restrict__ spread) {
+    constexpr uint32_t kRows = 4096, kPer = kRows / 256;
     __shared__ float red[8];
-    const uint32_t j = blockIdx.x, m = min(n, 4096u);
-    float s = 0.f;
-    for (uint32_t i = threadIdx.x; i < m; i += 256) s += x[((uint64_t) i * n / m) * d + j];
+    __shared__ float mean;
+    const uint32_t j = blockIdx.x, m = min(n, kRows);
+    float v[kPer], s = 0.f;
+#pragma unroll
+    for (uint32_t t = 0; t < kPer; ++t) {
+        const uint32_t i = threadIdx.x + 256 * t;
+        v[t] = i < m ? x[((uint64_t) i * n / m) * d + j] : 0.f;
+        s += v[t];
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
@@ -784,21 +803,40 @@ __global__ void __launch_bounds__(256) tc_shift_kernel(const float *__restrict__
     if (threadIdx.x == 0) {
         for (int i = 1; i < 8; ++i) s += red[i];
         s /= (float) m;
-        shift[j] = fabsf(s) < 1e30f ? s : 0.f;
+        mean = shift[j] = fabsf(s) < 1e30f ? s : 0.f;
     }
+    __syncthreads();
+    float far = 0.f;
+#pragma unroll
+    for (uint32_t t = 0; t < kPer; ++t) {
+        const float u = fabsf(v[t] - mean);
+        if (threadIdx.x + 256 * t < m && u < 3e38f) far = fmaxf(far, u);
+    }
+    const uint32_t most = __reduce_max_sync(0xffffffffu, __float_as_uint(far));
+    if ((threadIdx.x & 31) == 0) atomicMax(spread, most);
+}
+
+// The power of two (exact to multiply by) that brings the spread to [0.5, 1).
+__device__ __forceinline__ float tc_scale(const uint32_t *spread) {
+    const float m = __uint_as_float(*spread);
+    if (!(m > 0.f)) return 1.f;
+    int e;
+    frexpf(m, &e);
+    return ldexpf(1.f, max(-126, min(126, -e)));
 }
 
 // One block per tile of kTcM positions from p0: its rows (row perm[p] of x, p
 // itself without perm; no row from `valid` on or where perm says ~0) go through
 // shared memory once and leave as
-//   operand rows less the shift, [hi (W) | lo (W)] BF16: A (row side) holds x's
-//   parts and three ones after the high one; B (column side) the parts of -2 x
-//   and ||x||^2 (float64 sum) in three parts, a position without a row a norm
-//   no threshold reaches;
-//   xn = ||x||^2, the maximum of the norms (float bits), *huge = 1 if a norm
-//   leaves float32's safe range;
+//   operand rows less the shift and scaled, [hi (W) | lo (W)] BF16: A (row side)
+//   holds x's parts and three ones after the high one; B (column side) the parts
+//   of -2 x and ||x||^2 (float64 sum) in three parts, a position without a row a
+//   norm no threshold reaches;
+//   xn = ||x||^2, the maximum of the norms (float bits), both of the scaled rows;
+//   *large |= TC_NORM_BAD where one is not below kTcLarge, TC_NORM_LARGE too where
+//   the row is finite;
 //   the tile's centre (mean of its rows) and radius (rounded up; a tile without
-//   rows gets one that puts it out of every reach), not shifted.
+//   rows gets one that puts it out of every reach), scaled, not shifted.
 // Null outputs are skipped. Bound by issue: a lane keeps its column pairs in
 // registers from the norm to the two operands. 1M x 96 as columns: 0.72 ms with
 // 440 instructions a row, 0.49 ms so.
@@ -807,9 +845,10 @@ constexpr int kPrepSteps = 5;  // 64-wide steps of an operand row: W <= 320
 __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict__ x, uint32_t n, uint32_t d,
                                                          const uint32_t *__restrict__ perm, uint32_t p0,
                                                          uint32_t valid, uint32_t W, const float *__restrict__ shift,
+                                                         const uint32_t *__restrict__ spread,
                                                          __nv_bfloat16 *__restrict__ A, __nv_bfloat16 *__restrict__ B,
                                                          float *__restrict__ xn, uint32_t *__restrict__ ymax,
-                                                         uint32_t *__restrict__ huge, float *__restrict__ centre,
+                                                         uint32_t *__restrict__ large, float *__restrict__ centre,
                                                          float *__restrict__ radius) {
     extern __shared__ __align__(16) float tile[];  // kTcM x d
     __shared__ uint32_t rows[kTcM];
@@ -823,7 +862,8 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
         filled = row < n;
         rows[tid] = filled ? row : kNone;
     }
-    if (tid < d) sh[tid] = shift[tid];
+    const float scale = tc_scale(spread);
+    if (tid < d) sh[tid] = shift[tid] * scale;
     const uint32_t count = (uint32_t) __syncthreads_count(filled);
     if (d % 4 == 0) {
         const uint32_t d4 = d / 4, di = 256 / d4, dq = 256 - di * d4;
@@ -848,12 +888,12 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
     }
     __syncthreads();
     float nm = 0.f;
-    bool big = false;
+    uint32_t bad = 0;
     const bool even = d % 2 == 0;
     for (uint32_t i = w; i < kTcM; i += 8) {
         const bool have = rows[i] != kNone;
         const float *xr = tile + (size_t) i * d;
-        // The lane's column pairs 2 lane + 64 t, shifted.
+        // The lane's column pairs 2 lane + 64 t, shifted and scaled.
         float2 v[kPrepSteps];
         double s = 0.0;
 #pragma unroll
@@ -863,9 +903,9 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
             if (64u * t >= d) continue;
             if (have && e + 1 < d) {
                 float2 y = even ? *reinterpret_cast<const float2 *>(xr + e) : make_float2(xr[e], xr[e + 1]);
-                v[t] = make_float2(y.x - sh[e], y.y - sh[e + 1]);
+                v[t] = make_float2(fmaf(y.x, scale, -sh[e]), fmaf(y.y, scale, -sh[e + 1]));
             } else if (have && e < d) {
-                v[t].x = xr[e] - sh[e];
+                v[t].x = fmaf(xr[e], scale, -sh[e]);
             }
             s = fma((double) v[t].x, (double) v[t].x, s);
             s = fma((double) v[t].y, (double) v[t].y, s);
@@ -874,8 +914,13 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         const float nf = (float) s;
         if (lane == 0 && xn) xn[t0 + i] = nf;
-        if (have && nf < 3e38f) nm = fmaxf(nm, nf);
-        big = big || (have && !(nf < 1e37f));
+        if (have && nf < kTcLarge) {
+            nm = fmaxf(nm, nf);
+        } else if (have) {  // the warp agrees: the same sum on every lane
+            bool finite = true;
+            for (uint32_t e = lane; e < d; e += 32) finite = finite && fabsf(xr[e]) < __int_as_float(0x7f800000);
+            bad |= __all_sync(0xffffffffu, finite) ? TC_NORM_BAD | TC_NORM_LARGE : TC_NORM_BAD;
+        }
         const __nv_bfloat16 n1 = __float2bfloat16_rn(have ? nf : 3e38f);
         const float r1 = have ? nf - __bfloat162float(n1) : 0.f;
         const __nv_bfloat16 n2 = __float2bfloat16_rn(r1);
@@ -912,7 +957,7 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
         }
     }
     if (lane == 0) nmax[w] = nm;
-    if (huge && lane == 0 && big) *huge = 1u;
+    if (large && lane == 0 && bad) atomicOr(large, bad);
     __syncthreads();
     if (ymax && tid == 0) {
         for (int i = 1; i < 8; ++i) nm = fmaxf(nm, nmax[i]);
@@ -922,7 +967,7 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
     if (tid < d) {  // positions without a row hold zeros
         float s = 0.f;
 #pragma unroll 16
-        for (uint32_t i = 0; i < kTcM; ++i) s += tile[(size_t) i * d + tid];
+        for (uint32_t i = 0; i < kTcM; ++i) s = fmaf(tile[(size_t) i * d + tid], scale, s);
         c[tid] = count ? s / (float) count : 0.f;
         centre[(size_t) blockIdx.x * d + tid] = c[tid];
     }
@@ -932,7 +977,7 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
         if (rows[i] == kNone) continue;
         float t = 0.f;
         for (uint32_t e = lane; e < d; e += 32) {
-            const float u = tile[(size_t) i * d + e] - c[e];
+            const float u = fmaf(tile[(size_t) i * d + e], scale, -c[e]);
             t = fmaf(u, u, t);
         }
 #pragma unroll
@@ -950,7 +995,8 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
 
 // need[i][t] = 0 when some query of row block i can have a vertex of tile t
 // within its radius, else +inf: max(0, |q - c_t| - r_t)^2 <= tau_q for one of
-// its 128 queries, each part rounded to the safe side. Per query rather than
+// its 128 queries (scaled here as the balls and radii are), each part rounded to
+// the safe side. Per query rather than
 // ball against ball: a block's queries may lie in several clusters. One block
 // per (row block, 64 tiles), 8 x 4 distances per thread.
 //
@@ -961,7 +1007,7 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
 // 0.76 ms so.
 __global__ void __launch_bounds__(256) tc_need_kernel(const float *__restrict__ q, const uint32_t *__restrict__ qperm,
                                                       uint32_t nq, const float *__restrict__ tau,
-                                                      const float *__restrict__ cb, const float *__restrict__ rb,
+                                                      const uint32_t *__restrict__ spread, const float *__restrict__ cb, const float *__restrict__ rb,
                                                       uint32_t nb, uint32_t d, float *__restrict__ need) {
     __shared__ __align__(16) float sa[2][16][kTcM + 4];
     __shared__ __align__(16) float sb[2][16][68];
@@ -976,6 +1022,7 @@ __global__ void __launch_bounds__(256) tc_need_kernel(const float *__restrict__ 
     if (tid < kTcM) st[tid] = i0 + tid < nq ? tau[i0 + tid] : -1.f;
     if (tid < 64) any[tid] = 0;
     float va[8], vc[4];
+    const float scale = tc_scale(spread);
     const bool quads = d % 4 == 0;
     auto fetch4 = [&](const float *r, uint32_t k, float *v) {
         if (quads && r && k < d) {
@@ -993,7 +1040,7 @@ __global__ void __launch_bounds__(256) tc_need_kernel(const float *__restrict__ 
     };
     auto store = [&](int buf) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) sa[buf][ka + e][ra] = va[e];
+        for (int e = 0; e < 8; ++e) sa[buf][ka + e][ra] = va[e] * scale;
 #pragma unroll
         for (int e = 0; e < 4; ++e) sb[buf][kc + e][rc] = vc[e];
     };
@@ -1186,9 +1233,12 @@ __global__ void tc_scatter_kernel(const uint32_t *__restrict__ cell, uint32_t n,
     if (i < n) perm[atomicAdd(start + cell[i], 1u)] = i;
 }
 
-__global__ void tc_tau_kernel(const double *__restrict__ tau, uint32_t nq, float *__restrict__ out) {
+// Squared radii in scaled units, rounded up.
+__global__ void tc_tau_kernel(const double *__restrict__ tau, uint32_t nq, const uint32_t *__restrict__ spread,
+                              float *__restrict__ out) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < nq) out[i] = __double2float_ru(tau[i]);
+    const double scale = (double) tc_scale(spread);
+    if (i < nq) out[i] = __double2float_ru(tau[i] * (scale * scale));
 }
 
 int make_map(CUtensorMap *map, const __nv_bfloat16 *x, uint64_t rows, uint32_t width) {
@@ -1306,8 +1356,8 @@ int tc_locality_order(const float *x, uint32_t n, uint32_t d, bool padded, uint3
 }
 
 int tc_screen_knn(const float *x, uint32_t n, uint32_t d, uint32_t k, uint32_t C, const uint32_t *perm, uint32_t slots,
-                  const TcCells *cells, uint32_t *cand, uint32_t *fail_rows, uint32_t *fail_count, int num_sms,
-                  cudaStream_t s) {
+                  const TcCells *cells, uint32_t *cand, uint32_t *fail_rows, uint32_t *fail_count, bool *safe,
+                  int num_sms, cudaStream_t s) {
     if (d == 0 || d > 256 || k == 0 || k + 1 > kTcCap - kTcM || C < k || n < 2)
         return set_error(PANNS_EINVAL, "tc screen: unsupported shape");
     const TcShape sh = tc_shape(d);
@@ -1315,7 +1365,7 @@ int tc_screen_knn(const float *x, uint32_t n, uint32_t d, uint32_t k, uint32_t C
     TBuf<__nv_bfloat16> A, B;
     TBuf<float> xn, centre, radius, lb2, shift;
     TBuf<uint2> lists;
-    TBuf<uint32_t> ctl;  // counter, error, ymax
+    TBuf<uint32_t> ctl;  // counter, error, ymax, large, spread
     // Row operands and bounds between tiles for a limited number of row blocks at a time.
     const bool skip = !cells && tiles > 32;
     uint32_t per = std::min(tiles, kTcKnnBlocks);
@@ -1328,14 +1378,15 @@ int tc_screen_knn(const float *x, uint32_t n, uint32_t d, uint32_t k, uint32_t C
     TCU(A.alloc((size_t) per * kTcM * 2 * sh.W, s));
     TCU(B.alloc((size_t) pad * 2 * sh.W, s));
     TCU(xn.alloc(pad, s));
-    TCU(ctl.alloc(4, s));
+    TCU(ctl.alloc(5, s));
     TCU(shift.alloc(d, s));
-    TCU(cudaMemsetAsync(ctl.p, 0, 16, s));
+    TCU(cudaMemsetAsync(ctl.p, 0, 20, s));
     TCU(cudaMemsetAsync(fail_count, 0, 4, s));
-    tc_shift_kernel<<<d, 256, 0, s>>>(x, n, d, shift.p);
+    const uint32_t *spread = ctl.p + 4;
+    tc_shift_kernel<<<d, 256, 0, s>>>(x, n, d, shift.p, ctl.p + 4);
     TCU(allow_shared((const void *) tc_prepare_kernel));
-    tc_prepare_kernel<<<tiles, 256, kTcM * d * 4, s>>>(x, n, d, perm, 0, slots, sh.W, shift.p,
-                                                       per == tiles ? A.p : nullptr, B.p, xn.p, ctl.p + 2, nullptr,
+    tc_prepare_kernel<<<tiles, 256, kTcM * d * 4, s>>>(x, n, d, perm, 0, slots, sh.W, shift.p, spread,
+                                                       per == tiles ? A.p : nullptr, B.p, xn.p, ctl.p + 2, ctl.p + 3,
                                                        centre.p, radius.p);
     TCU(cudaGetLastError());
     TCU(lists.alloc((size_t) std::min<uint32_t>(per, (uint32_t) num_sms) * kTcM * kTcCap, s));
@@ -1346,8 +1397,8 @@ int tc_screen_knn(const float *x, uint32_t n, uint32_t d, uint32_t k, uint32_t C
     for (uint32_t rb0 = 0; rb0 < tiles; rb0 += per) {
         const uint32_t m = std::min(per, tiles - rb0);
         if (per != tiles) {
-            tc_prepare_kernel<<<m, 256, kTcM * d * 4, s>>>(x, n, d, perm, rb0 * kTcM, slots, sh.W, shift.p, A.p, nullptr,
-                                                           nullptr, nullptr, nullptr, nullptr, nullptr);
+            tc_prepare_kernel<<<m, 256, kTcM * d * 4, s>>>(x, n, d, perm, rb0 * kTcM, slots, sh.W, shift.p, spread, A.p,
+                                                           nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
             TCU(cudaGetLastError());
         }
         if (skip) {
@@ -1388,7 +1439,11 @@ int tc_screen_knn(const float *x, uint32_t n, uint32_t d, uint32_t k, uint32_t C
         rc = tc_launch<TC_KNN>(ma, mb, a, sh.smem, num_sms, s);
         if (rc) return rc;
     }
-    return tc_check(ctl.p + 1, s);
+    uint32_t large = 0;
+    TCU(cudaMemcpyAsync(&large, ctl.p + 3, 4, cudaMemcpyDeviceToHost, s));
+    rc = tc_check(ctl.p + 1, s);
+    *safe = !(large & TC_NORM_LARGE);
+    return rc;
 }
 
 size_t tc_knn_bytes(uint64_t slots, uint32_t d) {
@@ -1417,7 +1472,7 @@ int tc_screen_range(const float *x, uint32_t n, uint32_t d, const uint32_t *perm
     const uint32_t ct = chunk / kTcM;
     TBuf<__nv_bfloat16> A, B;
     TBuf<float> xn, cb, rad, need, ft, shift;
-    TBuf<uint32_t> ctl;  // counter, error, ymax, huge
+    TBuf<uint32_t> ctl;  // counter, error, ymax, large, spread
     TCU(A.alloc((size_t) qpad * 2 * sh.W, s));
     TCU(B.alloc((size_t) chunk * 2 * sh.W, s));
     TCU(xn.alloc(qpad, s));
@@ -1426,14 +1481,15 @@ int tc_screen_range(const float *x, uint32_t n, uint32_t d, const uint32_t *perm
     TCU(need.alloc((size_t) rb * ct, s));
     TCU(ft.alloc(nq, s));
     TCU(shift.alloc(d, s));
-    TCU(ctl.alloc(4, s));
-    TCU(cudaMemsetAsync(ctl.p, 0, 16, s));
+    TCU(ctl.alloc(5, s));
+    TCU(cudaMemsetAsync(ctl.p, 0, 20, s));
     TCU(cudaMemsetAsync(cnt, 0, (size_t) splits * nq * 4, s));
-    tc_shift_kernel<<<d, 256, 0, s>>>(x, n, d, shift.p);
-    tc_tau_kernel<<<(nq + 255) / 256, 256, 0, s>>>(tau, nq, ft.p);
+    const uint32_t *spread = ctl.p + 4;
+    tc_shift_kernel<<<d, 256, 0, s>>>(x, n, d, shift.p, ctl.p + 4);
+    tc_tau_kernel<<<(nq + 255) / 256, 256, 0, s>>>(tau, nq, spread, ft.p);
     TCU(allow_shared((const void *) tc_prepare_kernel));
-    tc_prepare_kernel<<<rb, 256, kTcM * d * 4, s>>>(queries, kNone, d, qperm, 0, nq, sh.W, shift.p, A.p, nullptr, xn.p,
-                                                    nullptr, ctl.p + 3, nullptr, nullptr);
+    tc_prepare_kernel<<<rb, 256, kTcM * d * 4, s>>>(queries, kNone, d, qperm, 0, nq, sh.W, shift.p, spread, A.p, nullptr,
+                                                    xn.p, nullptr, ctl.p + 3, nullptr, nullptr);
     TCU(cudaGetLastError());
     CUtensorMap ma, mb;
     int rc = make_map(&ma, A.p, qpad, 2 * sh.W);
@@ -1442,9 +1498,10 @@ int tc_screen_range(const float *x, uint32_t n, uint32_t d, const uint32_t *perm
     for (uint64_t c0 = 0; c0 < slots; c0 += chunk) {
         const uint32_t m = (uint32_t) std::min<uint64_t>(chunk, slots - c0), mt = (m + kTcM - 1) / kTcM;
         TCU(cudaMemsetAsync(ctl.p + 2, 0, 4, s));
-        tc_prepare_kernel<<<mt, 256, kTcM * d * 4, s>>>(x, n, d, perm, (uint32_t) c0, slots, sh.W, shift.p, nullptr, B.p,
-                                                        nullptr, ctl.p + 2, ctl.p + 3, cb.p, rad.p);
-        tc_need_kernel<<<dim3((mt + 63) / 64, rb), 256, 0, s>>>(queries, qperm, nq, ft.p, cb.p, rad.p, mt, d, need.p);
+        tc_prepare_kernel<<<mt, 256, kTcM * d * 4, s>>>(x, n, d, perm, (uint32_t) c0, slots, sh.W, shift.p, spread, nullptr,
+                                                        B.p, nullptr, ctl.p + 2, ctl.p + 3, cb.p, rad.p);
+        tc_need_kernel<<<dim3((mt + 63) / 64, rb), 256, 0, s>>>(queries, qperm, nq, ft.p, spread, cb.p, rad.p, mt, d,
+                                                                need.p);
         TCU(cudaGetLastError());
         TcArgs a{};
         a.rows = nq;
@@ -1470,10 +1527,10 @@ int tc_screen_range(const float *x, uint32_t n, uint32_t d, const uint32_t *perm
         rc = tc_launch<TC_RANGE>(ma, mb, a, sh.smem, num_sms, s);
         if (rc) return rc;
     }
-    uint32_t huge = 0;
-    TCU(cudaMemcpyAsync(&huge, ctl.p + 3, 4, cudaMemcpyDeviceToHost, s));
+    uint32_t large = 0;
+    TCU(cudaMemcpyAsync(&large, ctl.p + 3, 4, cudaMemcpyDeviceToHost, s));
     rc = tc_check(ctl.p + 1, s);
-    *safe = !huge;
+    *safe = !large;
     return rc;
 }
 

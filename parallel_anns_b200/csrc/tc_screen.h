@@ -41,12 +41,14 @@ struct TcCells {
 // (n x d float32, device), ~0 where there are fewer, in no particular order.
 // They include the k nearest of the rows screened (all, or the cells' when
 // `cells` is given) unless row i is listed in fail_rows[0 .. *fail_count)
-// (device; for these rows cand is not written). perm (device, `slots`
+// (device; for these rows cand is not written). *safe = false: a finite row is so
+// far from the others that the error bound does not hold, cand is not to be used
+// for any row. perm (device, `slots`
 // entries, ~0 = no row; null = identity) is the order the rows are processed
 // in. Enqueued on `s` and synchronised.
 int tc_screen_knn(const float *x, uint32_t n, uint32_t d, uint32_t k, uint32_t C, const uint32_t *perm, uint32_t slots,
-                  const TcCells *cells, uint32_t *cand, uint32_t *fail_rows, uint32_t *fail_count, int num_sms,
-                  cudaStream_t s);
+                  const TcCells *cells, uint32_t *cand, uint32_t *fail_rows, uint32_t *fail_count, bool *safe,
+                  int num_sms, cudaStream_t s);
 
 // Device memory tc_screen_knn takes for this many positions (besides the tile bounds).
 size_t tc_knn_bytes(uint64_t slots, uint32_t d);
@@ -56,8 +58,9 @@ size_t tc_knn_bytes(uint64_t slots, uint32_t d);
 // too), and few others: the entry e of split p is lists[(p * nq + i) * cap + e]
 // = {screen distance bits, position in perm}, e < cnt[p * nq + i] (entries from
 // cap on are counted, not stored). perm (`slots` positions, ~0 = no row): the
-// order the rows of x are processed in. *safe = false: a vector's norm is outside the
-// range the error bound holds for, the lists are not to be used. splits: from
+// order the rows of x are processed in. *safe = false: a vector is not finite, or so
+// far from the others that the error bound does not hold; the lists are not to be
+// used. splits: from
 // tc_range_splits. Enqueued on `s` and synchronised.
 constexpr uint32_t kTcMaxSplits = 8;
 uint32_t tc_range_splits(uint32_t nq, int num_sms);

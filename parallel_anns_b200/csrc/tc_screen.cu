@@ -816,13 +816,11 @@ __global__ void __launch_bounds__(256) tc_shift_kernel(const float *__restrict__
     if ((threadIdx.x & 31) == 0) atomicMax(spread, most);
 }
 
-// The power of two (exact to multiply by) that brings the spread to [0.5, 1).
+// The power of two (exact to multiply by) that brings the spread to [0.5, 1), or as
+// near as float32's exponents allow; 1 for a spread of 0.
 __device__ __forceinline__ float tc_scale(const uint32_t *spread) {
-    const float m = __uint_as_float(*spread);
-    if (!(m > 0.f)) return 1.f;
-    int e;
-    frexpf(m, &e);
-    return ldexpf(1.f, max(-126, min(126, -e)));
+    const uint32_t bits = *spread, e = bits >> 23;  // biased exponent; 0 below the normal range
+    return bits ? __uint_as_float(max(1, 253 - (int) e) << 23) : 1.f;
 }
 
 // One block per tile of kTcM positions from p0: its rows (row perm[p] of x, p

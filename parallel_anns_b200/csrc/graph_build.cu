@@ -152,6 +152,14 @@ __global__ void __launch_bounds__(256) topk_tile_kernel(const float *__restrict_
 // itself) with the smallest (||y||^2 - 2 x.y, id), over tiles of kBV
 // candidates. 256 threads: thread (ty, tx) computes a 4 x 8 block of the
 // 64 x 128 tile; then warp w inserts the tile into the lists of rows 8w..8w+7.
+//
+// DIRECT: by the squared distance as a sum of squared differences, for the rows the
+// tensor-core screen hands on. It takes two instructions a term instead of one, but
+// its error follows the distance itself, wherever the origin and however far other
+// rows are, which those rows (runs of equal distances, clusters much smaller than
+// the base) depend on. Distances that overflow, or of a row with a NaN, count as
+// equal, so that a list is filled (by id) all the same.
+template <bool DIRECT>
 __global__ void __launch_bounds__(256) screen_kernel(const float *__restrict__ x, uint32_t n, uint32_t d,
                                                      const float *__restrict__ xn, uint32_t C,
                                                      const uint32_t *__restrict__ rows, uint32_t nr,
@@ -200,7 +208,10 @@ __global__ void __launch_bounds__(256) screen_kernel(const float *__restrict__ x
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                    for (int j = 0; j < 8; ++j) {
+                        const float t = DIRECT ? a[i] - b[j] : 0.f;
+                        acc[i][j] = DIRECT ? fmaf(t, t, acc[i][j]) : fmaf(a[i], b[j], acc[i][j]);
+                    }
             }
             __syncthreads();
         }
@@ -211,8 +222,8 @@ __global__ void __launch_bounds__(256) screen_kernel(const float *__restrict__ x
             for (int j = 0; j < 8; ++j) {
                 const uint32_t gv = v0 + tx * 8 + j;
                 const bool ok = gv < n && gv != gq;
-                D[(ty * 4 + i) * (kBV + 1) + tx * 8 + j] =
-                    ok ? fmaf(-2.f, acc[i][j], xn[gv]) : __int_as_float(0x7f800000);
+                const float v = DIRECT ? fminf(acc[i][j], 3.4e38f) : ok ? fmaf(-2.f, acc[i][j], xn[gv]) : 0.f;
+                D[(ty * 4 + i) * (kBV + 1) + tx * 8 + j] = ok ? v : __int_as_float(0x7f800000);
             }
         }
         __syncthreads();
@@ -236,16 +247,17 @@ __global__ void __launch_bounds__(256) screen_kernel(const float *__restrict__ x
 }
 
 // Float32 screen restricted to cells: block b screens up to kBQ rows of cell
-// blk_cell[b] (members[blk_row0[b] ..], within the cell) against the members
+// blk_cell[b], rows[blk_row0[b]] .. rows[blk_row0[b + 1]), against the members
 // of the cell itself and of its P nearest cells (near[c * P ..]), keeping per
 // row the C candidates with the smallest (||y||^2 - 2 x.y, id). The same
-// tiling and list insertion as screen_kernel; rows and candidates are read
-// through the members list (cell by cell, ids ascending within a cell).
+// tiling and list insertion as screen_kernel; candidates are read through the
+// members list (cell by cell, ids ascending within a cell). DIRECT as there.
+template <bool DIRECT>
 __global__ void __launch_bounds__(256) screen_cells_kernel(
     const float *__restrict__ x, uint32_t n, uint32_t d, const float *__restrict__ xn, uint32_t C,
     const uint32_t *__restrict__ members, const uint32_t *__restrict__ cstart, const uint32_t *__restrict__ near,
-    uint32_t P, const uint32_t *__restrict__ blk_cell, const uint32_t *__restrict__ blk_row0,
-    uint32_t *__restrict__ out_ids) {
+    uint32_t P, const uint32_t *__restrict__ rows, const uint32_t *__restrict__ blk_cell,
+    const uint32_t *__restrict__ blk_row0, uint32_t *__restrict__ out_ids) {
     extern __shared__ __align__(16) uint8_t sm[];
     float *Qs = reinterpret_cast<float *>(sm);                 // [kBK][kBQ]
     float *Vs = Qs + kBK * kBQ;                                // [kBK][kBV]
@@ -257,10 +269,10 @@ __global__ void __launch_bounds__(256) screen_cells_kernel(
     uint32_t *vid = qid + kBQ;                                 // [kBV] candidate ids of the tile (~0: none)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t cell = blk_cell[blockIdx.x];
-    const uint32_t p0 = blk_row0[blockIdx.x], pend = cstart[cell + 1];
+    const uint32_t p0 = blk_row0[blockIdx.x], pend = blk_row0[blockIdx.x + 1];
     for (int i = tid; i < kBQ; i += 256) {
         cnt[i] = 0;
-        qid[i] = p0 + i < pend ? members[p0 + i] : 0xffffffffu;
+        qid[i] = p0 + i < pend ? rows[p0 + i] : 0xffffffffu;
     }
     const int ty = tid / 16, tx = tid % 16;  // rows ty*4.., cols tx*8..
     __syncthreads();
@@ -298,7 +310,10 @@ __global__ void __launch_bounds__(256) screen_cells_kernel(
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                        for (int j = 0; j < 8; ++j) {
+                        const float t = DIRECT ? a[i] - b[j] : 0.f;
+                        acc[i][j] = DIRECT ? fmaf(t, t, acc[i][j]) : fmaf(a[i], b[j], acc[i][j]);
+                    }
                 }
                 __syncthreads();
             }
@@ -309,8 +324,8 @@ __global__ void __launch_bounds__(256) screen_cells_kernel(
                 for (int j = 0; j < 8; ++j) {
                     const uint32_t gv = vid[tx * 8 + j];
                     const bool ok = gv < n && gv != gq;
-                    D[(ty * 4 + i) * (kBV + 1) + tx * 8 + j] =
-                        ok ? fmaf(-2.f, acc[i][j], xn[gv]) : __int_as_float(0x7f800000);
+                    const float v = DIRECT ? fminf(acc[i][j], 3.4e38f) : ok ? fmaf(-2.f, acc[i][j], xn[gv]) : 0.f;
+                    D[(ty * 4 + i) * (kBV + 1) + tx * 8 + j] = ok ? v : __int_as_float(0x7f800000);
                 }
             }
             __syncthreads();
@@ -904,12 +919,14 @@ __global__ void __launch_bounds__(256) parent_kernel(const uint32_t *__restrict_
 
 }  // namespace
 
-// The float32 screen of nr rows (of the list `rows`, or all without it).
+// The float32 screen of all rows, or (DIRECT) of the nr rows in the list `rows` (all
+// without it).
+template <bool DIRECT>
 static int screen_fp32(const float *x, uint32_t n, uint32_t d, const float *xn, uint32_t C, const uint32_t *rows,
                        uint32_t nr, uint32_t *cand, cudaStream_t s) {
     const size_t smem = (size_t) (kBK * kBQ + kBK * kBV + kBQ * (kBV + 1)) * 4 + (size_t) kBQ * C * 8 + kBQ * 8;
-    GCU(allow_shared((const void *) screen_kernel));
-    screen_kernel<<<(nr + kBQ - 1) / kBQ, 256, smem, s>>>(x, n, d, xn, C, rows, nr, cand);
+    GCU(allow_shared((const void *) screen_kernel<DIRECT>));
+    screen_kernel<DIRECT><<<(nr + kBQ - 1) / kBQ, 256, smem, s>>>(x, n, d, xn, C, rows, nr, cand);
     GCU(cudaGetLastError());
     return PANNS_OK;
 }
@@ -1200,12 +1217,12 @@ int panns_build_nsg_ex(int device, const float *base, uint32_t n, uint32_t d, ui
         if (safe) GCU(cudaMemcpyAsync(&nf, nfail.p, 4, cudaMemcpyDeviceToHost, s));
         GCU(cudaStreamSynchronize(s));
         if (nf) {
-            rc = screen_fp32(x.p, n, d, xn.p, C, safe ? fail.p : nullptr, nf, cand.p, s);
+            rc = screen_fp32<true>(x.p, n, d, xn.p, C, safe ? fail.p : nullptr, nf, cand.p, s);
             if (rc) return rc;
             GCU(cudaStreamSynchronize(s));
         }
     } else if (!tc) {
-        const int rc = screen_fp32(x.p, n, d, xn.p, C, nullptr, n, cand.p, s);
+        const int rc = screen_fp32<false>(x.p, n, d, xn.p, C, nullptr, n, cand.p, s);
         if (rc) return rc;
     } else {
         // -2 x.y for tiles of TR rows x TC candidates by TF32 tensor-core GEMMs
@@ -1322,11 +1339,13 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
     GCU(cudaMemsetAsync(cand.p, 0xff, (size_t) n * C * 4, s));
     // Tensor-core screen: every cell padded to whole tiles, a row block of one
     // cell against the tiles of the cell and of its near cells. Where padding
-    // would more than double the rows (cells of a few dozen rows), or its
-    // lists cannot settle a row, the float32 screen runs.
+    // would more than double the rows (cells of a few dozen rows) the float32
+    // screen runs, and it runs for the rows whose lists cannot be settled.
     uint64_t slots = 0;
     for (uint32_t c = 0; c < cells; ++c) slots += (cstart[c + 1] - cstart[c] + kTcM - 1) / kTcM * (uint64_t) kTcM;
-    bool screened = false;
+    std::vector<uint32_t> left;  // rows for the float32 screen, cell by cell
+    bool all_left = true;
+    bool direct = false;  // the tensor-core screen ran
     size_t free_b = 0, total_b = 0;
     GCU(cudaMemGetInfo(&free_b, &total_b));
     if (d <= 256 && n >= kTcMinRows && slots <= 2ull * n && slots <= 0x7fffffffull &&
@@ -1365,32 +1384,54 @@ int panns_build_nsg_cells(int device, const float *base, uint32_t n, uint32_t d,
         const int rc = tc_screen_knn(x.p, n, d, k, C, dorder.p, (uint32_t) slots, &tc, cand.p, fail.p, nfail.p, &safe,
                                      num_sms, s);
         if (rc) return rc;
-        uint32_t nf = 0;
-        GCU(cudaMemcpyAsync(&nf, nfail.p, 4, cudaMemcpyDeviceToHost, s));
-        GCU(cudaStreamSynchronize(s));
-        screened = safe && nf == 0;
+        direct = true;
+        all_left = !safe;
+        if (safe) {
+            uint32_t nf = 0;
+            GCU(cudaMemcpyAsync(&nf, nfail.p, 4, cudaMemcpyDeviceToHost, s));
+            GCU(cudaStreamSynchronize(s));
+            left.resize(nf);
+            if (nf) GCU(cudaMemcpyAsync(left.data(), fail.p, (size_t) nf * 4, cudaMemcpyDeviceToHost, s));
+            GCU(cudaStreamSynchronize(s));
+            std::sort(left.begin(), left.end(), [&cellh](uint32_t a, uint32_t b) {
+                return cellh[a] != cellh[b] ? cellh[a] < cellh[b] : a < b;
+            });
+        }
     }
-    if (!screened) {
+    if (all_left || !left.empty()) {
         // Blocks of up to kBQ rows of one cell.
         std::vector<uint32_t> blk_cell, blk_row0;
-        for (uint32_t c = 0; c < cells; ++c)
-            for (uint32_t r = cstart[c]; r < cstart[c + 1]; r += kBQ) {
-                blk_cell.push_back(c);
-                blk_row0.push_back(r);
+        const uint32_t rows = all_left ? n : (uint32_t) left.size();
+        for (uint32_t r = 0, c = 0; r < rows;) {
+            uint32_t end;
+            if (all_left) {
+                while (cstart[c + 1] <= r) ++c;
+                end = std::min(cstart[c + 1], r + kBQ);
+            } else {
+                c = cellh[left[r]];
+                for (end = r + 1; end < rows && end < r + kBQ && cellh[left[end]] == c;) ++end;
             }
-        Buf<uint32_t> dnear, dbc, dbr;
+            blk_cell.push_back(c);
+            blk_row0.push_back(r);
+            r = end;
+        }
+        blk_row0.push_back(rows);
+        Buf<uint32_t> dnear, dbc, dbr, drows;
         GCU(dnear.alloc(nearh.size(), s));
         GCU(dbc.alloc(blk_cell.size(), s));
         GCU(dbr.alloc(blk_row0.size(), s));
-        GCU(cudaMemsetAsync(cand.p, 0xff, (size_t) n * C * 4, s));
+        GCU(drows.alloc(left.size(), s));
+        if (!left.empty())
+            GCU(cudaMemcpyAsync(drows.p, left.data(), left.size() * 4, cudaMemcpyHostToDevice, s));
         GCU(cudaMemcpyAsync(dnear.p, nearh.data(), nearh.size() * 4, cudaMemcpyHostToDevice, s));
         GCU(cudaMemcpyAsync(dbc.p, blk_cell.data(), blk_cell.size() * 4, cudaMemcpyHostToDevice, s));
         GCU(cudaMemcpyAsync(dbr.p, blk_row0.data(), blk_row0.size() * 4, cudaMemcpyHostToDevice, s));
         const size_t smem = (size_t) (kBK * kBQ + kBK * kBV + kBQ * (kBV + 1)) * 4 + (size_t) kBQ * C * 8 +
                             (size_t) kBQ * 8 + (size_t) kBV * 4;
-        GCU(allow_shared((const void *) screen_cells_kernel));
-        screen_cells_kernel<<<(unsigned) blk_cell.size(), 256, smem, s>>>(x.p, n, d, xn.p, C, dmem.p, dstart.p,
-                                                                           dnear.p, P, dbc.p, dbr.p, cand.p);
+        const auto kern = direct ? screen_cells_kernel<true> : screen_cells_kernel<false>;
+        GCU(allow_shared((const void *) kern));
+        kern<<<(unsigned) blk_cell.size(), 256, smem, s>>>(x.p, n, d, xn.p, C, dmem.p, dstart.p, dnear.p, P,
+                                                           all_left ? dmem.p : drows.p, dbc.p, dbr.p, cand.p);
         GCU(cudaGetLastError());
         GCU(cudaStreamSynchronize(s));
     }

@@ -816,11 +816,16 @@ __global__ void __launch_bounds__(256) tc_shift_kernel(const float *__restrict__
     if ((threadIdx.x & 31) == 0) atomicMax(spread, most);
 }
 
-// The power of two (exact to multiply by) that brings the spread to [0.5, 1), or as
-// near as float32's exponents allow; 1 for a spread of 0.
-__device__ __forceinline__ float tc_scale(const uint32_t *spread) {
+// The d shifts in scaled units, in place, and the scale after them: element j of a
+// row goes into the screen as x_j * frame[d] - frame[j]. The scale is the power of
+// two (exact to multiply by) that brings the spread to [0.5, 1), or as near as
+// float32's exponents allow; 1 for a spread of 0. One block.
+__global__ void __launch_bounds__(256) tc_frame_kernel(float *__restrict__ frame, const uint32_t *__restrict__ spread,
+                                                       uint32_t d) {
     const uint32_t bits = *spread, e = bits >> 23;  // biased exponent; 0 below the normal range
-    return bits ? __uint_as_float(max(1, 253 - (int) e) << 23) : 1.f;
+    const float scale = bits ? __uint_as_float(max(1, 253 - (int) e) << 23) : 1.f;
+    for (uint32_t j = threadIdx.x; j < d; j += 256) frame[j] *= scale;
+    if (threadIdx.x == 0) frame[d] = scale;
 }
 
 // One block per tile of kTcM positions from p0: its rows (row perm[p] of x, p
@@ -842,8 +847,7 @@ constexpr int kPrepSteps = 5;  // 64-wide steps of an operand row: W <= 320
 
 __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict__ x, uint32_t n, uint32_t d,
                                                          const uint32_t *__restrict__ perm, uint32_t p0,
-                                                         uint32_t valid, uint32_t W, const float *__restrict__ shift,
-                                                         const uint32_t *__restrict__ spread,
+                                                         uint32_t valid, uint32_t W, const float *__restrict__ frame,
                                                          __nv_bfloat16 *__restrict__ A, __nv_bfloat16 *__restrict__ B,
                                                          float *__restrict__ xn, uint32_t *__restrict__ ymax,
                                                          uint32_t *__restrict__ large, float *__restrict__ centre,
@@ -860,8 +864,8 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
         filled = row < n;
         rows[tid] = filled ? row : kNone;
     }
-    const float scale = tc_scale(spread);
-    if (tid < d) sh[tid] = shift[tid] * scale;
+    const float scale = frame[d];
+    if (tid < d) sh[tid] = frame[tid];
     const uint32_t count = (uint32_t) __syncthreads_count(filled);
     if (d % 4 == 0) {
         const uint32_t d4 = d / 4, di = 256 / d4, dq = 256 - di * d4;
@@ -1005,7 +1009,7 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
 // 0.76 ms so.
 __global__ void __launch_bounds__(256) tc_need_kernel(const float *__restrict__ q, const uint32_t *__restrict__ qperm,
                                                       uint32_t nq, const float *__restrict__ tau,
-                                                      const uint32_t *__restrict__ spread, const float *__restrict__ cb, const float *__restrict__ rb,
+                                                      const float *__restrict__ scale_at, const float *__restrict__ cb, const float *__restrict__ rb,
                                                       uint32_t nb, uint32_t d, float *__restrict__ need) {
     __shared__ __align__(16) float sa[2][16][kTcM + 4];
     __shared__ __align__(16) float sb[2][16][68];
@@ -1020,7 +1024,7 @@ __global__ void __launch_bounds__(256) tc_need_kernel(const float *__restrict__ 
     if (tid < kTcM) st[tid] = i0 + tid < nq ? tau[i0 + tid] : -1.f;
     if (tid < 64) any[tid] = 0;
     float va[8], vc[4];
-    const float scale = tc_scale(spread);
+    const float scale = *scale_at;
     const bool quads = d % 4 == 0;
     auto fetch4 = [&](const float *r, uint32_t k, float *v) {
         if (quads && r && k < d) {
@@ -1232,10 +1236,10 @@ __global__ void tc_scatter_kernel(const uint32_t *__restrict__ cell, uint32_t n,
 }
 
 // Squared radii in scaled units, rounded up.
-__global__ void tc_tau_kernel(const double *__restrict__ tau, uint32_t nq, const uint32_t *__restrict__ spread,
+__global__ void tc_tau_kernel(const double *__restrict__ tau, uint32_t nq, const float *__restrict__ scale_at,
                               float *__restrict__ out) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const double scale = (double) tc_scale(spread);
+    const double scale = (double) *scale_at;
     if (i < nq) out[i] = __double2float_ru(tau[i] * (scale * scale));
 }
 
@@ -1361,7 +1365,7 @@ int tc_screen_knn(const float *x, uint32_t n, uint32_t d, uint32_t k, uint32_t C
     const TcShape sh = tc_shape(d);
     const uint32_t tiles = (slots + kTcM - 1) / kTcM, pad = tiles * kTcM;
     TBuf<__nv_bfloat16> A, B;
-    TBuf<float> xn, centre, radius, lb2, shift;
+    TBuf<float> xn, centre, radius, lb2, frame;
     TBuf<uint2> lists;
     TBuf<uint32_t> ctl;  // counter, error, ymax, large, spread
     // Row operands and bounds between tiles for a limited number of row blocks at a time.
@@ -1377,13 +1381,13 @@ int tc_screen_knn(const float *x, uint32_t n, uint32_t d, uint32_t k, uint32_t C
     TCU(B.alloc((size_t) pad * 2 * sh.W, s));
     TCU(xn.alloc(pad, s));
     TCU(ctl.alloc(5, s));
-    TCU(shift.alloc(d, s));
     TCU(cudaMemsetAsync(ctl.p, 0, 20, s));
     TCU(cudaMemsetAsync(fail_count, 0, 4, s));
-    const uint32_t *spread = ctl.p + 4;
-    tc_shift_kernel<<<d, 256, 0, s>>>(x, n, d, shift.p, ctl.p + 4);
+    TCU(frame.alloc(d + 1, s));
+    tc_shift_kernel<<<d, 256, 0, s>>>(x, n, d, frame.p, ctl.p + 4);
+    tc_frame_kernel<<<1, 256, 0, s>>>(frame.p, ctl.p + 4, d);
     TCU(allow_shared((const void *) tc_prepare_kernel));
-    tc_prepare_kernel<<<tiles, 256, kTcM * d * 4, s>>>(x, n, d, perm, 0, slots, sh.W, shift.p, spread,
+    tc_prepare_kernel<<<tiles, 256, kTcM * d * 4, s>>>(x, n, d, perm, 0, slots, sh.W, frame.p,
                                                        per == tiles ? A.p : nullptr, B.p, xn.p, ctl.p + 2, ctl.p + 3,
                                                        centre.p, radius.p);
     TCU(cudaGetLastError());
@@ -1395,7 +1399,7 @@ int tc_screen_knn(const float *x, uint32_t n, uint32_t d, uint32_t k, uint32_t C
     for (uint32_t rb0 = 0; rb0 < tiles; rb0 += per) {
         const uint32_t m = std::min(per, tiles - rb0);
         if (per != tiles) {
-            tc_prepare_kernel<<<m, 256, kTcM * d * 4, s>>>(x, n, d, perm, rb0 * kTcM, slots, sh.W, shift.p, spread, A.p,
+            tc_prepare_kernel<<<m, 256, kTcM * d * 4, s>>>(x, n, d, perm, rb0 * kTcM, slots, sh.W, frame.p, A.p,
                                                            nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
             TCU(cudaGetLastError());
         }
@@ -1469,7 +1473,7 @@ int tc_screen_range(const float *x, uint32_t n, uint32_t d, const uint32_t *perm
                                       std::max<uint64_t>(kTcM, std::min(by_rows, by_need) / kTcM * kTcM));
     const uint32_t ct = chunk / kTcM;
     TBuf<__nv_bfloat16> A, B;
-    TBuf<float> xn, cb, rad, need, ft, shift;
+    TBuf<float> xn, cb, rad, need, ft, frame;
     TBuf<uint32_t> ctl;  // counter, error, ymax, large, spread
     TCU(A.alloc((size_t) qpad * 2 * sh.W, s));
     TCU(B.alloc((size_t) chunk * 2 * sh.W, s));
@@ -1478,15 +1482,15 @@ int tc_screen_range(const float *x, uint32_t n, uint32_t d, const uint32_t *perm
     TCU(rad.alloc(ct, s));
     TCU(need.alloc((size_t) rb * ct, s));
     TCU(ft.alloc(nq, s));
-    TCU(shift.alloc(d, s));
+    TCU(frame.alloc(d + 1, s));
     TCU(ctl.alloc(5, s));
     TCU(cudaMemsetAsync(ctl.p, 0, 20, s));
     TCU(cudaMemsetAsync(cnt, 0, (size_t) splits * nq * 4, s));
-    const uint32_t *spread = ctl.p + 4;
-    tc_shift_kernel<<<d, 256, 0, s>>>(x, n, d, shift.p, ctl.p + 4);
-    tc_tau_kernel<<<(nq + 255) / 256, 256, 0, s>>>(tau, nq, spread, ft.p);
+    tc_shift_kernel<<<d, 256, 0, s>>>(x, n, d, frame.p, ctl.p + 4);
+    tc_frame_kernel<<<1, 256, 0, s>>>(frame.p, ctl.p + 4, d);
+    tc_tau_kernel<<<(nq + 255) / 256, 256, 0, s>>>(tau, nq, frame.p + d, ft.p);
     TCU(allow_shared((const void *) tc_prepare_kernel));
-    tc_prepare_kernel<<<rb, 256, kTcM * d * 4, s>>>(queries, kNone, d, qperm, 0, nq, sh.W, shift.p, spread, A.p, nullptr,
+    tc_prepare_kernel<<<rb, 256, kTcM * d * 4, s>>>(queries, kNone, d, qperm, 0, nq, sh.W, frame.p, A.p, nullptr,
                                                     xn.p, nullptr, ctl.p + 3, nullptr, nullptr);
     TCU(cudaGetLastError());
     CUtensorMap ma, mb;
@@ -1496,10 +1500,10 @@ int tc_screen_range(const float *x, uint32_t n, uint32_t d, const uint32_t *perm
     for (uint64_t c0 = 0; c0 < slots; c0 += chunk) {
         const uint32_t m = (uint32_t) std::min<uint64_t>(chunk, slots - c0), mt = (m + kTcM - 1) / kTcM;
         TCU(cudaMemsetAsync(ctl.p + 2, 0, 4, s));
-        tc_prepare_kernel<<<mt, 256, kTcM * d * 4, s>>>(x, n, d, perm, (uint32_t) c0, slots, sh.W, shift.p, spread, nullptr,
+        tc_prepare_kernel<<<mt, 256, kTcM * d * 4, s>>>(x, n, d, perm, (uint32_t) c0, slots, sh.W, frame.p, nullptr,
                                                         B.p, nullptr, ctl.p + 2, ctl.p + 3, cb.p, rad.p);
-        tc_need_kernel<<<dim3((mt + 63) / 64, rb), 256, 0, s>>>(queries, qperm, nq, ft.p, spread, cb.p, rad.p, mt, d,
-                                                                need.p);
+        tc_need_kernel<<<dim3((mt + 63) / 64, rb), 256, 0, s>>>(queries, qperm, nq, ft.p, frame.p + d, cb.p, rad.p,
+                                                                mt, d, need.p);
         TCU(cudaGetLastError());
         TcArgs a{};
         a.rows = nq;

@@ -7,6 +7,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <memory>
@@ -853,33 +854,57 @@ static uint32_t block_buffer(uint32_t max_deg, uint32_t M, uint32_t W) {
 }
 
 // Warps per query where the caller leaves the choice open (same ids either
-// way). More warps shorten a query but fewer queries are resident at once, and a
-// batch takes as many waves as its residents make it, so the choice is the
-// smallest waves x cost, cost relative to one warp. Measured on 1M x 96, M = 8
-// (ms per wave at L = 384, float32: 1.33 / 0.82 / 0.55 / 0.36-0.42 / 0.33 with 1 /
-// 2 / 4 / 8 / 16 warps; the ratios at L = 100 and 1,024 and with the FP8 copy are
-// within a fifth of it, but at L = 1,024 16 warps take 0.92 against 0.78 ms with
-// 8) and on 100k x 128 at L = 2,048 (9.8 / 3.5 / 2.0 / 1.7). Examples, ms with 1 /
-// 2 / 4 / 8 warps: 220 queries 1.34 / 0.82 / 0.52 / 0.42, 500 1.33 / 0.85 / 0.58 /
-// 0.80, 740 1.37 / 0.88 / 1.02 / 1.16, 1,480 1.48 / 1.68 / 1.57 / 1.98; 1,000 at
-// L = 2,048 10.6 / 9.1 / 6.4 / 7.1.
+// way): the W with the smallest estimate of the batch's time
+//     cost(W) * waves * (1 + 0.6 fill).
+// More warps shorten a query (cost, relative to one warp), but fewer queries are
+// resident at once, so a batch takes more waves: queries over residents, rounded up
+// for 0.8 and not for 0.2, since a wave's short queries make room for the next one's.
+// fill, the resident warps over the 24 that one-warp queries reach on an SM, stands
+// for what full SMs add to a query's time. Residents are those the launch takes
+// (blocks_in_196kb). cost depends on the neighbours of a step, M x the mean degree:
+// the more, the more warps have to do; below 64, several warps share a candidate's
+// row and eight gain nothing over four. A batch of more than one wave of one-warp
+// queries that fill at least two thirds of the SM takes one warp each.
+//
+// The constants are fitted to 942 measurements: M = 1, 8 and 33, L = 32 to 3,000 and 1
+// to 5,000 queries on 1M x 96 (mean degree 19; float32 and FP8) and 100,000 x 128 (45),
+// each with 1, 2, 4 and 8 warps. The choice is 1 % slower than the best of them in
+// the mean, up to 1.4 times in single cases. One table up to L = 2,047 and one from there on, more
+// residents than the launch takes and whole waves were 4 % slower in the mean and up
+// to 1.8 times. Examples, ms with 1 / 2 / 4 / 8 warps, the choice in brackets: 1M x 96,
+// float32, M = 8, L = 384: 300 queries 1.14 / 0.83 / [0.50] / 0.69, 1,000 1.18 / [0.97] /
+// 1.10 / 1.53, 1,480 [1.30] / 1.78 / 1.60 / 2.17; L = 2,047: 1,000 4.96 / 7.20 / [4.33] /
+// 6.40. 100,000 x 128, 1,000 queries: L = 100 0.61 / 0.59 / [0.52] / 0.61, L = 1,200 5.05 /
+// 5.67 / [4.00] / 4.40.
+// 16 warps serve up to one query per SM, L <= 512 (64 queries at L = 384: 0.33 ms, 0.34
+// with 8), unless the visited bits fit shared memory beside 8 warps but not beside 16
+// (M = 33, L = 100: 0.28 against 0.20).
 static int choose_warps(panns_index *h, const panns_search_params *p, uint32_t kind, int CL, uint32_t M, uint32_t nq,
                         uint32_t &wpq) {
     static const uint32_t warps[5] = {1, 2, 4, 8, 16};
-    static const float short_cost[5] = {1.f, 0.61f, 0.40f, 0.28f, 0.25f};
-    static const float long_cost[5] = {1.f, 0.36f, 0.20f, 0.175f, 0.2f};
-    const float *cost = p->L < 2048 ? short_cost : long_cost;
+    // below 64, below 250 and from 250 neighbours of a step on
+    static const float cost[3][5] = {{1.f, 0.70f, 0.50f, 0.60f, 0.80f},
+                                     {1.f, 0.80f, 0.42f, 0.31f, 0.25f},
+                                     {1.f, 0.60f, 0.31f, 0.235f, 0.19f}};
+    const double step = (double) M * (double) h->nbrs.size() / h->n;
+    const float *rel = cost[step < 64.0 ? 0 : step < 250.0 ? 1 : 2];
     const uint32_t qcap = ((p->L + 31) / 32) * 32;
+    const uint32_t words = (h->n + 31) / 32;
+    auto block_bytes = [&](uint32_t W, uint32_t vis) {
+        return (size_t) block_smem_bytes(qcap, W, block_buffer(h->max_deg, M, W), vis);
+    };
     float best = 0.f;
     wpq = 1;
     for (int i = 0; i < 5; ++i) {
         const uint32_t W = warps[i];
         if (W == 16 && (p->L > 512 || nq > (uint32_t) h->num_sms)) continue;
+        if (W == 16 && (size_t) words * 4 < kSmemLimit && block_bytes(8, words) <= kSmemLimit &&
+            block_bytes(16, words) > kSmemLimit)
+            continue;
         uint32_t wpb = 4;
         if (W == 1)
             while (wpb > 1 && wpb * warp_smem_bytes(qcap) > kSmemLimit) --wpb;
-        const size_t smem = W == 1 ? (size_t) wpb * warp_smem_bytes(qcap)
-                                   : (size_t) block_smem_bytes(qcap, W, block_buffer(h->max_deg, M, W), 0);
+        const size_t smem = W == 1 ? (size_t) wpb * warp_smem_bytes(qcap) : block_bytes(W, 0);
         if (smem > kSmemLimit) continue;
         const void *kern = W == 1 ? search_kernel_ptr(kind, ORDER_PANNS, CL, p->storage)
                                   : search_block_kernel_ptr(kind, CL, W, p->storage);
@@ -888,9 +913,12 @@ static int choose_warps(panns_index *h, const panns_search_params *p, uint32_t k
         const int rc = resident_blocks(h, kern, (int) (W == 1 ? wpb : W) * 32, smem, r);
         if (rc) return rc;
         if (r.per_sm < 1) continue;
-        const uint32_t at_once = (uint32_t) r.per_sm * (uint32_t) h->num_sms * (W == 1 ? wpb : 1u);
-        if (W == 1 && p->L < 2048 && nq > at_once) break;  // one warp each keeps every SM full
-        const float c = (float) ((nq + at_once - 1) / at_once) * cost[i];
+        const uint32_t at_once = blocks_in_196kb(r.per_sm, smem) * (uint32_t) h->num_sms * (W == 1 ? wpb : 1u);
+        const float x = (float) nq / (float) at_once;
+        const float waves = x <= 1.f ? 1.f : 0.8f * std::ceil(x) + 0.2f * x;
+        const float fill = (float) std::min(nq, at_once) * (float) W / (24.f * (float) h->num_sms);
+        if (W == 1 && x > 1.f && fill >= 0.66f) break;
+        const float c = rel[i] * waves * (1.f + 0.6f * fill);
         if (best == 0.f || c < best) {
             best = c;
             wpq = W;

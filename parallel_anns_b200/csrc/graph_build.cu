@@ -1471,8 +1471,7 @@ int panns_graph_copy(const panns_graph *g, uint64_t *offsets, uint32_t *nbrs, ui
     if (offsets) memcpy(offsets, g->off.data(), g->off.size() * 8);
     if (nbrs && !g->nbrs.empty()) memcpy(nbrs, g->nbrs.data(), g->nbrs.size() * 4);
     if (knn && g->knn_dev) {
-        GCU(cudaSetDevice(g->device));
-        GCU(cudaMemcpy(knn, g->knn_dev, (size_t) g->n * g->k * 4, cudaMemcpyDeviceToHost));
+        GCU(g->copy_knn(knn));
     } else if (knn) {
         memcpy(knn, g->knn.data(), g->knn.size() * 4);
     }

@@ -52,13 +52,29 @@ struct panns_graph {
     panns::HostWords knn;
     uint32_t *knn_dev = nullptr;
     int device = 0;
-    ~panns_graph() {
-        if (!knn_dev) return;
+    // Calls on the lists in device memory go to the calling thread's own stream, in a
+    // mode that a stream capture under way does not object to (the legacy stream
+    // would become part of it), and leave the thread's device as it was.
+    template <typename F>
+    cudaError_t on_device(F call) const {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
         int before = 0;
         cudaGetDevice(&before);
-        cudaSetDevice(device);
-        panns::scratch_free(knn_dev, nullptr);
+        cudaError_t e = cudaSetDevice(device);
+        if (e == cudaSuccess) e = call(cudaStreamPerThread);
         cudaSetDevice(before);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        return e;
+    }
+    cudaError_t copy_knn(uint32_t *out) const {
+        return on_device([&](cudaStream_t s) {
+            const cudaError_t e = cudaMemcpyAsync(out, knn_dev, (size_t) n * k * 4, cudaMemcpyDeviceToHost, s);
+            return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+        });
+    }
+    ~panns_graph() {
+        if (knn_dev) on_device([&](cudaStream_t s) { return cudaFreeAsync(knn_dev, s); });
     }
     uint32_t k = 0;
     uint32_t repaired = 0;

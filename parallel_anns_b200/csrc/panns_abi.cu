@@ -1154,15 +1154,14 @@ static int stage_init(panns_index *h, const panns_search_params *p, const uint32
         d_init = h->init_def.p;
         return PANNS_OK;
     }
+    // efanna2e's default lists begin with the entry's neighbours as the graph holds
+    // them (the rest is drawn without repeats): one that is there twice is in every list.
+    if (efanna && !init_ids && std::min<uint64_t>(L, h->off[h->entry + 1] - h->off[h->entry]) > h->entry_distinct)
+        return fail(PANNS_EINVAL, "search: duplicate init id");
     std::vector<uint32_t> buf;
     const uint32_t *ids = init_ids;
     if (!ids) {
         if (efanna) {
-            // The lists begin with the entry's neighbours as the graph holds them
-            // (the rest is drawn without repeats), so one that is there twice is in
-            // every list.
-            if (std::min<uint64_t>(L, h->off[h->entry + 1] - h->off[h->entry]) > h->entry_distinct)
-                return fail(PANNS_EINVAL, "search: duplicate init id");
             int32_t st[40];
             panns_rand_seed(st, 1);
             buf.resize((size_t) nq * L);

@@ -173,6 +173,7 @@ struct panns_index {
     DevBuf<float> base_raw, vec, norms;
     DevBuf<uint8_t> vec_lo;         // reduced copy (BF16 or FP8 rows)
     DevBuf<float> norms_lo, scales; // its norms; FP8 per-dimension scales
+    float q8_scale = 1.f;           // FP8: power of two that queries are multiplied by
     bool ready = false;             // vec/norms/head built for the current base + graph
     std::vector<uint32_t> perm, inv;  // device id -> original id, and back
     std::vector<uint32_t> cell_start; // device ids of each cell of the layout order (cells + 1)
@@ -403,6 +404,21 @@ int panns_set_graph(panns_index *h, uint32_t width, uint32_t entry, const uint64
     return PANNS_OK;
 }
 
+// The power of two that FP8 searches multiply a query by (after the per-dimension
+// scales) before it becomes half precision, whose normal range is 6e-5 to 65,504;
+// `most`: the largest such product (without it) of a base vector. 2^12 where that
+// puts `most` between 2^-6, which leaves room for much smaller elements, and an
+// eighth of the upper end, which leaves room for larger queries; else what puts it
+// just below that eighth. Results do not depend on it while no element leaves the
+// range. (2^12 for every base made infinities of integers up to 255.)
+static float fp8_query_scale(double most) {
+    const double room = 65504.0 / 8;
+    if (!(most > 0.0) || (most * 4096.0 <= room && most * 4096.0 >= 1.0 / 64)) return 4096.f;
+    int e = 0;
+    std::frexp(room / most, &e);  // 2^(e - 1) <= room / most < 2^e
+    return std::ldexp(1.f, std::max(-100, std::min(100, e - 1)));
+}
+
 // Build the search layout from the current base + graph: the locality order
 // (vertices grouped by their nearest of C pivot vertices, original id order
 // inside a group), chain-major rows and norms in that order, head rows and
@@ -471,13 +487,16 @@ static int finalize(panns_index *h) {
             absmax_kernel<<<h->num_sms * 8, 256, 0, h->stream>>>(h->base_raw.p, n, (int) h->d, amax.p);
             CU(cudaGetLastError());
             std::vector<unsigned int> am(h->d);
+            double most = 0.0;  // largest base value times its dimension's scale
             CU(cudaMemcpyAsync(am.data(), amax.p, h->d * 4ull, cudaMemcpyDeviceToHost, h->stream));
             CU(cudaStreamSynchronize(h->stream));
             for (uint32_t e = 0; e < h->d; ++e) {
                 float m;
                 memcpy(&m, &am[e], 4);
                 sc[e] = m > 0.f ? m / 448.0f : 1.0f;  // E4M3 largest finite value: 448
+                most = std::max(most, m < INFINITY ? (double) m * sc[e] : 0.0);
             }
+            h->q8_scale = fp8_query_scale(most);
         }
         CU(cudaMemcpyAsync(h->scales.p, sc.data(), h->dpad * 4ull, cudaMemcpyHostToDevice, h->stream));
         const int blocks = std::max(1, (int) std::min<uint32_t>((n + 127) / 128, h->num_sms * 16u));
@@ -1076,6 +1095,8 @@ static int launch_search(panns_index *h, const panns_search_params *p, float *d_
     a.vec_lo = h->vec_lo.p;
     a.norms_lo = h->norms_lo.p;
     a.scales = h->scales.p;
+    a.q8_scale = h->q8_scale;
+    a.q8_m2 = -2.0f / h->q8_scale;
     a.d = h->d;
     a.n = h->n;
     a.queries = reinterpret_cast<const float4 *>(d_queries_cm);

@@ -113,6 +113,7 @@ struct SearchArgs {
     const void *vec_lo;       // reduced rows, natural element order: n x dpad (BF16 or FP8)
     const float *norms_lo;    // ||v||^2 of the dequantised rows
     const float *scales;      // FP8: per-dimension scale (dpad)
+    float q8_scale, q8_m2;    // FP8: the power of two queries are multiplied by, and -2 over it
     uint32_t d;               // dimension
     const uint32_t *Lq;       // per-query queue length (K <= Lq[q] <= L), or null: L for all
     const uint32_t *decisions;  // per-query records of the entry / L-budget network (mlp_decide), or null
@@ -586,13 +587,14 @@ static __device__ __forceinline__ int chain_major_pos(int d, int e) {
 // query once.
 template <int KIND, int CL, int STORE>
 struct Dist {
-    // FP8 with PANNS_FP8_MIXED: the query (times the per-dimension scales and
-    // 2^12, which keeps it in half precision's normal range) as half pairs,
-    // multiplied with the E4M3 rows converted to half pairs by mixed-precision
-    // FMAs (half x half products are exact in float32, float32 accumulation);
-    // the 2^-12 is taken back in the final norm-trick FMA.
+    // FP8 with PANNS_FP8_MIXED: the query (times the per-dimension scales and a
+    // power of two of the index, which keep it in half precision's normal range;
+    // what is larger than a half can be is cut off there) as half pairs, multiplied
+    // with the E4M3 rows converted to half pairs by mixed-precision FMAs (half x
+    // half products are exact in float32, float32 accumulation); the power of two is
+    // taken back in the final norm-trick FMA.
     static constexpr bool kMixed = STORE == STORE_FP8 && PANNS_FP8_MIXED;
-    static constexpr float kMixedScale = 4096.0f;
+    static constexpr float kHalfMax = 65504.0f;
     float ql[kMixed ? 1 : 8 * CL];
     uint32_t qh[kMixed ? 4 * CL : 1];
     __device__ __forceinline__ void load(const SearchArgs &a, uint32_t q, int lane) {
@@ -606,7 +608,7 @@ struct Dist {
                 float x = e < (int) a.d ? __ldg(qrow + chain_major_pos((int) a.d, e)) : 0.f;
                 if (STORE == STORE_FP8) x *= __ldg(a.scales + e);
                 if constexpr (kMixed) {
-                    const __half h = __float2half_rn(x * kMixedScale);
+                    const __half h = __float2half_rn(fminf(fmaxf(x * a.q8_scale, -kHalfMax), kHalfMax));
                     const uint32_t hb = (uint32_t) __half_as_ushort(h);
                     if (j & 1) qh[4 * i + j / 2] |= hb << 16;
                     else qh[4 * i + j / 2] = hb;
@@ -715,7 +717,7 @@ struct Dist {
             s = __fadd2_rn(s, make_float2(__shfl_xor_sync(kFull, s.x, 1), __shfl_xor_sync(kFull, s.y, 1)));
             s = __fadd2_rn(s, make_float2(__shfl_xor_sync(kFull, s.x, 2), __shfl_xor_sync(kFull, s.y, 2)));
             if (t == 0) {
-                const float m2 = kMixed ? -2.f / kMixedScale : -2.f;
+                const float m2 = kMixed ? a.q8_m2 : -2.f;
                 const float2 r = __ffma2_rn(make_float2(m2, m2), s, make_float2(n0, n1));
                 if (act0) out[b] = ordered(r.x);
                 if (act1) out[bb] = ordered(r.y);

@@ -156,3 +156,46 @@ def test_efanna_build_with_nan_rows():
     a, b = efanna_build(xn, knn, 60, 12, 80), efanna_build(xi, knn, 60, 12, 80)
     assert a.entry < n and a.nbrs.max() < n
     assert np.array_equal(a.offsets, b.offsets) and np.array_equal(a.nbrs, b.nbrs)
+
+
+@pytest.mark.parametrize("warps", [1, 4])
+def test_fp8_search_at_any_scale(warps):
+    """Base and queries times a power of two: the FP8 rows are the same, their scales
+    and the queries follow, so the ids do too. (No element is near zero, so none
+    leaves half precision's range for another reason.)"""
+    from parallel_anns_b200 import native as N
+    from parallel_anns_b200.searching import Index
+    rng = np.random.default_rng(2)
+    n, d, K, L = 5000, 64, 20, 60
+
+    def rows(m):
+        return ((0.5 + 0.5 * rng.random((m, d))) * rng.choice([-1, 1], (m, d))).astype(np.float32)
+
+    x, q, g = rows(n), rows(50), _graph(n, 24, 4)
+    want = None
+    for e in (0, -30, -12, -6, -5, 5, 6, 7, 8, 20):
+        with Index(0) as ix:
+            ix.set_base(np.ldexp(x, e), storage=N.STORE_FP8)
+            ix.set_graph(g)
+            ids, _ = ix.search(np.ldexp(q, e), K=K, L=L, mode=N.MODE_TOP_M, M=4, storage=N.STORE_FP8,
+                               warps_per_query=warps)
+        want = ids if want is None else want
+        assert np.array_equal(ids, want), e
+
+
+def test_fp8_search_of_integers():
+    """Integers up to 255: queries times their scales and 2^12 are past half precision.
+    The FP8 search finds what the float32 search finds, but for a few."""
+    from parallel_anns_b200 import datasets as ds
+    from parallel_anns_b200 import native as N
+    from parallel_anns_b200.graph import build_nsg
+    from parallel_anns_b200.searching import Index
+    x, q = ds.uint8_cube(12_000, 128, seed=3), ds.uint8_cube(200, 128, seed=4)
+    with Index(0) as ix:
+        ix.set_base(x, storage=N.STORE_FP8)
+        ix.set_graph(build_nsg(x, R=64, knn_k=64))
+        a, _ = ix.search(q, K=50, L=400, mode=N.MODE_TOP_M, M=4)
+        b, _ = ix.search(q, K=50, L=400, mode=N.MODE_TOP_M, M=4, storage=N.STORE_FP8)
+        far, _ = ix.search(q * np.float32(1000), K=50, L=400, mode=N.MODE_TOP_M, M=4, storage=N.STORE_FP8)
+    assert np.mean([np.intersect1d(u, v).size / 50 for u, v in zip(a, b)]) > 0.95
+    assert far.max() < 12_000 and all(np.unique(r).size == 50 for r in far)

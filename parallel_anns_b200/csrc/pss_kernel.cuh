@@ -57,8 +57,9 @@ struct PssMem {
 template <int KIND, int CL>
 __device__ uint32_t pss_flush(const SearchArgs &a, const PssMem &m, uint32_t nb, float *qd, uint32_t *qi,
                               uint32_t *sz, uint32_t cap, const Dist<KIND, CL, STORE_FP32> &D, int lane) {
-    // 16 rows in flight; eight or fewer left over in a pass of eight.
-    const uint32_t wide = (nb & 15u) > 8u ? nb : nb & ~15u;
+    // 16 rows in flight; eight or fewer left over in a pass of eight. From CL = 6 on
+    // only the narrower passes: four rows a group spill there.
+    const uint32_t wide = CL >= 6 ? 0u : (nb & 15u) > 8u ? nb : nb & ~15u;
     float *tmp = reinterpret_cast<float *>(m.bk);
     if (wide) distances_wide<KIND, CL>(a, D.qv, m.bi, m.bd, wide, lane, tmp);
     if (wide < nb) D.distances(a, m.bi + wide, m.bd + wide, nb - wide, lane, tmp);

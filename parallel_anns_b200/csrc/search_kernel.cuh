@@ -504,11 +504,14 @@ struct Dist<KIND, CL, STORE_FP32> {
 #pragma unroll
         for (int i = 0; i < CL; ++i) qv[i] = __ldg(qrow + 8 * i + (lane & 7));
     }
-    // 32 vertices at a time, 8 rows in flight (2 per 8-lane group). The lanes
-    // leave their chains in tmp (256 floats), then lane i adds the eight of vertex
-    // i in order: a store per lane and vertex and one sum per 32 vertices, where
-    // shuffling the sum together on every lane took as many instructions as
-    // the rest of the pass.
+    // 32 vertices at a time, 8 rows in flight (2 per 8-lane group); from CL = 6 on
+    // 4 rows, since the registers of a one-warp query (80) hold one row's loads and
+    // the query's terms but not two rows': asked for two, the compiler loaded them a
+    // piece at a time (53,739 x 144, M = 1, 6,000 queries: 4.8 ms with two rows, 3.7
+    // with one; 30,000 x 256 5.4 and 4.3). The lanes leave their chains in tmp (256
+    // floats), then lane i adds the eight of vertex i in order: a store per lane and
+    // vertex and one sum per 32 vertices, where shuffling the sum together on every
+    // lane took as many instructions as the rest of the pass.
     __device__ __forceinline__ void distances(const SearchArgs &a, const uint32_t *ids, float *out, uint32_t nb,
                                               int lane, float *tmp) const {
         const uint32_t g = lane >> 3, c = lane & 7;
@@ -517,18 +520,28 @@ struct Dist<KIND, CL, STORE_FP32> {
             const bool have = (uint32_t) lane < m;
             const uint32_t mine = have ? ids[b0 + lane] & kIdMask : 0u;
             const float nrm = KIND == KIND_IP && have ? __ldg(a.norms + mine) : 0.f;
-            for (uint32_t p = 0; p < m; p += 8) {
-                const bool a0 = p + g < m, a1 = p + 4 + g < m;
-                const float4 *r0 = a.vec + (size_t) __shfl_sync(kFull, mine, p + g) * (CL * 8) + c;
-                const float4 *r1 = a.vec + (size_t) __shfl_sync(kFull, mine, p + 4 + g) * (CL * 8) + c;
-                float4 x0[CL], x1[CL];
+            if constexpr (CL >= 6) {
+                for (uint32_t p = 0; p < m; p += 4) {  // (row 0 past the last vertex)
+                    const float4 *r = a.vec + (size_t) __shfl_sync(kFull, mine, p + g) * (CL * 8) + c;
+                    float4 x[CL];
 #pragma unroll
-                for (int i = 0; i < CL; ++i) {
-                    x0[i] = a0 ? __ldg(r0 + 8 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    x1[i] = a1 ? __ldg(r1 + 8 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int i = 0; i < CL; ++i) x[i] = __ldg(r + 8 * i);
+                    tmp[p * 8 + lane] = chain<KIND, CL>(x, qv);
                 }
-                tmp[p * 8 + lane] = chain<KIND, CL>(x0, qv);
-                tmp[p * 8 + 32 + lane] = chain<KIND, CL>(x1, qv);
+            } else {
+                for (uint32_t p = 0; p < m; p += 8) {
+                    const bool a0 = p + g < m, a1 = p + 4 + g < m;
+                    const float4 *r0 = a.vec + (size_t) __shfl_sync(kFull, mine, p + g) * (CL * 8) + c;
+                    const float4 *r1 = a.vec + (size_t) __shfl_sync(kFull, mine, p + 4 + g) * (CL * 8) + c;
+                    float4 x0[CL], x1[CL];
+#pragma unroll
+                    for (int i = 0; i < CL; ++i) {
+                        x0[i] = a0 ? __ldg(r0 + 8 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        x1[i] = a1 ? __ldg(r1 + 8 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+                    tmp[p * 8 + lane] = chain<KIND, CL>(x0, qv);
+                    tmp[p * 8 + 32 + lane] = chain<KIND, CL>(x1, qv);
+                }
             }
             __syncwarp();
             if (have) out[b0 + lane] = finish_sum<KIND>(tmp + lane * 8, nrm);
@@ -691,6 +704,23 @@ struct Dist {
     __device__ __forceinline__ void distances(const SearchArgs &a, const uint32_t *ids, float *out, uint32_t nb,
                                               int lane, float *) const {
         const int g = lane >> 2, t = lane & 3;
+        if constexpr (STORE == STORE_BF16 && CL >= 4) {
+            // 8 vertices per round, one per 4-lane group: two rows' loads beside the
+            // query's terms pass the registers (60,000 x 224, 7,000 queries, M = 1:
+            // 2.7 ms with two, 2.5 with one).
+            for (uint32_t b0 = 0; b0 < nb; b0 += 8) {
+                const uint32_t b = b0 + g;
+                const bool act = b < nb;
+                const uint32_t v = act ? ids[b] & kIdMask : 0u;  // (row 0 past the last vertex)
+                const float n0 = act ? __ldg(a.norms_lo + v) : 0.f;
+                float s0 = dot_row_bf16(a.vec_lo, v, t);
+                s0 += __shfl_xor_sync(kFull, s0, 1);
+                s0 += __shfl_xor_sync(kFull, s0, 2);
+                if (t == 0 && act) out[b] = ordered(fmaf(-2.f, s0, n0));
+            }
+            __syncwarp();
+            return;
+        }
         // 16 vertices per round (2 per 4-lane group, loads issued together).
         for (uint32_t b0 = 0; b0 < nb; b0 += 16) {
             const uint32_t b = b0 + g, bb = b0 + 8 + g;
@@ -1085,8 +1115,16 @@ __device__ void search_one(const SearchArgs &a, const WarpMem &m, uint32_t q, ui
     __syncwarp();
 }
 
+// Resident blocks that registers are kept for: six (80 registers), but five for BF16
+// rows of 97 to 128 elements, which spill at six (7,782 queries, L = 127, M = 8, ms
+// with six and five: 174,925 x 112 integers 3.64 / 2.81, 200,000 x 112 1.41 / 1.17;
+// 10,000 queries, L = 384, where five take a wave more: 9.46 / 8.78 and 2.95 / 3.11).
+constexpr int search_min_blocks(int CL, int STORE) {
+    return STORE == STORE_BF16 && CL == 4 ? 5 : PANNS_SEARCH_MIN_BLOCKS;
+}
+
 template <int KIND, int ORDER, int CL, int STORE>
-__global__ void __launch_bounds__(128, PANNS_SEARCH_MIN_BLOCKS) search_kernel(SearchArgs a) {
+__global__ void __launch_bounds__(128, search_min_blocks(CL, STORE)) search_kernel(SearchArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
     const int lane = threadIdx.x & 31;
     const int wid = threadIdx.x >> 5;

@@ -881,8 +881,8 @@ static uint32_t block_buffer(uint32_t max_deg, uint32_t M, uint32_t W) {
 // fill, the resident warps over the 24 that one-warp queries reach on an SM, stands
 // for what full SMs add to a query's time. Residents are those the launch takes
 // (blocks_in_196kb). cost depends on the neighbours of a step, M x the mean degree:
-// the more, the more warps have to do; below 64, several warps share a candidate's
-// row and eight gain nothing over four. A batch of more than one wave of one-warp
+// the more, the more warps have to do; where a step is one long row (M = 1), four warps
+// share it as fast as eight. A batch of more than one wave of one-warp
 // queries that fill at least two thirds of the SM takes one warp each.
 //
 // The constants are fitted to 942 measurements: M = 1, 8 and 33, L = 32 to 3,000 and 1
@@ -897,16 +897,19 @@ static uint32_t block_buffer(uint32_t max_deg, uint32_t M, uint32_t W) {
 // 5.67 / [4.00] / 4.40.
 // 16 warps serve up to one query per SM, L <= 512 (64 queries at L = 384: 0.33 ms, 0.34
 // with 8), unless the visited bits fit shared memory beside 8 warps but not beside 16
-// (M = 33, L = 100: 0.28 against 0.20).
+// (M = 33, L = 100: 0.28 against 0.20), or the rows are BF16 of more than 192
+// elements, for which 512 threads have too few registers (50,000 x 224 integers, 140
+// queries: M = 33 0.43 against 0.23, M = 8 0.27 against 0.23).
 static int choose_warps(panns_index *h, const panns_search_params *p, uint32_t kind, int CL, uint32_t M, uint32_t nq,
                         uint32_t &wpq) {
     static const uint32_t warps[5] = {1, 2, 4, 8, 16};
-    // below 64, below 250 and from 250 neighbours of a step on
-    static const float cost[3][5] = {{1.f, 0.70f, 0.50f, 0.60f, 0.80f},
+    // below 64 neighbours of a step, one row of 32 and more, below 250 and from 250 on
+    static const float cost[4][5] = {{1.f, 0.70f, 0.54f, 0.44f, 0.60f},
+                                     {1.f, 0.70f, 0.50f, 0.60f, 0.80f},
                                      {1.f, 0.80f, 0.42f, 0.31f, 0.25f},
                                      {1.f, 0.60f, 0.31f, 0.235f, 0.19f}};
-    const double step = (double) M * (double) h->nbrs.size() / h->n;
-    const float *rel = cost[step < 64.0 ? 0 : step < 250.0 ? 1 : 2];
+    const double degree = (double) h->nbrs.size() / h->n, step = M * degree;
+    const float *rel = cost[M == 1 ? (degree < 32.0 ? 0 : 1) : step < 64.0 ? 0 : step < 250.0 ? 2 : 3];
     const uint32_t qcap = ((p->L + 31) / 32) * 32;
     const uint32_t words = (h->n + 31) / 32;
     auto block_bytes = [&](uint32_t W, uint32_t vis) {
@@ -916,7 +919,8 @@ static int choose_warps(panns_index *h, const panns_search_params *p, uint32_t k
     wpq = 1;
     for (int i = 0; i < 5; ++i) {
         const uint32_t W = warps[i];
-        if (W == 16 && (p->L > 512 || nq > (uint32_t) h->num_sms)) continue;
+        if (W == 16 && (p->L > 512 || nq > (uint32_t) h->num_sms || (p->storage == PANNS_STORE_BF16 && CL == 8)))
+            continue;
         if (W == 16 && (size_t) words * 4 < kSmemLimit && block_bytes(8, words) <= kSmemLimit &&
             block_bytes(16, words) > kSmemLimit)
             continue;

@@ -650,6 +650,21 @@ int panns_efanna_init_ids(const panns_index *h, uint32_t L, uint32_t nq, int32_t
     if (L == 0 || L > n) return fail(PANNS_EINVAL, "panns_efanna_init_ids: need 0 < L <= N");
     std::vector<uint8_t> flags(n, 0);
     const uint64_t e0 = h->off[h->entry], deg = h->off[h->entry + 1] - e0;
+    // rand_next with the table's two places in registers (a draw is a dependent chain
+    // of a few cycles, and there are L a query).
+    int32_t *const tbl = st, *const end = st + 31;
+    int32_t *f = st + st[31], *r = st + st[32];
+    auto draw = [&]() -> uint32_t {
+        const uint32_t val = (uint32_t) *f + (uint32_t) *r;
+        *f = (int32_t) val;
+        if (++f >= end) {
+            f = tbl;
+            ++r;
+        } else if (++r >= end) {
+            r = tbl;
+        }
+        return val >> 1;
+    };
     for (uint32_t q = 0; q < nq; ++q) {
         uint32_t *ids = out + (size_t) q * L;
         uint32_t t = 0;
@@ -658,13 +673,15 @@ int panns_efanna_init_ids(const panns_index *h, uint32_t L, uint32_t nq, int32_t
             flags[ids[t]] = 1;
         }
         while (t < L) {
-            const uint32_t id = (uint32_t) rand_next(st) % n;
+            const uint32_t id = draw() % n;
             if (flags[id]) continue;
             flags[id] = 1;
             ids[t++] = id;
         }
         for (uint32_t i = 0; i < L; ++i) flags[ids[i]] = 0;
     }
+    st[31] = (int32_t) (f - st);
+    st[32] = (int32_t) (r - st);
     return PANNS_OK;
 }
 
@@ -1204,8 +1221,11 @@ static int stage_init(panns_index *h, const panns_search_params *p, const uint32
     // over as device ids in the same order.
     const uint32_t groups = efanna ? nq : 1;
     std::vector<uint32_t> dev((size_t) groups * L);
-    if (!init_ids)
-        for (size_t i = 0; i < dev.size(); ++i) dev[i] = h->inv[ids[i]];
+    if (!init_ids) {
+        const uint32_t *inv = h->inv.data();
+        uint32_t *to = dev.data();
+        for (size_t i = 0, m = dev.size(); i < m; ++i) to[i] = inv[ids[i]];
+    }
     const bool by_sort = (uint64_t) groups * L * 16 < h->n;
     std::vector<uint8_t> seen(by_sort || !init_ids ? 0 : h->n, 0);
     std::vector<uint32_t> tmp;

@@ -94,8 +94,9 @@ typedef struct {
                                  without PANNS_FLAG_LEARNED), for small batches and long queues; same
                                  ids and counts.
                                  0: chosen (1, 2, 4, 8 or 16) by how many waves of queries each
-                                 takes and how long a wave is, when the mode allows it and
-                                 warps_per_block and blocks_per_sm are 0, else 1 */
+                                 takes and how long a wave is (from L, M, the mean degree and the
+                                 batch), when the mode allows it and warps_per_block and
+                                 blocks_per_sm are 0, else 1 */
 } panns_search_params;
 
 /* Enqueue the launch (per-call memsets, query layout and the search kernel)

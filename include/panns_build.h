@@ -32,12 +32,14 @@ typedef struct panns_graph panns_graph;
  * candidates per row; by TF32 tensor-core GEMMs (cuBLAS) keeping k + 32; or
  * by the library's own tcgen05 kernel (operands split in two BF16 parts, TMA
  * into shared memory, accumulators in tensor memory), which hands on every
- * pair within a threshold that provably holds all k nearest, and skips tiles
- * whose ball is out of reach. Either way the candidates are ranked exactly in
- * float64. AUTO: the tcgen05 kernel for n >= 1,024 and d <= 256 (rows it
- * cannot settle - non-finite values, more equal distances than its lists
- * hold - go through the float32 screen), else float32 below 100,000 vectors
- * and TF32 from there on. Chosen by name, PANNS_SCREEN_TC asks for d a
+ * pair within a threshold that provably holds all k nearest, at any scale of the
+ * data, and skips tiles whose ball is out of reach. Either way the candidates are
+ * ranked exactly in float64. AUTO: the tcgen05 kernel for n >= 1,024 and d <= 256
+ * (rows it cannot settle - non-finite values, more equal distances or a cluster
+ * with more rows within the error bound than its lists hold - go through a float32
+ * screen by squared differences, alone; all rows do where one is 10^18 times
+ * further from the mean than the rest), else float32 below 100,000 vectors and
+ * TF32 from there on. Chosen by name, PANNS_SCREEN_TC asks for d a
  * multiple of 32 up to 128. */
 #define PANNS_SCREEN_AUTO 0u
 #define PANNS_SCREEN_FP32 1u
@@ -62,8 +64,9 @@ int panns_build_nsg_ex(int device, const float *base, uint32_t n, uint32_t d, ui
  * members of a's cell and of the `probe` cells whose centroids are nearest to
  * it (by float64 squared distance, then index). The candidates come from the
  * tcgen05 screen with every cell padded to whole tiles where d <= 256, padding
- * at most doubles the rows and its operands fit the free memory, else from a
- * float32 screen keeping k + 8 per row; they are ranked exactly in float64.
+ * at most doubles the rows and its operands fit the free memory (rows it cannot
+ * settle again alone in float32), else from a float32 screen; that keeps k + 16
+ * per row, at most 136. They are ranked exactly in float64.
  * Prune, entry and repair are those of panns_build_nsg. probe <= 8; a list with
  * fewer than knn_k candidates is shorter. With `reverse` set, before the
  * repair every pruned edge a -> b (a ascending, then list order) also gives
@@ -93,7 +96,10 @@ int panns_graph_copy(const panns_graph *g, uint64_t *offsets, uint32_t *nbrs, ui
 int panns_graph_save_nsg(const panns_graph *g, const char *path);
 
 /* Release the graph. Its k-NN lists stay in device memory until then (lists of
- * more than 4 GiB are kept on the host). */
+ * more than 4 GiB are kept on the host). Copying and releasing work beside a
+ * stream capture. What constructions and training give back stays with the library,
+ * up to 2 GiB a device, until an index on that device is closed; a program
+ * without one can open and close one for that (panns_open, panns_close). */
 int panns_graph_free(panns_graph *g);
 
 /* efanna2e's own NSG construction, IndexNSG::Build

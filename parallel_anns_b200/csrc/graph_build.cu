@@ -14,12 +14,15 @@
 //     in-edge from the first reached vertex of its k-NN list (else the entry),
 //     then everything it reaches is marked (index_nsg.cpp:638-718 plays this
 //     part with a DFS tree).
-// The k-NN search screens all pairs (||y||^2 - 2 x.y) either in float32 on CUDA
-// cores (tiled here, C = k + 8 candidates kept per row) or with TF32
-// tensor-core GEMMs (cuBLAS) folded tile by tile into the rows' lists (C = k +
-// 32), and ranks the C survivors by d64; the result equals the exact k-NN
-// unless a true neighbour falls outside the screen's top C, which needs the
-// screen's rounding to move it past 8 (float32) or 32 (TF32) others.
+// A screen finds each row's candidates, which are then ranked by d64. By default
+// (n >= 1,024, d <= 256) it is the tcgen05 screen of tc_screen.cu, whose threshold
+// provably holds all k nearest; the rows it reports (runs of equal distances longer
+// than a list, clusters much smaller than the base, non-finite values) are screened
+// here in float32 by squared differences. Else, or by name, all pairs are screened
+// (||y||^2 - 2 x.y) in float32 on CUDA cores (tiled here, C = k + 8 candidates kept
+// per row) or with TF32 tensor-core GEMMs (cuBLAS) folded tile by tile into the
+// rows' lists (C = k + 32); these two equal the exact k-NN unless their rounding
+// moves a true neighbour past 8 or 32 others.
 #include <cublas_v2.h>
 #include <cuda_runtime.h>
 

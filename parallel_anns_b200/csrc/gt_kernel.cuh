@@ -5,9 +5,10 @@
 // It is enough to collect the vertices whose float64 distance is <= tau (about
 // k of them for a good search); an exact (distance, id) sort gives the top k.
 // The collection is the tensor-core range screen (tc_screen.cu), whose lists
-// gt_rank_kernel evaluates in float64 and ranks; where its lists do not fit
-// (k > kGtMaxK, or a bound so loose that refining it does not help) one tiled
-// float64 pass over the base collects instead (gt_collect_kernel).
+// gt_rank_kernel evaluates in float64 and ranks; one tiled float64 pass over the
+// base collects instead (gt_collect_kernel) for a few queries, where the screen's
+// fixed cost is more, and where its lists do not fit or do not hold (k > kGtMaxK, a
+// bound so loose that refining it does not help, vectors past the screen's range).
 // 10,000 queries x 1M x 96, k = 100: 174 ms in gt_collect_kernel, 3 ms in the
 // screen, its operands and gt_rank_kernel.
 // Distances are sum over dimensions, in order, of fma(t, t, acc) with

@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(WR *WC * 32) gemm_kernel(const TA *__restrict_
                                  As[buf][ia(wm + g, kk + tq + 4)], As[buf][ia(wm + g + 8, kk + tq + 4)]};
 #pragma unroll
             for (int i = 0; i < 4; ++i) split_tf32(av[i], ah[i], al[i]);
-uint32_t bh[TN][2], bl[TN][2];
+            uint32_t bh[TN][2], bl[TN][2];
 #pragma unroll
             for (int nt = 0; nt < TN; ++nt) {
                 const float b0 = Bs[buf][ib(kk + tq, wn + nt * 8 + g)], b1 = Bs[buf][ib(kk + tq + 4, wn + nt * 8 + g)];

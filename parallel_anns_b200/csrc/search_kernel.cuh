@@ -718,39 +718,38 @@ struct Dist {
                 s0 += __shfl_xor_sync(kFull, s0, 2);
                 if (t == 0 && act) out[b] = ordered(fmaf(-2.f, s0, n0));
             }
-            __syncwarp();
-            return;
-        }
-        // 16 vertices per round (2 per 4-lane group, loads issued together).
-        for (uint32_t b0 = 0; b0 < nb; b0 += 16) {
-            const uint32_t b = b0 + g, bb = b0 + 8 + g;
-            const bool act0 = b < nb, act1 = bb < nb;
-            const uint32_t v0 = act0 ? ids[b] & kIdMask : 0u, v1 = act1 ? ids[bb] & kIdMask : 0u;
-            const float n0 = act0 ? __ldg(a.norms_lo + v0) : 0.f;
-            const float n1 = act1 ? __ldg(a.norms_lo + v1) : 0.f;
-            if constexpr (STORE == STORE_BF16) {
-                float s0 = act0 ? dot_row_bf16(a.vec_lo, v0, t) : 0.f;
-                float s1 = act1 ? dot_row_bf16(a.vec_lo, v1, t) : 0.f;
-                s0 += __shfl_xor_sync(kFull, s0, 1);
-                s1 += __shfl_xor_sync(kFull, s1, 1);
-                s0 += __shfl_xor_sync(kFull, s0, 2);
-                s1 += __shfl_xor_sync(kFull, s1, 2);
-                if (t == 0) {
-                    if (act0) out[b] = ordered(fmaf(-2.f, s0, n0));
-                    if (act1) out[bb] = ordered(fmaf(-2.f, s1, n1));
+        } else {
+            // 16 vertices per round (2 per 4-lane group, loads issued together).
+            for (uint32_t b0 = 0; b0 < nb; b0 += 16) {
+                const uint32_t b = b0 + g, bb = b0 + 8 + g;
+                const bool act0 = b < nb, act1 = bb < nb;
+                const uint32_t v0 = act0 ? ids[b] & kIdMask : 0u, v1 = act1 ? ids[bb] & kIdMask : 0u;
+                const float n0 = act0 ? __ldg(a.norms_lo + v0) : 0.f;
+                const float n1 = act1 ? __ldg(a.norms_lo + v1) : 0.f;
+                if constexpr (STORE == STORE_BF16) {
+                    float s0 = act0 ? dot_row_bf16(a.vec_lo, v0, t) : 0.f;
+                    float s1 = act1 ? dot_row_bf16(a.vec_lo, v1, t) : 0.f;
+                    s0 += __shfl_xor_sync(kFull, s0, 1);
+                    s1 += __shfl_xor_sync(kFull, s1, 1);
+                    s0 += __shfl_xor_sync(kFull, s0, 2);
+                    s1 += __shfl_xor_sync(kFull, s1, 2);
+                    if (t == 0) {
+                        if (act0) out[b] = ordered(fmaf(-2.f, s0, n0));
+                        if (act1) out[bb] = ordered(fmaf(-2.f, s1, n1));
+                    }
+                    continue;
                 }
-                continue;
-            }
-            const float2 p0 = act0 ? dot_row2(a.vec_lo, v0, t) : make_float2(0.f, 0.f);
-            const float2 p1 = act1 ? dot_row2(a.vec_lo, v1, t) : make_float2(0.f, 0.f);
-            float2 s = __fadd2_rn(make_float2(p0.x, p1.x), make_float2(p0.y, p1.y));
-            s = __fadd2_rn(s, make_float2(__shfl_xor_sync(kFull, s.x, 1), __shfl_xor_sync(kFull, s.y, 1)));
-            s = __fadd2_rn(s, make_float2(__shfl_xor_sync(kFull, s.x, 2), __shfl_xor_sync(kFull, s.y, 2)));
-            if (t == 0) {
-                const float m2 = kMixed ? a.q8_m2 : -2.f;
-                const float2 r = __ffma2_rn(make_float2(m2, m2), s, make_float2(n0, n1));
-                if (act0) out[b] = ordered(r.x);
-                if (act1) out[bb] = ordered(r.y);
+                const float2 p0 = act0 ? dot_row2(a.vec_lo, v0, t) : make_float2(0.f, 0.f);
+                const float2 p1 = act1 ? dot_row2(a.vec_lo, v1, t) : make_float2(0.f, 0.f);
+                float2 s = __fadd2_rn(make_float2(p0.x, p1.x), make_float2(p0.y, p1.y));
+                s = __fadd2_rn(s, make_float2(__shfl_xor_sync(kFull, s.x, 1), __shfl_xor_sync(kFull, s.y, 1)));
+                s = __fadd2_rn(s, make_float2(__shfl_xor_sync(kFull, s.x, 2), __shfl_xor_sync(kFull, s.y, 2)));
+                if (t == 0) {
+                    const float m2 = kMixed ? a.q8_m2 : -2.f;
+                    const float2 r = __ffma2_rn(make_float2(m2, m2), s, make_float2(n0, n1));
+                    if (act0) out[b] = ordered(r.x);
+                    if (act1) out[bb] = ordered(r.y);
+                }
             }
         }
         __syncwarp();
